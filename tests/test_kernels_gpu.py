@@ -91,6 +91,26 @@ def test_gemm_generic(dtype, m, n, k, accumulate):
     assert (err <= 1e-6 * bound + 1e-6 * want.abs() + 1e-7).all(), f"worst {err.max():.3g}"
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 33, 4), (8, 9473, 132), (9, 17, 260), (16, 9480, 36), (17, 31, 100), (64, 70, 128), (65, 4104, 68),
+                                   (300, 2500, 52)])
+def test_gemm_float32_tiles(m, n, k):
+    """Every tile of the float32 product, at its edges in rows, columns and slices of k, alone and onto what is there; a row's
+    bits do not depend on how many rows stand beside it."""
+    g = torch.Generator().manual_seed(m + n + k)
+    a, w, out0 = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g), torch.randn(m, n, generator=g)
+    bound = a.double().abs() @ w.double().abs().T
+    for accumulate in (False, True):
+        out = out0.clone().to(DEV)
+        ops().gemm(a.to(DEV), w.to(DEV), out, accumulate=accumulate)
+        want = ref_ops.gemm(a, w, out0 if accumulate else None)
+        err = (out.double().cpu() - want).abs()
+        assert (err <= 1e-6 * bound + 1e-6 * want.abs() + 1e-7).all(), f"worst {err.max():.3g}"
+        if not accumulate:
+            alone = torch.empty(1, n, device=DEV)
+            ops().gemm(a[-1:].to(DEV), w.to(DEV), alone)
+            assert torch.equal(alone[0], out[-1])
+
+
 def make_paged(rng, n_slots, lens, G, hd, pt, dtype, extra_pages=3):
     """Random cache contents in scattered pages; returns (k_pages, v_pages, block_table, k, v) with
     k, v the dense float64 [slot][len, G, hd] contents (already rounded to `dtype`)."""
