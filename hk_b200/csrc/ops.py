@@ -776,13 +776,39 @@ def tanh_cols(x: torch.Tensor, out: torch.Tensor) -> None:
 # ---- recurrent mixers ---------------------------------------------------------------------
 
 
+DELTA_CHUNK = 32    # tokens of a chunk of the recurrences' chunked form (`csrc/delta_chunks.cu`)
+
+
+def delta_chunks_take(key_dim: int, value_dim: int, decay_scale: float = 0.0) -> bool:
+    """Whether the chunked form takes a recurrent mixer of these sizes (and, for the generalised delta rule, decays that a
+    chunk's product cannot bring below 2^-64)."""
+    return key_dim % 4 == 0 and key_dim <= 64 and value_dim % 4 == 0 and 0.0 <= decay_scale <= 1.38
+
+
+def _chunk_tables(chunks, requests, what: str):
+    _need(chunks, "chunks", torch.int32, 2)
+    _need(requests, "requests", torch.int32, 2)
+    if chunks.shape[1] != 2 or requests.shape[1] != 3:
+        raise KernelError(f"{what}: chunks must be [n, 2] and requests [n, 3]")
+    return _ptr(chunks), int(chunks.shape[0]), _ptr(requests), int(requests.shape[0])
+
+
+def _chunk_scratch(lib, chunks, H: int, dk: int, dvp: int, removal: bool, device):
+    lib.hk_delta_chunks_scratch.restype = ctypes.c_longlong
+    return torch.empty(int(lib.hk_delta_chunks_scratch(int(chunks.shape[0]), H, dk, dvp, 1 if removal else 0)), dtype=torch.float32,
+                       device=device)
+
+
 def delta_rule_scan(r, k, v, a_logit, w_logit, a_bias, w_bias, segments, state, out, n_heads: int, key_dim: int,
-                    value_dim: int, decay_scale: float, key_eps: float) -> None:
+                    value_dim: int, decay_scale: float, key_eps: float, chunks=None, requests=None, most_rows: int = 0) -> None:
     """Generalised delta rule over the rows of every segment (slot, first row, rows) of `segments` int32 [n_seg, 3]:
         S <- diag(d) S - (a * u) (u^T S) + k v^T,  out = S^T r      per head, S = state[slot, head] float32 [dk, dv]
     d = exp(-decay_scale * sigmoid(w_logit + w_bias)), a = sigmoid(a_logit + a_bias), u = k / sqrt(sum k^2 + key_eps).
     r, k, a_logit [n, H*dk] and v [n, H*dv] are float32 column slices of ONE matrix (one row stride); w_logit is
-    float32 [n, H*dk] with its own.  out: float32 [n, H*dv]."""
+    float32 [n, H*dk] with its own.  out: float32 [n, H*dv].
+    `chunks` int32 [n_chunks, 2] = (first row, rows) and `requests` int32 [n_requests, 3] = (slot, first chunk, chunks): further
+    requests that are walked in chunks of up to DELTA_CHUNK tokens (sizes that `delta_chunks_take`, 16-byte aligned slices); a
+    request's chunks stand side by side, full ones first.  `segments` then holds the others, none of more than `most_rows` rows."""
     H, dk, dv = n_heads, key_dim, value_dim
     ld = _cols(r, "r", H * dk)
     if _cols(k, "k", H * dk) != ld or _cols(a_logit, "a_logit", H * dk) != ld or _cols(v, "v", H * dv) != ld:
@@ -797,13 +823,22 @@ def delta_rule_scan(r, k, v, a_logit, w_logit, a_bias, w_bias, segments, state, 
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(out.shape) != (n, H * dv) or segments.shape[1] != 3 \
             or a_bias.shape[0] != H * dk or w_bias.shape[0] != H * dk:
         raise KernelError("delta_rule_scan: shapes do not fit")
+    if chunks is not None and chunks.shape[0]:
+        lib = build.load("delta_chunks")
+        scratch = _chunk_scratch(lib, chunks, H, dk, dv, True, out.device)
+        _check(lib.hk_delta_rule_chunks(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ctypes.c_longlong(ld), _ptr(w_logit),
+                                        ctypes.c_longlong(ldw), _ptr(a_bias), _ptr(w_bias), *_chunk_tables(chunks, requests, "delta_rule_scan"),
+                                        _ptr(scratch), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
+                                        ctypes.c_float(key_eps), _stream()), "delta_rule_scan (chunks)", launches=2)
+    if not segments.shape[0]:
+        return
     lib = build.load("recurrent")
     # what every token brings to the scan (decay, removal times unit key, unit key, key, receptance, value), made by a
     # kernel of its own for all tokens at once
     rec = torch.empty(n * H * int(lib.hk_delta_rule_record(dk, dv)), dtype=torch.float32, device=out.device)
     _check(lib.hk_delta_rule_scan(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ctypes.c_longlong(ld), _ptr(w_logit),
                                   ctypes.c_longlong(ldw), _ptr(a_bias), _ptr(w_bias), _ptr(segments), int(segments.shape[0]), n,
-                                  _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
+                                  int(most_rows), _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
                                   ctypes.c_float(key_eps), _stream()), "delta_rule_scan", launches=2)
 
 
@@ -867,12 +902,14 @@ def short_conv(x, weight, segments, tail, out, act: str = "silu", bias=None) -> 
 
 
 def gated_delta_scan(q, k, v, b_logit, a_logit, a_log, dt_bias, segments, state, out, n_heads: int, n_qk_heads: int,
-                     key_dim: int, value_dim: int, q_scale: float, unit_eps: float) -> None:
+                     key_dim: int, value_dim: int, q_scale: float, unit_eps: float, chunks=None, requests=None,
+                     most_rows: int = 0) -> None:
     """Gated delta rule over the rows of every segment, per head, S = state[slot, head] float32 [dk, dv]:
         S <- g S;  u = beta (v - S^T k);  S <- S + k u^T;  out = S^T q
     with q, k made unit vectors per head (x / sqrt(sum x^2 + unit_eps)), q times q_scale, beta = sigmoid(b_logit),
     g = exp(-exp(a_log) * softplus(a_logit + dt_bias)).  q, k [n, G*dk] and v [n, H*dv]: float32 column slices of ONE
-    matrix; b_logit, a_logit [n, H] slices of one; value head h reads query/key head h // (H/G).  out float32 [n, H*dv]."""
+    matrix; b_logit, a_logit [n, H] slices of one; value head h reads query/key head h // (H/G).  out float32 [n, H*dv].
+    `chunks`, `requests` and `most_rows` as in `delta_rule_scan`."""
     H, G, dk, dv = n_heads, n_qk_heads, key_dim, value_dim
     ld = _cols(q, "q", G * dk)
     if _cols(k, "k", G * dk) != ld or _cols(v, "v", H * dv) != ld:
@@ -889,21 +926,32 @@ def gated_delta_scan(q, k, v, b_logit, a_logit, a_log, dt_bias, segments, state,
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(out.shape) != (n, H * dv) or segments.shape[1] != 3 \
             or a_log.shape[0] != H or dt_bias.shape[0] != H or H % G:
         raise KernelError("gated_delta_scan: shapes do not fit")
+    if chunks is not None and chunks.shape[0]:
+        lib = build.load("delta_chunks")
+        scratch = _chunk_scratch(lib, chunks, H, dk, dv, True, out.device)
+        _check(lib.hk_gated_delta_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(b_logit), _ptr(a_logit),
+                                         ctypes.c_longlong(ldg), _ptr(a_log), _ptr(dt_bias),
+                                         *_chunk_tables(chunks, requests, "gated_delta_scan"), _ptr(scratch), _ptr(state), _ptr(out), H, G, dk,
+                                         dv, ctypes.c_float(q_scale), ctypes.c_float(unit_eps), _stream()), "gated_delta_scan (chunks)",
+               launches=2)
+    if not segments.shape[0]:
+        return
     lib = build.load("recurrent")
     rec = torch.empty(n * H * int(lib.hk_delta_rule_record(dk, dv)), dtype=torch.float32, device=out.device)
     _check(lib.hk_gated_delta_scan(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(b_logit), _ptr(a_logit),
                                    ctypes.c_longlong(ldg), _ptr(a_log), _ptr(dt_bias), _ptr(segments), int(segments.shape[0]), n,
-                                   _ptr(rec), _ptr(state), _ptr(out), H, G, dk, dv, ctypes.c_float(q_scale),
+                                   int(most_rows), _ptr(rec), _ptr(state), _ptr(out), H, G, dk, dv, ctypes.c_float(q_scale),
                                    ctypes.c_float(unit_eps), _stream()), "gated_delta_scan", launches=2)
 
 
 def retention_scan(q, k, v, cos, sin, rotary_dim: int, positions, decay, segments, state, out, n_heads: int, key_dim: int,
-                   value_dim: int, k_scale: float) -> None:
+                   value_dim: int, k_scale: float, chunks=None, requests=None, most_rows: int = 0) -> None:
     """Retention over the rows of every segment, per head, S = state[slot, head] float32 [dk, dv]:
         S <- decay[h] S + k v^T;  out = S^T q
     with q and k turned by position on their first `rotary_dim` dims (dim i paired with i + rotary_dim / 2; tables
     cos, sin float32 [positions, rotary_dim / 2]; 0: no rotation) and k then times k_scale.  q, k [n, H*dk] and v
-    [n, H*dv]: float32 column slices of ONE matrix; decay float32 [H]; out float32 [n, H*dv]."""
+    [n, H*dv]: float32 column slices of ONE matrix; decay float32 [H]; out float32 [n, H*dv].
+    `chunks`, `requests` and `most_rows` as in `delta_rule_scan`."""
     H, dk, dv = n_heads, key_dim, value_dim
     ld = _cols(q, "q", H * dk)
     if _cols(k, "k", H * dk) != ld or _cols(v, "v", H * dv) != ld:
@@ -922,11 +970,20 @@ def retention_scan(q, k, v, cos, sin, rotary_dim: int, positions, decay, segment
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(out.shape) != (n, H * dv) or segments.shape[1] != 3 \
             or decay.shape[0] != H or positions.shape[0] != n:
         raise KernelError("retention_scan: shapes do not fit")
+    if chunks is not None and chunks.shape[0]:
+        lib = build.load("delta_chunks")
+        scratch = _chunk_scratch(lib, chunks, H, dk, dv, False, out.device)
+        _check(lib.hk_retention_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(cos if rotary_dim > 0 else None),
+                                       _ptr(sin if rotary_dim > 0 else None), int(rotary_dim), _ptr(positions), _ptr(decay),
+                                       *_chunk_tables(chunks, requests, "retention_scan"), _ptr(scratch), _ptr(state), _ptr(out), H, dk, dv,
+                                       ctypes.c_float(k_scale), _stream()), "retention_scan (chunks)", launches=3)
+    if not segments.shape[0]:
+        return
     lib = build.load("recurrent")
     rec = torch.empty(n * H * int(lib.hk_delta_rule_record(dk, dv)), dtype=torch.float32, device=out.device)
     _check(lib.hk_retention_scan(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(cos if rotary_dim > 0 else None),
                                  _ptr(sin if rotary_dim > 0 else None), int(rotary_dim), _ptr(positions), _ptr(decay), _ptr(segments),
-                                 int(segments.shape[0]), n, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(k_scale),
+                                 int(segments.shape[0]), n, int(most_rows), _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(k_scale),
                                  _stream()), "retention_scan", launches=2)
 
 
@@ -1056,13 +1113,14 @@ def mlstm_padded(value_dim: int) -> int:
 
 
 def mlstm_scan(q, k, v, i_logit, f_logit, i_bias, f_bias, segments, state, m_state, out, gates, n_heads: int, key_dim: int,
-               value_dim: int, cap: float, q_scale: float) -> None:
+               value_dim: int, cap: float, q_scale: float, long_segments=None, chunks=None, requests=None, most_rows: int = 0) -> None:
     """Matrix memory with exponential gates over the rows of every segment, per head (S, n zero and m = 0 at a
     request's start): i = cap tanh((i_logit + i_bias) / cap), f = logsigmoid(cap tanh((f_logit + f_bias) / cap)),
         m' = max(f + m, i);  S <- e^(f + m - m') S + e^(i - m') k v^T;  n likewise with k alone.
     state float32 [slots, H, dk, dvp] holds S and, as column dv, n (dvp = mlstm_padded(dv)); m_state [slots, H].
     out float32 [n, H*dvp]: per head S^T (q q_scale) and, at column dv, n . (q q_scale); gates float32 [n, H, 3]
-    receives (e^(f + m - m'), e^(i - m'), e^(-m')) per token.  q, k, v, i_logit, f_logit: slices of ONE float32 matrix."""
+    receives (e^(f + m - m'), e^(i - m'), e^(-m')) per token.  q, k, v, i_logit, f_logit: slices of ONE float32 matrix.
+    `chunks`, `requests` and `most_rows` as in `delta_rule_scan`; `long_segments`: the requests in chunks as segments."""
     H, dk, dv = n_heads, key_dim, value_dim
     dvp = mlstm_padded(dv)
     ld = _cols(q, "q", H * dk)
@@ -1081,9 +1139,23 @@ def mlstm_scan(q, k, v, i_logit, f_logit, i_bias, f_bias, segments, state, m_sta
             or tuple(gates.shape) != (n, H, 3) or segments.shape[1] != 3 or i_bias.shape[0] != H or f_bias.shape[0] != H:
         raise KernelError("mlstm_scan: shapes do not fit")
     lib = build.load("recurrent")
+    if chunks is not None and chunks.shape[0]:
+        _need(long_segments, "long_segments", torch.int32, 2)
+        if long_segments.shape[1] != 3:
+            raise KernelError("mlstm_scan: long_segments must be [n, 3]")
+        tables = _chunk_tables(chunks, requests, "mlstm_scan")
+        wide = build.load("delta_chunks")
+        scratch = _chunk_scratch(wide, chunks, H, dk, dvp, False, out.device)
+        _check(lib.hk_mlstm_gates(_ptr(i_logit), _ptr(f_logit), ctypes.c_longlong(ld), _ptr(i_bias), _ptr(f_bias), _ptr(long_segments),
+                                  int(long_segments.shape[0]), _ptr(gates), _ptr(m_state), H, ctypes.c_float(cap), _stream()),
+               "mlstm_scan (gates)")
+        _check(wide.hk_mlstm_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(gates), *tables, _ptr(scratch), _ptr(state),
+                                    _ptr(out), H, dk, dv, ctypes.c_float(q_scale), _stream()), "mlstm_scan (chunks)", launches=3)
+    if not segments.shape[0]:
+        return
     rec = torch.empty(n * H * int(lib.hk_delta_rule_record(dk, dvp)), dtype=torch.float32, device=out.device)
     _check(lib.hk_mlstm_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(i_logit), _ptr(f_logit), ctypes.c_longlong(ld), _ptr(i_bias),
-                             _ptr(f_bias), _ptr(segments), int(segments.shape[0]), n, _ptr(rec), _ptr(gates), _ptr(state),
+                             _ptr(f_bias), _ptr(segments), int(segments.shape[0]), n, int(most_rows), _ptr(rec), _ptr(gates), _ptr(state),
                              _ptr(m_state), _ptr(out), H, dk, dv, ctypes.c_float(cap), ctypes.c_float(q_scale), _stream()),
            "mlstm_scan", launches=3)
 

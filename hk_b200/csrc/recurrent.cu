@@ -23,6 +23,20 @@
 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 
+// The rows that a preparation kernel works on: all of the step's (segs null), or those of the segments in blockIdx.y (up to
+// `most` rows each) when the step's other rows are not walked token by token.  `item` becomes the row's and head's number.
+__device__ __forceinline__ bool prep_item(long long& item, const int* segs, long long items, int H) {
+  if (item >= items) return false;
+  if (segs == nullptr) return true;
+  const int row0 = segs[blockIdx.y * 3 + 1], count = segs[blockIdx.y * 3 + 2];
+  if (item >= (long long)count * H) return false;
+  item += (long long)row0 * H;
+  return true;
+}
+static dim3 prep_grid(long long items, const int* segs, int n_seg) {
+  return dim3((unsigned)((items + 7) / 8), segs == nullptr ? 1u : (unsigned)n_seg);
+}
+
 // ------------------------------------------------------------------ generalised delta rule: what a token brings
 // One warp per (token, head) writes the record that the scan reads: five vectors of P = L * RPT floats (d, a*u, u, k, r;
 // P >= dk, the rest zero) and the dv values.  Inside a vector, entry i sits at (i % L) * RPT + i / L: lane `sub` of a
@@ -31,10 +45,10 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf
 __global__ void delta_rule_prep_kernel(const float* __restrict__ r, const float* __restrict__ k, const float* __restrict__ v,
                                        const float* __restrict__ al, long long ld, const float* __restrict__ wl, long long ldw,
                                        const float* __restrict__ a_bias, const float* __restrict__ w_bias, float* __restrict__ rec,
-                                       long long items, int H, int dk, int dv, int L, int RPT, float decay_scale, float key_eps) {
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+                                       const int* __restrict__ psegs, long long items, int H, int dk, int dv, int L, int RPT, float decay_scale, float key_eps) {
+  long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (item >= items) return;
+  if (!prep_item(item, psegs, items, H)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const size_t hoff = (size_t)h * dk;
@@ -338,8 +352,9 @@ static int dr_scan_records(const float* rec, const int* segs, int n_seg, float* 
 }
 
 // `rec`: scratch of n_rows * H * hk_delta_rule_record(dk, dv) floats (16-byte aligned) that the call fills and reads.
+// `most_rows` > 0: the segments do not hold all of the step's rows, and none holds more than so many; only theirs are prepared.
 HK_API int hk_delta_rule_scan(const float* r, const float* k, const float* v, const float* al, long long ld, const float* wl,
-                              long long ldw, const float* a_bias, const float* w_bias, const int* segs, int n_seg, int n_rows,
+                              long long ldw, const float* a_bias, const float* w_bias, const int* segs, int n_seg, int n_rows, int most_rows,
                               float* rec, float* state, float* out, int H, int dk, int dv, float decay_scale, float key_eps,
                               void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
@@ -348,9 +363,10 @@ HK_API int hk_delta_rule_scan(const float* r, const float* k, const float* v, co
   int L, rpt;
   if (!dr_plan(n_seg, H, dk, dv, &L, &rpt)) return HK_ERR_UNSUPPORTED;
   {
-    const long long items = (long long)n_rows * H;
-    int e = hk_launch(delta_rule_prep_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, r, k, v, al, ld, wl, ldw, a_bias,
-                      w_bias, rec, items, H, dk, dv, L, rpt, decay_scale, key_eps);
+    const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
+    const int* psegs = most_rows ? segs : nullptr;
+    int e = hk_launch(delta_rule_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, r, k, v, al, ld, wl, ldw, a_bias,
+                      w_bias, rec, psegs, items, H, dk, dv, L, rpt, decay_scale, key_eps);
     if (e) return e;
   }
   return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, s);
@@ -496,11 +512,11 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log
 __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                         long long ld, const float* __restrict__ bl, const float* __restrict__ al, long long ldg,
                                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ rec,
-                                        long long items, int H, int G, int dk, int dv, int L, int RPT, float q_scale,
+                                        const int* __restrict__ psegs, long long items, int H, int G, int dk, int dv, int L, int RPT, float q_scale,
                                         float unit_eps) {
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (item >= items) return;
+  if (!prep_item(item, psegs, items, H)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const int g = h / (H / G);
@@ -540,7 +556,7 @@ __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float
 // q, k [n, G*dk] and v [n, H*dv] are column slices of one float32 matrix (row stride ld), already convolved and
 // activated; b_logit and a_logit [n, H] slices of one (row stride ldg).  `rec` as for hk_delta_rule_scan.
 HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, long long ld, const float* bl, const float* al,
-                               long long ldg, const float* a_log, const float* dt_bias, const int* segs, int n_seg, int n_rows,
+                               long long ldg, const float* a_log, const float* dt_bias, const int* segs, int n_seg, int n_rows, int most_rows,
                                float* rec, float* state, float* out, int H, int G, int dk, int dv, float q_scale, float unit_eps,
                                void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
@@ -548,9 +564,10 @@ HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, l
   cudaStream_t s = (cudaStream_t)stream;
   int L, rpt;
   if (!dr_plan(n_seg, H, dk, dv, &L, &rpt)) return HK_ERR_UNSUPPORTED;
-  const long long items = (long long)n_rows * H;
-  int e = hk_launch(gated_delta_prep_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, q, k, v, ld, bl, al, ldg, a_log,
-                    dt_bias, rec, items, H, G, dk, dv, L, rpt, q_scale, unit_eps);
+  const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
+  const int* psegs = most_rows ? segs : nullptr;
+  int e = hk_launch(gated_delta_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, bl, al, ldg, a_log,
+                    dt_bias, rec, psegs, items, H, G, dk, dv, L, rpt, q_scale, unit_eps);
   if (e) return e;
   return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, s);
 }
@@ -566,10 +583,10 @@ HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, l
 __global__ void retention_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                       long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot,
                                       const int* __restrict__ positions, const float* __restrict__ decay, float* __restrict__ rec,
-                                      long long items, int H, int dk, int dv, int L, int RPT, float k_scale, int lean) {
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+                                      const int* __restrict__ psegs, long long items, int H, int dk, int dv, int L, int RPT, float k_scale, int lean) {
+  long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (item >= items) return;
+  if (!prep_item(item, psegs, items, H)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const float* qp = q + row * ld + (size_t)h * dk;
@@ -748,17 +765,18 @@ static int ret_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s
 // q, k [n, H*dk] and v [n, H*dv] are column slices of one float32 matrix (row stride ld); decay float32 [H]; `rec` as for
 // hk_delta_rule_scan.  Blocks, columns a block and columns a lane group are chosen as for the delta rule's scan.
 HK_API int hk_retention_scan(const float* q, const float* k, const float* v, long long ld, const float* cos_t, const float* sin_t,
-                             int rot, const int* positions, const float* decay, const int* segs, int n_seg, int n_rows, float* rec,
+                             int rot, const int* positions, const float* decay, const int* segs, int n_seg, int n_rows, int most_rows, float* rec,
                              float* state, float* out, int H, int dk, int dv, float k_scale, void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
   if (H < 1 || dk < 1 || dv < 1 || dk > 2048 || rot < 0 || rot > dk || (rot & 1) || ((uintptr_t)rec & 15)) return HK_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
   int L, rpt;
   if (!dr_plan(n_seg, H, dk, dv, &L, &rpt)) return HK_ERR_UNSUPPORTED;
-  const long long items = (long long)n_rows * H;
+  const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
+  const int* psegs = most_rows ? segs : nullptr;
   const int lean = (dv & 3) == 0;
-  int e = hk_launch(retention_prep_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, q, k, v, ld, cos_t, sin_t, rot,
-                    positions, decay, rec, items, H, dk, dv, L, rpt, k_scale, lean);
+  int e = hk_launch(retention_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, cos_t, sin_t, rot,
+                    positions, decay, rec, psegs, items, H, dk, dv, L, rpt, k_scale, lean);
   if (e) return e;
   if (!lean) return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, s);
   const int R = 2 * L * rpt + dv;
@@ -840,12 +858,21 @@ mlstm_gates_kernel(const float* __restrict__ il, const float* __restrict__ fl, l
   if (lane == 0) m_state[(size_t)slot * H + h] = m;
 }
 
+// The maxima and the three exponentials per token alone, for requests whose matrix part another kernel runs.
+HK_API int hk_mlstm_gates(const float* il, const float* fl, long long ld, const float* i_bias, const float* f_bias, const int* segs,
+                          int n_seg, float* gates, float* m_state, int H, float cap, void* stream) {
+  if (n_seg <= 0) return 0;
+  if (H < 1 || !(cap > 0.f)) return HK_ERR_UNSUPPORTED;
+  return hk_launch(mlstm_gates_kernel, dim3((unsigned)((n_seg * H + 3) / 4)), dim3(128), 0, (cudaStream_t)stream, il, fl, ld, i_bias, f_bias,
+                   segs, m_state, gates, n_seg, H, cap);
+}
+
 __global__ void mlstm_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                  long long ld, const float* __restrict__ gates, float* __restrict__ rec, long long items, int H,
+                                  long long ld, const float* __restrict__ gates, float* __restrict__ rec, const int* __restrict__ psegs, long long items, int H,
                                   int dk, int dv, int dvp, int L, int RPT, float q_scale) {
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (item >= items) return;
+  if (!prep_item(item, psegs, items, H)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const float keep = gates[item * 3], take = gates[item * 3 + 1];
@@ -871,7 +898,7 @@ HK_API int hk_mlstm_padded(int dv) { return (dv + 1 + 3) & ~3; }
 // q, k [n, H*dk], v [n, H*dv], il, fl [n, H]: column slices of one float32 matrix (row stride ld).  state
 // [slots, H, dk, dvp], m_state [slots, H], gates scratch [n, H, 3] (kept: the output's gate reads e^(-m)), out [n, H*dvp].
 HK_API int hk_mlstm_scan(const float* q, const float* k, const float* v, const float* il, const float* fl, long long ld,
-                         const float* i_bias, const float* f_bias, const int* segs, int n_seg, int n_rows, float* rec,
+                         const float* i_bias, const float* f_bias, const int* segs, int n_seg, int n_rows, int most_rows, float* rec,
                          float* gates, float* state, float* m_state, float* out, int H, int dk, int dv, float cap, float q_scale,
                          void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
@@ -883,9 +910,9 @@ HK_API int hk_mlstm_scan(const float* q, const float* k, const float* v, const f
   int e = hk_launch(mlstm_gates_kernel, dim3((unsigned)((n_seg * H + 3) / 4)), dim3(128), 0, s, il, fl, ld, i_bias, f_bias, segs,
                     m_state, gates, n_seg, H, cap);
   if (e) return e;
-  const long long items = (long long)n_rows * H;
-  e = hk_launch(mlstm_prep_kernel, dim3((unsigned)((items + 7) / 8)), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, items,
-                H, dk, dv, dvp, L, rpt, q_scale);
+  const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
+  const int* psegs = most_rows ? segs : nullptr;
+  e = hk_launch(mlstm_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, psegs, items,                 H, dk, dv, dvp, L, rpt, q_scale);
   if (e) return e;
   return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dvp, L, rpt, s);
 }

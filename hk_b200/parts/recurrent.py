@@ -97,7 +97,52 @@ class _SegmentScan(Part):
         return ctx.tables[SEGMENTS_KEY][0]["segments"]
 
 
-class GeneralDeltaRule(_SegmentScan):
+class _ChunkedScan(_SegmentScan):
+    """A recurrence that, when serving in bfloat16, walks a request that brings `CHUNKS_FROM` tokens or more to a step in chunks
+    of tokens (`csrc/delta_chunks.cu`) and the others token by token; the lists of requests and chunks are host-built tables
+    that all such mixers of a model share."""
+    CHUNKS_FROM = 64        # where the two are level, 30 to 50 us; at 128 tokens the chunks take two thirds of the walk's time
+    CHUNK_KEY = ("chunked_segments",)
+    _chunks = False                 # set at bind: the chunked form takes this mixer's sizes
+
+    def kernel_libraries(self, bfloat16: bool):
+        return ("recurrent",) + (("delta_chunks",) if bfloat16 and ops.delta_chunks_take(self.dk, self.dv) else ())
+
+    def _bind_chunks(self, precision: Precision, row: int, decay_scale: float = 0.0) -> None:
+        """`row`: the length of the rows that the recurrence reads, which wide loads want in whole 16-byte pieces."""
+        self._chunks = precision.compute == torch.bfloat16 and row % 4 == 0 and ops.delta_chunks_take(self.dk, self.dv, decay_scale)
+
+    def step_tables_key(self):
+        return self.CHUNK_KEY if self._chunks else SEGMENTS_KEY
+
+    def step_tables(self, ctx):
+        tables = segment_tables(ctx)
+        if not self._chunks:
+            return tables
+        seg = tables.arrays["segments"]
+        long = seg[:, 2] >= self.CHUNKS_FROM
+        chunks, requests = [], []
+        for slot, row, count in seg[long].tolist():
+            first = len(chunks)
+            chunks += [(row + t, min(ops.DELTA_CHUNK, count - t)) for t in range(0, count, ops.DELTA_CHUNK)]
+            requests.append((slot, first, len(chunks) - first))
+        return StepTables({"segments": seg, "short": seg[~long], "long": seg[long], "chunks": np.asarray(chunks, dtype=np.int32).reshape(-1, 2),
+                           "requests": np.asarray(requests, dtype=np.int32).reshape(-1, 3)})
+
+    def _scan_tables(self, ctx):
+        """(the segments that are walked token by token, the further arguments of a scan)."""
+        if not self._chunks:
+            return self._segments(ctx), {}
+        t = ctx.tables[self.CHUNK_KEY][0]
+        return t["short"], {"chunks": t["chunks"], "requests": t["requests"],
+                            "most_rows": self.CHUNKS_FROM - 1 if t["chunks"].shape[0] else 0}
+
+    def _all_segments(self, ctx) -> torch.Tensor:
+        """Every request of the step as a segment, whichever way it is walked."""
+        return ctx.tables[self.CHUNK_KEY][0]["segments"] if self._chunks else self._segments(ctx)
+
+
+class GeneralDeltaRule(_ChunkedScan):
     def __init__(self, hidden: int, n_heads: int, key_dim: int, prefix: str, norm_eps: float,
                  value_dim: Optional[int] = None, decay_rank: Optional[int] = None,
                  decay_scale: float = math.exp(-0.5), key_eps: float = 1e-6, names: Optional[Dict[str, str]] = None):
@@ -140,6 +185,7 @@ class GeneralDeltaRule(_SegmentScan):
         self.w_o = tensors[p + nm["o"]]
         self.a_bias, self.w_bias = tensors[p + nm["a_bias"]], tensors[p + nm["w_bias"]]
         self.norm_weight = tensors[p + nm["norm"]]
+        self._bind_chunks(precision, int(self.w_in.shape[0]), self.decay_scale)
 
     def forward(self, xb: torch.Tensor, residual: torch.Tensor, ctx, cache, write_cache: bool = True,
                 accumulate: bool = True) -> None:
@@ -154,8 +200,9 @@ class GeneralDeltaRule(_SegmentScan):
         wl = torch.empty((n, K), dtype=torch.float32, device=xb.device)
         ops.gemm(hid, self.w_w2, wl)
         o = torch.empty((n, V), dtype=torch.float32, device=xb.device)
-        ops.delta_rule_scan(r, k, v, al, wl, self.a_bias, self.w_bias, self._segments(ctx), cache.state, o,
-                            self.H, self.dk, self.dv, self.decay_scale, self.key_eps)
+        short, chunked = self._scan_tables(ctx)
+        ops.delta_rule_scan(r, k, v, al, wl, self.a_bias, self.w_bias, short, cache.state, o,
+                            self.H, self.dk, self.dv, self.decay_scale, self.key_eps, **chunked)
         og = torch.empty((n, V), dtype=xb.dtype, device=xb.device)
         ops.head_norm_gate(o, g, self.norm_weight, self.norm_eps, og, self.H, self.dv)
         ops.gemm(og, self.w_o, residual, accumulate=accumulate)
@@ -197,8 +244,9 @@ class MinGRU(_SegmentScan):
         ops.gemm(out, self.w_o, residual, accumulate=accumulate)
 
 
-class GatedDeltaRule(_SegmentScan):
-    kernel_libraries = ("recurrent", "short_conv")
+class GatedDeltaRule(_ChunkedScan):
+    def kernel_libraries(self, bfloat16: bool):
+        return super().kernel_libraries(bfloat16) + ("short_conv",)
 
     def __init__(self, hidden: int, n_heads: int, kv_heads: int, key_dim: int, value_dim: int, taps: int, prefix: str,
                  norm_eps: float, unit_eps: float = 1e-6, q_scale: Optional[float] = None, out_scale: float = 1.0,
@@ -249,26 +297,28 @@ class GatedDeltaRule(_SegmentScan):
         self.norm_weight = tensors[p + nm["norm"]]
         if self.out_scale != 1.0:
             self.norm_weight = (self.norm_weight * self.out_scale).contiguous()
+        self._bind_chunks(precision, self.channels)
 
     def forward(self, xb: torch.Tensor, residual: torch.Tensor, ctx, cache, write_cache: bool = True,
                 accumulate: bool = True) -> None:
         n = xb.shape[0]
         K, V, C, H = self.G * self.dk, self.H * self.dv, self.channels, self.H
         state, tail = cache[0].state, cache[1].state
-        segs = self._segments(ctx)
+        segs = self._all_segments(ctx)
+        short, chunked = self._scan_tables(ctx)
         proj = torch.empty((n, self.w_in.shape[0]), dtype=torch.float32, device=xb.device)
         ops.gemm(xb, self.w_in, proj)
         act = torch.empty((n, C), dtype=torch.float32, device=xb.device)
         ops.short_conv(proj[:, :C], self.conv, segs, tail, act)
         o = torch.empty((n, V), dtype=torch.float32, device=xb.device)
         ops.gated_delta_scan(act[:, :K], act[:, K:2 * K], act[:, 2 * K:], proj[:, C + V:C + V + H], proj[:, C + V + H:],
-                             self.a_log, self.dt_bias, segs, state, o, H, self.G, self.dk, self.dv, self.q_scale, self.unit_eps)
+                             self.a_log, self.dt_bias, short, state, o, H, self.G, self.dk, self.dv, self.q_scale, self.unit_eps, **chunked)
         og = torch.empty((n, V), dtype=xb.dtype, device=xb.device)
         ops.head_out_gate(o, proj[:, C:C + V], self.norm_weight, self.norm_eps, og, H, self.dv, act="silu")
         ops.gemm(og, self.w_o, residual, accumulate=accumulate)
 
 
-class Retention(_SegmentScan):
+class Retention(_ChunkedScan):
     def __init__(self, hidden: int, n_heads: int, key_dim: int, value_dim: int, decay, prefix: str, norm_eps: float,
                  position=None, k_scale: Optional[float] = None, names: Optional[Dict[str, str]] = None):
         decay = [float(x) for x in decay]
@@ -303,6 +353,7 @@ class Retention(_SegmentScan):
         self.w_in = torch.cat([t.to(wide) for t in mats], dim=0).contiguous()
         self.w_o = tensors[p + nm["o"]]
         self.decay = torch.tensor(self.decay_values, dtype=torch.float64).to(torch.float32).to(precision.device)
+        self._bind_chunks(precision, int(self.w_in.shape[0]))
 
     def forward(self, xb: torch.Tensor, residual: torch.Tensor, ctx, cache, write_cache: bool = True,
                 accumulate: bool = True) -> None:
@@ -315,8 +366,9 @@ class Retention(_SegmentScan):
         if self.position is not None:
             cos, sin, rot = self.position.tables()
         o = torch.empty((n, V), dtype=torch.float32, device=xb.device)
+        short, chunked = self._scan_tables(ctx)
         ops.retention_scan(proj[:, :K], proj[:, K:2 * K], proj[:, 2 * K:2 * K + V], cos, sin, rot, ctx.positions, self.decay,
-                           self._segments(ctx), cache.state, o, self.H, self.dk, self.dv, self.k_scale)
+                           short, cache.state, o, self.H, self.dk, self.dv, self.k_scale, **chunked)
         og = torch.empty((n, V), dtype=xb.dtype, device=xb.device)
         ops.head_out_gate(o, proj[:, 2 * K + V:], None, self.norm_eps, og, self.H, self.dv, act="silu")
         ops.gemm(og, self.w_o, residual, accumulate=accumulate)
@@ -530,7 +582,7 @@ class GatedLinearAttention(_SegmentScan):
         ops.gemm(og, self.w_o, residual, accumulate=accumulate)
 
 
-class MLSTM(_SegmentScan):
+class MLSTM(_ChunkedScan):
     def __init__(self, hidden: int, n_heads: int, key_dim: int, value_dim: int, gate_cap: float, prefix: str, norm_eps: float,
                  den_eps: float = 1e-6, q_scale: Optional[float] = None, names: Optional[Dict[str, str]] = None):
         if not gate_cap > 0:
@@ -566,6 +618,7 @@ class MLSTM(_SegmentScan):
         self.w_o = tensors[p + nm["o"]]
         self.i_bias, self.f_bias = tensors[p + nm["i_bias"]], tensors[p + nm["f_bias"]]
         self.norm_weight = tensors[p + nm["norm"]]
+        self._bind_chunks(precision, int(self.w_in.shape[0]))
 
     def forward(self, xb: torch.Tensor, residual: torch.Tensor, ctx, cache, write_cache: bool = True,
                 accumulate: bool = True) -> None:
@@ -575,9 +628,12 @@ class MLSTM(_SegmentScan):
         ops.gemm(xb, self.w_in, proj)
         o = torch.empty((n, H * self.dvp), dtype=torch.float32, device=xb.device)
         gates = torch.empty((n, H, 3), dtype=torch.float32, device=xb.device)
+        short, chunked = self._scan_tables(ctx)
+        if chunked:
+            chunked["long_segments"] = ctx.tables[self.CHUNK_KEY][0]["long"]
         ops.mlstm_scan(proj[:, :K], proj[:, K:2 * K], proj[:, 2 * K:2 * K + V], proj[:, 2 * K + 2 * V:2 * K + 2 * V + H],
-                       proj[:, 2 * K + 2 * V + H:], self.i_bias, self.f_bias, self._segments(ctx), cache[0].state,
-                       cache[1].state, o, gates, H, self.dk, self.dv, self.cap, self.q_scale)
+                       proj[:, 2 * K + 2 * V + H:], self.i_bias, self.f_bias, short, cache[0].state,
+                       cache[1].state, o, gates, H, self.dk, self.dv, self.cap, self.q_scale, **chunked)
         og = torch.empty((n, V), dtype=xb.dtype, device=xb.device)
         ops.head_out_gate(o, proj[:, 2 * K + V:2 * K + 2 * V], self.norm_weight, self.norm_eps, og, H, self.dv, act="sigmoid",
                           gates=gates, den_eps=self.den_eps)
