@@ -312,3 +312,55 @@ def run_latent(q, pages, block_table, out, H: int, dk: int, dv: int, page_tokens
                                                _ptr(out), q.shape[0], H, dv, stream)
         ops._check(code, "latent attention (combine)")
     return True
+
+
+# ---- attention over keys and values made from a compressed cache (csrc/attention_prefill_tc.cu) ------------------
+
+MADE_FIRST = 16         # positions from a request's start whose values are not rounded (FIRST_ROWS in csrc/attention_latent.cu)
+MADE_TOKENS = 256       # query tokens of a work item: two query tiles of one head
+
+
+def made_supported(plain_dim: int, rot_dim: int, v_head_dim: int, rank: int) -> bool:
+    return plain_dim == 128 and v_head_dim == 128 and rot_dim in (0, 64) and rank % 8 == 0
+
+
+def made_items(slots, q_starts, q_lens, start_positions, window: int):
+    """(items int32 [n, 8], segments int32 [requests, 4], firsts int32 [m, 4], rows): the work items of requests whose visible
+    cache rows are laid side by side, longest key ranges first, where those rows come from (`ops.latent_rows`), and which of the
+    step's rows stand at a request's start."""
+    items, segments, firsts, row = [], [], [], 0
+    for slot, qs, ql, p0 in zip(slots, q_starts, q_lens, start_positions):
+        first = max(0, p0 - window + 1) if window > 0 else 0
+        base = row - first                     # the row of position 0, were it there
+        for b0 in range(0, ql, MADE_TOKENS):
+            n, pos0 = min(MADE_TOKENS, ql - b0), p0 + b0
+            lo = max(0, pos0 - window + 1) if window > 0 else 0
+            items.append((qs + b0, n, base, pos0, lo, pos0 + n, -1, 0))
+        segments.append((slot, first, p0 + ql - first, row))
+        if p0 < MADE_FIRST:
+            firsts.append((qs, base, p0, min(ql, MADE_FIRST - p0)))
+        row += p0 + ql - first
+    items.sort(key=lambda r: r[4] - r[5])
+    return np.asarray(items, dtype=np.int32).reshape(-1, 8), np.asarray(segments, dtype=np.int32).reshape(-1, 4), \
+        np.asarray(firsts, dtype=np.int32).reshape(-1, 4), row
+
+
+def run_made(q, kv, rope, items, out, H: int, window: int, scale: float, c, w_uv, firsts, gate=None, gate_per_head: bool = False,
+             gate_scale: float = 1.0) -> None:
+    """out bf16 [n, H * 128] of the items' rows, from q bf16 [n, H * (128 + 64)] (128 without `rope`), kv bf16 [rows, H * 256] =
+    per head 128 key dims and 128 value dims, and rope bf16 [rows, 64], the key dims that all heads share (or None).  c bf16
+    [rows, r] and w_uv bf16 [H, 128, r]: what the values were made of, for the rows of `firsts`."""
+    from . import gemm_fast, ops
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    gated = (_ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), 1 if gate_per_head else 0, ctypes.c_float(gate_scale))
+    scale_log2 = ctypes.c_float(scale * math.log2(math.e))
+    lib = build.load("attention_prefill_tc")
+    code = lib.hk_attention_prefill_made(_ptr(q), _ptr(kv), _ptr(rope), ctypes.c_longlong(kv.shape[0]), _ptr(items), int(items.shape[0]),
+                                         _ptr(out), H, int(window), scale_log2, _ptr(gemm_fast.status_flag(q.device)), *gated, stream)
+    ops._check(code, "latent attention (made keys and values)")
+    if not firsts.shape[0]:
+        return
+    code = build.load("attention_latent").hk_latent_first_rows(
+        _ptr(q), _ptr(kv), _ptr(rope), _ptr(c), _ptr(w_uv), _ptr(firsts), int(firsts.shape[0]), _ptr(out), H,
+        int(rope.shape[1]) if rope is not None else 0, int(c.shape[1]), int(window), scale_log2, *gated, stream)
+    ops._check(code, "latent attention (first rows)")

@@ -652,3 +652,131 @@ HK_API int hk_attention_latent_combine(const float* part_o, const float* part_ml
 }
 
 HK_API int hk_attention_latent_rows() { return ROWS; }
+
+// ------------------------------------------------------------------ the first rows of a prompt
+// Where keys and values are made for a step, a value is rounded to bf16 before the attention's sum, not behind it.  The sums over
+// few keys are the largest (a prompt's first rows hold a third of its results' energy), so the first FIRST_ROWS positions of a
+// request are taken here again with values that are never rounded: out = W_uv,h (sum_j p_j c_j) [* gate], all in float32 behind
+// the scores.  A block per (head, request, 32 value dims), everything it reads staged in shared memory; 26 us at 32 heads.  Relative
+// error of a 2,048-token prompt through the mixer: 3.34e-3 in the latent space, 3.45e-3 without this, 3.19e-3 with it.
+constexpr int FIRST_ROWS = 16;
+
+struct FirstRows {
+  int q_row, row0, pos0, count;       // first of its rows of the step, the row of position 0 among the made rows
+};
+
+__global__ void __launch_bounds__(256)
+latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv, const bf16* __restrict__ rope, const bf16* __restrict__ c,
+                         const bf16* __restrict__ w_uv, const FirstRows* __restrict__ firsts, bf16* __restrict__ out, int H, int dr, int r,
+                         int window, float scale_log2, const float* __restrict__ gate, long long gate_ld, int gate_heads, float gate_scale) {
+  extern __shared__ __align__(16) float lat[];          // [FIRST_ROWS][r + 4], then bf16 [FIRST_ROWS][r + 8] of cache rows
+  constexpr int LDQ = 192 + 8;                          // 16-byte pieces of neighbouring rows lie in different banks
+  __shared__ __align__(16) bf16 qs[FIRST_ROWS][LDQ], ks[FIRST_ROWS][LDQ];
+  __shared__ float prob[FIRST_ROWS][FIRST_ROWS];
+  const int h = blockIdx.x, d0 = blockIdx.z * 32, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ldl = r + 4, ldc = r + 8;
+  bf16* cs = reinterpret_cast<bf16*>(lat + FIRST_ROWS * ldl);
+  const FirstRows f = firsts[blockIdx.y];
+  const int wide = 128 + dr, last = f.pos0 + f.count;   // keys are positions 0 .. last - 1
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  for (int e = tid; e < FIRST_ROWS * 24; e += 256) {
+    const int i = e / 24, p = (e % 24) * 8;
+    const bool q_in = i < f.count && p < wide, k_in = i < last && p < wide;
+    *reinterpret_cast<uint4*>(&qs[i][p]) = q_in ? *reinterpret_cast<const uint4*>(q + ((size_t)(f.q_row + i) * H + h) * wide + p) : zero;
+    const bf16* kp = p < 128 ? kv + ((size_t)(f.row0 + i) * H + h) * 256 + p : rope + (size_t)(f.row0 + i) * dr + p - 128;
+    *reinterpret_cast<uint4*>(&ks[i][p]) = k_in ? *reinterpret_cast<const uint4*>(kp) : zero;
+  }
+  for (int e = tid; e < FIRST_ROWS * (r / 8); e += 256) {
+    const int j = e / (r / 8), p = (e % (r / 8)) * 8;
+    *reinterpret_cast<uint4*>(cs + j * ldc + p) = j < last ? *reinterpret_cast<const uint4*>(c + (size_t)(f.row0 + j) * r + p) : zero;
+  }
+  __syncthreads();
+  auto halves = [](const uint4& v, float* x) {          // eight bf16 as floats
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      x[2 * e] = __uint_as_float(w[e] << 16);
+      x[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+    }
+  };
+  {                                                     // a score a thread; a row's 16 in one half of a warp
+    const int i = tid >> 4, j = tid & 15, pos = f.pos0 + i, lo = window > 0 ? max(0, pos - window + 1) : 0;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll 4
+    for (int p = 0; p < 192; p += 8) {
+      float a[8], b[8];
+      halves(*reinterpret_cast<const uint4*>(&qs[i][p]), a);
+      halves(*reinterpret_cast<const uint4*>(&ks[j][p]), b);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        s0 = fmaf(a[e], b[e], s0);
+        s1 = fmaf(a[e + 1], b[e + 1], s1);
+      }
+    }
+    const float s = j >= lo && j <= pos ? (s0 + s1) * scale_log2 : -INFINITY;
+    float m = s;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float p = m == -INFINITY ? 0.f : exp2f(s - m);
+    float total = p;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+    prob[i][j] = total > 0.f ? p / total : 0.f;
+  }
+  __syncthreads();
+  for (int e = tid; e < FIRST_ROWS * (r / 8); e += 256) {     // their sums in the latent space
+    const int i = e / (r / 8), p = (e % (r / 8)) * 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int j = 0; j < FIRST_ROWS; ++j) {
+      float x[8];
+      halves(*reinterpret_cast<const uint4*>(cs + j * ldc + p), x);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] = fmaf(prob[i][j], x[k], acc[k]);
+    }
+    *reinterpret_cast<float4*>(lat + i * ldl + p) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4*>(lat + i * ldl + p + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+  __syncthreads();
+  const int d = d0 + lane, i0 = warp * 2;               // a lane per value dim, a warp per two rows
+  const uint4* wp = reinterpret_cast<const uint4*>(w_uv + ((size_t)h * 128 + d) * r);
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 8
+  for (int k = 0; k < r; k += 8) {
+    float w[8];
+    halves(wp[k >> 3], w);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 x = *reinterpret_cast<const float4*>(lat + (i0 + i) * ldl + k), y = *reinterpret_cast<const float4*>(lat + (i0 + i) * ldl + k + 4);
+      acc[i][0] = fmaf(w[6], y.z, fmaf(w[4], y.x, fmaf(w[2], x.z, fmaf(w[0], x.x, acc[i][0]))));
+      acc[i][1] = fmaf(w[7], y.w, fmaf(w[5], y.y, fmaf(w[3], x.w, fmaf(w[1], x.y, acc[i][1]))));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (i0 + i >= f.count) continue;
+    const size_t row = (size_t)f.q_row + i0 + i;
+    float y = acc[i][0] + acc[i][1];
+    if (gate) y *= gate_scale / (1.0f + expf(-gate[row * gate_ld + (gate_heads ? h : h * 128 + d)]));
+    out[(row * H + h) * 128 + d] = __float2bfloat16_rn(y);
+  }
+}
+
+HK_API int hk_latent_first_rows_count() { return FIRST_ROWS; }
+
+// q, kv, rope, out and gate as for hk_attention_prefill_made; c bf16 [rows, r] the cache rows that kv was made from; w_uv bf16
+// [H, 128, r]; firsts int32 [n, 4] = (first row of the step, made row of position 0, position, rows with pos0 + rows <= 16).
+HK_API int hk_latent_first_rows(const void* q, const void* kv, const void* rope, const void* c, const void* w_uv, const void* firsts,
+                                int n_firsts, void* out, int H, int dr, int r, int window, float scale_log2, const float* gate,
+                                long long gate_ld, int gate_heads, float gate_scale, void* stream) {
+  if (n_firsts <= 0) return 0;
+  if (H < 1 || n_firsts > 65535 || (dr != 0 && dr != 64) || (dr != 0) != (rope != nullptr) || r < 8 || (r & 7) ||
+      (((uintptr_t)w_uv | (uintptr_t)q | (uintptr_t)kv | (uintptr_t)rope | (uintptr_t)c) & 15))
+    return HK_ERR_UNSUPPORTED;
+  const size_t smem = (size_t)FIRST_ROWS * ((r + 4) * sizeof(float) + (r + 8) * sizeof(bf16));
+  if (smem > 200 * 1024) return HK_ERR_UNSUPPORTED;
+  static HkSmemCache cache;
+  if (int e = hk_allow_smem(latent_first_rows_kernel, smem, cache)) return e;
+  return hk_launch(latent_first_rows_kernel, dim3((unsigned)H, (unsigned)n_firsts, 4), dim3(256), smem, (cudaStream_t)stream, (const bf16*)q,
+                   (const bf16*)kv, (const bf16*)rope, (const bf16*)c, (const bf16*)w_uv, (const FirstRows*)firsts, (bf16*)out, H, dr, r, window,
+                   scale_log2, gate, gate_ld, gate_heads, gate_scale);
+}

@@ -58,6 +58,7 @@ struct ScoreOpts {
   float gate_scale;
   const float* dist;    // [H, dist_n] in the base-2 domain: added to the score of a key n positions back, at
   int dist_n;           //   min(n, dist_n - 1); null: none
+  int gate_heads;       // 1 (made keys and values only): gate holds one logit per query head, [tokens, gate_ld >= H]
 };
 
 // eight values of a row of O, normalised and (with a gate) gated, packed into bfloat16
@@ -606,11 +607,12 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-template <int HD>
+template <int HD, int HDK>
 struct Smem2 {
-  alignas(1024) uint8_t q[2][ROWS * HD * 2];
-  alignas(1024) uint8_t k[2][TK * HD * 2];
-  alignas(1024) uint8_t v[2][TK * HD * 2];
+  static constexpr int VST = HDK > 128 ? 1 : 2;     // V stages: wider keys leave room for one
+  alignas(1024) uint8_t q[2][ROWS * HDK * 2];
+  alignas(1024) uint8_t k[2][TK * HDK * 2];
+  alignas(1024) uint8_t v[VST][TK * HD * 2];
   alignas(8) uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_full[2], o_done[2];
   uint32_t tmem_base;
   int abort_flag;
@@ -618,15 +620,21 @@ struct Smem2 {
 };
 
 // DIST: with a bias by distance (an instance of its own, so that the softmax of a model without one issues nothing for it)
-template <int HD, bool DIST>
+// MADE: keys and values made for the step from a compressed cache (a latent attention's prompt portions), not pages: every
+// query head has its own (H == G); a request's rows stand side by side, the row of position 0 at item.slot (which may lie
+// before the first row there is); map_k and map_v see [rows, H][128 key dims | 128 value dims], map_r the 64 key dims that all
+// heads share (HDK = HD + 64; without them HDK = HD).  2,048 tokens at 32 heads: 112 us (384 TFLOP/s of the visible pairs), where
+// the same scores and sums in the latent space (576 and 512 numbers a row instead of 192 and 128) took 876 us on mma.sync.
+template <int HD, int HDK, bool DIST, bool MADE>
 __global__ void __launch_bounds__(NT2, 1)
 attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                             const bf16* __restrict__ q, const int* __restrict__ block_table, int table_stride,
+                             const __grid_constant__ CUtensorMap map_r, const bf16* __restrict__ q, const int* __restrict__ block_table, int table_stride,
                              const Item* __restrict__ items, bf16* __restrict__ out, int H, int G, int page_tokens, int window,
                              float scale_log2, ScoreOpts so, int pages_cap, int* __restrict__ status) {
-  constexpr int CPR = HD / 8;
-  constexpr int KSTEPS = HD / 16;
-  constexpr int HALVES = HD / 64;
+  constexpr int CPR = HDK / 8;
+  constexpr int KSTEPS = HDK / 16;
+  constexpr int HALVES = HD / 64, KHALVES = HDK / 64;
+  constexpr int VST = Smem2<HD, HDK>::VST;
   constexpr uint32_t TMEM_COLS = 512;
   constexpr uint32_t SP_COL[2] = {0, 128};
   constexpr uint32_t O_COL[2] = {256, 256 + HD};
@@ -634,28 +642,31 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   constexpr uint32_t IDESC_O = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
 
   extern __shared__ uint8_t smem_raw[];
-  Smem2<HD>& sm = *reinterpret_cast<Smem2<HD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  Smem2<HD, HDK>& sm = *reinterpret_cast<Smem2<HD, HDK>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   volatile int* abort_flag = &sm.abort_flag;
 
   const Item it = items[blockIdx.x / G];
   const int g = blockIdx.x % G;
   const int group = H / G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int* bt = block_table + (size_t)it.slot * table_stride;
   const int t_begin = it.kv_lo / TK;
   const int t_end = (it.kv_hi + TK - 1) / TK;
   const int n_rows = it.n_tokens * group;
   const bool two = n_rows > ROWS;                 // the second tile has rows at all
   int* pages = sm.pages;
-  const int page_lo = it.kv_lo / page_tokens;
-  const int n_pages = it.kv_hi > it.kv_lo ? min((it.kv_hi - 1) / page_tokens - page_lo + 1, pages_cap) : 0;
-  for (int i = threadIdx.x; i < n_pages; i += NT2) pages[i] = bt[page_lo + i];
+  const int page_lo = MADE ? 0 : it.kv_lo / page_tokens;
+  const int n_pages = !MADE && it.kv_hi > it.kv_lo ? min((it.kv_hi - 1) / page_tokens - page_lo + 1, pages_cap) : 0;
+  if (!MADE) {
+    const int* bt = block_table + (size_t)it.slot * table_stride;
+    for (int i = threadIdx.x; i < n_pages; i += NT2) pages[i] = bt[page_lo + i];
+  }
   // The V stages start as zeros: a box that is not copied (a page outside the key range, or one that the request
   // does not hold) leaves its rows as they are, and whatever is there is multiplied by a probability of zero, which
-  // must not meet a NaN pattern.  K needs none: a score of such a key is masked before it is looked at.
-  {
+  // must not meet a NaN pattern.  K needs none: a score of such a key is masked before it is looked at.  (Made values come
+  // in whole boxes: rows that are not there as zeros, rows of other requests as they are.)
+  if (!MADE) {
     uint4* z = reinterpret_cast<uint4*>(sm.v[0]);
-    constexpr int N16 = 2 * TK * HD * 2 / 16;
+    constexpr int N16 = VST * TK * HD * 2 / 16;
     for (int i = threadIdx.x; i < N16; i += NT2) z[i] = make_uint4(0u, 0u, 0u, 0u);
   }
   if (threadIdx.x == 0) {
@@ -681,7 +692,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const int qt = warp >> 2, r = threadIdx.x & 127, row = qt * ROWS + r;
     const bool ok = row < n_rows;
     const int tok = ok ? row / group : 0, head = ok ? row - tok * group : 0;
-    const bf16* src = q + ((size_t)(it.q_row0 + tok) * H + g * group + head) * HD;
+    const bf16* src = q + ((size_t)(it.q_row0 + tok) * H + g * group + head) * HDK;
     const uint32_t qs = smem_u32(sm.q[qt]);
 #pragma unroll
     for (int c = 0; c < CPR; ++c) cp_async16(qs + swz(r, c, ROWS), src + c * 8, ok);
@@ -702,8 +713,25 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const int boxes = TK / box_rows;                                   // at most 16
     const uint32_t box_bytes = (uint32_t)box_rows * 128u;
     for (int n = 0; n < n_tiles; ++n) {
-      const int t = t_begin + n, st = n & 1;
-      const uint32_t par = (uint32_t)(((n >> 1) & 1) ^ 1);            // a fresh barrier lets the first fill through
+      const int t = t_begin + n, st_k = n & 1, st_v = n % VST;
+      // a fresh barrier lets the first fill through
+      const uint32_t par_k = (uint32_t)(((n >> 1) & 1) ^ 1), par_v = (uint32_t)(((n / VST) & 1) ^ 1);
+      if (MADE) {
+        if (lane != 0) continue;
+        const int row = it.slot + t * TK;
+        if (!mbar_wait(&sm.k_empty[st_k], par_k, abort_flag)) break;
+        mbar_expect_tx(&sm.k_full[st_k], TK * HDK * 2);
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h)
+          tma_load_3d(smem_u32(sm.k[st_k]) + (uint32_t)h * (TK * 128), &map_k, &sm.k_full[st_k], 0, row, g * 2 * HALVES + h);
+        if (HDK > HD) tma_load_3d(smem_u32(sm.k[st_k]) + (uint32_t)HALVES * (TK * 128), &map_r, &sm.k_full[st_k], 0, row, 0);
+        if (!mbar_wait(&sm.v_empty[st_v], par_v, abort_flag)) break;
+        mbar_expect_tx(&sm.v_full[st_v], TK * HD * 2);
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h)
+          tma_load_3d(smem_u32(sm.v[st_v]) + (uint32_t)h * (TK * 128), &map_v, &sm.v_full[st_v], 0, row, g * 2 * HALVES + HALVES + h);
+        continue;
+      }
       // this lane's box of the tile: does it hold keys of the range, and does the request hold its page?
       int row = -1;
       if (lane < boxes) {
@@ -715,10 +743,10 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
       const uint32_t bytes = (uint32_t)__popc(__ballot_sync(0xffffffffu, row >= 0)) * box_bytes * HALVES;
       bool alive = true;
       for (int kv = 0; kv < 2 && alive; ++kv) {
-        uint64_t* full = kv == 0 ? &sm.k_full[st] : &sm.v_full[st];
+        uint64_t* full = kv == 0 ? &sm.k_full[st_k] : &sm.v_full[st_v];
         int go = 1;
         if (lane == 0) {
-          go = mbar_wait(kv == 0 ? &sm.k_empty[st] : &sm.v_empty[st], par, abort_flag) ? 1 : 0;
+          go = mbar_wait(kv == 0 ? &sm.k_empty[st_k] : &sm.v_empty[st_v], kv == 0 ? par_k : par_v, abort_flag) ? 1 : 0;
           if (go) {
             if (bytes == 0) mbar_arrive(full);
             else mbar_expect_tx(full, bytes);
@@ -727,7 +755,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         go = __shfl_sync(0xffffffffu, go, 0);
         if (!go) { alive = false; break; }
         if (row >= 0) {
-          const uint32_t base = smem_u32(kv == 0 ? sm.k[st] : sm.v[st]) + (uint32_t)(lane * box_rows) * 128u;
+          const uint32_t base = smem_u32(kv == 0 ? sm.k[st_k] : sm.v[st_v]) + (uint32_t)(lane * box_rows) * 128u;
           const CUtensorMap* map = kv == 0 ? &map_k : &map_v;
 #pragma unroll
           for (int h = 0; h < HALVES; ++h) tma_load_3d(base + (uint32_t)h * (TK * 128), map, full, 0, row, h);
@@ -757,11 +785,11 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         }
       }
       for (int n = 0; n < n_tiles && ok; ++n) {
-        const int st = n & 1;
+        const int st = n % VST;
         const uint32_t vs = smem_u32(sm.v[st]);
         for (int qt = 0; qt < nq && ok; ++qt) {
           if (!mbar_wait(&sm.p_full[qt], (uint32_t)(n & 1), abort_flag)) { ok = false; break; }
-          if (qt == 0 && !mbar_wait(&sm.v_full[st], (uint32_t)((n >> 1) & 1), abort_flag)) { ok = false; break; }
+          if (qt == 0 && !mbar_wait(&sm.v_full[st], (uint32_t)((n / VST) & 1), abort_flag)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk)
@@ -902,10 +930,11 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         tc_fence_after();
         float l = l0 + l1;
         if (so.sink && valid) l += exp2f((so.sinks ? so.sinks[g * group + row % group] * 1.4426950408889634f : 0.f) - m);
-        const float inv = l > 0.f ? 1.0f / l : 0.f;
+        float inv = l > 0.f ? 1.0f / l : 0.f;
         const int out_row = it.q_row0 + (valid ? tq : 0), out_head = g * group + (valid ? row % group : 0);
         bf16* op = out + ((size_t)out_row * H + out_head) * HD;
-        const float* gp = so.gate ? so.gate + (size_t)out_row * so.gate_ld + (size_t)out_head * HD : nullptr;
+        const float* gp = so.gate && !so.gate_heads ? so.gate + (size_t)out_row * so.gate_ld + (size_t)out_head * HD : nullptr;
+        if (MADE && so.gate && so.gate_heads) inv *= so.gate_scale / (1.0f + __expf(-so.gate[(size_t)out_row * so.gate_ld + out_head]));
         // the whole row of O at once (the registers that held scores are free now): one wait instead of HD / 32
         uint32_t o[HD];
 #pragma unroll
@@ -960,22 +989,23 @@ bool make_page_map(CUtensorMap* map, const void* ptr, unsigned long long rows, i
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int HD, bool DIST>
+template <int HD, bool DIST, int HDK = HD, bool MADE = false>
 int launch2(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, const int* bt, int stride, const void* items, int n_items,
-            void* out, int H, int G, int pt, int window, float scale_log2, ScoreOpts so, int pages_cap, int* status, cudaStream_t s) {
-  const size_t smem = sizeof(Smem2<HD>) + 1024 + (size_t)pages_cap * sizeof(int);
-  if (smem > 225 * 1024) return HK_ERR_UNSUPPORTED;
+            void* out, int H, int G, int pt, int window, float scale_log2, ScoreOpts so, int pages_cap, int* status, cudaStream_t s,
+            const CUtensorMap* mr = nullptr) {
+  const size_t smem = sizeof(Smem2<HD, HDK>) + 1024 + (size_t)pages_cap * sizeof(int);
+  if (smem > (MADE ? 227 : 225) * 1024) return HK_ERR_UNSUPPORTED;
   static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_prefill_tc2_kernel<HD, DIST>, smem, allowed)) return e;
+  if (int e = hk_allow_smem(attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>, smem, allowed)) return e;
   dim3 grid((unsigned)n_items * (unsigned)G);
-  return hk_launch(attention_prefill_tc2_kernel<HD, DIST>, grid, dim3(NT2), smem, s, mk, mv, (const bf16*)q, bt, stride, (const Item*)items,
-                   (bf16*)out, H, G, pt, window, scale_log2, so, pages_cap, status);
+  return hk_launch(attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>, grid, dim3(NT2), smem, s, mk, mv, mr ? *mr : mk, (const bf16*)q, bt, stride,
+                   (const Item*)items, (bf16*)out, H, G, pt, window, scale_log2, so, pages_cap, status);
 }
 
 ScoreOpts make_opts(int sink, const float* sinks, float softcap, float scale_log2, int chunk, const float* gate, long long gate_ld,
                     float gate_scale, const float* dist, int dist_n) {
   ScoreOpts so = {sink, sink ? sinks : nullptr, 0.f, 0.f, chunk > 0 ? chunk : 0, gate, gate_ld, gate_scale, dist_n > 0 ? dist : nullptr,
-                  dist_n};
+                  dist_n, 0};
   if (softcap > 0.f) {
     so.cap_log2 = softcap * 1.4426950408889634f;
     so.cap_in2 = 2.8853900817779268f * scale_log2 / so.cap_log2;       // 2 log2(e) scale / softcap
@@ -1037,3 +1067,25 @@ HK_API int hk_attention_prefill_tc2(const void* q, const void* k_pages, const vo
          : launch2<64, false>(mk, mv, q, block_table, table_stride, items, n_items, out, H, G, page_tokens, window, scale_log2, so, pages_cap, status, s);
 }
 
+// Keys and values that were made for the step (see the kernel's MADE).  q bf16 [n, H, 128 (+ 64 with rope)]; kv bf16 [rows, H,
+// 128 key dims | 128 value dims]; rope bf16 [rows, 64], the key dims that all heads share behind their own 128, or null; items
+// as above for groups of one head (up to 256 query tokens), with the row of the request's position 0 in the place of its slot;
+// out bf16 [n, H, 128].  gate (or null): float32 logits [n, gate_ld], one per output (16-byte aligned rows) or, with gate_heads,
+// one per head.
+HK_API int hk_attention_prefill_made(const void* q, const void* kv, const void* rope, long long rows, const void* items, int n_items,
+                                     void* out, int H, int window, float scale_log2, int* status, const float* gate, long long gate_ld,
+                                     int gate_heads, float gate_scale, void* stream) {
+  if (n_items <= 0) return 0;
+  if (H < 1 || H > 16383 || rows < 1 || rows > 0x7fffffffLL || !(scale_log2 > 0.f)) return HK_ERR_UNSUPPORTED;
+  if (gate != nullptr && !gate_heads && ((((uintptr_t)gate) & 15) != 0 || (gate_ld & 3) != 0 || gate_ld < (long long)H * 128)) return HK_ERR_UNSUPPORTED;
+  if ((((uintptr_t)q | (uintptr_t)out) & 15) != 0 || (((uintptr_t)kv | (uintptr_t)rope) & 127) != 0) return HK_ERR_UNSUPPORTED;
+  ScoreOpts so = make_opts(0, nullptr, 0.f, scale_log2, 0, gate, gate_ld, gate_scale, nullptr, 0);
+  so.gate_heads = gate_heads;
+  CUtensorMap mk, mr;
+  if (!make_page_map(&mk, kv, (unsigned long long)rows, H * 256, TK)) return HK_ERR_UNSUPPORTED;
+  if (rope != nullptr && !make_page_map(&mr, rope, (unsigned long long)rows, 64, TK)) return HK_ERR_UNSUPPORTED;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (rope != nullptr)
+    return launch2<128, false, 192, true>(mk, mk, q, nullptr, 0, items, n_items, out, H, H, TK, window, scale_log2, so, 0, status, s, &mr);
+  return launch2<128, false, 128, true>(mk, mk, q, nullptr, 0, items, n_items, out, H, H, TK, window, scale_log2, so, 0, status, s);
+}

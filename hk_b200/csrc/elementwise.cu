@@ -1005,16 +1005,17 @@ HK_API int hk_sigmoid_gate(const void* x, int x_dtype, const float* gate, long l
 // A mixer that caches one compressed vector per token instead of keys and values.  One warp per (token, item) of two
 // fp32 projection outputs, the query heads q[n, H (dn + dr)] (row stride ldq) and the compressed row kv[n, r + dr] (row
 // stride ldkv; both may be slices of one matrix):
-//   query head h: its first dn dims go unchanged to q_plain[t, h, :dn] (they are multiplied with the keys' up-projection
-//                 afterwards); its last dr dims are rotated by the token's position into q_full[t, h, r : r + dr];
+//   query head h: its first dn dims go unchanged to q_plain[t, h, :dn] (heads `plain_head` elements apart; they are multiplied
+//                 with the keys' up-projection afterwards, or meet keys made with it); its last dr dims are rotated by the
+//                 token's position into q_rot[t, h, :dr] (heads `rot_head` apart);
 //   the compressed row: its first r dims are RMS-normed with `c_w` (the latent), its last dr dims are rotated (the one
 //                 rotated key part that all heads share); both go to the token's cache row [page][1][page_tokens][r + dr].
 // The rotation turns the first `rot` of the dr dims, pairing 0: (i, i + rot/2), 1: (2i, 2i + 1); the tables carry any
 // magnitude factor.  With write_kv == 0 only the queries are produced.
 template <typename T>
 __global__ void __launch_bounds__(128)
-latent_prep_kernel(const float* __restrict__ q, long long ldq, const float* __restrict__ kv, long long ldkv, T* __restrict__ q_plain, T* __restrict__ q_full,
-                   const float* __restrict__ c_w, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+latent_prep_kernel(const float* __restrict__ q, long long ldq, const float* __restrict__ kv, long long ldkv, T* __restrict__ q_plain, int plain_head,
+                   T* __restrict__ q_rot, int rot_head, const float* __restrict__ c_w, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                    int rot, int pairing, const int* __restrict__ positions, const int* __restrict__ slot_of_token,
                    const int* __restrict__ block_table, int table_stride, T* __restrict__ pages, int n, int H, int dn, int dr,
                    int r, int page_tokens, int write_kv) {
@@ -1033,10 +1034,10 @@ latent_prep_kernel(const float* __restrict__ q, long long ldq, const float* __re
   T* dst;             // where they go
   if (it < H) {
     const float* qh = q + (size_t)t * ldq + (size_t)it * (dn + dr);
-    T* qp = q_plain + ((size_t)t * H + it) * dn;
+    T* qp = q_plain + ((size_t)t * H + it) * plain_head;
     for (int i = lane; i < dn; i += 32) qp[i] = from_f32<T>(qh[i]);
     src = qh + dn;
-    dst = q_full + ((size_t)t * H + it) * (r + dr) + r;
+    dst = q_rot + ((size_t)t * H + it) * rot_head;
   } else {
     const int page = block_table[(size_t)slot_of_token[t] * table_stride + pos / page_tokens];
     if (page < 0) return;   // the host never schedules this; keeps a stale table from writing out of bounds
@@ -1059,7 +1060,8 @@ latent_prep_kernel(const float* __restrict__ q, long long ldq, const float* __re
   for (int i = rot + lane; i < dr; i += 32) dst[i] = from_f32<T>(src[i]);
 }
 
-HK_API int hk_latent_prep(const float* q, long long ldq, const float* kv, long long ldkv, void* q_plain, void* q_full, int dtype, const float* c_w, float eps,
+HK_API int hk_latent_prep(const float* q, long long ldq, const float* kv, long long ldkv, void* q_plain, int plain_head, void* q_rot, int rot_head,
+                          int dtype, const float* c_w, float eps,
                           const float* cos_t, const float* sin_t, int rot, int pairing, const int* positions,
                           const int* slot_of_token, const int* block_table, int table_stride, void* pages, int n, int H, int dn,
                           int dr, int r, int page_tokens, int write_kv, void* stream) {
@@ -1069,14 +1071,41 @@ HK_API int hk_latent_prep(const float* q, long long ldq, const float* kv, long l
   const long long items = (long long)n * (H + (write_kv ? 1 : 0));
   const dim3 grid((unsigned)((items + 3) / 4)), block(128);
   if (dtype == HK_F32)
-    return hk_launch_pdl(latent_prep_kernel<float>, grid, block, 0, s, q, ldq, kv, ldkv, (float*)q_plain, (float*)q_full, c_w, eps, cos_t,
+    return hk_launch_pdl(latent_prep_kernel<float>, grid, block, 0, s, q, ldq, kv, ldkv, (float*)q_plain, plain_head, (float*)q_rot, rot_head, c_w, eps, cos_t,
                          sin_t, rot, pairing, positions, slot_of_token, block_table, table_stride, (float*)pages, n, H, dn, dr, r,
                          page_tokens, write_kv);
   if (dtype == HK_BF16)
-    return hk_launch_pdl(latent_prep_kernel<bf16>, grid, block, 0, s, q, ldq, kv, ldkv, (bf16*)q_plain, (bf16*)q_full, c_w, eps, cos_t,
+    return hk_launch_pdl(latent_prep_kernel<bf16>, grid, block, 0, s, q, ldq, kv, ldkv, (bf16*)q_plain, plain_head, (bf16*)q_rot, rot_head, c_w, eps, cos_t,
                          sin_t, rot, pairing, positions, slot_of_token, block_table, table_stride, (bf16*)pages, n, H, dn, dr, r,
                          page_tokens, write_kv);
   return HK_ERR_UNSUPPORTED;
+}
+
+// The cache rows of whole requests side by side, for keys and values that are made for the step: segs int32 [n, 4] = (slot, first
+// position, rows, first row of the result); a row's first r numbers go to c[row, :r], the other dr to rope[row, :dr] (both in
+// 16-byte pieces).  Bound by its bytes, each read and written once.
+__global__ void latent_rows_kernel(const bf16* __restrict__ pages, const int* __restrict__ block_table, int table_stride,
+                                   const int* __restrict__ segs, bf16* __restrict__ c, bf16* __restrict__ rope, int r, int dr, int page_tokens) {
+  const int* seg = segs + 4 * blockIdx.y;
+  const int pieces = (r + dr) >> 3;
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (long long)seg[2] * pieces) return;
+  const int t = (int)(e / pieces), i = (int)(e % pieces) * 8, pos = seg[1] + t;
+  const int page = block_table[(size_t)seg[0] * table_stride + pos / page_tokens];
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (page >= 0) v = *reinterpret_cast<const uint4*>(pages + ((size_t)page * page_tokens + pos % page_tokens) * (r + dr) + i);
+  const size_t row = (size_t)seg[3] + t;
+  *reinterpret_cast<uint4*>(i < r ? c + row * r + i : rope + row * dr + i - r) = v;
+}
+
+HK_API int hk_latent_rows(const void* pages, const int* block_table, int table_stride, const int* segs, int n_segs, int most_rows, void* c,
+                          void* rope, int r, int dr, int page_tokens, void* stream) {
+  if (n_segs <= 0 || most_rows <= 0) return 0;
+  if (r < 8 || (r & 7) || dr < 0 || (dr & 7) || page_tokens < 1 || n_segs > 65535 || (((uintptr_t)pages | (uintptr_t)c | (uintptr_t)rope) & 15))
+    return HK_ERR_UNSUPPORTED;
+  const long long items = (long long)most_rows * ((r + dr) >> 3);
+  return hk_launch(latent_rows_kernel, dim3((unsigned)((items + 255) / 256), (unsigned)n_segs), dim3(256), 0, (cudaStream_t)stream, (const bf16*)pages,
+                   block_table, table_stride, segs, (bf16*)c, (bf16*)rope, r, dr, page_tokens);
 }
 
 // ----------------------------------------------------------------------------- sums of float32 streams

@@ -301,6 +301,24 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
     return True
 
 
+def run_narrow(a, w, out) -> bool:
+    """out (bf16 [M, N]) = a w^T on the tcgen05 kernel.  False when it refuses the shape."""
+    from . import ops
+    M, K = a.shape
+    N = w.shape[0]
+    if not _aligned(a, w):
+        return False
+    lib = build.load("gemm_tc")
+    bn, splits = tc_config(M, N, K, _sms(a.device))
+    partial = _tc_partial(lib, M, N, splits, a.device)
+    code = lib.hk_gemm_tc_narrow(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), bn, splits,
+                                 _ptr(partial) if splits > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)), _stream())
+    if code == _UNSUPPORTED:
+        return False
+    ops._check(code, "gemm, narrowed (tcgen05)")
+    return True
+
+
 GROUPED_ROWS = 128      # rows of a tile of the grouped tcgen05 product: an expert's rows start on a multiple of it
 
 

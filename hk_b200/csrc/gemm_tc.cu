@@ -40,11 +40,11 @@ constexpr int RING_BYTES = 227 * 1024 - 2 * 1024;   // what is left of an SM's s
 constexpr uint32_t TMEM_COLS = 2 * MAX_BN;
 constexpr uint32_t WAIT_LIMIT = 1u << 24;
 
-enum Epilogue { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2, EPI_GEGLU = 3, EPI_CLAMPGLU = 4, EPI_SQRELU = 5 };
+enum Epilogue { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2, EPI_GEGLU = 3, EPI_CLAMPGLU = 4, EPI_SQRELU = 5, EPI_NARROW = 6 };
 // The first two gated epilogues differ in the gate's activation alone: silu, or the tanh form of gelu, which is
 // g * sigmoid(2 * sqrt(2 / pi) * (g + 0.044715 g^3)).  The third clamps both halves first: with g = min(gate, limit) and
 // u = clamp(up, -limit, limit) it gives g * sigmoid(slope * g) * (u + 1); limit and slope travel as kernel arguments.
-// EPI_SQRELU has no gate: slope * max(z, 0)^2 narrowed to bf16 (slope is a factor on the result).
+// EPI_SQRELU has no gate: slope * max(z, 0)^2 narrowed to bf16 (slope is a factor on the result).  EPI_NARROW: z itself in bf16.
 #define IS_GLU(e) ((e) == EPI_SWIGLU || (e) == EPI_GEGLU || (e) == EPI_CLAMPGLU)
 struct GluParams {
   float limit, slope;
@@ -214,9 +214,13 @@ __device__ __forceinline__ void load_chunk(const float* o, int c0, float4* y) {
   for (int j = 0; j < 8; ++j) y[j] = *reinterpret_cast<const float4*>(o + c0 + 4 * j);
 }
 
-// W columns as W bf16 outputs slope * max(z, 0)^2.
-template <int W>
-__device__ __forceinline__ void sqrelu_chunk(uint32_t taddr, bf16* o, int c0, int n_out, bool row_ok, bool vec_ok, GluParams gp) {
+// W columns as W bf16 outputs, slope * max(z, 0)^2 or z itself.
+template <int EPI>
+__device__ __forceinline__ bf16 narrowed(float z, GluParams gp) {
+  return EPI == EPI_NARROW ? __float2bfloat16_rn(z) : squared_relu(z, gp);
+}
+template <int W, int EPI>
+__device__ __forceinline__ void narrow_chunk(uint32_t taddr, bf16* o, int c0, int n_out, bool row_ok, bool vec_ok, GluParams gp) {
   uint32_t v[W];
   tmem_ld<W>(taddr + (uint32_t)c0, v);
   tmem_ld_wait();
@@ -228,15 +232,15 @@ __device__ __forceinline__ void sqrelu_chunk(uint32_t taddr, bf16* o, int c0, in
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         __nv_bfloat162 p;
-        p.x = squared_relu(__uint_as_float(v[j + 2 * e]), gp);
-        p.y = squared_relu(__uint_as_float(v[j + 2 * e + 1]), gp);
+        p.x = narrowed<EPI>(__uint_as_float(v[j + 2 * e]), gp);
+        p.y = narrowed<EPI>(__uint_as_float(v[j + 2 * e + 1]), gp);
         packed[e] = *reinterpret_cast<uint32_t*>(&p);
       }
       *reinterpret_cast<uint4*>(o + c0 + j) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     }
   } else {
     for (int j = 0; j < W; ++j)
-      if (c0 + j < n_out) o[c0 + j] = squared_relu(__uint_as_float(v[j]), gp);
+      if (c0 + j < n_out) o[c0 + j] = narrowed<EPI>(__uint_as_float(v[j]), gp);
   }
 }
 
@@ -434,14 +438,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll 1
         for (; c0 + 32 <= h; c0 += 32) swiglu_chunk<32, EPI>(taddr, o, c0, h, n_out, row_ok, vec_ok, gp);
         if (c0 < h) swiglu_chunk<16, EPI>(taddr, o, c0, h, n_out, row_ok, vec_ok, gp);
-      } else if (EPI == EPI_SQRELU) {
+      } else if (EPI == EPI_SQRELU || EPI == EPI_NARROW) {
         bf16* o = reinterpret_cast<bf16*>(out) + (size_t)row * ldo + nt * bn;
         const int n_out = N - nt * bn;
         const bool vec_ok = (ldo & 7) == 0 && ((nt * bn) & 7) == 0;
         int c0 = 0;
 #pragma unroll 1
-        for (; c0 + 32 <= bn; c0 += 32) sqrelu_chunk<32>(taddr, o, c0, n_out, row_ok, vec_ok, gp);
-        if (c0 < bn) sqrelu_chunk<16>(taddr, o, c0, n_out, row_ok, vec_ok, gp);
+        for (; c0 + 32 <= bn; c0 += 32) narrow_chunk<32, EPI>(taddr, o, c0, n_out, row_ok, vec_ok, gp);
+        if (c0 < bn) narrow_chunk<16, EPI>(taddr, o, c0, n_out, row_ok, vec_ok, gp);
       } else {
         const int n0 = nt * bn;
         float* o = reinterpret_cast<float*>(out) + (size_t)row * ldo + n0;
@@ -523,7 +527,7 @@ int sm_count() {
 
 // Adds the K slices of a split product in slice order.  mode 0: out fp32 = sum; 1: out fp32 += sum;
 // 2 (silu), 3 (tanh gelu) and 4 (clamped): out bf16 [M, N/2] = act(gate) * up, the partial sums' columns in tiles of [bn / 2 gates | their bn / 2 ups];
-// 5: out bf16 [M, N] = slope * max(sum, 0)^2.
+// 5: out bf16 [M, N] = slope * max(sum, 0)^2; 6: out bf16 [M, N] = sum.
 template <int MODE>
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, void* __restrict__ out, int M, int N, long long ldo,
                                      int splits, int bn, GluParams gp) {
@@ -548,8 +552,8 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, void* __
     const int m = (int)(i / N), n = (int)(i % N);
     float sum = 0.f;
     for (int s = 0; s < splits; ++s) sum += partial[s * slice + i];
-    if (MODE == EPI_SQRELU) {
-      reinterpret_cast<bf16*>(out)[(size_t)m * ldo + n] = squared_relu(sum, gp);
+    if (MODE == EPI_SQRELU || MODE == EPI_NARROW) {
+      reinterpret_cast<bf16*>(out)[(size_t)m * ldo + n] = narrowed<MODE>(sum, gp);
       return;
     }
     float* o = reinterpret_cast<float*>(out) + (size_t)m * ldo + n;
@@ -622,7 +626,7 @@ static int gemm_tc_run(const void* a, const void* w, void* out, int M, int N, in
                        int splits, float* partial, int* status, GluParams gp, void* stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || (K & 7) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return HK_ERR_UNSUPPORTED;
-  if (epilogue < EPI_STORE || epilogue > EPI_SQRELU) return HK_ERR_UNSUPPORTED;
+  if (epilogue < EPI_STORE || epilogue > EPI_NARROW) return HK_ERR_UNSUPPORTED;
   if (bn < 16 || bn > MAX_BN || (bn & 15)) return HK_ERR_UNSUPPORTED;
   if (IS_GLU(epilogue) && ((N & 1) || (bn & 31))) return HK_ERR_UNSUPPORTED;
   if (splits < 1 || splits > (K + BK - 1) / BK || (splits > 1 && partial == nullptr)) return HK_ERR_UNSUPPORTED;
@@ -635,6 +639,7 @@ static int gemm_tc_run(const void* a, const void* w, void* out, int M, int N, in
   if (epilogue == EPI_GEGLU) return launch<EPI_GEGLU>(ma, mw, out, M, N, K, ldo, bn, splits, partial, status, s);
   if (epilogue == EPI_CLAMPGLU) return launch<EPI_CLAMPGLU>(ma, mw, out, M, N, K, ldo, bn, splits, partial, status, s, nullptr, gp);
   if (epilogue == EPI_SQRELU) return launch<EPI_SQRELU>(ma, mw, out, M, N, K, ldo, bn, splits, partial, status, s, nullptr, gp);
+  if (epilogue == EPI_NARROW) return launch<EPI_NARROW>(ma, mw, out, M, N, K, ldo, bn, splits, partial, status, s);
   return launch<EPI_SWIGLU>(ma, mw, out, M, N, K, ldo, bn, splits, partial, status, s);
 }
 
@@ -655,6 +660,12 @@ HK_API int hk_gemm_tc_clamped(const void* a, const void* w, void* out, int M, in
 HK_API int hk_gemm_tc_sqrelu(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, int bn, int splits,
                              float* partial, int* status, float factor, void* stream) {
   return gemm_tc_run(a, w, out, M, N, K, ldo, EPI_SQRELU, bn, splits, partial, status, GluParams{0.f, factor}, stream);
+}
+
+// The product narrowed (epilogue 6): out bf16 [M, N] = a w^T.
+HK_API int hk_gemm_tc_narrow(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, int bn, int splits,
+                             float* partial, int* status, void* stream) {
+  return gemm_tc_run(a, w, out, M, N, K, ldo, EPI_NARROW, bn, splits, partial, status, GluParams{0.f, 1.f}, stream);
 }
 
 // Floats of scratch that `hk_gemm_tc` needs for `splits` K slices.

@@ -597,24 +597,34 @@ def sigmoid_gate(x: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, scale: 
 
 
 def latent_prep(q, kv, q_plain, q_full, c_weight, eps, cos, sin, rotary_dim, pairing, positions, slot_of_token, block_table,
-                pages, n_heads, plain_dim, rot_dim, rank, page_tokens, write_kv=True) -> None:
+                pages, n_heads, plain_dim, rot_dim, rank, page_tokens, write_kv=True, q_packed=None) -> None:
     """What a token brings to a latent attention, from two float32 column slices: q [n, H*(dn+dr)] = H query heads of (dn
     plain | dr to rotate), and kv [n, r + dr] = r compressed dims, then the dr dims of the shared rotated key:
     q_plain[n, H*dn] takes the queries' plain parts, q_full[n, H*(r+dr)] their rotated parts in its last dr dims per
     head (the first r are left for the absorbed product), and the token's cache row [page, 0, place, r+dr] takes the
-    compressed dims RMS-normed with `c_weight` and the rotated key part."""
+    compressed dims RMS-normed with `c_weight` and the rotated key part.  With `q_packed` [n, H*(dn+dr)] a head's plain and
+    rotated parts go there side by side instead (q_plain and q_full are then not looked at)."""
     if pairing not in PAIRINGS:
         raise KernelError(f"latent_prep: pairing {pairing!r} is neither 'half' nor 'adjacent'")
     H, dn, dr, r = n_heads, plain_dim, rot_dim, rank
-    _need(q_plain, "q_plain", dims=2)
-    _need(q_full, "q_full", q_plain.dtype, 2)
+    if q_packed is not None:
+        _need(q_packed, "q_packed", dims=2)
+        q_plain, rot_out, plain_head, rot_head = q_packed, q_packed.data_ptr() + dn * q_packed.element_size(), dn + dr, dn + dr
+        if q_packed.shape[1] != H * (dn + dr):
+            raise KernelError("latent_prep: q_packed has the wrong shape")
+    else:
+        _need(q_plain, "q_plain", dims=2)
+        _need(q_full, "q_full", q_plain.dtype, 2)
+        rot_out, plain_head, rot_head = q_full.data_ptr() + r * q_full.element_size(), dn, r + dr
+        if tuple(q_plain.shape) != (q_full.shape[0], H * dn) or q_full.shape[1] != H * (r + dr):
+            raise KernelError("latent_prep: q_plain or q_full has the wrong shape")
     _need(c_weight, "c_weight", torch.float32, 1)
     n = q_plain.shape[0]
     ldq, ldkv = _cols(q, "q", H * (dn + dr)), _cols(kv, "kv", r + dr)
     if q.shape[0] != n or kv.shape[0] != n:
         raise KernelError("latent_prep: one row of q and kv per token")
-    if tuple(q_plain.shape) != (n, H * dn) or tuple(q_full.shape) != (n, H * (r + dr)) or c_weight.shape[0] != r:
-        raise KernelError("latent_prep: q_plain, q_full or the norm weight has the wrong shape")
+    if c_weight.shape[0] != r:
+        raise KernelError("latent_prep: the norm weight has the wrong shape")
     if rotary_dim > 0:
         _need(cos, "cos", torch.float32, 2)
         _need(sin, "sin", torch.float32, 2)
@@ -629,11 +639,43 @@ def latent_prep(q, kv, q_plain, q_full, c_weight, eps, cos, sin, rotary_dim, pai
             raise KernelError("latent_prep: cache pages must be [pages, 1, page_tokens, rank + rot_dim]")
     lib = build.load("elementwise")
     _check(lib.hk_latent_prep(
-        _ptr(q), ctypes.c_longlong(ldq), _ptr(kv), ctypes.c_longlong(ldkv), _ptr(q_plain), _ptr(q_full), _dt(q_plain), _ptr(c_weight),
+        _ptr(q), ctypes.c_longlong(ldq), _ptr(kv), ctypes.c_longlong(ldkv), _ptr(q_plain), int(plain_head),
+        ctypes.c_void_p(rot_out), int(rot_head), _dt(q_plain), _ptr(c_weight),
         ctypes.c_float(eps), _ptr(cos if rotary_dim > 0 else None), _ptr(sin if rotary_dim > 0 else None), int(rotary_dim),
         PAIRINGS[pairing], _ptr(positions), _ptr(slot_of_token), _ptr(block_table if write_kv else None),
         int(block_table.shape[1]) if write_kv else 0, _ptr(pages if write_kv else None), n, H, dn, dr, r, int(page_tokens),
         1 if write_kv else 0, _stream()), "latent_prep")
+
+
+def latent_rows(pages, block_table, segments, most_rows: int, c, rope) -> None:
+    """The cache rows of whole requests side by side: `segments` int32 [n, 4] = (slot, first position, rows, first row of the
+    result), none of more than `most_rows` rows; c [rows, r] and rope [rows, dr] (None where a row has no such part), bfloat16."""
+    _need(pages, "pages", torch.bfloat16, 4)
+    _need(block_table, "block_table", torch.int32, 2)
+    _need(segments, "segments", torch.int32, 2)
+    _need(c, "c", torch.bfloat16, 2)
+    dr = 0
+    if rope is not None:
+        _need(rope, "rope", torch.bfloat16, 2)
+        dr = int(rope.shape[1])
+    r = int(c.shape[1])
+    if segments.shape[1] != 4 or pages.shape[1] != 1 or pages.shape[3] != r + dr or (rope is not None and rope.shape[0] != c.shape[0]):
+        raise KernelError("latent_rows: shapes do not fit")
+    lib = build.load("elementwise")
+    _check(lib.hk_latent_rows(_ptr(pages), _ptr(block_table), int(block_table.shape[1]), _ptr(segments), int(segments.shape[0]), int(most_rows),
+                              _ptr(c), _ptr(rope), r, dr, int(pages.shape[2]), _stream()), "latent_rows")
+
+
+def gemm_narrow(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+    """out bfloat16 [M, N] = a @ w^T, both bfloat16 (float32 sums, rounded once)."""
+    _need(a, "a", torch.bfloat16, 2)
+    _need(w, "w", torch.bfloat16, 2)
+    _need(out, "out", torch.bfloat16, 2)
+    if a.shape[1] != w.shape[1] or tuple(out.shape) != (a.shape[0], w.shape[0]):
+        raise KernelError("gemm_narrow: shapes do not fit")
+    from . import gemm_fast
+    if not gemm_fast.run_narrow(a, w, out):
+        raise KernelError("gemm_narrow: the tcgen05 kernel refuses this shape")
 
 
 def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n_heads: int, gate: Optional[torch.Tensor] = None,

@@ -16,20 +16,46 @@ the output gate are parameters; `names` renames the tensors (keys q, dkv, dkv_no
   `q_rank`: the queries come through a latent of their own, q = W_uq (rms(W_dq x) * weight), instead of W_q x;
   `gate="head"`: one gate number per head (tensor [n_heads, hidden]) instead of one per output of a head;
   `out_scale` is a factor on the mixer's result that the gate carries.
+
+Prompt portions, when serving in bfloat16 with heads of 128 plain dims, 64 rotated ones (or none) and values of 128: a query
+meets 128 + 64 numbers of a key and 128 of a value instead of kv_rank + rot_dim and kv_rank of a cache row, a third of the
+arithmetic, where enough queries share the making of keys and values.  A request that brings `MADE_FROM` tokens or more to a
+step has them made from the cache rows it sees (one product for all heads) and runs on the tcgen05 prompt kernel; the others
+stay in the latent space.
 """
 from __future__ import annotations
 
-from typing import Dict, Optional
+from dataclasses import dataclass
+from types import SimpleNamespace
+from typing import Dict, List, Optional, Tuple
 
 import torch
 
 from ..csrc import ops
-from .base import KVCacheSpec, MATRIX, VECTOR, ParamSpec, Part, Precision, register_part, stacked_rows
+from .base import KVCacheSpec, MATRIX, VECTOR, ParamSpec, Part, Precision, StepTables, register_part, stacked_rows
 from .position import RotaryEmbedding
+
+
+@dataclass
+class LatentInfo:
+    """The host-side facts of a step in which requests have their keys and values made: the latent kernel's plan for the others
+    (or None), runs of neighbouring rows (first, one past the last, made or not), and the made rows."""
+    plan: object
+    single_tokens: bool
+    runs: List[Tuple[int, int, bool]]
+    rows: int
+    most_rows: int
 
 
 class LatentAttention(Part):
     graph_safe = True   # reads the batch from device tensors only
+    # Measured at 32 heads, prompt mixer alone, latent space against made: 2,048 tokens 1,213 us against 364; 128 tokens behind
+    # 4,000 348 against 220, 64 behind 2,000 176 against 172 (level: 32 rows made for a query); 64 to 128 tokens level, bound by
+    # the launches.  Rows made are bounded to 16 a query, which bounds their memory too.
+    MADE_FROM = 64
+    MADE_ROWS = 16
+    MADE_BESIDE = 256   # beside requests that stay in the latent space: so many tokens at least, for the further launches
+    MADE_RUNS = 4       # a step whose kinds of requests alternate more often stays in the latent space: every run is launched apart
 
     def __init__(self, hidden: int, n_heads: int, plain_dim: int, rot_dim: int, v_head_dim: int, kv_rank: int, prefix: str,
                  norm_eps: float, scale: float, position: Optional[RotaryEmbedding] = None, gate=False,
@@ -57,6 +83,7 @@ class LatentAttention(Part):
         self._tables_key = None        # set at bind: the flash kernels' work items, when they take a row of this size
         self._sm_count = 0
         self._wide = False             # set at bind: the row is too wide for the flash kernels, the latent kernel takes it
+        self._w_ukv = None             # set at bind, where prompt portions have keys and values made: per head [W_uk,h | W_uv,h]
 
     def _flash_takes(self) -> bool:
         """The flash kernels run H query heads over ONE key/value head whose keys and values are both the cache row
@@ -69,12 +96,20 @@ class LatentAttention(Part):
         from ..csrc import attention_fast
         return attention_fast.latent_supported(self.H, self.r + self.dr, self.r)
 
+    def _made_takes(self) -> bool:
+        """The tcgen05 prompt kernel takes keys and values of these sizes (and the gate's logits lie on 16-byte boundaries)."""
+        from ..csrc import attention_fast
+        first = self.q_rank if self.q_rank is not None else self.H * (self.dn + self.dr)
+        return attention_fast.made_supported(self.dn, self.dr, self.vd, self.r) \
+            and (not self.gate or self.gate_per_head or (first + self.r + self.dr) % 4 == 0)
+
     def kernel_libraries(self, bfloat16: bool):
         from ..csrc import attention_fast
         if not bfloat16:
             return ()
         if not self._flash_takes():
-            return ("gemm_heads", "attention_latent") if self._latent_kernel_takes() else ("gemm_heads",)
+            made = ("attention_prefill_tc",) if self._made_takes() else ()
+            return ("gemm_heads", "attention_latent") + made if self._latent_kernel_takes() else ("gemm_heads",)
         return ("gemm_heads", "attention_flash", "attention_prefill_tc") if attention_fast.tc_prefill_supported(self.r + self.dr, self.H) \
             else ("gemm_heads", "attention_flash")
 
@@ -83,10 +118,47 @@ class LatentAttention(Part):
 
     def step_tables(self, ctx):
         from .attention import flash_step_tables
+        if self._w_ukv is not None and not ctx.fixed_shape:
+            tables = self._made_tables(ctx)
+            if tables is not None:
+                return tables
         if self._wide:
             # items of at most 64 / H tokens, all heads of a token in one item; never the tcgen05 prompt kernels' tiles
             return flash_step_tables(ctx, self.H, 1, self.r + self.dr, self.window or 0, 0, self._sm_count, tensor_prompt=False)
         return flash_step_tables(ctx, self.H, 1, self.r + self.dr, self.window or 0, 0, self._sm_count)
+
+    def _made_tables(self, ctx) -> Optional[StepTables]:
+        from ..csrc import attention_fast
+        from .attention import flash_step_tables
+        window = self.window or 0
+        seen = [int(c) + (min(int(p), window - 1) if window else int(p)) for c, p in zip(ctx.q_lens, ctx.start_positions)]
+        made = [int(c) >= self.MADE_FROM and v <= self.MADE_ROWS * int(c) for c, v in zip(ctx.q_lens, seen)]
+        runs: List[Tuple[int, int, bool]] = []
+        for start, count, m in zip(ctx.q_starts, ctx.q_lens, made):
+            if runs and runs[-1][2] == m:
+                runs[-1] = (runs[-1][0], start + count, m)
+            else:
+                runs.append((start, start + count, m))
+        if not any(made) or len(runs) > self.MADE_RUNS:
+            return None
+        if not all(made) and sum(int(c) for c, m in zip(ctx.q_lens, made) if m) < self.MADE_BESIDE:
+            return None
+
+        def those(kind):
+            return [[x for x, m in zip(xs, made) if m == kind] for xs in (ctx.slots, ctx.q_starts, ctx.q_lens, ctx.start_positions)]
+
+        items, segments, firsts, rows = attention_fast.made_items(*those(True), window)
+        arrays, plan, single = {"made_items": items, "made_segments": segments, "made_firsts": firsts}, None, False
+        if not all(made):
+            slots, q_starts, q_lens, starts = those(False)
+            rest = SimpleNamespace(slots=slots, q_starts=q_starts, q_lens=q_lens, start_positions=starts, n_tokens=ctx.n_tokens,
+                                   fixed_shape=False, max_context=ctx.max_context, page_tokens=ctx.page_tokens)
+            got = flash_step_tables(rest, self.H, 1, self.r + self.dr, window, 0, self._sm_count, tensor_prompt=False)
+            if got is None:
+                return None
+            arrays.update(got.arrays)
+            plan, single = got.info, all(int(c) == 1 for c in q_lens)
+        return StepTables(arrays, LatentInfo(plan, single, runs, rows, int(segments[:, 2].max())))
 
     def children(self):
         return (self.position,) if self.position is not None else ()
@@ -134,6 +206,47 @@ class LatentAttention(Part):
             self._wide = True
             self._tables_key = ("latent_attention_items", self.window or 0, self.H, self.r + self.dr)
             self._sm_count = torch.cuda.get_device_properties(precision.device).multi_processor_count
+            if self._made_takes() and (not self.gate or self.gate_per_head or self.w_in.shape[0] % 4 == 0):
+                self._tables_key += (self.dn, self.dr, self.vd)
+                self._w_ukv = torch.cat([tensors[p + nm["uk"]].to(dt).view(H, self.dn, self.r), self.w_uv], dim=1) \
+                    .reshape(H * (self.dn + self.vd), self.r).contiguous()
+
+    def _forward_made(self, q, proj, at: int, xb, ctx, cache, rotation, write_cache: bool, gate, att) -> None:
+        """The attention of a step in which some requests (or all) have their keys and values made: rows of `att`."""
+        from ..csrc import attention_fast
+        arrays, info = ctx.tables[self._tables_key]
+        n, dev, dt = xb.shape[0], xb.device, xb.dtype
+        H, dn, dr, r, vd = self.H, self.dn, self.dr, self.r, self.vd
+        packed = torch.empty((n, H * (dn + dr)), dtype=dt, device=dev)
+        q_full = torch.empty((n, H * (r + dr)), dtype=dt, device=dev) if info.plan is not None else None
+        plain = {}
+        for a, b, made in info.runs:
+            if not made:
+                plain[a] = torch.empty((b - a, H * dn), dtype=dt, device=dev)
+            ops.latent_prep(q[a:b], proj[a:b, at:at + r + dr], plain.get(a), None if made else q_full[a:b], self.c_norm, self.norm_eps,
+                            *rotation, ctx.positions[a:b], ctx.slot_of_token[a:b], cache.block_table, cache.k_pages, H, dn, dr, r,
+                            cache.page_tokens, write_kv=write_cache, q_packed=packed[a:b] if made else None)
+        c = torch.empty((info.rows, r), dtype=dt, device=dev)
+        rope = torch.empty((info.rows, dr), dtype=dt, device=dev) if dr else None
+        ops.latent_rows(cache.k_pages, cache.block_table, arrays["made_segments"], info.most_rows, c, rope)
+        kv = torch.empty((info.rows, H * (dn + vd)), dtype=dt, device=dev)
+        ops.gemm_narrow(c, self._w_ukv, kv)
+        attention_fast.run_made(packed, kv, rope, arrays["made_items"], att, H, self.window or 0, self.scale, c, self.w_uv,
+                                arrays["made_firsts"], gate, self.gate_per_head, self.out_scale)
+        if info.plan is None:
+            return
+        for a, b, made in info.runs:
+            if not made:
+                ops.gemm_heads(plain[a].view(b - a, H, dn), self.w_uk_t, q_full[a:b].view(b - a, H, r + dr)[:, :, :r], H)
+        lat = torch.empty((n, H * r), dtype=dt, device=dev)
+        plan = attention_fast.plan_on_device(info.plan, arrays["items"], arrays.get("merge"))
+        if not attention_fast.run_latent(q_full, cache.k_pages, cache.block_table, lat, H, r + dr, r, cache.page_tokens, self.window or 0,
+                                         self.scale, plan, single_tokens=info.single_tokens):
+            raise ops.KernelError("latent attention: the kernel refuses a step that its plan was made for")
+        for a, b, made in info.runs:
+            if not made:
+                ops.gemm_heads(lat[a:b].view(b - a, H, r), self.w_uv, att[a:b].view(b - a, H, vd), H, gate=gate[a:b] if gate is not None else None,
+                               gate_scale=self.out_scale, gate_per_head=self.gate_per_head)
 
     def _attend(self, q_full: torch.Tensor, ctx, cache) -> torch.Tensor:
         """The attention over the cache rows: a view [n, H, kv_rank] of the heads' latent sums.  In bfloat16 a tensor-core
@@ -176,21 +289,27 @@ class LatentAttention(Part):
             ops.rms_norm(proj[:, :at], self.q_norm, self.norm_eps, c_q)
             q = torch.empty((n, H * (dn + dr)), dtype=torch.float32, device=dev)
             ops.gemm(c_q, self.w_uq, q)
-        q_plain = torch.empty((n, H * dn), dtype=dt, device=dev)
-        q_full = torch.empty((n, H * (r + dr)), dtype=dt, device=dev)
         cos = sin = None
         rot, pairing = 0, "half"
         if self.position is not None:
             cos, sin, rot = self.position.tables()
             pairing = self.position.pairing
+        # the output gate's logits, which the last step of either way applies
+        gate = proj[:, at + r + dr:at + r + dr + (H if self.gate_per_head else H * vd)] if self.gate else None
+        att = torch.empty((n, H * vd), dtype=dt, device=dev)
+        if self._w_ukv is not None and dt == torch.bfloat16 and ops.forced("attention") != "generic" \
+                and isinstance(ctx.tables.get(self._tables_key, (None, None))[1], LatentInfo):
+            self._forward_made(q, proj, at, xb, ctx, cache, (cos, sin, rot, pairing), write_cache, gate, att)
+            ops.gemm(att, self.w_o, residual, accumulate=accumulate)
+            return
+        q_plain = torch.empty((n, H * dn), dtype=dt, device=dev)
+        q_full = torch.empty((n, H * (r + dr)), dtype=dt, device=dev)
         ops.latent_prep(q, proj[:, at:at + r + dr], q_plain, q_full, self.c_norm, self.norm_eps, cos, sin, rot, pairing, ctx.positions,
                         ctx.slot_of_token, cache.block_table, cache.k_pages, H, dn, dr, r, cache.page_tokens,
                         write_kv=write_cache)
         ops.gemm_heads(q_plain.view(n, H, dn), self.w_uk_t, q_full.view(n, H, r + dr)[:, :, :r], H)
         lat = self._attend(q_full, ctx, cache)                  # [n, H, r]: sum_j p_j c_j per head
-        att = torch.empty((n, H * vd), dtype=dt, device=dev)
         # the values' up-projection per head, with the output gate in its epilogue
-        gate = proj[:, at + r + dr:at + r + dr + (H if self.gate_per_head else H * vd)] if self.gate else None
         ops.gemm_heads(lat, self.w_uv, att.view(n, H, vd), H, gate=gate, gate_scale=self.out_scale, gate_per_head=self.gate_per_head)
         ops.gemm(att, self.w_o, residual, accumulate=accumulate)
 
