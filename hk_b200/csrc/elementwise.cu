@@ -456,6 +456,100 @@ qk_norm_rope_kv_write_vec_kernel(
   }
 }
 
+// The same for heads of 128 dims that turn whole with dim i paired with i + 64: sixteen lanes hold a head, four dims of its
+// first half and the four that they are paired with each, so a rotation needs no exchange and a sum four of them for two heads.
+// A CTA takes a token (or, where the tokens are few, a third of one), a warp two heads at a time; the token's position, page,
+// angles and the norms' weights are read once.  Between its bytes and its instructions:
+// 48 heads by 2,048 tokens 48 -> 32 us (2.4 TB/s), by 8,192 147 -> 87 (3.5 TB/s), by 527 24 -> 15, by 64 19 -> 14 (L2 cold; the
+// kernel above, which other sizes take, is bound by 180 instructions a warp and head).  Three CTAs a token below two a SM.
+#define QKH_WARPS 8
+template <typename T>
+__global__ void __launch_bounds__(QKH_WARPS * 32)
+qk_norm_rope_kv_write_halves_kernel(const float* __restrict__ qkv, T* __restrict__ q_out, const float* __restrict__ q_w,
+                                    const float* __restrict__ k_w, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                    const int* __restrict__ positions, const int* __restrict__ slot_of_token,
+                                    const int* __restrict__ block_table, int table_stride, T* __restrict__ k_pages, T* __restrict__ v_pages,
+                                    int H, int G, int page_tokens, int write_kv, const float* __restrict__ bias, int norm_after, long long ld,
+                                    QueryFactor qt) {
+  constexpr int HD = 128;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d0 = (lane & 15) * 4;
+  const int heads = H + (write_kv ? 2 * G : 0), step = 2 * QKH_WARPS * gridDim.y;
+  const float* src = qkv + (size_t)t * (size_t)ld + d0;
+  const int pos = positions[t];
+  const float4 c = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * (HD / 2) + d0);
+  const float4 sn = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * (HD / 2) + d0);
+  int page = -1;
+  if (write_kv) page = block_table[(size_t)slot_of_token[t] * table_stride + pos / page_tokens];
+  const size_t place = ((size_t)max(page, 0) * G * page_tokens + pos % page_tokens) * HD + d0;      // of key head 0
+  const float one = 1.0f, factor = qt.every > 0 ? query_factor(qt, pos) : one;
+  auto normed = [&](float4& a, float4& b, const float* w) {
+    float ss = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, a.w * a.w)));
+    ss += fmaf(b.x, b.x, fmaf(b.y, b.y, fmaf(b.z, b.z, b.w * b.w)));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float inv = 1.0f / sqrtf(ss / (float)HD + eps);
+    const float4 g = w ? *reinterpret_cast<const float4*>(w + d0) : make_float4(1.f, 1.f, 1.f, 1.f);
+    const float4 h = w ? *reinterpret_cast<const float4*>(w + d0 + HD / 2) : make_float4(1.f, 1.f, 1.f, 1.f);
+    a = make_float4(a.x * inv * g.x, a.y * inv * g.y, a.z * inv * g.z, a.w * inv * g.w);
+    b = make_float4(b.x * inv * h.x, b.y * inv * h.y, b.z * inv * h.z, b.w * inv * h.w);
+  };
+  auto store = [](T* dst, const float4& v) {
+    if (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(dst)) = v;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  };
+  const int first = 2 * (warp + QKH_WARPS * blockIdx.y) + (lane >> 4);
+#pragma unroll 3
+  for (int hh = first; hh - (lane >> 4) < heads; hh += step) {        // a whole warp or none: its sums meet by shuffle
+    const bool in = hh < heads;
+    const float* p = src + (size_t)(in ? hh : 0) * HD;
+    float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + HD / 2);
+    if (bias) {
+      const float4 x = *reinterpret_cast<const float4*>(bias + (size_t)(in ? hh : 0) * HD + d0);
+      const float4 y = *reinterpret_cast<const float4*>(bias + (size_t)(in ? hh : 0) * HD + d0 + HD / 2);
+      a = make_float4(a.x + x.x, a.y + x.y, a.z + x.z, a.w + x.w);
+      b = make_float4(b.x + y.x, b.y + y.y, b.z + y.z, b.w + y.w);
+    }
+    const bool value = hh >= H + G;
+    const float* w = hh < H ? q_w : k_w;
+    if (!norm_after && (q_w || k_w)) {
+      float4 x = a, y = b;
+      normed(x, y, w);
+      if (w && !value) a = x, b = y;
+    }
+    if (!value) {
+      // x' = a c - b s, y' = a s + b c
+      const float4 x = a, y = b;
+      a = make_float4(x.x * c.x - y.x * sn.x, x.y * c.y - y.y * sn.y, x.z * c.z - y.z * sn.z, x.w * c.w - y.w * sn.w);
+      b = make_float4(x.x * sn.x + y.x * c.x, x.y * sn.y + y.y * c.y, x.z * sn.z + y.z * c.z, x.w * sn.w + y.w * c.w);
+    }
+    if (norm_after) {
+      float4 x = a, y = b;
+      normed(x, y, w);
+      if (!value) a = x, b = y;
+    }
+    if (!in) continue;
+    T* dst;
+    if (hh < H) {
+      if (qt.every > 0) {
+        a = make_float4(a.x * factor, a.y * factor, a.z * factor, a.w * factor);
+        b = make_float4(b.x * factor, b.y * factor, b.z * factor, b.w * factor);
+      }
+      dst = q_out + ((size_t)t * H + hh) * HD + d0;
+    } else {
+      if (page < 0) continue;                          // the host never schedules this
+      dst = (value ? v_pages : k_pages) + place + (size_t)(value ? hh - H - G : hh - H) * page_tokens * HD;
+    }
+    store(dst, a);
+    store(dst + HD / 2, b);
+  }
+}
+
 HK_API int hk_qk_norm_rope_kv_write(const float* qkv, void* q_out, int dtype, const float* q_w,
                                     const float* k_w, float eps, const float* cos_t, const float* sin_t,
                                     int rot, const int* positions, const int* slot_of_token,
@@ -473,6 +567,18 @@ HK_API int hk_qk_norm_rope_kv_write(const float* qkv, void* q_out, int dtype, co
   long long items = (long long)n * (H + (write_kv ? (tied_v ? G : 2 * G) : 0));
   const bool aligned = ((((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)q_w |
                           (uintptr_t)k_w | (uintptr_t)cos_t | (uintptr_t)sin_t | (uintptr_t)bias) & 15) == 0);
+  if (hd == 128 && vd == 128 && rot == 128 && pairing == 0 && !tied_v && (ld & 3) == 0 && aligned) {
+    const dim3 grid((unsigned)n, n < 2 * 148 ? 3u : 1u), block(QKH_WARPS * 32);
+    if (dtype == HK_F32)
+      return hk_launch_pdl(qk_norm_rope_kv_write_halves_kernel<float>, grid, block, 0, s, qkv, (float*)q_out, q_w, k_w, eps, cos_t, sin_t,
+                           positions, slot_of_token, block_table, table_stride, (float*)k_pages, (float*)v_pages, H, G, page_tokens,
+                           write_kv, bias, norm_after, ld, qt);
+    if (dtype == HK_BF16)
+      return hk_launch_pdl(qk_norm_rope_kv_write_halves_kernel<bf16>, grid, block, 0, s, qkv, (bf16*)q_out, q_w, k_w, eps, cos_t, sin_t,
+                           positions, slot_of_token, block_table, table_stride, (bf16*)k_pages, (bf16*)v_pages, H, G, page_tokens,
+                           write_kv, bias, norm_after, ld, qt);
+    return HK_ERR_UNSUPPORTED;
+  }
   if (hd <= 128 && vd <= 128 && (hd & 3) == 0 && (vd & 3) == 0 && (rot & 7) == 0 && (ld & 3) == 0 && aligned) {
     unsigned vblocks = (unsigned)((items + QKV_WARPS - 1) / QKV_WARPS);
     if (dtype == HK_F32)

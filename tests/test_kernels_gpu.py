@@ -210,6 +210,33 @@ def test_qk_norm_rope_kv_write_many_tokens(dtype, H, G, hd, pt, rot, norm, ntok)
 
 
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
+@pytest.mark.parametrize("H,G,ntok,norms", [(3, 1, 1, "qk"), (1, 1, 295, "q"), (3, 1, 297, "k"), (40, 8, 33, ""), (7, 7, 296, "qk")])
+def test_qk_norm_rope_kv_write_two_heads_a_warp(dtype, H, G, ntok, norms):
+    # heads of 128 that turn whole: odd numbers of heads, as many as take a warp several turns, tokens on both sides of where a
+    # token gets one CTA instead of three, a norm on one side only
+    rng = np.random.default_rng(H * 7 + ntok)
+    k_pages, v_pages, bt, _, _ = make_paged(rng, 1, [ntok + 3], G, 128, 16, dtype)
+    k_pages.zero_()
+    v_pages.zero_()
+    slot, pos = torch.zeros(ntok, dtype=torch.int32), torch.arange(3, ntok + 3, dtype=torch.int32)
+    qkv = torch.from_numpy(rng.standard_normal((ntok, (H + 2 * G) * 128))).float() * 2
+    qw, kw = ((1 + 0.2 * torch.from_numpy(rng.standard_normal(128))).float() if c in norms else None for c in "qk")
+    ang = torch.arange(ntok + 3, dtype=torch.float64)[:, None] * torch.from_numpy(rng.uniform(0.001, 1.0, 64))[None, :]
+    cos, sin = torch.cos(ang).float(), torch.sin(ang).float()
+    q_out = torch.empty(ntok, H * 128, dtype=dtype, device=DEV)
+    kp, vp = k_pages.to(DEV), v_pages.to(DEV)
+    d = lambda t: None if t is None else t.to(DEV)
+    ops().qk_norm_rope_kv_write(qkv.to(DEV), q_out, d(qw), d(kw), 1e-6, d(cos), d(sin), 128, pos.to(DEV), slot.to(DEV), bt.to(DEV), kp, vp,
+                                H, G, 128, 16)
+    q, k, v = ref_ops.qk_norm_rope(qkv, qw, kw, 1e-6, cos, sin, 128, pos, H, G, 128)
+    close(q_out, q.reshape(ntok, H * 128), dtype)
+    rk, rv = torch.zeros_like(k_pages, dtype=torch.float64), torch.zeros_like(v_pages, dtype=torch.float64)
+    ref_ops.write_pages(k, v, rk, rv, bt, slot, pos, 16)
+    close(kp, rk, dtype)
+    close(vp, rv, dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
 @pytest.mark.parametrize("H,G,hd,pt,rot", [(4, 2, 16, 4, 16), (5, 1, 48, 16, 24), (8, 8, 128, 16, 128), (3, 1, 40, 8, 24), (2, 1, 24, 4, 22),
                                             (4, 2, 160, 16, 160), (6, 2, 64, 16, 32)])
 @pytest.mark.parametrize("pairing,with_bias", [("adjacent", False), ("adjacent", True), ("half", True)])
