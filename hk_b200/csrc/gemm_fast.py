@@ -13,6 +13,7 @@ Shapes all of them refuse (K not a multiple of 8, unaligned operands) go to the 
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -54,7 +55,8 @@ def _ptr(t):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    from .ops import _stream as current
+    return current()
 
 
 def _aligned(a, w) -> bool:
@@ -75,17 +77,44 @@ _tc_splits = 0        # ... and the number of K slices of the tcgen05 kernel
 TC_TILE_FIXED = 150   # a tile's fixed cost in columns: tiles of 128 measured 30-45 % slower per flop than tiles of 256
 
 
+@functools.lru_cache(maxsize=4096)
+def _tc_ragged_config(M: int, N: int, K: int, sms: int, swiglu: bool):
+    """Tile width and K slices for two or more row tiles, by a model of the time in us that was fitted to 900 measured
+    (shape, width, slices), 130 to 1,500 rows by the products of layers 2,048 and 4,096 wide (relative error 9 %): what it picks
+    is 1.4 % slower than the best on average, "256 wide, or 128 wide with slices where the tiles do not fill the SMs" was 8 %.
+    At 527 rows: 4,096 x 12,288 92 us with tiles of 256 (80 tiles on 148 SMs), 74 with 144 (145 tiles); 4,096 x 4,096 43 and
+    36; at 300 rows 72 (128 wide) and 54 (256 wide, three slices)."""
+    m_tiles, step = -(-M // 128), 32 if swiglu else 16
+    k_blocks = -(-K // 64)
+    best = None
+    for bn in range(256, 63, -step):
+        tiles = m_tiles * -(-N // bn)
+        for splits in (1, 2, 3, 4, 6, 8):
+            if splits > 1 and (tiles * splits > sms or k_blocks < 8 * splits or (swiglu and (N // 2) % (bn // 2))):
+                break
+            waves = -(-tiles * splits // sms)
+            cost = waves * (k_blocks / splits * (0.198 + 0.000521 * bn) + 0.013 * bn)
+            if splits > 1:
+                cost += 1.5 + M * N * splits * 1.46e-6        # partial sums written and read, and the launch that adds them
+            if best is None or cost < best[0]:
+                best = (cost, bn, splits)
+    return best[1:]
+
+
 def tc_config(M: int, N: int, K: int, sms: int, swiglu: bool = False):
     """Tile width (a multiple of 16, of 32 with the SwiGLU epilogue) and number of K slices for the tcgen05 kernel.
-    Many rows (prefill): the width, from 256 down to 192, whose tiles leave the least of the last wave of SMs
-    empty, a tile costing its width plus a fixed part.  Few output tiles (decode batches, narrow outputs):
-    with the SwiGLU epilogue the widest tile that gives every SM one (no slices: the epilogue cannot run on partial
-    sums without a second kernel); else 128- or 256-wide tiles with K cut into slices so that every SM streams a
-    share of the weights.  (A finer cost model that also weighed wave tails chose more slices and measured slower:
+    Very many tiles (prefill): the width, from 256 down to 192, whose tiles leave the least of the last wave of SMs
+    empty, a tile costing its width plus a fixed part.  Several row tiles but few waves: `_tc_ragged_config`.  One row tile
+    (decode batches): with the SwiGLU epilogue the widest tile that gives every SM one (no slices: the epilogue cannot run on
+    partial sums without a second kernel); else 128- or 256-wide tiles with K cut into slices so that every SM streams a
+    share of the weights.  (A finer cost model that also weighed wave tails chose more slices there and measured slower:
     the second kernel that adds the slices has a fixed cost.)"""
     m_tiles = -(-M // 128)
     step = 32 if swiglu else 16
     k_blocks = -(-K // 64)
+    if not _tc_bn and m_tiles > 1 and m_tiles * -(-N // 256) < 8 * sms:
+        bn, splits = _tc_ragged_config(M, N, K, sms, swiglu)
+        return bn, min(_tc_splits, k_blocks) if _tc_splits else splits
     if _tc_bn:
         bn = _tc_bn
     elif m_tiles * -(-N // 256) >= sms:

@@ -11,3 +11,18 @@ def test_tile_widths_the_tcgen05_product_chooses():
     assert splits == 1 and bn % 32 == 0 and 120 <= -(-24576 // bn) <= 148
     bn, splits = cfg(64, 4096, 12288, 148)
     assert bn in (128, 256) and splits > 1                               # narrow output: K slices
+
+
+def test_tile_widths_of_a_few_hundred_rows():
+    """Several row tiles, few waves: every choice is one that the kernel takes, and none leaves half of the SMs idle."""
+    from hk_b200.csrc import gemm_fast
+    for m in (129, 200, 257, 384, 527, 1000):
+        for n, k in ((4096, 4096), (4096, 12288), (6144, 4096), (2056, 2048), (72, 512), (10304, 2048)):
+            bn, splits = gemm_fast.tc_config(m, n, k, 148)
+            assert bn % 16 == 0 and 64 <= bn <= 256 and 1 <= splits <= -(-k // 64)
+            tiles = -(-m // 128) * -(-n // bn) * splits
+            assert n < 4000 or tiles > 74
+        for n, k in ((24576, 4096), (12288, 2048), (1056, 256)):
+            bn, splits = gemm_fast.tc_config(m, n, k, 148, swiglu=True)
+            assert bn % 32 == 0 and (splits == 1 or (n // 2) % (bn // 2) == 0)
+    assert gemm_fast.tc_config(527, 4096, 12288, 148) == (144, 1)       # 145 tiles in one wave
