@@ -224,7 +224,7 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
     gate_args = (_ptr(gate if fused_gate else None), ctypes.c_longlong(gate.stride(0) if fused_gate else 0), ctypes.c_float(gate_scale))
     done = GATED if fused_gate else True
     lib = build.load("attention_flash")
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = ops._stream()
     rows = 16 * plan.nw
     part_o = part_ml = None
     if plan.n_parts:
@@ -296,7 +296,7 @@ def run_latent(q, pages, block_table, out, H: int, dk: int, dv: int, page_tokens
     if not latent_supported(H, dk, dv) or plan is None:
         return False
     lib = build.load("attention_latent")
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = ops._stream()
     part_o = part_ml = None
     if plan.n_parts:
         part_o = torch.empty((plan.n_parts, LATENT_ROWS, dv), dtype=torch.float32, device=q.device)
@@ -351,7 +351,7 @@ def run_made(q, kv, rope, items, out, H: int, window: int, scale: float, c, w_uv
     per head 128 key dims and 128 value dims, and rope bf16 [rows, 64], the key dims that all heads share (or None).  c bf16
     [rows, r] and w_uv bf16 [H, 128, r]: what the values were made of, for the rows of `firsts`."""
     from . import gemm_fast, ops
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = ops._stream()
     gated = (_ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), 1 if gate_per_head else 0, ctypes.c_float(gate_scale))
     scale_log2 = ctypes.c_float(scale * math.log2(math.e))
     lib = build.load("attention_prefill_tc")

@@ -38,7 +38,8 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream, as its handle (an object around it would cost two microseconds a launch)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, dims: Optional[int] = None) -> None:
