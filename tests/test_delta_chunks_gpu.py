@@ -130,3 +130,30 @@ def test_chunks_refuse_what_they_cannot_do():
         ops.delta_rule_scan(z[:, :64], z[:, 64:128], z[:, 128:192], z[:, 192:], z[:, :64], z[0, :64], z[0, :64], short,
                             torch.zeros(1, 1, 64, 64, device=DEV), torch.zeros(64, 64, device=DEV), 1, 64, 64, 2.0, 1e-6, chunks=chunks,
                             requests=requests)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,dv,act,weight,memory", [(3, 4, "silu", "shared", False), (5, 32, "sigmoid", "all", False), (2, 36, "silu", None, False),
+                                                    (7, 64, "sigmoid", "all", True), (3, 68, "silu", "shared", False), (1, 128, "sigmoid", "all", True)])
+def test_head_out_gate_of_whole_pieces(dtype, H, dv, act, weight, memory):
+    """A head's norm and gate with 8, 16 and 32 lanes a head, heads that leave lanes idle, items that leave a block unfilled."""
+    from hk_b200.csrc import ops
+    g = torch.Generator(DEV).manual_seed(dv * 10 + H)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)       # noqa: E731
+    n, ldo = 37, ops.mlstm_padded(dv) if memory else dv
+    o, logits = rand(n, H * ldo), rand(n, H * dv + 8)[:, 4:4 + H * dv]
+    w = None if weight is None else rand(dv if weight == "shared" else H * dv)
+    gates = rand(n, H, 3).abs() if memory else None
+    out = torch.empty(n, H * dv, dtype=dtype, device=DEV)
+    ops.head_out_gate(o, logits, w, 1e-5, out, H, dv, act=act, gates=gates, den_eps=1e-6)
+    x = o.double().view(n, H, ldo)
+    if memory:
+        x = x / (torch.maximum(x[..., dv:dv + 1].abs(), gates[..., 2:].double()) + 1e-6)
+    x = x[..., :dv]
+    y = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5)
+    if w is not None:
+        y = y * w.double().view(-1, dv)
+    z = logits.double().view(n, H, dv)
+    want = (y * torch.sigmoid(z) * (z if act == "silu" else 1.0)).flatten(1)
+    rel = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5              # half a unit of the storage type; float32 rounding
+    assert bool(((out.double() - want).abs() <= rel * want.abs() + 1e-6).all())
