@@ -13,6 +13,7 @@ import contextlib
 import ctypes
 from typing import Optional
 
+import numpy as np
 import torch
 
 from . import build
@@ -512,9 +513,24 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool =
 # ---- attention ------------------------------------------------------------------------
 
 
+RUN_ROWS = 32       # (token, head of the group) rows of a run of the float32 kernel
+
+
+def float32_runs(slots, q_starts, q_lens, start_positions, group: int):
+    """The step's rows as runs of at most RUN_ROWS / group tokens of a request, int32 [m, 4] = (first row, tokens, slot, position
+    of the first), those with the most keys first; None for groups that the kernel does not take."""
+    if group > RUN_ROWS:
+        return None
+    per = RUN_ROWS // group
+    runs = [(qs + b, min(per, ql - b), slot, p0 + b) for slot, qs, ql, p0 in zip(slots, q_starts, q_lens, start_positions)
+            for b in range(0, ql, per)]
+    runs.sort(key=lambda r: -r[3])
+    return np.asarray(runs, dtype=np.int32)
+
+
 def paged_attention(q, k_pages, v_pages, block_table, positions, slot_of_token, out, n_heads, n_kv_heads,
                     head_dim, page_tokens, window: int, scale: float, plan=None, sink: bool = False, sinks=None,
-                    softcap: float = 0.0, chunk: int = 0, gate=None, gate_scale: float = 1.0, dist=None, dist_log2=None) -> None:
+                    softcap: float = 0.0, chunk: int = 0, gate=None, gate_scale: float = 1.0, dist=None, dist_log2=None, runs=None) -> None:
     """out[t, h, :] = softmax_j(scale * q[t, h] . k[j]) v[j] over the keys j in
     [max(0, p - window + 1), p] (all of [0, p] when window <= 0) of the token's request, read
     through its block-table row; p = positions[t].  `plan` carries the per-request tiling the
@@ -526,7 +542,8 @@ def paged_attention(q, k_pages, v_pages, block_table, positions, slot_of_token, 
     `softcap` c > 0: scores become c * tanh(score / c).  `chunk` s > 0: a token sees no key before the start of its own
     block of s positions.  `gate` (a float32 column slice [n, H*vd] of a projection's output): the result is
     multiplied by gate_scale * sigmoid(gate).  `dist` float32 [H, N]: dist[h, min(n, N - 1)] is added to the (scaled, capped)
-    score of a key n positions back; `dist_log2`: the same table times log2(e), which the flash kernels read."""
+    score of a key n positions back; `dist_log2`: the same table times log2(e), which the flash kernels read.  `runs` (float32
+    only) int32 [m, 4]: the step's rows as runs of a request's tokens (`float32_runs`), which a kernel of its own takes."""
     _need(q, "q", dims=2)
     _need(out, "out", q.dtype, 2)
     _need(k_pages, "k_pages", q.dtype, 4)
@@ -575,6 +592,16 @@ def paged_attention(q, k_pages, v_pages, block_table, positions, slot_of_token, 
         if choice is not None:
             raise KernelError(f"paged_attention: the '{choice}' kernel refuses head_dim={hd} page_tokens={page_tokens}")
     lib = build.load("attention_generic")
+    if runs is not None and q.dtype == torch.float32 and choice != "generic":
+        _need(runs, "runs", torch.int32, 2)
+        code = lib.hk_attention_f32(
+            _ptr(q), _ptr(k_pages), _ptr(v_pages if v_pages is not None else k_pages), _ptr(block_table), int(block_table.shape[1]), _ptr(runs),
+            int(runs.shape[0]), _ptr(out), H, G, hd, int(page_tokens), int(window), ctypes.c_float(scale), vd, 1 if sink else 0, _ptr(sinks),
+            ctypes.c_float(softcap), int(chunk), vd if v_pages is not None else hd, _ptr(gate), ctypes.c_longlong(gate_ld),
+            ctypes.c_float(gate_scale), _ptr(dist), int(dist.shape[1]) if dist is not None else 0, _stream())
+        if code != _ERR_UNSUPPORTED:
+            _check(code, "paged_attention (float32 runs)")
+            return
     _check(lib.hk_attention_generic(
         _ptr(q), _ptr(k_pages), _ptr(v_pages if v_pages is not None else k_pages), _dt(q), _ptr(block_table),
         int(block_table.shape[1]), _ptr(positions), _ptr(slot_of_token), _ptr(out), n, H, G, hd, int(page_tokens), int(window),

@@ -286,6 +286,8 @@ class GQAAttention(Part):
         if precision.compute == torch.bfloat16 and self._flash_takes():
             self._tables_key = ("paged_attention_items", self.window or 0, self.H, self.G, self.hd, self.sink, self.chunk, bool(self.softcap))
             self._sm_count = torch.cuda.get_device_properties(precision.device).multi_processor_count
+        elif precision.compute == torch.float32:
+            self._tables_key = ("float32_attention_runs", self.H // self.G)
 
     # -- the step's work items (host-built; see parts.base) --------------------------------
     def step_tables_key(self):
@@ -293,7 +295,11 @@ class GQAAttention(Part):
 
     def step_tables(self, ctx):
         """Cuts the batch into the flash kernels' work items (csrc/attention_fast.py).  In a step whose shape must
-        not change (a captured decode graph) every request's keys go to the same number of splits."""
+        not change (a captured decode graph) every request's keys go to the same number of splits.  In 32-bit: the runs of the
+        float32 kernel."""
+        if self._tables_key[0] == "float32_attention_runs":
+            runs = ops.float32_runs(ctx.slots, ctx.q_starts, ctx.q_lens, ctx.start_positions, self.H // self.G)
+            return StepTables({} if runs is None else {"runs": runs})
         return flash_step_tables(ctx, self.H, self.G, self.hd, self.window or 0, self.chunk, self._sm_count)
 
     def _plan(self, ctx):
@@ -317,6 +323,7 @@ class GQAAttention(Part):
         n = xb.shape[0]
         H, G, hd = self.H, self.G, self.hd
         plan = self._plan(ctx) if xb.dtype == torch.bfloat16 else None
+        runs = ctx.tables.get(self._tables_key, ({}, None))[0].get("runs") if xb.dtype == torch.float32 else None
         if proj is None:
             proj = torch.empty((n, self.w_qkv.shape[0]), dtype=torch.float32, device=xb.device)
             ops.gemm(xb, self.w_qkv, proj)
@@ -345,7 +352,7 @@ class GQAAttention(Part):
         ops.paged_attention(q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.slot_of_token,
                             att, H, G, hd, cache.page_tokens, self.window or 0, self.scale,
                             plan=plan, sink=self.sink, sinks=self.sinks, softcap=self.softcap, chunk=self.chunk, gate=gate,
-                            gate_scale=self.out_scale, dist=self.dist, dist_log2=self.dist_log2)
+                            gate_scale=self.out_scale, dist=self.dist, dist_log2=self.dist_log2, runs=runs)
         ops.gemm(att, self.w_o, residual, accumulate=accumulate, bias=self.b_o if add_bias else None)
 
 
