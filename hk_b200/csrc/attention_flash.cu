@@ -551,9 +551,17 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_p
 // CTAs per SM keep about 128 KB in flight per SM.  Boxes outside the item's key range are not requested; what
 // the stage then holds is masked (K) or finite and multiplied by zero (V: the stages are zeroed once at the
 // start).  Every wait is bounded; on time-out the CTA sets `status`, writes nothing and leaves.
-constexpr int TW = 4;             // consumer warps (a fifth warp produces)
-constexpr int TT = 64;            // keys per tile
+//
+// TW, the consumer warps, is 4 (tiles of 64 keys, two CTAs an SM at a head of 128) or 2 (tiles of 32 keys, half the
+// shared memory, four CTAs an SM with the same bytes in flight between them).  The kernel is bound by the HBM, and CTAs
+// that run together share it evenly; what is lost is the last wave, whose few CTAs do not have enough on their way to
+// fill it.  A batch that is more than one wave of wide CTAs and at most one of narrow ones therefore loses nothing as
+// narrow ones; `narrow_pays` has the rule.  Microseconds at 2,048 keys, 32 / 8 heads of 128, wide and narrow: 48 requests
+// 91 and 74, 64: 98 and 93, 80: 138 and 156 (stays wide), 128: 189 and 172; 64 requests
+// of 300 keys: 35 and 27; heads of 64: 64 requests 69 and 55, 80: 74 and 64, 170: 135 and 121.
 constexpr int TS = 3;             // stages
+// CTAs an SM holds at once, by registers (about 160 a thread at a head of 128, 120 at 64) and shared memory
+constexpr int decode_tma_slots(int hd, int tw) { return (tw == 4 ? 2 : 4) + (hd == 64 ? 1 : 0); }
 constexpr uint32_t T_WAIT_LIMIT = 1u << 22;
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -590,8 +598,8 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
 }
 
 // DIST: with a bias by distance (an instance of its own, so that the steps of a model without one issues nothing for it)
-template <int HD, bool DIST>
-__global__ void __launch_bounds__((TW + 1) * 32, 2)
+template <int HD, bool DIST, int TW>
+__global__ void __launch_bounds__((TW + 1) * 32, decode_tma_slots(HD, TW))
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                             const bf16* __restrict__ q, const int* __restrict__ block_table, int table_stride,
                             const Item* __restrict__ items, bf16* __restrict__ out, float* __restrict__ part_o,
@@ -599,6 +607,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                             float scale_log2, ScoreOpts so, int pages_cap, int* __restrict__ status) {
   constexpr int ROWS = 16;
   constexpr int KSTEPS = HD / 16;
+  constexpr int TT = TW * 16;                        // keys per tile
   constexpr int TILE_BYTES = TT * HD * 2;            // K (or V) of one stage
   extern __shared__ uint8_t smem_dyn[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -1022,16 +1031,47 @@ bool make_page_map(CUtensorMap* map, const void* ptr, unsigned long long rows, i
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int HD, bool DIST>
+int sm_count() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return n;
+}
+
+template <int HD>
+size_t decode_tma_smem(int tile, int pages_cap) {
+  return 1024 + (size_t)2 * TS * tile * HD * 2 + 2 * TS * sizeof(uint64_t) + 8 + (size_t)pages_cap * sizeof(int);
+}
+
+// Which width `ctas` CTAs of about equal length take less time in.  The unit is the time in which the HBM delivers one
+// CTA's keys: a full wave of c CTAs takes c, a thinner one no less than `least` (what one CTA has on its way bounds its
+// own rate), and a wave's start and end about S / 8 of S SMs.  `least` is fitted over batches of 48 to 256 requests at
+// heads of 128 and 64: 4/3 S wide and 2 S narrow, twice that at a head of 64, where a CTA's bytes on their way are half;
+// with it the model is within 5 % of every measured time.
+bool narrow_pays(long long ctas, int hd, int pages_cap) {
+  const long long S = sm_count(), scale = 128 / hd;
+  const size_t smem = hd == 64 ? decode_tma_smem<64>(32, pages_cap) : decode_tma_smem<128>(32, pages_cap);
+  if (decode_tma_slots(hd, 2) * (smem + 1024) > 228 * 1024) return false;    // a long page list: fewer fit than the rule counts on
+  auto cost = [&](long long slots, long long least) {
+    const long long full = ctas / slots, rest = ctas % slots, ends = S / 8 * scale;
+    return full * (slots + ends) + (rest ? (rest > least ? rest : least) + ends : 0);
+  };
+  return cost(S * decode_tma_slots(hd, 2), 2 * S * scale) < cost(S * decode_tma_slots(hd, 4), 4 * S * scale / 3);
+}
+
+template <int HD, bool DIST, int TW>
 int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, const int* bt, int stride, const void* items,
                       int n_items, void* out, float* part_o, float* part_ml, int H, int G, int pt, int box_rows, int window,
                       float scale_log2, ScoreOpts so, int pages_cap, int* status, cudaStream_t s) {
-  const size_t smem = 1024 + (size_t)2 * TS * TT * HD * 2 + 2 * TS * sizeof(uint64_t) + 8 + (size_t)pages_cap * sizeof(int);
+  const size_t smem = decode_tma_smem<HD>(TW * 16, pages_cap);
   if (smem > 110 * 1024) return HK_ERR_UNSUPPORTED;
   static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_decode_tma_kernel<HD, DIST>, smem, allowed)) return e;
+  if (int e = hk_allow_smem(attention_decode_tma_kernel<HD, DIST, TW>, smem, allowed)) return e;
   dim3 grid((unsigned)n_items, (unsigned)G);
-  return hk_launch_pdl(attention_decode_tma_kernel<HD, DIST>, grid, dim3((TW + 1) * 32), smem, s, mk, mv, (const bf16*)q, bt, stride,
+  return hk_launch_pdl(attention_decode_tma_kernel<HD, DIST, TW>, grid, dim3((TW + 1) * 32), smem, s, mk, mv, (const bf16*)q, bt, stride,
                        (const Item*)items, (bf16*)out, part_o, part_ml, H, G, pt, box_rows, window, scale_log2, so, pages_cap, status);
 }
 
@@ -1050,16 +1090,22 @@ HK_API int hk_attention_decode_tma(const void* q, const void* k_pages, const voi
   if (G < 1 || H % G != 0 || (H / G) > 16 || G > 65535) return HK_ERR_UNSUPPORTED;
   if ((hd != 64 && hd != 128) || page_tokens < 16 || (page_tokens & (page_tokens - 1))) return HK_ERR_UNSUPPORTED;
   if (((uintptr_t)k_pages & 127) || ((uintptr_t)v_pages & 127)) return HK_ERR_UNSUPPORTED;
-  const int box_rows = page_tokens < TT ? page_tokens : TT;
+  const bool narrow = narrow_pays((long long)n_items * G, hd, pages_cap);
+  const int tile = narrow ? 32 : 64;
+  const int box_rows = page_tokens < tile ? page_tokens : tile;
   const unsigned long long rows = (unsigned long long)num_pages * G * page_tokens;
   CUtensorMap mk, mv;
   if (!make_page_map(&mk, k_pages, rows, hd, box_rows) || !make_page_map(&mv, v_pages, rows, hd, box_rows)) return HK_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
-#define HK_TMA(D, WITH)                                                                                                      \
-  launch_decode_tma<D, WITH>(mk, mv, q, block_table, table_stride, items, n_items, out, part_o, part_ml, H, G, page_tokens, \
+#define HK_TMA(D, WITH, W)                                                                                                   \
+  launch_decode_tma<D, WITH, W>(mk, mv, q, block_table, table_stride, items, n_items, out, part_o, part_ml, H, G, page_tokens, \
                              box_rows, window, scale_log2, so, pages_cap, status, s)
-  if (hd == 64) return so.dist ? HK_TMA(64, true) : HK_TMA(64, false);
-  return so.dist ? HK_TMA(128, true) : HK_TMA(128, false);
+  if (narrow) {
+    if (hd == 64) return so.dist ? HK_TMA(64, true, 2) : HK_TMA(64, false, 2);
+    return so.dist ? HK_TMA(128, true, 2) : HK_TMA(128, false, 2);
+  }
+  if (hd == 64) return so.dist ? HK_TMA(64, true, 4) : HK_TMA(64, false, 4);
+  return so.dist ? HK_TMA(128, true, 4) : HK_TMA(128, false, 4);
 #undef HK_TMA
 }
 
