@@ -219,6 +219,49 @@ def run_stream(a, w, out, epilogue: int, ldo: int, limit: float = 0.0, slope: fl
     return True
 
 
+# Clusters of CTAs with a whole SM's shared memory each that are resident at once on 148 SMs (asked of the driver's occupancy
+# call): the groups of SMs a cluster must sit in are not multiples of it.
+CLUSTERS_AT_ONCE = {2: 74, 3: 45, 4: 33, 6: 22, 8: 15}
+CLUSTER_M = 128
+
+
+@functools.lru_cache(maxsize=4096)
+def cluster_config(M: int, N: int, K: int, sms: int):
+    """(tile width, K slices) of the product whose slices are added inside a cluster, or None where the sliced kernel with its
+    second launch stays.  It takes what would be cut into three slices or more: with two the partial sums are few, and 64 and
+    128 rows by 8,192 x 4,096 measured 19.3 and 21.7 us that way, 19.7 and 23.2 in clusters.  All clusters run at once; among
+    the widths and slices that allow it a model picks (a K block costs a fixed part and its bytes; then the tile goes through
+    shared memory), within 4 % of the best of all 27 measured shapes of 24 to 128 rows.  64 rows, us before and now: 4,096 x
+    4,096 13.9 and 12.8, 6,144 x 4,096 17.0 and 16.1, 4,096 x 12,288 26.9 and 24.9, 2,560 x 2,560 10.6 and 8.9."""
+    if M > CLUSTER_M or N % 4 or tc_config(M, N, K, sms)[1] < 3:
+        return None
+    k_blocks, rows = -(-K // 64), -(-M // 8) * 8
+    best = None
+    for slices, clusters in CLUSTERS_AT_ONCE.items():
+        if k_blocks < 4 * slices:
+            break
+        for bn in range(64, 257, 32):
+            if -(-N // bn) > clusters * sms // 148:
+                continue
+            cost = k_blocks / slices * (0.25 + 0.0007 * (rows + bn)) + 1.3e-4 * M * bn
+            if best is None or cost < best[0]:
+                best = (cost, bn, slices)
+    return best and best[1:]
+
+
+def run_cluster(a, w, out, accumulate: bool, bn: int, slices: int) -> bool:
+    """out (fp32) = a w^T (+ out) with the K slices added inside clusters.  False when the kernel refuses."""
+    from . import ops
+    M, K = a.shape
+    N = w.shape[0]
+    code = build.load("gemm_tc").hk_gemm_tc_cluster(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), 1 if accumulate else 0,
+                                                    bn, slices, _ptr(status_flag(a.device)), _stream())
+    if code == _UNSUPPORTED:
+        return False
+    ops._check(code, "gemm (tcgen05, clusters)")
+    return True
+
+
 def _tc_partial(lib, M: int, N: int, splits: int, device):
     """Scratch for the partial sums of `splits` K slices (None without slices)."""
     if splits <= 1:
@@ -248,6 +291,9 @@ def run(a, w, out, accumulate: bool, choice: Optional[str]) -> bool:
         if code == _UNSUPPORTED:
             return False
         ops._check(code, "gemm (small-M)")
+        return True
+    clusters = None if _tc_bn or _tc_splits else cluster_config(M, N, K, _sms(a.device))
+    if clusters is not None and run_cluster(a, w, out, accumulate, *clusters):
         return True
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))

@@ -12,7 +12,8 @@
 // Two accumulator buffers (2 x 256 columns of tensor memory) let the epilogue of one tile overlap
 // the main loop of the next.  Every mbarrier wait is bounded: on time-out the CTA records an
 // error in `status`, all roles leave their loops, tensor memory is freed and the kernel returns.
-// No cluster multicast is used anywhere: every CTA loads its own tiles.
+// No cluster multicast is used anywhere: every CTA loads its own tiles.  `gemm_tc_cluster_kernel` below is the form for up to
+// 128 rows whose K slices are added inside a cluster.
 //
 // Reference counterpart: `gemm_tc_<fmt>` (mma.sync, 64 x 128 blocks), src/cuda_device.zig:348-499.
 #include <cuda.h>
@@ -484,6 +485,148 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
+// ---- K slices added inside a cluster ---------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 load_peer(uint32_t addr, uint32_t rank) {
+  float4 v;
+  uint32_t peer;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer) : "memory");
+  return v;
+}
+
+__host__ __device__ inline int cluster_rows(int M) { return (M + 7) & ~7; }        // rows of a stage's a tile
+__host__ __device__ inline uint32_t cluster_stage_bytes(int M, int bn) { return (uint32_t)(cluster_rows(M) + bn) * (BK * 2); }
+constexpr int CLUSTER_PITCH = 4;        // floats between the rows of a partial tile beyond bn: eight rows' 16 bytes fall in all 32 banks
+
+// out (fp32) = or += a w^T for M <= 128 rows: the cluster's CTAs each take a slice of K of one tile of bn columns, leave
+// their partial sums in their own shared memory (in the ring, whose stages are used up) and add the slices there, each a
+// share of the rows, slice after slice.  Against partial sums in global memory and a second kernel that is one launch
+// and one trip through L2 less: 64 rows by 4,096 x 4,096 13.9 -> 12.8 us, 4,096 x 12,288 26.9 -> 24.9, 2,560 x 2,560 10.6 ->
+// 8.9 (back to back, weights from the HBM).  Bound by how soon a CTA's loads start and by the K blocks' own latency: the
+// weights alone would take 5.0, 15.1 and 2.0.  The a tile holds M rows, not 128: the tensor core's other rows read whatever follows
+// in the stage (bn >= 64 weight rows and more: inside the ring) and end in accumulator rows nobody stores.
+template <bool ADD>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, float* __restrict__ out,
+                       int M, int N, int K, long long ldo, int bn, int stages, int* __restrict__ status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  Control& sm = *reinterpret_cast<Control*>(base);
+  uint8_t* ring = base + CONTROL_BYTES;
+  volatile int* abort_flag = &sm.abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank(), slices = (int)cluster_size();
+  const int n0 = ((int)blockIdx.x / slices) * bn;
+  const int k_blocks = (K + BK - 1) / BK;
+  const int kb0 = (int)((long long)k_blocks * rank / slices), kb1 = (int)((long long)k_blocks * (rank + 1) / slices);
+  const uint32_t stage_bytes = cluster_stage_bytes(M, bn), a_bytes = (uint32_t)cluster_rows(M) * (BK * 2);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(&sm.full[s], 1);
+      mbar_init(&sm.empty[s], 1);
+    }
+    mbar_init(&sm.tmem_full[0], 1);
+    sm.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"((uint32_t)MAX_BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sm.tmem_base;
+  pdl_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int issued = 0;
+      for (int kb = kb0; kb < kb1; ++kb, ++issued) {
+        const int stage = issued % stages;
+        if (!mbar_wait(&sm.empty[stage], ((uint32_t)(issued / stages) & 1u) ^ 1u, abort_flag)) break;
+        uint8_t* st = ring + (size_t)stage * stage_bytes;
+        mbar_expect_tx(&sm.full[stage], stage_bytes);
+        tma_load_2d(st + a_bytes, &map_w, &sm.full[stage], kb * BK, n0);
+        tma_load_2d(st, &map_a, &sm.full[stage], kb * BK, 0);
+      }
+      pdl_launch_dependents();
+      if (*abort_flag) {      // giving up: let the copies that are still on their way land before the shared memory goes away
+        for (int i = issued > stages ? issued - stages : 0; i < issued; ++i)
+          for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin)
+            if (mbar_try_wait(&sm.full[i % stages], (uint32_t)(i / stages) & 1u)) break;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const int i = kb - kb0, stage = i % stages;
+        if (!mbar_wait(&sm.full[stage], (uint32_t)(i / stages) & 1u, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t st = smem_u32(ring + (size_t)stage * stage_bytes);
+        const uint64_t da = make_smem_desc(st), db = make_smem_desc(st + a_bytes);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_bf16(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&sm.empty[stage]);
+      }
+      if (ok) umma_commit(&sm.tmem_full[0]);
+    }
+  } else {
+    const int quarter = warp & 3;
+    const int row = quarter * 32 + lane;
+    // (for a whole warp or not at all: the tensor-memory loads below are warp-wide instructions)
+    if (__all_sync(0xffffffffu, mbar_wait(&sm.tmem_full[0], 0u, abort_flag))) {
+      tc_fence_after();
+      // every stage is read (the accumulator is complete): the ring is free for the partial tile
+      float* mine = reinterpret_cast<float*>(ring) + (size_t)row * (bn + CLUSTER_PITCH);
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+      if (quarter * 32 < M)
+#pragma unroll 1
+        for (int c0 = 0; c0 < bn; c0 += 32) store_chunk<32, false>(taddr, mine, c0, bn, row < M, true);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  const bool gave_up = sm.abort_flag != 0;
+  if (threadIdx.x == 0 && gave_up) atomicExch(status, 1);
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)MAX_BN) : "memory");
+  }
+  cluster_sync();
+  // this CTA's share of the tile's rows, the columns that exist (N and bn are multiples of 4)
+  const int r0 = M * rank / slices, r1 = M * (rank + 1) / slices;
+  const int quads = (min(bn, N - n0)) >> 2;
+  const uint32_t tile = smem_u32(ring);
+  for (int i = threadIdx.x; i < (r1 - r0) * quads; i += NUM_THREADS) {
+    const int r = r0 + i / quads, c = (i % quads) * 4;
+    float4* o = reinterpret_cast<float4*>(out + (size_t)r * ldo + n0 + c);
+    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ADD) y = *o;
+    const uint32_t at = tile + (uint32_t)(r * (bn + CLUSTER_PITCH) + c) * 4u;
+    float4 sum = load_peer(at, 0);
+    for (int s = 1; s < slices; ++s) {
+      const float4 p = load_peer(at, (uint32_t)s);
+      sum.x += p.x; sum.y += p.y; sum.z += p.z; sum.w += p.w;
+    }
+    if (ADD) { sum.x += y.x; sum.y += y.y; sum.z += y.z; sum.w += y.w; }
+    *o = sum;
+  }
+  cluster_sync();     // nobody leaves while its tile may still be read
+}
+
 // ---- host side: tensor maps ------------------------------------------------------------------
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -612,7 +755,49 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int M, int N
   return hk_launch_pdl(splitk_reduce_kernel<EPI>, dim3(blocks), dim3(256), 0, s, (const float*)partial, out, M, N, ldo, splits, bn, gp);
 }
 
+template <bool ADD>
+int launch_cluster(const CUtensorMap& ma, const CUtensorMap& mw, float* out, int M, int N, int K, long long ldo, int bn, int slices,
+                   int* status, cudaStream_t s) {
+  static HkSmemCache allowed = {};
+  const uint32_t stage_bytes = cluster_stage_bytes(M, bn);
+  int stages = (RING_BYTES - 16 * 1024) / (int)stage_bytes;       // 16 KB: what the tensor core may read past the last stage's a rows
+  if (stages > MAX_STAGES) stages = MAX_STAGES;
+  const size_t smem = (size_t)RING_BYTES + CONTROL_BYTES + 1024;
+  if (int e = hk_allow_smem(gemm_tc_cluster_kernel<ADD>, smem, allowed)) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((N + bn - 1) / bn * slices));
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)slices;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<ADD>, ma, mw, out, M, N, K, ldo, bn, stages, status);
+}
+
 }  // namespace
+
+// out (fp32 [M, N]) = a w^T, or += with `add`, for M <= 128 with K cut into `slices` (2 to 8) that one cluster adds in its
+// shared memory.  Refuses (HK_ERR_UNSUPPORTED) what hk_gemm_tc refuses, tiles that are not 64 to 256 columns in steps of 32,
+// N or ldo that are not multiples of 4 and an `out` off a 16-byte boundary.
+HK_API int hk_gemm_tc_cluster(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, int add, int bn,
+                              int slices, int* status, void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || (K & 7) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || ((uintptr_t)out & 15)) return HK_ERR_UNSUPPORTED;
+  if (M > BM || (N & 3) || (ldo & 3) || bn < 64 || bn > MAX_BN || (bn & 31)) return HK_ERR_UNSUPPORTED;
+  if (slices < 2 || slices > 8 || slices > (K + BK - 1) / BK) return HK_ERR_UNSUPPORTED;
+  CUtensorMap ma, mw;
+  if (!make_map(&ma, a, M, K, cluster_rows(M)) || !make_map(&mw, w, N, K, bn)) return HK_ERR_UNSUPPORTED;
+  cudaStream_t s = (cudaStream_t)stream;
+  float* o = reinterpret_cast<float*>(out);
+  return add ? launch_cluster<true>(ma, mw, o, M, N, K, ldo, bn, slices, status, s)
+             : launch_cluster<false>(ma, mw, o, M, N, K, ldo, bn, slices, status, s);
+}
 
 // out = a w^T.  epilogue 0: out fp32 [M, N] stored; 1: out fp32 [M, N] += ; 2: out bf16 [M, N/2] =
 // silu(gate) * up with w = [N/2 gate rows | N/2 up rows].  `bn` is the tile width: a multiple of 16 from 16 to 256
