@@ -6,7 +6,8 @@
 // its own key was written by the cache-write kernel earlier in the same step.  Four warps take
 // the keys round-robin, each keeping an online softmax state (max, sum, weighted values); the
 // four states are merged in a fixed order.  Nothing depends on which other tokens are in the
-// batch, so the result at a position is the same under every way of cutting the work.
+// batch, so the result at a position is the same under every way of cutting the work.  In float, heads and values of up
+// to 128 take `attention_f32_kernel` further down (a block per run of a request's rows and key head), with the same promise.
 // Values may have another width than keys (`vd`: pages [page][G][page_tokens][vd], out [n, H * vd]).  With
 // `sink` = 1 the softmax has one more term in its denominator, a key whose score is 0 and that has no value:
 // p_j = exp(s_j) / (1 + sum exp(s_j)); with `sinks` (one float per query head) that key's score is sinks[h] instead of 0.

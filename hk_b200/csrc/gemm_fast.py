@@ -6,7 +6,8 @@
   * 9 to 16 rows: the streaming kernel at every shape;
   * more rows (larger decode batches, prefill, mixed batches): the persistent tcgen05 kernel (`gemm_tc.cu`) with
     the tile width that fills whole waves of SMs (`tc_config`), cutting K into slices when the output has fewer
-    tiles than the GPU has SMs.
+    tiles than the GPU has SMs; up to 128 rows and from three slices on, the slices are added inside a cluster
+    (`cluster_config`).
 The choice depends on the shape alone, so a token's logits do not depend on what else a process ran before.
 Shapes all of them refuse (K not a multiple of 8, unaligned operands) go to the generic kernel.
 """
