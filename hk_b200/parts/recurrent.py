@@ -4,9 +4,9 @@ Both keep their state in float32 in the request's state slot (`StateSpec`) and f
 of a step through one host-built table, `segments` int32 [requests of the step, 3] = (slot, first row, rows),
 shared by all recurrent mixers of a model.  The scans (`csrc/recurrent.cu`) walk a request's rows in order, so
 what a position computes does not depend on how the prompt was cut, on the batch or on the slot.  In bfloat16 a request's
-portion of 64 rows or more is taken in chunks instead (`csrc/delta_chunks.cu`; the state-space and the key-gated recurrence
-have chunks of their own): the same float32 sums, grouped by chunk, so there a prompt's cut moves a result by rounding, while
-the batch and the slot still do not.  Projections
+portion of 64 rows or more is taken in chunks instead: the delta rules, the matrix memory and retention with the same float32
+sums grouped by chunk (`csrc/delta_chunks.cu`), the state-space and the key-gated recurrence with kernels of their own.  There
+a prompt's cut moves a result by rounding; the batch and the slot still do not.  Projections
 are products in the compute type with float32 results; everything from there to the state and the scan's
 output is float32.
 
