@@ -4,8 +4,8 @@
 // A step's batch is described by a segment table int32 [n_seg, 3] = (state slot, first row, rows): the rows
 // of a request are consecutive and in increasing position.  Every scan walks a segment's rows in order, one
 // token after the other, whatever the cut of the prompt was, so the state after a token (and every sum's
-// order) depends on the tokens before it alone: never on the portion sizes, the batch or the slot.  (Portions of 64 rows
-// or more in bfloat16 models take `delta_chunks.cu` instead; these scans are the 32-bit path, decode and short portions.)
+// order) depends on the tokens before it alone: never on the portion sizes, the batch or the slot.  (Steps with a long
+// portion take `delta_chunks.cu` instead in bfloat16 models; these scans are the 32-bit path, decode and shorter portions.)
 //
 //   * generalised delta rule (per head a matrix state S [dk, dv]):
 //         S_t = diag(d_t) S_(t-1) - (a_t * u_t) (u_t^T S_(t-1)) + k_t v_t^T,   o_t = S_t^T r_t

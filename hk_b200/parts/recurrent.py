@@ -3,10 +3,10 @@
 Both keep their state in float32 in the request's state slot (`StateSpec`) and find the rows of every request
 of a step through one host-built table, `segments` int32 [requests of the step, 3] = (slot, first row, rows),
 shared by all recurrent mixers of a model.  The scans (`csrc/recurrent.cu`) walk a request's rows in order, so
-what a position computes does not depend on how the prompt was cut, on the batch or on the slot.  In bfloat16 a request's
-portion of 64 rows or more is taken in chunks instead: the delta rules, the matrix memory and retention with the same float32
-sums grouped by chunk (`csrc/delta_chunks.cu`), the state-space and the key-gated recurrence with kernels of their own.  There
-a prompt's cut moves a result by rounding; the batch and the slot still do not.  Projections
+what a position computes does not depend on how the prompt was cut, on the batch or on the slot.  In bfloat16 steps
+with a long portion take it in chunks instead: the delta rules, the matrix memory and retention with the same float32 sums
+grouped by chunk (`csrc/delta_chunks.cu`), the state-space and the key-gated recurrence with kernels of their own.  There a
+prompt's cut, and through the choice the step's other requests, move a result by float32 rounding.  Projections
 are products in the compute type with float32 results; everything from there to the state and the scan's
 output is float32.
 
@@ -101,11 +101,19 @@ class _SegmentScan(Part):
 
 
 class _ChunkedScan(_SegmentScan):
-    """A recurrence that, when serving in bfloat16, walks a request that brings `CHUNKS_FROM` tokens or more to a step in chunks
-    of tokens (`csrc/delta_chunks.cu`) and the others token by token; the lists of requests and chunks are host-built tables
-    that all such mixers of a model share."""
-    CHUNKS_FROM = 64        # where the two are level, 30 to 50 us; at 128 tokens the chunks take two thirds of the walk's time
-    CHUNK_KEY = ("chunked_segments",)
+    """A recurrence that, when serving in bfloat16, walks the requests of a step in chunks of tokens (`csrc/delta_chunks.cu`)
+    where a long one sets the time of the walk token by token; the lists of requests and chunks are host-built tables that the
+    mixers with as many heads share.
+
+    A walk's time grows with the longest request until requests times heads fill the SMs; the chunks' with all rows.  So a step
+    takes chunks when its longest request brings `LONGEST_FROM` tokens and all rows to be chunked times the heads are at most
+    `BESIDE` times the longest; then every request of `CHUNKS_FROM` tokens or more goes that way.  Scan kernels of the delta
+    rule with 64 heads, us in chunks and walked: one request of 2,048 tokens 423 and 988, one of 512 120 and 249, four of 512
+    423 and 576, nine of 227 474 and 373 (over the limit: walked); with 32 heads one of 512 76 and 193, nine of 100 137 and 121.
+    Requests of 128 to 256 tokens gain up to 50 us of kernels, which the launches and tables of the longer route cost the host."""
+    CHUNKS_FROM = 64
+    LONGEST_FROM = 320
+    BESIDE = 256
     _chunks = False                 # set at bind: the chunked form takes this mixer's sizes
 
     def kernel_libraries(self, bfloat16: bool):
@@ -116,7 +124,10 @@ class _ChunkedScan(_SegmentScan):
         self._chunks = precision.compute == torch.bfloat16 and row % 4 == 0 and ops.delta_chunks_take(self.dk, self.dv, decay_scale)
 
     def step_tables_key(self):
-        return self.CHUNK_KEY if self._chunks else SEGMENTS_KEY
+        return ("chunked_segments", self._beside()) if self._chunks else SEGMENTS_KEY
+
+    def _beside(self) -> int:
+        return max(1, self.BESIDE // self.H)
 
     def step_tables(self, ctx):
         tables = segment_tables(ctx)
@@ -124,6 +135,9 @@ class _ChunkedScan(_SegmentScan):
             return tables
         seg = tables.arrays["segments"]
         long = seg[:, 2] >= self.CHUNKS_FROM
+        longest = int(seg[:, 2].max(initial=0))
+        if longest < self.LONGEST_FROM or int(seg[long, 2].sum()) > self._beside() * longest:
+            long[:] = False
         chunks, requests = [], []
         for slot, row, count in seg[long].tolist():
             first = len(chunks)
@@ -136,13 +150,13 @@ class _ChunkedScan(_SegmentScan):
         """(the segments that are walked token by token, the further arguments of a scan)."""
         if not self._chunks:
             return self._segments(ctx), {}
-        t = ctx.tables[self.CHUNK_KEY][0]
+        t = ctx.tables[self.step_tables_key()][0]
         return t["short"], {"chunks": t["chunks"], "requests": t["requests"],
                             "most_rows": self.CHUNKS_FROM - 1 if t["chunks"].shape[0] else 0}
 
     def _all_segments(self, ctx) -> torch.Tensor:
         """Every request of the step as a segment, whichever way it is walked."""
-        return ctx.tables[self.CHUNK_KEY][0]["segments"] if self._chunks else self._segments(ctx)
+        return ctx.tables[self.step_tables_key()][0]["segments"] if self._chunks else self._segments(ctx)
 
 
 class GeneralDeltaRule(_ChunkedScan):
@@ -633,7 +647,7 @@ class MLSTM(_ChunkedScan):
         gates = torch.empty((n, H, 3), dtype=torch.float32, device=xb.device)
         short, chunked = self._scan_tables(ctx)
         if chunked:
-            chunked["long_segments"] = ctx.tables[self.CHUNK_KEY][0]["long"]
+            chunked["long_segments"] = ctx.tables[self.step_tables_key()][0]["long"]
         ops.mlstm_scan(proj[:, :K], proj[:, K:2 * K], proj[:, 2 * K:2 * K + V], proj[:, 2 * K + 2 * V:2 * K + 2 * V + H],
                        proj[:, 2 * K + 2 * V + H:], self.i_bias, self.f_bias, short, cache[0].state,
                        cache[1].state, o, gates, H, self.dk, self.dv, self.cap, self.q_scale, **chunked)

@@ -26,3 +26,32 @@ def test_tile_widths_of_a_few_hundred_rows():
             bn, splits = gemm_fast.tc_config(m, n, k, 148, swiglu=True)
             assert bn % 32 == 0 and (splits == 1 or (n // 2) % (bn // 2) == 0)
     assert gemm_fast.tc_config(527, 4096, 12288, 148) == (144, 1)       # 145 tiles in one wave
+
+
+def test_which_steps_of_a_recurrence_go_in_chunks():
+    import types
+
+    import numpy as np
+
+    from hk_b200.parts import recurrent
+    part = types.SimpleNamespace()
+
+    def taken(heads, rows):
+        scan = recurrent._ChunkedScan.__new__(recurrent._ChunkedScan)
+        scan.H, scan._chunks = heads, True
+        starts = np.cumsum([0] + rows[:-1])
+        seg = np.asarray([(i, int(s), n) for i, (s, n) in enumerate(zip(starts, rows))], dtype=np.int32).reshape(-1, 3)
+        part.arrays = {"segments": seg}
+        old, recurrent.segment_tables = recurrent.segment_tables, lambda ctx: part
+        try:
+            t = scan.step_tables(None).arrays
+        finally:
+            recurrent.segment_tables = old
+        assert sorted(t["short"].tolist() + t["long"].tolist()) == sorted(seg.tolist()) and len(t["requests"]) == len(t["long"])
+        assert int(t["chunks"][:, 1].sum()) == int(t["long"][:, 2].sum())
+        return t["long"][:, 2].tolist()
+
+    assert taken(64, [319]) == [] and taken(64, [320]) == [320] and taken(64, [1] * 9) == []
+    assert taken(64, [512] * 4) == [512] * 4 and taken(64, [512] * 5) == [] and taken(32, [512] * 8) == [512] * 8
+    assert taken(32, [700, 301, 77, 1]) == [700, 301, 77] and taken(32, [1500, 100, 63]) == [1500, 100]
+    assert taken(300, [400]) == [400] and taken(300, [400, 64]) == []
