@@ -106,13 +106,16 @@ class _ChunkedScan(_SegmentScan):
     mixers with as many heads share.
 
     A walk's time grows with the longest request until requests times heads fill the SMs; the chunks' with all rows.  So a step
-    takes chunks when its longest request brings `LONGEST_FROM` tokens and all rows to be chunked times the heads are at most
+    takes chunks when its longest request brings `LONGEST_FROM` tokens (half that with many heads: tokens times heads at least
+    `ROWS_FROM`) and all rows to be chunked times the heads are at most
     `BESIDE` times the longest; then every request of `CHUNKS_FROM` tokens or more goes that way.  Scan kernels of the delta
     rule with 64 heads, us in chunks and walked: one request of 2,048 tokens 423 and 988, one of 512 120 and 249, four of 512
     423 and 576, nine of 227 474 and 373 (over the limit: walked); with 32 heads one of 512 76 and 193, nine of 100 137 and 121.
-    Requests of 128 to 256 tokens gain up to 50 us of kernels, which the launches and tables of the longer route cost the host."""
+    Below, the kernels still gain (one request of 512 tokens over 32 heads, see above), but the launches and tables of the longer
+    route cost the host as much: requests of 34 and 471 tokens took 288 us walked and 309 with the longer one in chunks."""
     CHUNKS_FROM = 64
-    LONGEST_FROM = 320
+    LONGEST_FROM = 640
+    ROWS_FROM = 320 * 64
     BESIDE = 256
     _chunks = False                 # set at bind: the chunked form takes this mixer's sizes
 
@@ -124,10 +127,7 @@ class _ChunkedScan(_SegmentScan):
         self._chunks = precision.compute == torch.bfloat16 and row % 4 == 0 and ops.delta_chunks_take(self.dk, self.dv, decay_scale)
 
     def step_tables_key(self):
-        return ("chunked_segments", self._beside()) if self._chunks else SEGMENTS_KEY
-
-    def _beside(self) -> int:
-        return max(1, self.BESIDE // self.H)
+        return ("chunked_segments", self.H) if self._chunks else SEGMENTS_KEY
 
     def step_tables(self, ctx):
         tables = segment_tables(ctx)
@@ -136,7 +136,8 @@ class _ChunkedScan(_SegmentScan):
         seg = tables.arrays["segments"]
         long = seg[:, 2] >= self.CHUNKS_FROM
         longest = int(seg[:, 2].max(initial=0))
-        if longest < self.LONGEST_FROM or int(seg[long, 2].sum()) > self._beside() * longest:
+        worth = longest >= self.LONGEST_FROM or (2 * longest >= self.LONGEST_FROM and longest * self.H >= self.ROWS_FROM)
+        if not worth or int(seg[long, 2].sum()) > max(1, self.BESIDE // self.H) * longest:
             long[:] = False
         chunks, requests = [], []
         for slot, row, count in seg[long].tolist():

@@ -52,6 +52,7 @@ def test_which_steps_of_a_recurrence_go_in_chunks():
         return t["long"][:, 2].tolist()
 
     assert taken(64, [319]) == [] and taken(64, [320]) == [320] and taken(64, [1] * 9) == []
-    assert taken(64, [512] * 4) == [512] * 4 and taken(64, [512] * 5) == [] and taken(32, [512] * 8) == [512] * 8
+    assert taken(64, [512] * 4) == [512] * 4 and taken(64, [512] * 5) == [] and taken(32, [640] * 8) == [640] * 8
     assert taken(32, [700, 301, 77, 1]) == [700, 301, 77] and taken(32, [1500, 100, 63]) == [1500, 100]
+    assert taken(32, [639]) == [] and taken(8, [1000]) == [1000] and taken(320, [319]) == []
     assert taken(300, [400]) == [400] and taken(300, [400, 64]) == []
