@@ -676,18 +676,26 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
   const int h = blockIdx.x, d0 = blockIdx.z * 32, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ldl = r + 4, ldc = r + 8;
   bf16* cs = reinterpret_cast<bf16*>(lat + FIRST_ROWS * ldl);
   const FirstRows f = firsts[blockIdx.y];
-  const int wide = 128 + dr, last = f.pos0 + f.count;   // keys are positions 0 .. last - 1
+  // keys are positions first .. last - 1: a window below FIRST_ROWS may leave out a request's first positions, and where they
+  // would stand among the made rows another request stands, or nothing (row0 is then negative)
+  const int wide = 128 + dr, last = f.pos0 + f.count, first = window > 0 ? max(0, f.pos0 - window + 1) : 0;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   for (int e = tid; e < FIRST_ROWS * 24; e += 256) {
     const int i = e / 24, p = (e % 24) * 8;
-    const bool q_in = i < f.count && p < wide, k_in = i < last && p < wide;
+    const bool q_in = i < f.count && p < wide;
     *reinterpret_cast<uint4*>(&qs[i][p]) = q_in ? *reinterpret_cast<const uint4*>(q + ((size_t)(f.q_row + i) * H + h) * wide + p) : zero;
-    const bf16* kp = p < 128 ? kv + ((size_t)(f.row0 + i) * H + h) * 256 + p : rope + (size_t)(f.row0 + i) * dr + p - 128;
-    *reinterpret_cast<uint4*>(&ks[i][p]) = k_in ? *reinterpret_cast<const uint4*>(kp) : zero;
+    uint4 key = zero;
+    if (i >= first && i < last && p < wide) {
+      const size_t row = (size_t)(f.row0 + i);
+      key = *reinterpret_cast<const uint4*>(p < 128 ? kv + (row * H + h) * 256 + p : rope + row * dr + p - 128);
+    }
+    *reinterpret_cast<uint4*>(&ks[i][p]) = key;
   }
   for (int e = tid; e < FIRST_ROWS * (r / 8); e += 256) {
     const int j = e / (r / 8), p = (e % (r / 8)) * 8;
-    *reinterpret_cast<uint4*>(cs + j * ldc + p) = j < last ? *reinterpret_cast<const uint4*>(c + (size_t)(f.row0 + j) * r + p) : zero;
+    uint4 latent = zero;
+    if (j >= first && j < last) latent = *reinterpret_cast<const uint4*>(c + (size_t)(f.row0 + j) * r + p);
+    *reinterpret_cast<uint4*>(cs + j * ldc + p) = latent;
   }
   __syncthreads();
   auto halves = [](const uint4& v, float* x) {          // eight bf16 as floats
