@@ -318,28 +318,32 @@ def run_latent(q, pages, block_table, out, H: int, dk: int, dv: int, page_tokens
 
 MADE_FIRST = 16         # positions from a request's start whose values are not rounded (FIRST_ROWS in csrc/attention_latent.cu)
 MADE_TOKENS = 256       # query tokens of a work item: two query tiles of one head
+MADE_TILE = 128         # made rows that the prompt kernel loads at once (TK in csrc/attention_prefill_tc.cu)
 
 
 def made_supported(plain_dim: int, rot_dim: int, v_head_dim: int, rank: int) -> bool:
     return plain_dim == 128 and v_head_dim == 128 and rot_dim in (0, 64) and rank % 8 == 0
 
 
-def made_items(slots, q_starts, q_lens, start_positions, window: int):
+def made_items(slots, q_starts, q_lens, start_positions, window: int, tile: int = 1):
     """(items int32 [n, 8], segments int32 [requests, 4], firsts int32 [m, 4], rows): the work items of requests whose visible
     cache rows are laid side by side, longest key ranges first, where those rows come from (`ops.latent_rows`), and which of the
-    step's rows stand at a request's start."""
+    step's rows stand at a request's start.  Position 0 of a request lies (or would) on a multiple of `tile` rows and the request
+    takes whole tiles: what a tile of the prompt kernel holds beside a request's rows is filled up and not another request's, whose
+    values, were they NaN or Inf, a probability of zero would not keep out of the sums."""
     items, segments, firsts, row = [], [], [], 0
     for slot, qs, ql, p0 in zip(slots, q_starts, q_lens, start_positions):
         first = max(0, p0 - window + 1) if window > 0 else 0
-        base = row - first                     # the row of position 0, were it there
+        start = first // tile * tile           # the position that the request's first row would have
+        base = row - start                     # the row of position 0, were it there
         for b0 in range(0, ql, MADE_TOKENS):
             n, pos0 = min(MADE_TOKENS, ql - b0), p0 + b0
             lo = max(0, pos0 - window + 1) if window > 0 else 0
             items.append((qs + b0, n, base, pos0, lo, pos0 + n, -1, 0))
-        segments.append((slot, first, p0 + ql - first, row))
+        segments.append((slot, first, p0 + ql - first, base + first))
         if p0 < MADE_FIRST:
             firsts.append((qs, base, p0, min(ql, MADE_FIRST - p0)))
-        row += p0 + ql - first
+        row += -(-(p0 + ql - start) // tile) * tile
     items.sort(key=lambda r: r[4] - r[5])
     return np.asarray(items, dtype=np.int32).reshape(-1, 8), np.asarray(segments, dtype=np.int32).reshape(-1, 4), \
         np.asarray(firsts, dtype=np.int32).reshape(-1, 4), row

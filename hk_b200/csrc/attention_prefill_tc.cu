@@ -622,7 +622,7 @@ struct Smem2 {
 // DIST: with a bias by distance (an instance of its own, so that the softmax of a model without one issues nothing for it)
 // MADE: keys and values made for the step from a compressed cache (a latent attention's prompt portions), not pages: every
 // query head has its own (H == G); a request's rows stand side by side, the row of position 0 at item.slot (which may lie
-// before the first row there is); map_k and map_v see [rows, H][128 key dims | 128 value dims], map_r the 64 key dims that all
+// before the first row there is), a multiple of TK unless the request is alone: a box holds no other request's rows; map_k and map_v see [rows, H][128 key dims | 128 value dims], map_r the 64 key dims that all
 // heads share (HDK = HD + 64; without them HDK = HD).  2,048 tokens at 32 heads: 112 us (384 TFLOP/s of the visible pairs), where
 // the same scores and sums in the latent space (576 and 512 numbers a row instead of 192 and 128) took 876 us on mma.sync.
 template <int HD, int HDK, bool DIST, bool MADE>
@@ -663,7 +663,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   // The V stages start as zeros: a box that is not copied (a page outside the key range, or one that the request
   // does not hold) leaves its rows as they are, and whatever is there is multiplied by a probability of zero, which
   // must not meet a NaN pattern.  K needs none: a score of such a key is masked before it is looked at.  (Made values come
-  // in whole boxes: rows that are not there as zeros, rows of other requests as they are.)
+  // in whole boxes: the rows of a box that are not the request's are zeros, in the array or behind its end.)
   if (!MADE) {
     uint4* z = reinterpret_cast<uint4*>(sm.v[0]);
     constexpr int N16 = VST * TK * HD * 2 / 16;
@@ -1069,7 +1069,8 @@ HK_API int hk_attention_prefill_tc2(const void* q, const void* k_pages, const vo
 
 // Keys and values that were made for the step (see the kernel's MADE).  q bf16 [n, H, 128 (+ 64 with rope)]; kv bf16 [rows, H,
 // 128 key dims | 128 value dims]; rope bf16 [rows, 64], the key dims that all heads share behind their own 128, or null; items
-// as above for groups of one head (up to 256 query tokens), with the row of the request's position 0 in the place of its slot;
+// as above for groups of one head (up to 256 query tokens), with the row of the request's position 0 in the place of its slot (a
+// multiple of 128 where several requests share the arrays: a request's rows fill whole boxes of 128, with zeros beside its own);
 // out bf16 [n, H, 128].  gate (or null): float32 logits [n, gate_ld], one per output (16-byte aligned rows) or, with gate_heads,
 // one per head.
 HK_API int hk_attention_prefill_made(const void* q, const void* kv, const void* rope, long long rows, const void* items, int n_items,

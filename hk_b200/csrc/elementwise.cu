@@ -1189,29 +1189,33 @@ HK_API int hk_latent_prep(const float* q, long long ldq, const float* kv, long l
 
 // The cache rows of whole requests side by side, for keys and values that are made for the step: segs int32 [n, 4] = (slot, first
 // position, rows, first row of the result); a row's first r numbers go to c[row, :r], the other dr to rope[row, :dr] (both in
-// 16-byte pieces).  Bound by its bytes, each read and written once.
+// 16-byte pieces).  The rows before and behind a segment's own in its tiles of `tile` rows become zeros, up to row `all` of the
+// result.  Bound by its bytes, each read and written once.
 __global__ void latent_rows_kernel(const bf16* __restrict__ pages, const int* __restrict__ block_table, int table_stride,
-                                   const int* __restrict__ segs, bf16* __restrict__ c, bf16* __restrict__ rope, int r, int dr, int page_tokens) {
+                                   const int* __restrict__ segs, int tile, bf16* __restrict__ c, bf16* __restrict__ rope, int all, int r, int dr,
+                                   int page_tokens) {
   const int* seg = segs + 4 * blockIdx.y;
   const int pieces = (r + dr) >> 3;
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long long)seg[2] * pieces) return;
-  const int t = (int)(e / pieces), i = (int)(e % pieces) * 8, pos = seg[1] + t;
-  const int page = block_table[(size_t)seg[0] * table_stride + pos / page_tokens];
+  const int before = seg[3] % tile, i = (int)(e % pieces) * 8;
+  const long long t = e / pieces - before, row = seg[3] + t;       // t: the row of the segment, below 0 in front of it
+  if (row >= all || t >= seg[2] + (tile - (before + seg[2]) % tile) % tile) return;
   uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (page >= 0) v = *reinterpret_cast<const uint4*>(pages + ((size_t)page * page_tokens + pos % page_tokens) * (r + dr) + i);
-  const size_t row = (size_t)seg[3] + t;
+  if (t >= 0 && t < seg[2]) {
+    const int pos = seg[1] + (int)t, page = block_table[(size_t)seg[0] * table_stride + pos / page_tokens];
+    if (page >= 0) v = *reinterpret_cast<const uint4*>(pages + ((size_t)page * page_tokens + pos % page_tokens) * (r + dr) + i);
+  }
   *reinterpret_cast<uint4*>(i < r ? c + row * r + i : rope + row * dr + i - r) = v;
 }
 
-HK_API int hk_latent_rows(const void* pages, const int* block_table, int table_stride, const int* segs, int n_segs, int most_rows, void* c,
-                          void* rope, int r, int dr, int page_tokens, void* stream) {
+HK_API int hk_latent_rows(const void* pages, const int* block_table, int table_stride, const int* segs, int n_segs, int most_rows, int tile,
+                          void* c, void* rope, int all, int r, int dr, int page_tokens, void* stream) {
   if (n_segs <= 0 || most_rows <= 0) return 0;
-  if (r < 8 || (r & 7) || dr < 0 || (dr & 7) || page_tokens < 1 || n_segs > 65535 || (((uintptr_t)pages | (uintptr_t)c | (uintptr_t)rope) & 15))
+  if (tile < 1 || tile > 65536 || r < 8 || (r & 7) || dr < 0 || (dr & 7) || page_tokens < 1 || n_segs > 65535 || (((uintptr_t)pages | (uintptr_t)c | (uintptr_t)rope) & 15))
     return HK_ERR_UNSUPPORTED;
-  const long long items = (long long)most_rows * ((r + dr) >> 3);
+  const long long items = ((long long)most_rows + 2 * (tile - 1)) * ((r + dr) >> 3);
   return hk_launch(latent_rows_kernel, dim3((unsigned)((items + 255) / 256), (unsigned)n_segs), dim3(256), 0, (cudaStream_t)stream, (const bf16*)pages,
-                   block_table, table_stride, segs, (bf16*)c, (bf16*)rope, r, dr, page_tokens);
+                   block_table, table_stride, segs, tile, (bf16*)c, (bf16*)rope, all, r, dr, page_tokens);
 }
 
 // ----------------------------------------------------------------------------- sums of float32 streams

@@ -675,9 +675,10 @@ def latent_prep(q, kv, q_plain, q_full, c_weight, eps, cos, sin, rotary_dim, pai
         1 if write_kv else 0, _stream()), "latent_prep")
 
 
-def latent_rows(pages, block_table, segments, most_rows: int, c, rope) -> None:
+def latent_rows(pages, block_table, segments, most_rows: int, c, rope, tile: int = 1) -> None:
     """The cache rows of whole requests side by side: `segments` int32 [n, 4] = (slot, first position, rows, first row of the
-    result), none of more than `most_rows` rows; c [rows, r] and rope [rows, dr] (None where a row has no such part), bfloat16."""
+    result), none of more than `most_rows` rows; c [rows, r] and rope [rows, dr] (None where a row has no such part), bfloat16.
+    The rows beside a segment's own in its tiles of `tile` rows become zeros (no two segments share a tile)."""
     _need(pages, "pages", torch.bfloat16, 4)
     _need(block_table, "block_table", torch.int32, 2)
     _need(segments, "segments", torch.int32, 2)
@@ -691,7 +692,7 @@ def latent_rows(pages, block_table, segments, most_rows: int, c, rope) -> None:
         raise KernelError("latent_rows: shapes do not fit")
     lib = build.load("elementwise")
     _check(lib.hk_latent_rows(_ptr(pages), _ptr(block_table), int(block_table.shape[1]), _ptr(segments), int(segments.shape[0]), int(most_rows),
-                              _ptr(c), _ptr(rope), r, dr, int(pages.shape[2]), _stream()), "latent_rows")
+                              int(tile), _ptr(c), _ptr(rope), int(c.shape[0]), r, dr, int(pages.shape[2]), _stream()), "latent_rows")
 
 
 def gemm_narrow(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:

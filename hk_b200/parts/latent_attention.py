@@ -39,7 +39,8 @@ from .position import RotaryEmbedding
 @dataclass
 class LatentInfo:
     """The host-side facts of a step in which requests have their keys and values made: the latent kernel's plan for the others
-    (or None), runs of neighbouring rows (first, one past the last, made or not), and the made rows."""
+    (or None), runs of neighbouring rows (first, one past the last, made or not), the made rows with what fills their tiles up, and
+    the most that a request sees."""
     plan: object
     single_tokens: bool
     runs: List[Tuple[int, int, bool]]
@@ -147,7 +148,7 @@ class LatentAttention(Part):
         def those(kind):
             return [[x for x, m in zip(xs, made) if m == kind] for xs in (ctx.slots, ctx.q_starts, ctx.q_lens, ctx.start_positions)]
 
-        items, segments, firsts, rows = attention_fast.made_items(*those(True), window)
+        items, segments, firsts, rows = attention_fast.made_items(*those(True), window, attention_fast.MADE_TILE)
         arrays, plan, single = {"made_items": items, "made_segments": segments, "made_firsts": firsts}, None, False
         if not all(made):
             slots, q_starts, q_lens, starts = those(False)
@@ -228,7 +229,7 @@ class LatentAttention(Part):
                             cache.page_tokens, write_kv=write_cache, q_packed=packed[a:b] if made else None)
         c = torch.empty((info.rows, r), dtype=dt, device=dev)
         rope = torch.empty((info.rows, dr), dtype=dt, device=dev) if dr else None
-        ops.latent_rows(cache.k_pages, cache.block_table, arrays["made_segments"], info.most_rows, c, rope)
+        ops.latent_rows(cache.k_pages, cache.block_table, arrays["made_segments"], info.most_rows, c, rope, attention_fast.MADE_TILE)
         kv = torch.empty((info.rows, H * (dn + vd)), dtype=dt, device=dev)
         ops.gemm_narrow(c, self._w_ukv, kv)
         attention_fast.run_made(packed, kv, rope, arrays["made_items"], att, H, self.window or 0, self.scale, c, self.w_uv,

@@ -9,8 +9,9 @@ DEV = "cuda"
 H, R, DR, GUARD = 2, 64, 64, 256
 
 
-def made_case(spans, window, layout, seed=0):
-    """(out of `run_made`, the same in float64, positions): spans (cached, new) of requests whose rows lie as `layout` says."""
+def made_case(spans, window, layout, seed=0, tile=1, spoilt=(), spoil=float("nan")):
+    """(out of `run_made`, the same in float64, positions): spans (cached, new) of requests whose rows lie as `layout` says, the rest
+    of their tiles zeros; `spoilt` = (request, row of its own) whose cache row and values are `spoil`."""
     from hk_b200.csrc import attention_fast, gemm_fast
     g = torch.Generator(DEV).manual_seed(seed)
     rand = lambda *s: torch.randn(*s, generator=g, device=DEV)       # noqa: E731
@@ -26,7 +27,8 @@ def made_case(spans, window, layout, seed=0):
     n = sum(lens)
     q, want, pos = (rand(n, H * 192) * 0.5).bfloat16(), torch.empty(n, H, 128, dtype=torch.float64), []
     for (_, first, count, row0), qs, ql, p0 in zip(segments.tolist(), q_starts, lens, starts):
-        part = slice(row0, row0 + count)
+        part, whole = slice(row0, row0 + count), slice(row0 // tile * tile, -(-(row0 + count) // tile) * tile)
+        c[whole], rope[whole], kv[whole] = 0.0, 0.0, 0.0
         c[part], rope[part] = rand(count, R).bfloat16(), rand(count, DR).bfloat16()
         kv[part] = (c[part].float() @ w.float().flatten(0, 1).t()).bfloat16()
         keys = torch.cat([kv[part].view(count, H, 256)[..., :128], rope[part][:, None].expand(count, H, DR)], dim=2).double()
@@ -37,6 +39,8 @@ def made_case(spans, window, layout, seed=0):
             s = torch.einsum("hd,thd->ht", q[qs + i].view(H, 192).double(), keys[see]) * 192 ** -0.5
             want[qs + i] = torch.einsum("ht,thv->hv", torch.softmax(s, dim=1), values[see]).cpu()
             pos.append(p)
+    for request, own in spoilt:
+        c[segments[request][3] + own], kv[segments[request][3] + own] = spoil, spoil
     out = torch.full((n, H * 128), float("nan"), dtype=torch.bfloat16, device=DEV)
     attention_fast.run_made(q, kv, rope, torch.from_numpy(items).to(DEV), out, H, window, 192 ** -0.5, c, w[:, 128:].contiguous(),
                             torch.from_numpy(firsts).to(DEV))
@@ -54,3 +58,69 @@ def test_a_window_that_leaves_out_the_first_positions(span, window):
     # the first positions: values that are never rounded, so half a unit of the result and float32 sums
     early = pos < attention_fast.MADE_FIRST
     assert bool(((got - want).abs()[early] <= 2.0 ** -8 * want.abs()[early] + 1e-4 * scale).all())
+
+
+def tiled(*args):
+    from hk_b200.csrc import attention_fast
+    return attention_fast.made_items(*args, attention_fast.MADE_TILE)
+
+
+NEIGHBOURS = [([(0, 70), (0, 200), (0, 65)], 0), ([(0, 129), (37, 127), (200, 300)], 0), ([(300, 90), (0, 257), (5, 64)], 50),
+              ([(700, 129), (15, 64), (140, 70)], 130), ([(15, 64), (16, 64), (3, 70)], 7)]
+
+
+@pytest.mark.parametrize("spans,window", NEIGHBOURS)
+@pytest.mark.parametrize("spoil", [float("nan"), float("inf")])
+def test_a_request_that_is_not_finite_leaves_the_others_alone(spans, window, spoil):
+    clean, want, _ = made_case(spans, window, tiled, tile=128)
+    scale = float(want.abs().max())
+    assert float((clean - want).abs().max()) <= 3e-2 * scale       # probabilities and values in bfloat16
+    ends = np.cumsum([n for _, n in spans]).tolist()
+    for bad, (cached, n) in enumerate(spans):
+        rows = cached + n - max(0, cached - window + 1 if window else 0)
+        got, _, _ = made_case(spans, window, tiled, tile=128, spoilt=[(bad, i) for i in range(rows)], spoil=spoil)
+        own = slice(ends[bad] - n, ends[bad])
+        assert not bool(torch.isfinite(got[own]).any())
+        got[own] = clean[own]
+        assert torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("spans,window", NEIGHBOURS)
+def test_neighbours_in_a_step_of_the_part(spans, window):
+    """The same through `LatentAttention`: a request whose inputs are NaN and Inf, the others' results equal to the bit."""
+    from test_latent_made_gpu import part_of, run
+    from test_parts_gpu import bind_random
+    part = part_of(2, 64, 512, window or None)
+    prec, _ = bind_random(part, torch.bfloat16, std=0.08)
+    rows = [torch.randn(c + n, 192, device=DEV).to(torch.bfloat16) for c, n in spans]
+    clean, _ = run(part, prec, rows, spans, 64)
+    assert bool(torch.isfinite(clean).all())
+    ends = np.cumsum([n for _, n in spans]).tolist()
+    for bad, (_, n) in enumerate(spans):
+        spoilt = [x.clone() for x in rows]
+        spoilt[bad][::2], spoilt[bad][1::2] = float("nan"), float("inf")
+        got, _ = run(part, prec, spoilt, spans, 64)
+        own = slice(ends[bad] - n, ends[bad])
+        assert not bool(torch.isfinite(got[own]).any())
+        got[own] = clean[own]
+        assert torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("tile", [1, 128])
+@pytest.mark.parametrize("dr", [0, 8])
+def test_latent_rows_fill_up_their_tiles(tile, dr):
+    from hk_b200.csrc import attention_fast, ops
+    spans, r, pt = [(0, 127), (300, 90), (130, 129), (5, 123), (0, 128)], 16, 16
+    per = 32
+    pages = torch.randn(per * len(spans), 1, pt, r + dr, device=DEV).bfloat16()
+    table = torch.randperm(per * len(spans)).int().view(len(spans), per).to(DEV)
+    lens = [n for _, n in spans]
+    _, segments, _, rows = attention_fast.made_items(range(len(spans)), np.cumsum([0] + lens[:-1]).tolist(), lens, [c for c, _ in spans], 50, tile)
+    c = torch.full((rows, r), float("nan"), dtype=torch.bfloat16, device=DEV)
+    rope = torch.full((rows, dr), float("nan"), dtype=torch.bfloat16, device=DEV) if dr else None
+    ops.latent_rows(pages, table, torch.from_numpy(segments).to(DEV), int(segments[:, 2].max()), c, rope, tile)
+    want = torch.zeros(rows, r + dr, dtype=torch.bfloat16, device=DEV)
+    for slot, first, count, row in segments.tolist():
+        pos = torch.arange(first, first + count, device=DEV)
+        want[row:row + count] = pages[table[slot, pos // pt].long(), 0, pos % pt]
+    assert torch.equal(torch.cat([c, rope], dim=1) if dr else c, want)
