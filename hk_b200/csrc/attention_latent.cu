@@ -732,10 +732,11 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
   }
   __syncthreads();
   for (int e = tid; e < FIRST_ROWS * (r / 8); e += 256) {     // their sums in the latent space
-    const int i = e / (r / 8), p = (e % (r / 8)) * 8;
+    const int i = e / (r / 8), p = (e % (r / 8)) * 8, pos = f.pos0 + i;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    // over the keys that the row sees: a later one may be NaN or Inf, which a probability of zero would not keep out
 #pragma unroll 4
-    for (int j = 0; j < FIRST_ROWS; ++j) {
+    for (int j = window > 0 ? max(0, pos - window + 1) : 0; j <= min(pos, FIRST_ROWS - 1); ++j) {
       float x[8];
       halves(*reinterpret_cast<const uint4*>(cs + j * ldc + p), x);
 #pragma unroll

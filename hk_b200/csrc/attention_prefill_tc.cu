@@ -619,6 +619,57 @@ struct Smem2 {
   int pages[1];        // [pages_cap]
 };
 
+// A made row (below) whose sums came out NaN or Inf, once more over the keys [lo, pos] that it sees, by one warp: the tensor
+// core's product takes whole tiles of values, and a NaN or Inf among those that the row does not see (later tokens of its request)
+// would not be kept out by their probability of zero.  `row0`: the request's position 0, of `ld` numbers a row.
+template <int HDK>
+__device__ __noinline__ void made_row_again(const bf16* q, const bf16* row0, size_t ld, const bf16* rope0, int lo, int pos, float scale_log2,
+                                            float factor, const float* gate, float gate_scale, bf16* out) {
+  const int lane = threadIdx.x & 31;
+  auto dot8 = [](const bf16* a, const bf16* b, float s) {
+    const uint4 x = *reinterpret_cast<const uint4*>(a), y = *reinterpret_cast<const uint4*>(b);
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      s = fmaf(__uint_as_float(xs[e] << 16), __uint_as_float(ys[e] << 16), s);
+      s = fmaf(__uint_as_float(xs[e] & 0xffff0000u), __uint_as_float(ys[e] & 0xffff0000u), s);
+    }
+    return s;
+  };
+  float m = -CUDART_INF_F, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int j0 = lo; j0 <= pos; j0 += 32) {
+    const int j = j0 + lane;
+    float s = -CUDART_INF_F;
+    if (j <= pos) {
+      s = 0.f;
+      for (int d = 0; d < 128; d += 8) s = dot8(q + d, row0 + (size_t)j * ld + d, s);
+      for (int d = 128; d < HDK; d += 8) s = dot8(q + d, rope0 + (size_t)j * 64 + d - 128, s);
+      s *= scale_log2;
+    }
+    const float mn = fmaxf(m, warp_max(s)), safe = mn == -CUDART_INF_F ? 0.f : mn;
+    const float corr = exp2f(m - safe), p = j <= pos ? exp2f(s - safe) : 0.f;
+    l = fmaf(l, corr, warp_sum(p));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] *= corr;
+    for (int i = 0; i < min(32, pos - j0 + 1); ++i) {
+      const float w = __shfl_sync(0xffffffffu, p, i);
+      const uint2 v = *reinterpret_cast<const uint2*>(row0 + (size_t)(j0 + i) * ld + 128 + 4 * lane);
+      acc[0] = fmaf(w, __uint_as_float(v.x << 16), acc[0]);
+      acc[1] = fmaf(w, __uint_as_float(v.x & 0xffff0000u), acc[1]);
+      acc[2] = fmaf(w, __uint_as_float(v.y << 16), acc[2]);
+      acc[3] = fmaf(w, __uint_as_float(v.y & 0xffff0000u), acc[3]);
+    }
+    m = mn;
+  }
+  const float inv = (l > 0.f ? 1.0f / l : 0.f) * factor;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float y = acc[e] * inv;
+    if (gate) y *= gate_scale / (1.0f + __expf(-gate[4 * lane + e]));
+    out[4 * lane + e] = __float2bfloat16_rn(y);
+  }
+}
+
 // DIST: with a bias by distance (an instance of its own, so that the softmax of a model without one issues nothing for it)
 // MADE: keys and values made for the step from a compressed cache (a latent attention's prompt portions), not pages: every
 // query head has its own (H == G); a request's rows stand side by side, the row of position 0 at item.slot (which may lie
@@ -630,7 +681,8 @@ __global__ void __launch_bounds__(NT2, 1)
 attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                              const __grid_constant__ CUtensorMap map_r, const bf16* __restrict__ q, const int* __restrict__ block_table, int table_stride,
                              const Item* __restrict__ items, bf16* __restrict__ out, int H, int G, int page_tokens, int window,
-                             float scale_log2, ScoreOpts so, int pages_cap, int* __restrict__ status) {
+                             float scale_log2, ScoreOpts so, int pages_cap, int* __restrict__ status, const bf16* __restrict__ made,
+                             const bf16* __restrict__ made_rope) {
   constexpr int CPR = HDK / 8;
   constexpr int KSTEPS = HDK / 16;
   constexpr int HALVES = HD / 64, KHALVES = HDK / 64;
@@ -930,20 +982,35 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
         tc_fence_after();
         float l = l0 + l1;
         if (so.sink && valid) l += exp2f((so.sinks ? so.sinks[g * group + row % group] * 1.4426950408889634f : 0.f) - m);
-        float inv = l > 0.f ? 1.0f / l : 0.f;
+        float inv = l > 0.f ? 1.0f / l : 0.f, factor = 1.0f;
         const int out_row = it.q_row0 + (valid ? tq : 0), out_head = g * group + (valid ? row % group : 0);
         bf16* op = out + ((size_t)out_row * H + out_head) * HD;
         const float* gp = so.gate && !so.gate_heads ? so.gate + (size_t)out_row * so.gate_ld + (size_t)out_head * HD : nullptr;
-        if (MADE && so.gate && so.gate_heads) inv *= so.gate_scale / (1.0f + __expf(-so.gate[(size_t)out_row * so.gate_ld + out_head]));
+        if (MADE && so.gate && so.gate_heads) {
+          factor = so.gate_scale / (1.0f + __expf(-so.gate[(size_t)out_row * so.gate_ld + out_head]));
+          inv *= factor;
+        }
         // the whole row of O at once (the registers that held scores are free now): one wait instead of HD / 32
         uint32_t o[HD];
 #pragma unroll
         for (int c0 = 0; c0 < HD; c0 += 32) tmem_ld32(lane_addr + O_COL[qt] + (uint32_t)c0, o + c0);
         tmem_ld_wait();
-        if (valid) {
+        float z = 0.f;                                    // NaN where a sum is NaN or Inf
+        if (MADE)
+#pragma unroll
+          for (int i = 0; i < HD; ++i) z = fmaf(__uint_as_float(o[i]), 0.f, z);
+        if (valid && z == 0.f) {
 #pragma unroll
           for (int i = 0; i < HD; i += 8)
             *reinterpret_cast<uint4*>(op + i) = finish8(o + i, inv, gp ? gp + i : nullptr, so.gate_scale);
+        }
+        for (unsigned again = MADE ? __ballot_sync(0xffffffffu, valid && z != 0.f) : 0u; again; again &= again - 1) {
+          const int from = __ffs(again) - 1, p = __shfl_sync(0xffffffffu, pos, from), at = __shfl_sync(0xffffffffu, out_row, from);
+          const size_t cell = (size_t)at * H + g;          // a head of its own each: group 1
+          made_row_again<HDK>(q + cell * HDK, made + ((long long)it.slot * H + g) * 256, (size_t)H * 256, made_rope + (long long)it.slot * 64,
+                              __shfl_sync(0xffffffffu, lo, from), p, scale_log2, __shfl_sync(0xffffffffu, factor, from),
+                              so.gate && !so.gate_heads ? so.gate + (size_t)at * so.gate_ld + (size_t)g * HD : nullptr, so.gate_scale,
+                              out + cell * HD);
         }
       }
     }
@@ -992,14 +1059,14 @@ bool make_page_map(CUtensorMap* map, const void* ptr, unsigned long long rows, i
 template <int HD, bool DIST, int HDK = HD, bool MADE = false>
 int launch2(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, const int* bt, int stride, const void* items, int n_items,
             void* out, int H, int G, int pt, int window, float scale_log2, ScoreOpts so, int pages_cap, int* status, cudaStream_t s,
-            const CUtensorMap* mr = nullptr) {
+            const CUtensorMap* mr = nullptr, const void* made = nullptr, const void* made_rope = nullptr) {
   const size_t smem = sizeof(Smem2<HD, HDK>) + 1024 + (size_t)pages_cap * sizeof(int);
   if (smem > (MADE ? 227 : 225) * 1024) return HK_ERR_UNSUPPORTED;
   static HkSmemCache allowed = {};
   if (int e = hk_allow_smem(attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>, smem, allowed)) return e;
   dim3 grid((unsigned)n_items * (unsigned)G);
   return hk_launch(attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>, grid, dim3(NT2), smem, s, mk, mv, mr ? *mr : mk, (const bf16*)q, bt, stride,
-                   (const Item*)items, (bf16*)out, H, G, pt, window, scale_log2, so, pages_cap, status);
+                   (const Item*)items, (bf16*)out, H, G, pt, window, scale_log2, so, pages_cap, status, (const bf16*)made, (const bf16*)made_rope);
 }
 
 ScoreOpts make_opts(int sink, const float* sinks, float softcap, float scale_log2, int chunk, const float* gate, long long gate_ld,
@@ -1087,6 +1154,7 @@ HK_API int hk_attention_prefill_made(const void* q, const void* kv, const void* 
   if (rope != nullptr && !make_page_map(&mr, rope, (unsigned long long)rows, 64, TK)) return HK_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
   if (rope != nullptr)
-    return launch2<128, false, 192, true>(mk, mk, q, nullptr, 0, items, n_items, out, H, H, TK, window, scale_log2, so, 0, status, s, &mr);
-  return launch2<128, false, 128, true>(mk, mk, q, nullptr, 0, items, n_items, out, H, H, TK, window, scale_log2, so, 0, status, s);
+    return launch2<128, false, 192, true>(mk, mk, q, nullptr, 0, items, n_items, out, H, H, TK, window, scale_log2, so, 0, status, s, &mr, kv, rope);
+  return launch2<128, false, 128, true>(mk, mk, q, nullptr, 0, items, n_items, out, H, H, TK, window, scale_log2, so, 0, status, s, nullptr, kv,
+                                        nullptr);
 }

@@ -1,5 +1,6 @@
 """The two kernels over keys and values made for a step (`attention_fast.run_made`), on arrays whose every row outside a request's
-own is NaN: against the softmax in float64, windows shorter than a request's first rows among them."""
+own is NaN: against the softmax in float64, windows shorter than a request's first rows among them.  And what a row of the cache that
+holds NaN or Inf does to other requests of the step, and to rows of its own request that do not see it: nothing."""
 import numpy as np
 import pytest
 import torch
@@ -9,7 +10,7 @@ DEV = "cuda"
 H, R, DR, GUARD = 2, 64, 64, 256
 
 
-def made_case(spans, window, layout, seed=0, tile=1, spoilt=(), spoil=float("nan")):
+def made_case(spans, window, layout, seed=0, tile=1, spoilt=(), spoil=float("nan"), gate=None, dr=DR):
     """(out of `run_made`, the same in float64, positions): spans (cached, new) of requests whose rows lie as `layout` says, the rest
     of their tiles zeros; `spoilt` = (request, row of its own) whose cache row and values are `spoil`."""
     from hk_b200.csrc import attention_fast, gemm_fast
@@ -22,28 +23,31 @@ def made_case(spans, window, layout, seed=0, tile=1, spoilt=(), spoil=float("nan
     def guarded(width):
         """A matrix of `rows` rows, NaN, inside one with NaN on both sides."""
         return torch.full((GUARD + rows + GUARD, width), float("nan"), dtype=torch.bfloat16, device=DEV)[GUARD:GUARD + rows]
-    c, rope, kv = guarded(R), guarded(DR), guarded(H * 256)
+    c, rope, kv = guarded(R), guarded(dr), guarded(H * 256)
     w = (rand(H, 256, R) * R ** -0.5).bfloat16()
     n = sum(lens)
-    q, want, pos = (rand(n, H * 192) * 0.5).bfloat16(), torch.empty(n, H, 128, dtype=torch.float64), []
+    q, want, pos = (rand(n, H * (128 + dr)) * 0.5).bfloat16(), torch.empty(n, H, 128, dtype=torch.float64), []
     for (_, first, count, row0), qs, ql, p0 in zip(segments.tolist(), q_starts, lens, starts):
         part, whole = slice(row0, row0 + count), slice(row0 // tile * tile, -(-(row0 + count) // tile) * tile)
         c[whole], rope[whole], kv[whole] = 0.0, 0.0, 0.0
-        c[part], rope[part] = rand(count, R).bfloat16(), rand(count, DR).bfloat16()
+        c[part], rope[part] = rand(count, R).bfloat16(), rand(count, dr).bfloat16()
         kv[part] = (c[part].float() @ w.float().flatten(0, 1).t()).bfloat16()
-        keys = torch.cat([kv[part].view(count, H, 256)[..., :128], rope[part][:, None].expand(count, H, DR)], dim=2).double()
+        keys = torch.cat([kv[part].view(count, H, 256)[..., :128], rope[part][:, None].expand(count, H, dr)], dim=2).double()
         values = torch.einsum("tr,hvr->thv", c[part].double(), w[:, 128:].double())
         for i in range(ql):
             p, lo = p0 + i, max(0, p0 + i - window + 1) if window else 0
             see = slice(lo - first, p + 1 - first)
-            s = torch.einsum("hd,thd->ht", q[qs + i].view(H, 192).double(), keys[see]) * 192 ** -0.5
+            s = torch.einsum("hd,thd->ht", q[qs + i].view(H, 128 + dr).double(), keys[see]) * 192 ** -0.5
             want[qs + i] = torch.einsum("ht,thv->hv", torch.softmax(s, dim=1), values[see]).cpu()
             pos.append(p)
     for request, own in spoilt:
         c[segments[request][3] + own], kv[segments[request][3] + own] = spoil, spoil
     out = torch.full((n, H * 128), float("nan"), dtype=torch.bfloat16, device=DEV)
-    attention_fast.run_made(q, kv, rope, torch.from_numpy(items).to(DEV), out, H, window, 192 ** -0.5, c, w[:, 128:].contiguous(),
-                            torch.from_numpy(firsts).to(DEV))
+    logits = rand(n, H if gate == "head" else H * 128) if gate else None
+    if gate:
+        want *= 0.7 * torch.sigmoid(logits.double().cpu().view(n, H, -1))
+    attention_fast.run_made(q, kv, rope if dr else None, torch.from_numpy(items).to(DEV), out, H, window, 192 ** -0.5, c, w[:, 128:].contiguous(),
+                            torch.from_numpy(firsts).to(DEV), logits, gate == "head", 0.7)
     gemm_fast.check_status(torch.device(DEV, 0))
     return out.double().cpu().view(n, H, 128), want, np.asarray(pos)
 
@@ -124,3 +128,18 @@ def test_latent_rows_fill_up_their_tiles(tile, dr):
         pos = torch.arange(first, first + count, device=DEV)
         want[row:row + count] = pages[table[slot, pos // pt].long(), 0, pos % pt]
     assert torch.equal(torch.cat([c, rope], dim=1) if dr else c, want)
+
+
+@pytest.mark.parametrize("spans,window,gate,dr", [([(0, 70)], 0, None, 64), ([(0, 300), (37, 127)], 0, "each", 64), ([(300, 90), (0, 257)], 50, "head", 64),
+                                                  ([(15, 64), (3, 400)], 7, "each", 0), ([(0, 129)], 0, "head", 0)])
+@pytest.mark.parametrize("at", [0.0, 0.04, 0.5, 1.0])
+def test_rows_that_see_only_finite_rows_stay_finite(spans, window, gate, dr, at):
+    """One position of every request holds NaN: the rows before it, and those that it has left the window of, are as they were."""
+    places = [min(cached + n - 1, (max(0, cached - window + 1) if window else 0) + int(at * (cached + n))) for cached, n in spans]
+    spoilt = [(i, p - (max(0, cached - window + 1) if window else 0)) for i, (p, (cached, _)) in enumerate(zip(places, spans))]
+    got, want, pos = made_case(spans, window, tiled, tile=128, spoilt=spoilt, gate=gate, dr=dr)
+    place = np.concatenate([np.full(n, p) for p, (_, n) in zip(places, spans)])
+    sees = torch.from_numpy((place <= pos) & ((place > pos - window) if window else True))
+    scale = float(want.abs().max())
+    assert not bool(torch.isfinite(got[sees]).any()) and bool(torch.isfinite(got[~sees]).all())
+    assert bool(((got - want).abs()[~sees] <= 3e-2 * scale).all())       # probabilities and values in bfloat16
