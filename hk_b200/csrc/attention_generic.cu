@@ -26,6 +26,8 @@
 // warp per position, online softmax); scale on q first: src/engine/attention_kernel.zig:109.
 #include <math_constants.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 #define AG_WARPS 4
@@ -169,7 +171,9 @@ HK_API int hk_attention_generic(const void* q, const void* k_pages, const void* 
 // position of the first} for one key/value head, 32 rows = (token, head of the group) pairs, so 64 keys at a time are read once
 // for all of them.  Scores and sums are register tiles of multiply-adds over 16-byte loads of shared memory (4 x 4 scores a thread
 // along the head's dims, 4 x 8 sums); the next tile's keys arrive while this one's probabilities are made, the next values while
-// the next scores are.  Every option of the kernel above.  A row's result is the same to the bit whatever run it stands in.  Up
+// the next scores are.  Every option of the kernel above.  A row's result is the same to the bit whatever run it stands in, also
+// beside rows that are not finite: a tile with keys that some row does not see looks for NaN and Inf among its values (a
+// probability of zero would not keep them out) and, if there are any, adds for every row the keys that it sees alone.  Up
 // to 8 rows (single tokens) do a quarter of the arithmetic.  Bound by what shared memory delivers (two thirds of the fp32 rate).
 // 16 heads of 128 over 8, us, the kernel above and this: 509 tokens 484 and 132; single tokens behind 2,000: one 415 and 357, 64 (32
 // heads) 1,697 and 877; 2,048 tokens of 32 heads 13,658 and 2,009.
@@ -299,30 +303,49 @@ __device__ __forceinline__ void attention_f32_item(AfSmem& sm, const AfItem it, 
       if ((tid & 3) == 0) sm.corr[sr] = corr;
     }
     asm volatile("cp.async.wait_group 1;" ::: "memory");          // the values
-    __syncthreads();
+    float odd = 0.f;                                              // NaN with NaN or Inf among the pieces that this thread fetched
+    if (j0 < first_key(it.pos0 + it.n_tokens - 1) || j0 + AF_KEYS - 1 > it.pos0) {
+#pragma unroll 4
+      for (int e = tid; e < AF_KEYS * (AF_HD / 4); e += AF_TH) {
+        const float4 x = *reinterpret_cast<const float4*>(sm.v + (e / (AF_HD / 4)) * AF_LD + (e % (AF_HD / 4)) * 4);
+        odd = fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, fmaf(x.w, 0.f, odd))));
+      }
+    }
+    const bool apart = __syncthreads_or(odd != 0.f);
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const float c = sm.corr[ty + 8 * i];
 #pragma unroll
       for (int b = 0; b < 2; ++b) acc[i][b] = make_float4(acc[i][b].x * c, acc[i][b].y * c, acc[i][b].z * c, acc[i][b].w * c);
     }
+    const int c_end = min(AF_KEYS, kv_hi - j0);                   // behind the last row's own key there is nothing
+    auto add = [&](auto seen_alone) {
 #pragma unroll 2
-    for (int c = 0; c < AF_KEYS; c += 4) {
-      float4 p[RI];
+      for (int c = 0; c < c_end; c += 4) {
+        float4 p[RI];
 #pragma unroll
-      for (int i = 0; i < RI; ++i) p[i] = *reinterpret_cast<const float4*>(sm.p + (ty + 8 * i) * AF_LDP + c);
+        for (int i = 0; i < RI; ++i) p[i] = *reinterpret_cast<const float4*>(sm.p + (ty + 8 * i) * AF_LDP + c);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float4 v0 = *reinterpret_cast<const float4*>(sm.v + (c + e) * AF_LD + 4 * tx);
-        const float4 v1 = *reinterpret_cast<const float4*>(sm.v + (c + e) * AF_LD + 64 + 4 * tx);
+        for (int e = 0; e < 4; ++e) {
+          const float4 v0 = *reinterpret_cast<const float4*>(sm.v + (c + e) * AF_LD + 4 * tx);
+          const float4 v1 = *reinterpret_cast<const float4*>(sm.v + (c + e) * AF_LD + 64 + 4 * tx);
 #pragma unroll
-        for (int i = 0; i < RI; ++i) {
-          const float w = e == 0 ? p[i].x : e == 1 ? p[i].y : e == 2 ? p[i].z : p[i].w;
-          acc[i][0] = make_float4(fmaf(w, v0.x, acc[i][0].x), fmaf(w, v0.y, acc[i][0].y), fmaf(w, v0.z, acc[i][0].z), fmaf(w, v0.w, acc[i][0].w));
-          acc[i][1] = make_float4(fmaf(w, v1.x, acc[i][1].x), fmaf(w, v1.y, acc[i][1].y), fmaf(w, v1.z, acc[i][1].z), fmaf(w, v1.w, acc[i][1].w));
+          for (int i = 0; i < RI; ++i) {
+            if (decltype(seen_alone)::value) {
+              const int key = j0 + c + e, pos = it.pos0 + (ty + 8 * i) / group;
+              if (key > pos || key < first_key(pos)) continue;
+            }
+            const float w = e == 0 ? p[i].x : e == 1 ? p[i].y : e == 2 ? p[i].z : p[i].w;
+            acc[i][0] = make_float4(fmaf(w, v0.x, acc[i][0].x), fmaf(w, v0.y, acc[i][0].y), fmaf(w, v0.z, acc[i][0].z), fmaf(w, v0.w, acc[i][0].w));
+            acc[i][1] = make_float4(fmaf(w, v1.x, acc[i][1].x), fmaf(w, v1.y, acc[i][1].y), fmaf(w, v1.z, acc[i][1].z), fmaf(w, v1.w, acc[i][1].w));
+          }
         }
       }
-    }
+    };
+    if (apart)
+      add(std::true_type{});
+    else
+      add(std::false_type{});
     __syncthreads();
     if (t + 1 < tiles) fetch(v_pages, sm.v, t + 1, vd, opt.v_stride);
     else asm volatile("cp.async.commit_group;" ::: "memory");
