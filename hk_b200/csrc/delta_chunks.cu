@@ -19,6 +19,9 @@
 // channel (generalised delta rule) rows are scaled by P_t and 1 / P_s, which holds while a chunk's decay stays above 2^-64
 // (the launcher's condition on decay_scale).
 //
+// A value, key, gate or decay that is NaN or Inf reaches its own token and later ones, as in the walk: the products with triangular
+// matrices leave out what stands above the diagonal (`triangle_rows`), which a zero there would not keep out.
+//
 // One request of 2,048 tokens at 64 heads of 64 x 64 (walk token by token -> here): generalised rule 994 -> 435 us, gated rule
 // 989 -> 405, matrix memory 1,089 -> 296, retention 607 -> 211; of 1,000 at 32 heads 392 -> 144, 390 -> 138, 428 -> 111,
 // 241 -> 68; of 64 tokens level (39 -> 38, 42 -> 35, 57 -> 52, 30 -> 30), of 128 61 -> 38, 61 -> 38, 78 -> 54, 42 -> 31.
@@ -71,6 +74,32 @@ __device__ __forceinline__ void fma4(float4& c, float a, float4 b) {
   c.y = fmaf(a, b.y, c.y);
   c.z = fmaf(a, b.z, c.z);
   c.w = fmaf(a, b.w, c.w);
+}
+
+// acc[i] (N rows, row i's token ty + 8 (i & 3)) += sign * a[row i, s] * b[s, :] over the tokens s below limit(i), a row's own at most:
+// `a` row ty + 8 i with ROWS floats between rows, `b` four columns with LD between tokens.  The two values of ty in a warp lie
+// in one group of four tokens, so a warp skips the groups above the diagonal as one, half of all.
+template <int N, int ROWS, int SIGN, int NB, typename Limit>
+__device__ __forceinline__ void triangle_rows(float4 (&acc)[NB][N], const float* a, const float* (&b)[NB], int ty, Limit limit) {
+#pragma unroll 2
+  for (int s = 0; s < CQ; s += 4) {
+    float4 x[NB][4];
+#pragma unroll
+    for (int n = 0; n < NB; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[n][j] = ld4(b[n] + (s + j) * LD);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int end = limit(i);
+      if (s >= (end + 3 & ~3)) continue;
+      const float4 w = ld4(a + (ty + 8 * i) * ROWS + s);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (s + j < end)
+#pragma unroll
+          for (int n = 0; n < NB; ++n) fma4(acc[n][i], SIGN * at4(w, j), x[n][j]);
+    }
+  }
 }
 
 // The products of a chunk's decays, one number g[t] per token: gam[t][s] = g[s + 1] .. g[t] for s <= t (0 above), `from` [CQ]
@@ -207,7 +236,7 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
     float p = 1.f;
     if (tid < 64) {
 #pragma unroll 8
-      for (int t = 0; t < CQ; ++t) {
+      for (int t = 0; t < ch.count; ++t) {
         const float d = sm.a[t * LD + i];
         sm.ur[t * LD + i] *= p;
         p *= d;
@@ -216,7 +245,7 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
       sm.pc[i] = p;
     } else {
 #pragma unroll 8
-      for (int t = 0; t < CQ; ++t) {
+      for (int t = 0; t < ch.count; ++t) {
         p *= sm.a[t * LD + i];
         const float b = 1.0f / p;
         sm.ka[t * LD + i] *= b;
@@ -256,12 +285,12 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
         const int s = tx + 16 * (j & 1);
-        const bool in_tri = read ? s <= t : s < t;
+        const bool in_tri = (read ? s <= t : s < t) && t < ch.count;
         float x = in_tri ? pair_sum(acc[i][j]) : 0.f;
         float* dst = sm.a + (ty + 8 * i) * LD + tx + 16 * j;
         if (GATED) {
           x *= in_tri ? sm.w[(read ? t : t - 1) * LD + s] : 0.f;
-          dst[CQ] = x * sm.gb[s];
+          dst[CQ] = in_tri ? x * sm.gb[s] : 0.f;
         }
         *dst = x;
       }
@@ -284,27 +313,17 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
 
   // ---- [Auk ; Ark] V
   {
-    float4 acc[8];
+    float4 acc[1][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = zero;
-#pragma unroll 2
-    for (int s = 0; s < CQ; s += 4) {
-      float4 b[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ld4(sm.vs + (s + j) * LD + 4 * tx);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 a = ld4(sm.a + (ty + 8 * i) * LD + s);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) fma4(acc[i], at4(a, j), b[j]);
-      }
-    }
+    for (int i = 0; i < 8; ++i) acc[0][i] = zero;
+    const float* v[1] = {sm.vs + 4 * tx};
+    triangle_rows<8, LD, 1>(acc, sm.a, v, ty, [&](int i) { return ty + 8 * (i & 3) + (i >= 4 ? 1 : 0); });
     __syncthreads();            // everyone has read the k columns of the matrices
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int t = ty + 8 * i;
-      st4(sm.w + t * LD + 4 * tx, acc[i]);
-      st4(sm.a + (t + (tx >= 8 ? CQ : 0)) * LD + 4 * (tx & 7), acc[4 + i]);
+      st4(sm.w + t * LD + 4 * tx, acc[0][i]);
+      st4(sm.a + (t + (tx >= 8 ? CQ : 0)) * LD + 4 * (tx & 7), acc[0][4 + i]);
     }
   }
   __syncthreads();
@@ -338,36 +357,20 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
   const int col0 = blockIdx.y * NT, ncols = min(NT, dv - col0);
   // ---- Rq = R~ - Aru X,  Ov = Ark V - Aru W
   {
-    float4 r[4], o[4];
+    float4 ro[2][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int t = ty + 8 * i;
-      r[i] = ld4(sm.ur + (CQ + t) * LD + 4 * tx);
-      o[i] = ld4(sm.a + (t + (tx >= 8 ? CQ : 0)) * LD + 4 * (tx & 7));
+      ro[0][i] = ld4(sm.ur + (CQ + t) * LD + 4 * tx);
+      ro[1][i] = ld4(sm.a + (t + (tx >= 8 ? CQ : 0)) * LD + 4 * (tx & 7));
     }
-#pragma unroll 2
-    for (int s = 0; s < CQ; s += 4) {
-      float4 x[4], w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        x[j] = ld4(sm.ur + (s + j) * LD + 4 * tx);
-        w[j] = ld4(sm.w + (s + j) * LD + 4 * tx);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 a = ld4(sm.a + (CQ + ty + 8 * i) * LD + CQ + s);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          fma4(r[i], -at4(a, j), x[j]);
-          fma4(o[i], -at4(a, j), w[j]);
-        }
-      }
-    }
+    const float* xw[2] = {sm.ur + 4 * tx, sm.w + 4 * tx};
+    triangle_rows<4, LD, -1>(ro, sm.a + CQ * LD + CQ, xw, ty, [&](int i) { return ty + 8 * i + 1; });
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int t = ty + 8 * i;
-      if (blockIdx.y == 0) st4(rq + (item * CQ + t) * NT + 4 * tx, r[i]);
-      if (t < ch.count && 4 * tx < ncols) st4(out + ((size_t)(ch.row0 + t) * H + h) * dv + col0 + 4 * tx, o[i]);
+      if (blockIdx.y == 0) st4(rq + (item * CQ + t) * NT + 4 * tx, ro[0][i]);
+      if (t < ch.count && 4 * tx < ncols) st4(out + ((size_t)(ch.row0 + t) * H + h) * dv + col0 + 4 * tx, ro[1][i]);
     }
   }
   // ---- M = -AU'^T X and P,  B = K'^T V - AU'^T W
@@ -662,32 +665,30 @@ decay_out_kernel(const DecayIn in, const Chunk* __restrict__ chunks, const float
       }
       continue;
     }
-    float4 o[4], y[4];
+    float4 o[1][4], y[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto products = [&](const float* a, int lda, const float* b, int inner, float4* acc) {
+    for (int i = 0; i < 4; ++i) o[0][i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* values[1] = {sm.vs + 4 * tx};
+    triangle_rows<4, LA, 1>(o, sm.a, values, ty, [&](int i) { return ty + 8 * i + 1; });
 #pragma unroll 2
-      for (int s = 0; s < inner; s += 4) {
-        float4 v[4];
+    for (int s = 0; s < NT; s += 4) {
+      float4 v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = ld4(b + (s + j) * LD + 4 * tx);
+      for (int j = 0; j < 4; ++j) v[j] = ld4(sm.st + (s + j) * LD + 4 * tx);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 x = ld4(a + (ty + 8 * i) * lda + s);
+      for (int i = 0; i < 4; ++i) {
+        const float4 x = ld4(sm.q + (ty + 8 * i) * LD + s);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) fma4(acc[i], at4(x, j), v[j]);
-        }
+        for (int j = 0; j < 4; ++j) fma4(y[i], at4(x, j), v[j]);
       }
-    };
-    products(sm.a, LA, sm.vs, CQ, o);
-    products(sm.q, LD, sm.st, NT, y);
+    }
     if (4 * tx < ncols)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int t = ty + 8 * i;
         if (t < ch.count)
           st4(out + ((size_t)(ch.row0 + t) * H + h) * dvp + col0 + 4 * tx,
-              make_float4(o[i].x + y[i].x, o[i].y + y[i].y, o[i].z + y[i].z, o[i].w + y[i].w));
+              make_float4(o[0][i].x + y[i].x, o[0][i].y + y[i].y, o[0][i].z + y[i].z, o[0][i].w + y[i].w));
       }
   }
 }

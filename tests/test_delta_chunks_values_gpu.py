@@ -1,0 +1,78 @@
+"""The recurrences in chunks of tokens on values that are no ordinary numbers, against the walk token by token over the same inputs: what
+is NaN or Inf at a token reaches that token and later ones, the columns and requests that it reaches in the walk and no others."""
+import math
+
+import pytest
+import torch
+
+from test_delta_chunks_gpu import DEV, tables
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(kind, H, dk, dv, lengths, g):
+    from hk_b200.csrc import ops
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)       # noqa: E731
+    n, R, K, V = sum(lengths), len(lengths), H * dk, H * dv
+    dvp = ops.mlstm_padded(dv) if kind == "memory" else dv
+    t = {"proj": rand(n, 3 * K + V + 4 * H), "state": rand(R, H, dk, dvp), "m": rand(R, H), "bias": rand(2 * K) - 1.0, "wl": rand(n, K)}
+    if kind == "memory":
+        t["state"][..., dv + 1:] = 0.0
+    return t
+
+
+def scan(kind, H, dk, dv, lengths, t, first_chunked, eps=1e-6):
+    """(out, state) with the requests from `first_chunked` on in chunks."""
+    from hk_b200.csrc import ops
+    short, long, chunks, requests = tables(lengths, first_chunked)
+    more = {"chunks": chunks, "requests": requests, "most_rows": max(lengths)} if first_chunked < len(lengths) else {}
+    n, K, V, p, state = sum(lengths), H * dk, H * dv, t["proj"], t["state"].clone()
+    q, k, v, x, logits = p[:, :K], p[:, K:2 * K], p[:, 2 * K:2 * K + V], p[:, 2 * K + V:3 * K + V], p[:, 3 * K + V:]
+    out = torch.full((n, H * state.shape[3]), 7.0, device=DEV)
+    if kind == "general":
+        ops.delta_rule_scan(q, k, v, x, t["wl"], t["bias"][:K], t["bias"][K:], short, state, out, H, dk, dv, math.exp(-0.5), eps, **more)
+    elif kind == "gated":
+        ops.gated_delta_scan(q, k, v, logits[:, :H], logits[:, H:2 * H], t["bias"][:H].abs(), t["bias"][H:2 * H], short, state, out, H, H, dk, dv,
+                             dk ** -0.5, eps, **more)
+    elif kind == "retention":
+        pos = torch.cat([torch.arange(c) for c in lengths]).int().to(DEV)
+        angle = torch.arange(max(lengths), device=DEV)[:, None] * torch.rand(1, 2, generator=torch.Generator(DEV).manual_seed(1), device=DEV)
+        ops.retention_scan(q, k, v, angle.cos(), angle.sin(), 4, pos, 1 - t["bias"][:H].abs() * 0.05, short, state, out, H, dk, dv, 0.3, **more)
+    else:
+        gates = torch.empty(n, H, 3, device=DEV)
+        ops.mlstm_scan(q, k, v, logits[:, :H], logits[:, H:2 * H], t["bias"][:H], t["bias"][H:2 * H] + 4, short, state, t["m"].clone(), out, gates,
+                       H, dk, dv, 15.0, 0.5, **({**more, "long_segments": long} if more else {}))
+    return out, state
+
+
+def same(got, want, more_finite=False):
+    for a, b, what in zip(got, want, ("outputs", "states")):
+        finite = torch.isfinite(b)
+        # (the walk runs the matrix memory as a delta rule that removes nothing: 0 times a NaN entry reaches the column's others)
+        assert torch.equal(torch.isfinite(a) & finite if more_finite else torch.isfinite(a), finite), what
+        worst = float((a - b)[finite].abs().max() / b[finite].abs().max())
+        assert worst <= 6e-5, f"{what}: {worst:.3g} of the largest value"      # float32 rounding of both
+
+
+@pytest.mark.parametrize("kind", ["general", "gated", "retention", "memory"])
+@pytest.mark.parametrize("dk,dv", [(64, 64), (24, 20), (64, 132)])
+@pytest.mark.parametrize("what", ["value", "key", "read", "gate"])
+@pytest.mark.parametrize("at", [0, 17, 31, 63, 69])
+def test_what_is_not_finite_reaches_no_earlier_token(kind, dk, dv, what, at):
+    H, lengths = 2, [40, 70, 65]
+    if what == "gate" and kind == "retention":
+        return                          # its decays are the model's
+    t = inputs(kind, H, dk, dv, lengths, torch.Generator(DEV).manual_seed(dk + dv + at))
+    K, V, row = H * dk, H * dv, lengths[0] + at
+    col = {"read": 3, "key": K + 3, "value": 2 * K + dv // 2, "gate": 3 * K + V if kind in ("gated", "memory") else 2 * K + V + 3}[what]
+    for spoil in (float("nan"), float("inf")) if what == "value" else (float("nan"),):
+        t["proj"][row, col] = spoil     # of head 0 of the second request
+        want = scan(kind, H, dk, dv, lengths, t, len(lengths))
+        assert bool(torch.isfinite(want[0][:row]).all()) and not bool(torch.isfinite(want[0][row]).all())
+        same(scan(kind, H, dk, dv, lengths, t, 0), want, kind == "memory" and what == "key")
+        if kind == "gated" and what == "gate":      # the decay's logit instead of the step's
+            t["proj"][row, col], t["proj"][row, col + H] = 0.5, spoil
+            same(scan(kind, H, dk, dv, lengths, t, 0), scan(kind, H, dk, dv, lengths, t, len(lengths)))
+        if kind == "general" and what == "gate":    # the channel's decay
+            t["proj"][row, col], t["wl"][row, 3] = 0.5, spoil
+            same(scan(kind, H, dk, dv, lengths, t, 0), scan(kind, H, dk, dv, lengths, t, len(lengths)))
