@@ -176,12 +176,12 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
     }
     sk += __shfl_xor_sync(0xffffffffu, sk, 1);
     sk += __shfl_xor_sync(0xffffffffu, sk, 2);
-    const float kinv = 1.0f / sqrtf(sk + in.s1);
+    const float kinv = row_in ? 1.0f / sqrtf(sk + in.s1) : 0.f;      // (a row that is not there has no length)
     float beta = 0.f;
     if (GATED) {
       sq += __shfl_xor_sync(0xffffffffu, sq, 1);
       sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-      const float qinv = in.s0 / sqrtf(sq + in.s1);
+      const float qinv = row_in ? in.s0 / sqrtf(sq + in.s1) : 0.f;
       float g = 1.f;
       if (row_in) {
         beta = sigmoid_f(in.x[row * in.ldx + h]);

@@ -76,3 +76,13 @@ def test_what_is_not_finite_reaches_no_earlier_token(kind, dk, dv, what, at):
         if kind == "general" and what == "gate":    # the channel's decay
             t["proj"][row, col], t["wl"][row, 3] = 0.5, spoil
             same(scan(kind, H, dk, dv, lengths, t, 0), scan(kind, H, dk, dv, lengths, t, len(lengths)))
+
+
+@pytest.mark.parametrize("kind", ["general", "gated"])
+@pytest.mark.parametrize("lengths", [[33], [1, 70, 95]])
+def test_chunks_that_are_not_full_without_an_epsilon(kind, lengths):
+    """Rows that fill a chunk up have no key whose length could be divided by."""
+    t = inputs(kind, 2, 64, 64, lengths, torch.Generator(DEV).manual_seed(len(lengths)))
+    got, want = (scan(kind, 2, 64, 64, lengths, t, first, eps=0.0) for first in (0, len(lengths)))
+    assert all(bool(torch.isfinite(x).all()) for x in want)
+    same(got, want)
