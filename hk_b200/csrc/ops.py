@@ -864,13 +864,21 @@ def _chunk_tables(chunks, requests, what: str):
     return _ptr(chunks), int(chunks.shape[0]), _ptr(requests), int(requests.shape[0])
 
 
-def _walk_record(n: int, segments, H: int, dk: int, dv: int, device):
+def walk_rows(n: int, segments: int, most_rows: int):
+    """(rows of scratch, rows a segment) of a walk over so many segments of a step of n rows: with `most_rows` > 0 the segments leave
+    rows out, and the scratch holds `most_rows` for each of them where that is less than the step's rows (0: it holds the step's)."""
+    own = segments * most_rows
+    return (own, most_rows) if 0 < own < n else (n, 0)
+
+
+def _walk_record(n: int, segments, most_rows: int, H: int, dk: int, dv: int, device):
     """Scratch for what every token brings to a walk (decay, removal times unit key, unit key, key, receptance, value, made by a
-    kernel of its own for all tokens at once); None when no request is walked.  Taken before the chunks are launched: an
-    allocation that fails leaves every state as it was."""
+    kernel of its own for all tokens at once) and its rows a segment (`walk_rows`); (None, 0) when no request is walked.  Taken before
+    the chunks are launched: an allocation that fails leaves every state as it was."""
     if not segments.shape[0]:
-        return None
-    return torch.empty(n * H * int(build.load("recurrent").hk_delta_rule_record(dk, dv)), dtype=torch.float32, device=device)
+        return None, 0
+    rows, each = walk_rows(n, int(segments.shape[0]), int(most_rows))
+    return torch.empty(rows * H * int(build.load("recurrent").hk_delta_rule_record(dk, dv)), dtype=torch.float32, device=device), each
 
 
 def _chunk_scratch(lib, chunks, H: int, dk: int, dvp: int, removal: bool, device):
@@ -903,7 +911,7 @@ def delta_rule_scan(r, k, v, a_logit, w_logit, a_bias, w_bias, segments, state, 
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(out.shape) != (n, H * dv) or segments.shape[1] != 3 \
             or a_bias.shape[0] != H * dk or w_bias.shape[0] != H * dk:
         raise KernelError("delta_rule_scan: shapes do not fit")
-    rec = _walk_record(n, segments, H, dk, dv, out.device)
+    rec, rec_rows = _walk_record(n, segments, most_rows, H, dk, dv, out.device)
     if chunks is not None and chunks.shape[0]:
         lib = build.load("delta_chunks")
         scratch = _chunk_scratch(lib, chunks, H, dk, dv, True, out.device)
@@ -916,7 +924,7 @@ def delta_rule_scan(r, k, v, a_logit, w_logit, a_bias, w_bias, segments, state, 
     lib = build.load("recurrent")
     _check(lib.hk_delta_rule_scan(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ctypes.c_longlong(ld), _ptr(w_logit),
                                   ctypes.c_longlong(ldw), _ptr(a_bias), _ptr(w_bias), _ptr(segments), int(segments.shape[0]), n,
-                                  int(most_rows), _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
+                                  int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
                                   ctypes.c_float(key_eps), _stream()), "delta_rule_scan", launches=2)
 
 
@@ -1004,7 +1012,7 @@ def gated_delta_scan(q, k, v, b_logit, a_logit, a_log, dt_bias, segments, state,
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(out.shape) != (n, H * dv) or segments.shape[1] != 3 \
             or a_log.shape[0] != H or dt_bias.shape[0] != H or H % G:
         raise KernelError("gated_delta_scan: shapes do not fit")
-    rec = _walk_record(n, segments, H, dk, dv, out.device)
+    rec, rec_rows = _walk_record(n, segments, most_rows, H, dk, dv, out.device)
     if chunks is not None and chunks.shape[0]:
         lib = build.load("delta_chunks")
         scratch = _chunk_scratch(lib, chunks, H, dk, dv, True, out.device)
@@ -1018,7 +1026,7 @@ def gated_delta_scan(q, k, v, b_logit, a_logit, a_log, dt_bias, segments, state,
     lib = build.load("recurrent")
     _check(lib.hk_gated_delta_scan(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(b_logit), _ptr(a_logit),
                                    ctypes.c_longlong(ldg), _ptr(a_log), _ptr(dt_bias), _ptr(segments), int(segments.shape[0]), n,
-                                   int(most_rows), _ptr(rec), _ptr(state), _ptr(out), H, G, dk, dv, ctypes.c_float(q_scale),
+                                   int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, G, dk, dv, ctypes.c_float(q_scale),
                                    ctypes.c_float(unit_eps), _stream()), "gated_delta_scan", launches=2)
 
 
@@ -1048,7 +1056,7 @@ def retention_scan(q, k, v, cos, sin, rotary_dim: int, positions, decay, segment
     if tuple(state.shape[1:]) != (H, dk, dv) or tuple(out.shape) != (n, H * dv) or segments.shape[1] != 3 \
             or decay.shape[0] != H or positions.shape[0] != n:
         raise KernelError("retention_scan: shapes do not fit")
-    rec = _walk_record(n, segments, H, dk, dv, out.device)
+    rec, rec_rows = _walk_record(n, segments, most_rows, H, dk, dv, out.device)
     if chunks is not None and chunks.shape[0]:
         lib = build.load("delta_chunks")
         scratch = _chunk_scratch(lib, chunks, H, dk, dv, False, out.device)
@@ -1061,7 +1069,7 @@ def retention_scan(q, k, v, cos, sin, rotary_dim: int, positions, decay, segment
     lib = build.load("recurrent")
     _check(lib.hk_retention_scan(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(cos if rotary_dim > 0 else None),
                                  _ptr(sin if rotary_dim > 0 else None), int(rotary_dim), _ptr(positions), _ptr(decay), _ptr(segments),
-                                 int(segments.shape[0]), n, int(most_rows), _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(k_scale),
+                                 int(segments.shape[0]), n, int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(k_scale),
                                  _stream()), "retention_scan", launches=2)
 
 
@@ -1216,7 +1224,7 @@ def mlstm_scan(q, k, v, i_logit, f_logit, i_bias, f_bias, segments, state, m_sta
     if tuple(state.shape[1:]) != (H, dk, dvp) or tuple(m_state.shape[1:]) != (H,) or tuple(out.shape) != (n, H * dvp) \
             or tuple(gates.shape) != (n, H, 3) or segments.shape[1] != 3 or i_bias.shape[0] != H or f_bias.shape[0] != H:
         raise KernelError("mlstm_scan: shapes do not fit")
-    rec = _walk_record(n, segments, H, dk, dvp, out.device)
+    rec, rec_rows = _walk_record(n, segments, most_rows, H, dk, dvp, out.device)
     lib = build.load("recurrent")
     if chunks is not None and chunks.shape[0]:
         _need(long_segments, "long_segments", torch.int32, 2)
@@ -1233,7 +1241,7 @@ def mlstm_scan(q, k, v, i_logit, f_logit, i_bias, f_bias, segments, state, m_sta
     if rec is None:
         return
     _check(lib.hk_mlstm_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(i_logit), _ptr(f_logit), ctypes.c_longlong(ld), _ptr(i_bias),
-                             _ptr(f_bias), _ptr(segments), int(segments.shape[0]), n, int(most_rows), _ptr(rec), _ptr(gates), _ptr(state),
+                             _ptr(f_bias), _ptr(segments), int(segments.shape[0]), n, int(most_rows), rec_rows, _ptr(rec), _ptr(gates), _ptr(state),
                              _ptr(m_state), _ptr(out), H, dk, dv, ctypes.c_float(cap), ctypes.c_float(q_scale), _stream()),
            "mlstm_scan", launches=3)
 

@@ -25,12 +25,15 @@
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // The rows that a preparation kernel works on: all of the step's (segs null), or those of the segments in blockIdx.y (up to
-// `most` rows each) when the step's other rows are not walked token by token.  `item` becomes the row's and head's number.
-__device__ __forceinline__ bool prep_item(long long& item, const int* segs, long long items, int H) {
+// `most` rows each) when the step's other rows are not walked token by token.  `item` becomes the row's and head's number, `at`
+// the number of its record: the same, or with `rec_rows` > 0 that among the records of the segments alone, so many rows each.
+__device__ __forceinline__ bool prep_item(long long& item, long long& at, const int* segs, long long items, int H, int rec_rows) {
   if (item >= items) return false;
+  at = item;
   if (segs == nullptr) return true;
   const int row0 = segs[blockIdx.y * 3 + 1], count = segs[blockIdx.y * 3 + 2];
   if (item >= (long long)count * H) return false;
+  at += (long long)(rec_rows ? (int)blockIdx.y * rec_rows : row0) * H;
   item += (long long)row0 * H;
   return true;
 }
@@ -46,10 +49,11 @@ static dim3 prep_grid(long long items, const int* segs, int n_seg) {
 __global__ void delta_rule_prep_kernel(const float* __restrict__ r, const float* __restrict__ k, const float* __restrict__ v,
                                        const float* __restrict__ al, long long ld, const float* __restrict__ wl, long long ldw,
                                        const float* __restrict__ a_bias, const float* __restrict__ w_bias, float* __restrict__ rec,
-                                       const int* __restrict__ psegs, long long items, int H, int dk, int dv, int L, int RPT, float decay_scale, float key_eps) {
+                                       const int* __restrict__ psegs, int rec_rows, long long items, int H, int dk, int dv, int L, int RPT, float decay_scale, float key_eps) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long at;
   const int lane = threadIdx.x & 31;
-  if (!prep_item(item, psegs, items, H)) return;
+  if (!prep_item(item, at, psegs, items, H, rec_rows)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const size_t hoff = (size_t)h * dk;
@@ -62,7 +66,7 @@ __global__ void delta_rule_prep_kernel(const float* __restrict__ r, const float*
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss + key_eps);
   const int P = L * RPT;
-  float* out = rec + (size_t)item * (5 * P + dv);
+  float* out = rec + (size_t)at * (5 * P + dv);
   for (int j = lane; j < P; j += 32) {
     const int i = (j % RPT) * L + j / RPT;       // the entry that sits at place j
     float d = 0.f, au = 0.f, u = 0.f, kv = 0.f, rv = 0.f;
@@ -96,12 +100,12 @@ __device__ __forceinline__ void dr_cp_async16(void* dst, const void* src) {
 template <int RPT, int L, int CPT>     // CPT: columns a lane group owns (they share every load of the token's vectors)
 __global__ void __launch_bounds__(256)
 delta_rule_scan_kernel(const float* __restrict__ rec, const int* __restrict__ segs, float* __restrict__ state,
-                       float* __restrict__ out, int H, int dk, int dv, int cols, int chunk) {
+                       float* __restrict__ out, int H, int dk, int dv, int cols, int chunk, int rec_rows) {
   extern __shared__ __align__(16) float sm[];   // [2][chunk][5 P + dv]
   constexpr int P = L * RPT;
   const int R = 5 * P + dv;
   const int seg = blockIdx.x / H, h = blockIdx.x % H;
-  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], count = segs[seg * 3 + 2];
+  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], count = segs[seg * 3 + 2], rec0 = rec_rows ? seg * rec_rows : row0;
   const int col0 = blockIdx.y * cols;
   const int tid = threadIdx.x;
   const int sub = tid % L, cidx = (tid / L) * CPT;           // first of this lane group's columns, within the block
@@ -123,7 +127,7 @@ delta_rule_scan_kernel(const float* __restrict__ rec, const int* __restrict__ se
   auto fetch = [&](int c) {                     // chunk c -> stage c & 1
     const int t0 = c * chunk, tc = min(chunk, count - t0);
     float* dst = sm + (size_t)(c & 1) * chunk * R;
-    const float* src = rec + ((size_t)(row0 + t0) * H + h) * R;
+    const float* src = rec + ((size_t)(rec0 + t0) * H + h) * R;
     for (int t = 0; t < tc; ++t)
       for (int p = tid; p < pieces; p += blockDim.x) dr_cp_async16(dst + (size_t)t * R + 4 * p, src + (size_t)t * H * R + 4 * p);
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -216,11 +220,11 @@ delta_rule_scan_kernel(const float* __restrict__ rec, const int* __restrict__ se
 // The plain form of the scan for value sizes that are no multiple of 4 (records that are not whole 16-byte pieces):
 // the same recurrence, the state in shared memory, records read with plain loads, one token at a time.
 __global__ void delta_rule_scan_plain_kernel(const float* __restrict__ rec, const int* __restrict__ segs, float* __restrict__ state,
-                                             float* __restrict__ out, int H, int dk, int dv, int L, int RPT, int cols) {
+                                             float* __restrict__ out, int H, int dk, int dv, int L, int RPT, int cols, int rec_rows) {
   extern __shared__ __align__(16) float sm[];   // [blockDim / L][P] the state columns; then one record
   const int P = L * RPT, R = 5 * P + dv;
   const int seg = blockIdx.x / H, h = blockIdx.x % H;
-  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], count = segs[seg * 3 + 2];
+  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], count = segs[seg * 3 + 2], rec0 = rec_rows ? seg * rec_rows : row0;
   const int tid = threadIdx.x, sub = tid % L, cidx = tid / L, col = blockIdx.y * cols + cidx;
   const bool col_ok = cidx < cols && col < dv;
   float* Sc = sm + (size_t)cidx * P;             // this column's state, in the record's order of entries
@@ -232,7 +236,7 @@ __global__ void delta_rule_scan_plain_kernel(const float* __restrict__ rec, cons
   }
   for (int t = 0; t < count; ++t) {
     __syncthreads();
-    const float* src = rec + ((size_t)(row0 + t) * H + h) * R;
+    const float* src = rec + ((size_t)(rec0 + t) * H + h) * R;
     for (int p = tid; p < R; p += blockDim.x) recs[p] = src[p];
     __syncthreads();
     const float* mine = recs + sub * RPT;
@@ -285,14 +289,14 @@ HK_API int hk_delta_rule_record(int dk, int dv) {
 
 template <int RPT, int CPT>
 static int dr_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s, const float* rec, const int* segs, float* state,
-                     float* out, int H, int dk, int dv, int cols, int chunk) {
+                     float* out, int H, int dk, int dv, int cols, int chunk, int rec_rows) {
 #define DR_LAUNCH(LL)                                                                                                       \
   do {                                                                                                                      \
     static HkSmemCache cache;                                                                                               \
     int e = hk_allow_smem(delta_rule_scan_kernel<RPT, LL, CPT>, smem, cache);                                               \
     if (e) return e;                                                                                                        \
     return hk_launch(delta_rule_scan_kernel<RPT, LL, CPT>, grid, dim3(threads), smem, s, rec, segs, state, out, H, dk, dv, cols, \
-                     chunk);                                                                                                \
+                     chunk, rec_rows);                                                                                      \
   } while (0)
   switch (L) {
     case 1: DR_LAUNCH(1);
@@ -317,7 +321,7 @@ static int dr_plan(int n_seg, int H, int dk, int dv, int* L_out, int* rpt_out) {
 
 // The scan over records that a prep kernel wrote with the layout (L, rpt) of `dr_plan`.
 static int dr_scan_records(const float* rec, const int* segs, int n_seg, float* state, float* out, int H, int dk, int dv, int L,
-                           int rpt, cudaStream_t s) {
+                           int rpt, int rec_rows, cudaStream_t s) {
   const int R = 5 * L * rpt + dv;
   if (dv & 3) {
     const int cols = max(1, min(dv, 128 / L));
@@ -327,7 +331,7 @@ static int dr_scan_records(const float* rec, const int* segs, int n_seg, float* 
     int e = hk_allow_smem(delta_rule_scan_plain_kernel, smem, cache);
     if (e) return e;
     return hk_launch(delta_rule_scan_plain_kernel, dim3((unsigned)(n_seg * H), (unsigned)((dv + cols - 1) / cols)), dim3(threads), smem, s,
-                     rec, segs, state, out, H, dk, dv, L, rpt, cols);
+                     rec, segs, state, out, H, dk, dv, L, rpt, cols, rec_rows);
   }
   // a block takes as many columns as 256 threads hold (they share the records that the ring brings), fewer while the
   // blocks do not yet fill the SMs twice: one request of 2,048 tokens at 32 heads of 64 runs 808 us with 8 columns a
@@ -345,17 +349,18 @@ static int dr_scan_records(const float* rec, const int* segs, int n_seg, float* 
   while (chunk > 2 && (size_t)2 * chunk * R * sizeof(float) > 64 * 1024) chunk >>= 1;
   const size_t smem = (size_t)2 * chunk * R * sizeof(float);
   dim3 grid((unsigned)(n_seg * H), (unsigned)((dv + cols - 1) / cols));
-  if (rpt == 8 && cpt == 2) return dr_launch<8, 2>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk);
-  if (rpt == 8) return dr_launch<8, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk);
-  if (rpt == 16) return dr_launch<16, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk);
-  if (rpt == 32) return dr_launch<32, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk);
-  return dr_launch<64, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk);
+  if (rpt == 8 && cpt == 2) return dr_launch<8, 2>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk, rec_rows);
+  if (rpt == 8) return dr_launch<8, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk, rec_rows);
+  if (rpt == 16) return dr_launch<16, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk, rec_rows);
+  if (rpt == 32) return dr_launch<32, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk, rec_rows);
+  return dr_launch<64, 1>(L, grid, threads, smem, s, rec, segs, state, out, H, dk, dv, cols, chunk, rec_rows);
 }
 
 // `rec`: scratch of n_rows * H * hk_delta_rule_record(dk, dv) floats (16-byte aligned) that the call fills and reads.
 // `most_rows` > 0: the segments do not hold all of the step's rows, and none holds more than so many; only theirs are prepared.
+// With `rec_rows` (0, or at least most_rows) > 0 `rec` holds so many rows per segment instead, n_seg * rec_rows.
 HK_API int hk_delta_rule_scan(const float* r, const float* k, const float* v, const float* al, long long ld, const float* wl,
-                              long long ldw, const float* a_bias, const float* w_bias, const int* segs, int n_seg, int n_rows, int most_rows,
+                              long long ldw, const float* a_bias, const float* w_bias, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows,
                               float* rec, float* state, float* out, int H, int dk, int dv, float decay_scale, float key_eps,
                               void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
@@ -367,10 +372,10 @@ HK_API int hk_delta_rule_scan(const float* r, const float* k, const float* v, co
     const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
     const int* psegs = most_rows ? segs : nullptr;
     int e = hk_launch(delta_rule_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, r, k, v, al, ld, wl, ldw, a_bias,
-                      w_bias, rec, psegs, items, H, dk, dv, L, rpt, decay_scale, key_eps);
+                      w_bias, rec, psegs, rec_rows, items, H, dk, dv, L, rpt, decay_scale, key_eps);
     if (e) return e;
   }
-  return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, s);
+  return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, rec_rows, s);
 }
 
 // ------------------------------------------------------------------ minGRU
@@ -475,11 +480,12 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log
 __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                         long long ld, const float* __restrict__ bl, const float* __restrict__ al, long long ldg,
                                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ rec,
-                                        const int* __restrict__ psegs, long long items, int H, int G, int dk, int dv, int L, int RPT, float q_scale,
+                                        const int* __restrict__ psegs, int rec_rows, long long items, int H, int G, int dk, int dv, int L, int RPT, float q_scale,
                                         float unit_eps) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long at;
   const int lane = threadIdx.x & 31;
-  if (!prep_item(item, psegs, items, H)) return;
+  if (!prep_item(item, at, psegs, items, H, rec_rows)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const int g = h / (H / G);
@@ -497,7 +503,7 @@ __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float
   const float beta = sigmoid_f(bl[row * ldg + h]);
   const float decay = expf(-expf(a_log[h]) * softplus_f(al[row * ldg + h] + dt_bias[h]));
   const int P = L * RPT;
-  float* out = rec + (size_t)item * (5 * P + dv);
+  float* out = rec + (size_t)at * (5 * P + dv);
   for (int j = lane; j < P; j += 32) {
     const int i = (j % RPT) * L + j / RPT;       // the entry that sits at place j
     float d = 0.f, au = 0.f, u = 0.f, rv = 0.f;
@@ -519,7 +525,7 @@ __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float
 // q, k [n, G*dk] and v [n, H*dv] are column slices of one float32 matrix (row stride ld), already convolved and
 // activated; b_logit and a_logit [n, H] slices of one (row stride ldg).  `rec` as for hk_delta_rule_scan.
 HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, long long ld, const float* bl, const float* al,
-                               long long ldg, const float* a_log, const float* dt_bias, const int* segs, int n_seg, int n_rows, int most_rows,
+                               long long ldg, const float* a_log, const float* dt_bias, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows,
                                float* rec, float* state, float* out, int H, int G, int dk, int dv, float q_scale, float unit_eps,
                                void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
@@ -530,9 +536,9 @@ HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, l
   const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
   const int* psegs = most_rows ? segs : nullptr;
   int e = hk_launch(gated_delta_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, bl, al, ldg, a_log,
-                    dt_bias, rec, psegs, items, H, G, dk, dv, L, rpt, q_scale, unit_eps);
+                    dt_bias, rec, psegs, rec_rows, items, H, G, dk, dv, L, rpt, q_scale, unit_eps);
   if (e) return e;
-  return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, s);
+  return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, rec_rows, s);
 }
 
 // ------------------------------------------------------------------ retention
@@ -546,10 +552,11 @@ HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, l
 __global__ void retention_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                       long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot,
                                       const int* __restrict__ positions, const float* __restrict__ decay, float* __restrict__ rec,
-                                      const int* __restrict__ psegs, long long items, int H, int dk, int dv, int L, int RPT, float k_scale, int lean) {
+                                      const int* __restrict__ psegs, int rec_rows, long long items, int H, int dk, int dv, int L, int RPT, float k_scale, int lean) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long at;
   const int lane = threadIdx.x & 31;
-  if (!prep_item(item, psegs, items, H)) return;
+  if (!prep_item(item, at, psegs, items, H, rec_rows)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const float* qp = q + row * ld + (size_t)h * dk;
@@ -559,7 +566,7 @@ __global__ void retention_prep_kernel(const float* __restrict__ q, const float* 
   const float* s = sin_t + (size_t)positions[row] * half;
   const float dec = decay[h];
   const int P = L * RPT;
-  float* out = rec + (size_t)item * ((lean ? 2 : 5) * P + dv);
+  float* out = rec + (size_t)at * ((lean ? 2 : 5) * P + dv);
   for (int j = lane; j < P; j += 32) {
     const int i = (j % RPT) * L + j / RPT;       // the entry that sits at place j
     float kv = 0.f, qv = 0.f;
@@ -600,14 +607,14 @@ __global__ void retention_prep_kernel(const float* __restrict__ q, const float* 
 template <int RPT, int L, int CPT>
 __global__ void __launch_bounds__(256)
 retention_scan_kernel(const float* __restrict__ rec, const int* __restrict__ segs, const float* __restrict__ decay,
-                      float* __restrict__ state, float* __restrict__ out, int H, int dk, int dv, int cols, int chunk) {
+                      float* __restrict__ state, float* __restrict__ out, int H, int dk, int dv, int cols, int chunk, int rec_rows) {
   extern __shared__ __align__(16) float sm[];   // [2][chunk][2 P + dv] records, then [2][chunk][W] the lanes' shares
   constexpr int P = L * RPT;
   const int R = 2 * P + dv;
   const int W = blockDim.x * CPT;               // shares a token: one per (column of the block, lane)
   float* part = sm + (size_t)2 * chunk * R;
   const int seg = blockIdx.x / H, h = blockIdx.x % H;
-  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], count = segs[seg * 3 + 2];
+  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], count = segs[seg * 3 + 2], rec0 = rec_rows ? seg * rec_rows : row0;
   const int col0 = blockIdx.y * cols;
   const int tid = threadIdx.x;
   const int sub = tid % L, cidx = (tid / L) * CPT;
@@ -630,7 +637,7 @@ retention_scan_kernel(const float* __restrict__ rec, const int* __restrict__ seg
   auto fetch = [&](int c) {                     // chunk c -> stage c & 1
     const int t0 = c * chunk, tc = min(chunk, count - t0);
     float* dst = sm + (size_t)(c & 1) * chunk * R;
-    const float* src = rec + ((size_t)(row0 + t0) * H + h) * R;
+    const float* src = rec + ((size_t)(rec0 + t0) * H + h) * R;
     for (int t = 0; t < tc; ++t)
       for (int p = tid; p < pieces; p += blockDim.x) dr_cp_async16(dst + (size_t)t * R + 4 * p, src + (size_t)t * H * R + 4 * p);
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -705,14 +712,14 @@ retention_scan_kernel(const float* __restrict__ rec, const int* __restrict__ seg
 
 template <int RPT, int CPT>
 static int ret_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s, const float* rec, const int* segs,
-                      const float* decay, float* state, float* out, int H, int dk, int dv, int cols, int chunk) {
+                      const float* decay, float* state, float* out, int H, int dk, int dv, int cols, int chunk, int rec_rows) {
 #define RET_LAUNCH(LL)                                                                                                      \
   do {                                                                                                                      \
     static HkSmemCache cache;                                                                                               \
     int e = hk_allow_smem(retention_scan_kernel<RPT, LL, CPT>, smem, cache);                                                \
     if (e) return e;                                                                                                        \
     return hk_launch(retention_scan_kernel<RPT, LL, CPT>, grid, dim3(threads), smem, s, rec, segs, decay, state, out, H, dk, dv, \
-                     cols, chunk);                                                                                          \
+                     cols, chunk, rec_rows);                                                                                \
   } while (0)
   switch (L) {
     case 1: RET_LAUNCH(1);
@@ -728,7 +735,7 @@ static int ret_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s
 // q, k [n, H*dk] and v [n, H*dv] are column slices of one float32 matrix (row stride ld); decay float32 [H]; `rec` as for
 // hk_delta_rule_scan.  Blocks, columns a block and columns a lane group are chosen as for the delta rule's scan.
 HK_API int hk_retention_scan(const float* q, const float* k, const float* v, long long ld, const float* cos_t, const float* sin_t,
-                             int rot, const int* positions, const float* decay, const int* segs, int n_seg, int n_rows, int most_rows, float* rec,
+                             int rot, const int* positions, const float* decay, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows, float* rec,
                              float* state, float* out, int H, int dk, int dv, float k_scale, void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
   if (H < 1 || dk < 1 || dv < 1 || dk > 2048 || rot < 0 || rot > dk || (rot & 1) || ((uintptr_t)rec & 15)) return HK_ERR_UNSUPPORTED;
@@ -739,9 +746,9 @@ HK_API int hk_retention_scan(const float* q, const float* k, const float* v, lon
   const int* psegs = most_rows ? segs : nullptr;
   const int lean = (dv & 3) == 0;
   int e = hk_launch(retention_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, cos_t, sin_t, rot,
-                    positions, decay, rec, psegs, items, H, dk, dv, L, rpt, k_scale, lean);
+                    positions, decay, rec, psegs, rec_rows, items, H, dk, dv, L, rpt, k_scale, lean);
   if (e) return e;
-  if (!lean) return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, s);
+  if (!lean) return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dv, L, rpt, rec_rows, s);
   const int R = 2 * L * rpt + dv;
   int cols = max(1, min(dv, 256 / L));
   while (cols > 8 && cols * L > 64 && (long long)n_seg * H * ((dv + cols - 1) / cols) < 2 * 148) cols >>= 1;
@@ -752,11 +759,11 @@ HK_API int hk_retention_scan(const float* q, const float* k, const float* v, lon
   while (chunk > 2 && (size_t)2 * chunk * (R + threads * cpt) * sizeof(float) > 64 * 1024) chunk >>= 1;
   const size_t smem = (size_t)2 * chunk * (R + threads * cpt) * sizeof(float);       // records, and the lanes' shares of the outputs
   dim3 grid((unsigned)(n_seg * H), (unsigned)((dv + cols - 1) / cols));
-  if (rpt == 8 && cpt == 2) return ret_launch<8, 2>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk);
-  if (rpt == 8) return ret_launch<8, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk);
-  if (rpt == 16) return ret_launch<16, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk);
-  if (rpt == 32) return ret_launch<32, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk);
-  return ret_launch<64, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk);
+  if (rpt == 8 && cpt == 2) return ret_launch<8, 2>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk, rec_rows);
+  if (rpt == 8) return ret_launch<8, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk, rec_rows);
+  if (rpt == 16) return ret_launch<16, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk, rec_rows);
+  if (rpt == 32) return ret_launch<32, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk, rec_rows);
+  return ret_launch<64, 1>(L, grid, threads, smem, s, rec, segs, decay, state, out, H, dk, dv, cols, chunk, rec_rows);
 }
 
 // ------------------------------------------------------------------ matrix memory with exponential gates (mLSTM)
@@ -831,18 +838,19 @@ HK_API int hk_mlstm_gates(const float* il, const float* fl, long long ld, const 
 }
 
 __global__ void mlstm_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                  long long ld, const float* __restrict__ gates, float* __restrict__ rec, const int* __restrict__ psegs, long long items, int H,
+                                  long long ld, const float* __restrict__ gates, float* __restrict__ rec, const int* __restrict__ psegs, int rec_rows, long long items, int H,
                                   int dk, int dv, int dvp, int L, int RPT, float q_scale) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long at;
   const int lane = threadIdx.x & 31;
-  if (!prep_item(item, psegs, items, H)) return;
+  if (!prep_item(item, at, psegs, items, H, rec_rows)) return;
   const size_t row = (size_t)(item / H);
   const int h = (int)(item % H);
   const float keep = gates[item * 3], take = gates[item * 3 + 1];
   const float* qp = q + row * ld + (size_t)h * dk;
   const float* kp = k + row * ld + (size_t)h * dk;
   const int P = L * RPT;
-  float* out = rec + (size_t)item * (5 * P + dvp);
+  float* out = rec + (size_t)at * (5 * P + dvp);
   for (int j = lane; j < P; j += 32) {
     const int i = (j % RPT) * L + j / RPT;
     const bool in = i < dk;
@@ -861,7 +869,7 @@ HK_API int hk_mlstm_padded(int dv) { return (dv + 1 + 3) & ~3; }
 // q, k [n, H*dk], v [n, H*dv], il, fl [n, H]: column slices of one float32 matrix (row stride ld).  state
 // [slots, H, dk, dvp], m_state [slots, H], gates scratch [n, H, 3] (kept: the output's gate reads e^(-m)), out [n, H*dvp].
 HK_API int hk_mlstm_scan(const float* q, const float* k, const float* v, const float* il, const float* fl, long long ld,
-                         const float* i_bias, const float* f_bias, const int* segs, int n_seg, int n_rows, int most_rows, float* rec,
+                         const float* i_bias, const float* f_bias, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows, float* rec,
                          float* gates, float* state, float* m_state, float* out, int H, int dk, int dv, float cap, float q_scale,
                          void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
@@ -875,9 +883,9 @@ HK_API int hk_mlstm_scan(const float* q, const float* k, const float* v, const f
   if (e) return e;
   const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
   const int* psegs = most_rows ? segs : nullptr;
-  e = hk_launch(mlstm_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, psegs, items,                 H, dk, dv, dvp, L, rpt, q_scale);
+  e = hk_launch(mlstm_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, psegs, rec_rows, items,                 H, dk, dv, dvp, L, rpt, q_scale);
   if (e) return e;
-  return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dvp, L, rpt, s);
+  return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dvp, L, rpt, rec_rows, s);
 }
 
 // ------------------------------------------------------------------ the output of a head of a recurrent mixer

@@ -144,16 +144,17 @@ class _ChunkedScan(_SegmentScan):
             first = len(chunks)
             chunks += [(row + t, min(ops.DELTA_CHUNK, count - t)) for t in range(0, count, ops.DELTA_CHUNK)]
             requests.append((slot, first, len(chunks) - first))
+        # the info: the most rows of a request that is walked beside others in chunks
         return StepTables({"segments": seg, "short": seg[~long], "long": seg[long], "chunks": np.asarray(chunks, dtype=np.int32).reshape(-1, 2),
-                           "requests": np.asarray(requests, dtype=np.int32).reshape(-1, 3)})
+                           "requests": np.asarray(requests, dtype=np.int32).reshape(-1, 3)},
+                          int(seg[~long, 2].max(initial=0)) if requests else 0)
 
     def _scan_tables(self, ctx):
         """(the segments that are walked token by token, the further arguments of a scan)."""
         if not self._chunks:
             return self._segments(ctx), {}
-        t = ctx.tables[self.step_tables_key()][0]
-        return t["short"], {"chunks": t["chunks"], "requests": t["requests"],
-                            "most_rows": self.CHUNKS_FROM - 1 if t["chunks"].shape[0] else 0}
+        t, most_rows = ctx.tables[self.step_tables_key()]
+        return t["short"], {"chunks": t["chunks"], "requests": t["requests"], "most_rows": most_rows}
 
     def _all_segments(self, ctx) -> torch.Tensor:
         """Every request of the step as a segment, whichever way it is walked."""
