@@ -52,9 +52,12 @@ class LatentAttention(Part):
     graph_safe = True   # reads the batch from device tensors only
     # Measured at 32 heads, prompt mixer alone, latent space against made: 2,048 tokens 1,213 us against 364; 128 tokens behind
     # 4,000 348 against 220, 64 behind 2,000 176 against 172 (level: 32 rows made for a query); 64 to 128 tokens level, bound by
-    # the launches.  Rows made are bounded to 16 a query, which bounds their memory too.
+    # the launches.  Rows made are bounded to 16 a query.
     MADE_FROM = 64
     MADE_ROWS = 16
+    # What is made for a step takes at most so many bytes (16 KB a row at 32 heads), or where that is more what the latent space takes
+    # for the same queries (76 KB each at 32 heads and a rank of 512).  The requests with the most rows a query go first.
+    MADE_SCRATCH = 1 << 30
     MADE_BESIDE = 256   # beside requests that stay in the latent space: so many tokens at least, for the further launches
     MADE_RUNS = 4       # a step whose kinds of requests alternate more often stays in the latent space: every run is launched apart
 
@@ -134,6 +137,7 @@ class LatentAttention(Part):
         window = self.window or 0
         seen = [int(c) + (min(int(p), window - 1) if window else int(p)) for c, p in zip(ctx.q_lens, ctx.start_positions)]
         made = [int(c) >= self.MADE_FROM and v <= self.MADE_ROWS * int(c) for c, v in zip(ctx.q_lens, seen)]
+        self._fit_scratch(made, [int(c) for c in ctx.q_lens], seen, attention_fast.MADE_TILE)
         runs: List[Tuple[int, int, bool]] = []
         for start, count, m in zip(ctx.q_starts, ctx.q_lens, made):
             if runs and runs[-1][2] == m:
@@ -160,6 +164,18 @@ class LatentAttention(Part):
             arrays.update(got.arrays)
             plan, single = got.info, all(int(c) == 1 for c in q_lens)
         return StepTables(arrays, LatentInfo(plan, single, runs, rows, int(segments[:, 2].max())))
+
+    def _fit_scratch(self, made: List[bool], rows: List[int], seen: List[int], tile: int) -> None:
+        """Takes requests back into the latent space until the arrays of the others fit (MADE_SCRATCH)."""
+        def needed():       # packed queries, cache rows side by side, keys and values; two tiles a request may be filled up
+            return sum(2 * (c * self.H * (self.dn + self.dr) + (v + 2 * tile) * (self.r + self.dr + self.H * (self.dn + self.vd)))
+                       for c, v, m in zip(rows, seen, made) if m)
+
+        def latent():       # plain and absorbed queries, latent sums
+            return sum(2 * c * self.H * (self.dn + 2 * self.r + self.dr) for c, m in zip(rows, made) if m)
+        order = sorted((i for i, m in enumerate(made) if m), key=lambda i: seen[i] / rows[i])
+        while order and needed() > max(self.MADE_SCRATCH, latent()):
+            made[order.pop()] = False
 
     def children(self):
         return (self.position,) if self.position is not None else ()

@@ -40,3 +40,34 @@ def test_rows_side_by_side_without_tiles():
     assert firsts.tolist() == [[0, -5, 12, 4]] and segments.tolist() == [[0, 5, 77, 0]] and rows == 77
     _, segments, firsts, rows = attention_fast.made_items([0], [0], [70], [12], 8, 128)
     assert firsts.tolist() == [[0, 0, 12, 4]] and segments.tolist() == [[0, 5, 77, 5]] and rows == 128
+
+
+def latent_part(H=32):
+    from hk_b200.parts import LatentAttention
+    part = LatentAttention(4096, H, 128, 64, 128, 512, "m.", 1e-6, 192 ** -0.5)
+    part._w_ukv, part._wide, part._sm_count, part._tables_key = True, True, 148, ("latent",)      # as bound in bfloat16
+    return part
+
+
+@pytest.mark.parametrize("spans,stays", [
+    ([(30000, 2048)], []), ([(50000, 4096)], []), ([(120000, 8192)], [0]), ([(60000, 4000), (0, 4096)], [0]), ([(0, 100000)], []),
+    ([(30000, 2100), (20000, 1500), (15000, 1100)], [0]), ([(0, 64)] * 3, [])])
+def test_what_a_step_makes_is_bounded(spans, stays):
+    """The arrays of a step stay below MADE_SCRATCH or what the latent space would take; what does not fit stays there."""
+    from types import SimpleNamespace
+    part, T = latent_part(), 128
+    lens, starts = [n for _, n in spans], [c for c, _ in spans]
+    ctx = SimpleNamespace(slots=list(range(len(spans))), q_starts=[sum(lens[:i]) for i in range(len(lens))], q_lens=lens, start_positions=starts,
+                          n_tokens=sum(lens), fixed_shape=False, max_context=200000, page_tokens=16)
+    tables = part._made_tables(ctx)
+    if len(stays) == len(spans):
+        assert tables is None
+        return
+    kept = sorted(tables.arrays["made_segments"][:, 0].tolist())
+    assert kept == [i for i in range(len(spans)) if i not in stays]
+    n = sum(lens[i] for i in kept)
+    made = 2 * (n * 32 * 192 + tables.info.rows * (576 + 32 * 256))
+    assert made <= max(part.MADE_SCRATCH, 2 * n * 32 * (128 + 576 + 512))
+    # without the bound they would all have been made
+    part.MADE_SCRATCH = 1 << 50
+    assert sorted(part._made_tables(ctx).arrays["made_segments"][:, 0].tolist()) == list(range(len(spans)))
