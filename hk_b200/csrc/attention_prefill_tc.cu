@@ -1134,6 +1134,10 @@ HK_API int hk_attention_prefill_tc2(const void* q, const void* k_pages, const vo
          : launch2<64, false>(mk, mv, q, block_table, table_stride, items, n_items, out, H, G, page_tokens, window, scale_log2, so, pages_cap, status, s);
 }
 
+// Made rows that the kernel loads at once, and query tokens of an item of one head.
+HK_API int hk_attention_made_tile() { return TK; }
+HK_API int hk_attention_made_tokens() { return 2 * ROWS; }
+
 // Keys and values that were made for the step (see the kernel's MADE).  q bf16 [n, H, 128 (+ 64 with rope)]; kv bf16 [rows, H,
 // 128 key dims | 128 value dims]; rope bf16 [rows, 64], the key dims that all heads share behind their own 128, or null; items
 // as above for groups of one head (up to 256 query tokens), with the row of the request's position 0 in the place of its slot (a

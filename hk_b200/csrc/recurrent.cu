@@ -883,7 +883,8 @@ HK_API int hk_mlstm_scan(const float* q, const float* k, const float* v, const f
   if (e) return e;
   const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
   const int* psegs = most_rows ? segs : nullptr;
-  e = hk_launch(mlstm_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, psegs, rec_rows, items,                 H, dk, dv, dvp, L, rpt, q_scale);
+  e = hk_launch(mlstm_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, psegs,
+                rec_rows, items, H, dk, dv, dvp, L, rpt, q_scale);
   if (e) return e;
   return dr_scan_records(rec, segs, n_seg, state, out, H, dk, dvp, L, rpt, rec_rows, s);
 }

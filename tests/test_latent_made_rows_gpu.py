@@ -143,3 +143,22 @@ def test_rows_that_see_only_finite_rows_stay_finite(spans, window, gate, dr, at)
     scale = float(want.abs().max())
     assert not bool(torch.isfinite(got[sees]).any()) and bool(torch.isfinite(got[~sees]).all())
     assert bool(((got - want).abs()[~sees] <= 3e-2 * scale).all())       # probabilities and values in bfloat16
+
+
+@pytest.mark.parametrize("spans", [[(0, 64)], [(3, 70), (0, 200), (15, 64)]])
+def test_values_of_the_first_positions_are_never_rounded(spans):
+    """The first positions' results are off by half a unit of themselves and float32 sums; values in bfloat16 would show."""
+    from hk_b200.csrc import attention_fast
+    got, want, pos = made_case(spans, 0, tiled, tile=128)
+    scale, early = float(want.abs().max()), pos < attention_fast.MADE_FIRST
+    off = (got - want).abs() - 2.0 ** -8 * want.abs()
+    assert bool((off[early] <= 1e-4 * scale).all())
+    assert bool((off[~early] > 1e-4 * scale).any())         # (as later ones do)
+
+
+def test_sizes_that_the_host_shares_with_the_kernels():
+    from hk_b200.csrc import attention_fast, build, ops
+    made, first, runs = build.load("attention_prefill_tc"), build.load("attention_latent"), build.load("attention_generic")
+    assert made.hk_attention_made_tile() == attention_fast.MADE_TILE and made.hk_attention_made_tokens() == attention_fast.MADE_TOKENS
+    assert first.hk_latent_first_rows_count() == attention_fast.MADE_FIRST
+    assert [runs.hk_attention_f32_tokens(g) for g in (1, 3, 32, 33)] == [ops.RUN_ROWS, ops.RUN_ROWS // 3, 1, 0]
