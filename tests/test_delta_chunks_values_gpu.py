@@ -86,3 +86,32 @@ def test_chunks_that_are_not_full_without_an_epsilon(kind, lengths):
     got, want = (scan(kind, 2, 64, 64, lengths, t, first, eps=0.0) for first in (0, len(lengths)))
     assert all(bool(torch.isfinite(x).all()) for x in want)
     same(got, want)
+
+
+@pytest.mark.parametrize("first_chunked", [0, 2])
+def test_gates_and_maxima_of_the_matrix_memory(first_chunked):
+    """What `mlstm_scan` leaves in `gates` and `m_state`, for requests in chunks and beside them, from the logits alone."""
+    from hk_b200.csrc import ops
+    H, dk, dv, lengths, cap = 3, 8, 8, [5, 33, 70, 129], 15.0
+    g = torch.Generator(DEV).manual_seed(7)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)       # noqa: E731
+    n, R, at = sum(lengths), len(lengths), H * (2 * dk + dv)
+    wide, ib, fb, m0 = rand(n, at + 2 * H + 2) * 3, rand(H), rand(H) + 2, rand(R, H)
+    short, long, chunks, requests = tables(lengths, first_chunked)
+    state, m, gates = torch.zeros(R, H, dk, ops.mlstm_padded(dv), device=DEV), m0.clone(), torch.full((n, H, 3), 7.0, device=DEV)
+    out = torch.empty(n, H * ops.mlstm_padded(dv), device=DEV)
+    ops.mlstm_scan(wide[:, :H * dk], wide[:, H * dk:2 * H * dk], wide[:, 2 * H * dk:at], wide[:, at:at + H], wide[:, at + H:at + 2 * H], ib, fb,
+                   short, state, m, out, gates, H, dk, dv, cap, 0.5, long_segments=long, chunks=chunks, requests=requests, most_rows=max(lengths))
+    soft = lambda x: cap * torch.tanh(x.double() / cap)              # noqa: E731
+    i, f = soft(wide[:, at:at + H] + ib), torch.nn.functional.logsigmoid(soft(wide[:, at + H:at + 2 * H] + fb))
+    row = 0
+    for r, count in enumerate(lengths):
+        top = m0[r].double()
+        for t in range(row, row + count):
+            new = torch.maximum(f[t] + top, i[t])
+            want = torch.stack([torch.exp(f[t] + top - new), torch.exp(i[t] - new), torch.exp(-new)], dim=1)
+            # exponents of up to 2 cap and a sum of up to 129 terms, each rounded in float32
+            assert bool(((gates[t].double() - want).abs() <= 5e-5 * want + 1e-30).all())
+            top = new
+        assert bool(((m[r].double() - top).abs() <= 5e-5 * (1 + top.abs())).all())
+        row += count
