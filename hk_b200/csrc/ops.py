@@ -868,7 +868,7 @@ def walk_rows(n: int, segments: int, most_rows: int):
     """(rows of scratch, rows a segment) of a walk over so many segments of a step of n rows: with `most_rows` > 0 the segments leave
     rows out, and the scratch holds `most_rows` for each of them where that is less than the step's rows (0: it holds the step's)."""
     own = segments * most_rows
-    return (own, most_rows) if 0 < own < n else (n, 0)
+    return (own, most_rows) if 0 < own < n and segments <= 65535 else (n, 0)      # (more are prepared as the step's rows)
 
 
 def _walk_record(n: int, segments, most_rows: int, H: int, dk: int, dv: int, device):

@@ -37,6 +37,8 @@ __device__ __forceinline__ bool prep_item(long long& item, long long& at, const 
   item += (long long)row0 * H;
   return true;
 }
+// The segments that a preparation keeps to, or null: all of the step's rows (more segments than a grid is high, or no others).
+static const int* prep_segments(const int* segs, int n_seg, int most_rows) { return most_rows > 0 && n_seg <= 65535 ? segs : nullptr; }
 static dim3 prep_grid(long long items, const int* segs, int n_seg) {
   return dim3((unsigned)((items + 7) / 8), segs == nullptr ? 1u : (unsigned)n_seg);
 }
@@ -369,8 +371,9 @@ HK_API int hk_delta_rule_scan(const float* r, const float* k, const float* v, co
   int L, rpt;
   if (!dr_plan(n_seg, H, dk, dv, &L, &rpt)) return HK_ERR_UNSUPPORTED;
   {
-    const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
-    const int* psegs = most_rows ? segs : nullptr;
+    const int* psegs = prep_segments(segs, n_seg, most_rows);
+    const long long items = (long long)(psegs ? most_rows : n_rows) * H;
+    if (!psegs && rec_rows) return HK_ERR_UNSUPPORTED;
     int e = hk_launch(delta_rule_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, r, k, v, al, ld, wl, ldw, a_bias,
                       w_bias, rec, psegs, rec_rows, items, H, dk, dv, L, rpt, decay_scale, key_eps);
     if (e) return e;
@@ -533,8 +536,9 @@ HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, l
   cudaStream_t s = (cudaStream_t)stream;
   int L, rpt;
   if (!dr_plan(n_seg, H, dk, dv, &L, &rpt)) return HK_ERR_UNSUPPORTED;
-  const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
-  const int* psegs = most_rows ? segs : nullptr;
+  const int* psegs = prep_segments(segs, n_seg, most_rows);
+  const long long items = (long long)(psegs ? most_rows : n_rows) * H;
+  if (!psegs && rec_rows) return HK_ERR_UNSUPPORTED;
   int e = hk_launch(gated_delta_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, bl, al, ldg, a_log,
                     dt_bias, rec, psegs, rec_rows, items, H, G, dk, dv, L, rpt, q_scale, unit_eps);
   if (e) return e;
@@ -742,8 +746,9 @@ HK_API int hk_retention_scan(const float* q, const float* k, const float* v, lon
   cudaStream_t s = (cudaStream_t)stream;
   int L, rpt;
   if (!dr_plan(n_seg, H, dk, dv, &L, &rpt)) return HK_ERR_UNSUPPORTED;
-  const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
-  const int* psegs = most_rows ? segs : nullptr;
+  const int* psegs = prep_segments(segs, n_seg, most_rows);
+  const long long items = (long long)(psegs ? most_rows : n_rows) * H;
+  if (!psegs && rec_rows) return HK_ERR_UNSUPPORTED;
   const int lean = (dv & 3) == 0;
   int e = hk_launch(retention_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, cos_t, sin_t, rot,
                     positions, decay, rec, psegs, rec_rows, items, H, dk, dv, L, rpt, k_scale, lean);
@@ -881,8 +886,9 @@ HK_API int hk_mlstm_scan(const float* q, const float* k, const float* v, const f
   int e = hk_launch(mlstm_gates_kernel, dim3((unsigned)((n_seg * H + 3) / 4)), dim3(128), 0, s, il, fl, ld, i_bias, f_bias, segs,
                     m_state, gates, n_seg, H, cap);
   if (e) return e;
-  const long long items = (long long)(most_rows ? most_rows : n_rows) * H;
-  const int* psegs = most_rows ? segs : nullptr;
+  const int* psegs = prep_segments(segs, n_seg, most_rows);
+  const long long items = (long long)(psegs ? most_rows : n_rows) * H;
+  if (!psegs && rec_rows) return HK_ERR_UNSUPPORTED;
   e = hk_launch(mlstm_prep_kernel, prep_grid(items, psegs, n_seg), dim3(256), 0, s, q, k, v, ld, (const float*)gates, rec, psegs,
                 rec_rows, items, H, dk, dv, dvp, L, rpt, q_scale);
   if (e) return e;

@@ -115,3 +115,9 @@ def test_gates_and_maxima_of_the_matrix_memory(first_chunked):
             top = new
         assert bool(((m[r].double() - top).abs() <= 5e-5 * (1 + top.abs())).all())
         row += count
+
+
+def test_more_walked_requests_than_a_grid_is_high():
+    lengths = [1] * 65536 + [64]
+    t = inputs("general", 1, 4, 4, lengths, torch.Generator(DEV).manual_seed(3))
+    same(scan("general", 1, 4, 4, lengths, t, 65536), scan("general", 1, 4, 4, lengths, t, len(lengths)))

@@ -56,3 +56,12 @@ def test_which_steps_of_a_recurrence_go_in_chunks():
     assert taken(32, [700, 301, 77, 1]) == [700, 301, 77] and taken(32, [1500, 100, 63]) == [1500, 100]
     assert taken(32, [639]) == [] and taken(8, [1000]) == [1000] and taken(320, [319]) == []
     assert taken(300, [400]) == [400] and taken(300, [400, 64]) == []
+
+
+def test_scratch_of_a_walk_beside_chunks():
+    from hk_b200.csrc import ops
+    assert ops.walk_rows(1079, 1, 1) == (1, 1)              # one token beside 1,078 rows in chunks
+    assert ops.walk_rows(1079, 3, 63) == (189, 63) and ops.walk_rows(400, 20, 1) == (20, 1)
+    assert ops.walk_rows(206, 2, 130) == (206, 0)           # as many as the step has: its rows
+    assert ops.walk_rows(500, 7, 0) == (500, 0)             # nothing beside
+    assert ops.walk_rows(70000, 65536, 1) == (70000, 0) and ops.walk_rows(70000, 65535, 1) == (65535, 1)
