@@ -26,8 +26,6 @@
 // warp per position, online softmax); scale on q first: src/engine/attention_kernel.zig:109.
 #include <math_constants.h>
 
-#include <type_traits>
-
 #include "common.cuh"
 
 #define AG_WARPS 4
@@ -303,25 +301,27 @@ __device__ __forceinline__ void attention_f32_item(AfSmem& sm, const AfItem it, 
       if ((tid & 3) == 0) sm.corr[sr] = corr;
     }
     asm volatile("cp.async.wait_group 1;" ::: "memory");          // the values
-    float odd = 0.f;                                              // NaN with NaN or Inf among the pieces that this thread fetched
+    bool apart = false;                                           // NaN or Inf among values that some row does not see
     if (j0 < first_key(it.pos0 + it.n_tokens - 1) || j0 + AF_KEYS - 1 > it.pos0) {
+      float odd = 0.f;                                            // NaN if one of the pieces that this thread fetched holds any
 #pragma unroll 4
       for (int e = tid; e < AF_KEYS * (AF_HD / 4); e += AF_TH) {
         const float4 x = *reinterpret_cast<const float4*>(sm.v + (e / (AF_HD / 4)) * AF_LD + (e % (AF_HD / 4)) * 4);
         odd = fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, fmaf(x.w, 0.f, odd))));
       }
+      apart = __syncthreads_or(odd != 0.f);
+    } else {
+      __syncthreads();
     }
-    const bool apart = __syncthreads_or(odd != 0.f);
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const float c = sm.corr[ty + 8 * i];
 #pragma unroll
       for (int b = 0; b < 2; ++b) acc[i][b] = make_float4(acc[i][b].x * c, acc[i][b].y * c, acc[i][b].z * c, acc[i][b].w * c);
     }
-    const int c_end = min(AF_KEYS, kv_hi - j0);                   // behind the last row's own key there is nothing
-    auto add = [&](auto seen_alone) {
+    if (!apart) {
 #pragma unroll 2
-      for (int c = 0; c < c_end; c += 4) {
+      for (int c = 0; c < AF_KEYS; c += 4) {
         float4 p[RI];
 #pragma unroll
         for (int i = 0; i < RI; ++i) p[i] = *reinterpret_cast<const float4*>(sm.p + (ty + 8 * i) * AF_LDP + c);
@@ -331,21 +331,27 @@ __device__ __forceinline__ void attention_f32_item(AfSmem& sm, const AfItem it, 
           const float4 v1 = *reinterpret_cast<const float4*>(sm.v + (c + e) * AF_LD + 64 + 4 * tx);
 #pragma unroll
           for (int i = 0; i < RI; ++i) {
-            if (decltype(seen_alone)::value) {
-              const int key = j0 + c + e, pos = it.pos0 + (ty + 8 * i) / group;
-              if (key > pos || key < first_key(pos)) continue;
-            }
             const float w = e == 0 ? p[i].x : e == 1 ? p[i].y : e == 2 ? p[i].z : p[i].w;
             acc[i][0] = make_float4(fmaf(w, v0.x, acc[i][0].x), fmaf(w, v0.y, acc[i][0].y), fmaf(w, v0.z, acc[i][0].z), fmaf(w, v0.w, acc[i][0].w));
             acc[i][1] = make_float4(fmaf(w, v1.x, acc[i][1].x), fmaf(w, v1.y, acc[i][1].y), fmaf(w, v1.z, acc[i][1].z), fmaf(w, v1.w, acc[i][1].w));
           }
         }
       }
-    };
-    if (apart)
-      add(std::true_type{});
-    else
-      add(std::false_type{});
+    } else {
+#pragma unroll
+      for (int i = 0; i < RI; ++i) {
+        const int r = ty + 8 * i, pos = it.pos0 + r / group;
+#pragma unroll 1
+        for (int c = max(0, first_key(pos) - j0); c < min(AF_KEYS, pos + 1 - j0); ++c) {
+          const float w = sm.p[r * AF_LDP + c];
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const float4 x = *reinterpret_cast<const float4*>(sm.v + c * AF_LD + 64 * b + 4 * tx);
+            acc[i][b] = make_float4(fmaf(w, x.x, acc[i][b].x), fmaf(w, x.y, acc[i][b].y), fmaf(w, x.z, acc[i][b].z), fmaf(w, x.w, acc[i][b].w));
+          }
+        }
+      }
+    }
     __syncthreads();
     if (t + 1 < tiles) fetch(v_pages, sm.v, t + 1, vd, opt.v_stride);
     else asm volatile("cp.async.commit_group;" ::: "memory");
