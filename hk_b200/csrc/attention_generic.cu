@@ -173,8 +173,8 @@ HK_API int hk_attention_generic(const void* q, const void* k_pages, const void* 
 // beside rows that are not finite: a tile with keys that some row does not see looks for NaN and Inf among its values (a
 // probability of zero would not keep them out) and, if there are any, adds for every row the keys that it sees alone.  Up
 // to 8 rows (single tokens) do a quarter of the arithmetic.  Bound by what shared memory delivers (two thirds of the fp32 rate).
-// 16 heads of 128 over 8, us, the kernel above and this: 509 tokens 484 and 132; single tokens behind 2,000: one 415 and 357, 64 (32
-// heads) 1,697 and 877; 2,048 tokens of 32 heads 13,658 and 2,009.
+// 16 heads of 128 over 8, us, the kernel above and this: 509 tokens 484 and 139; single tokens behind 2,000: one 415 and 360, 64 (32
+// heads) 1,697 and 869; 2,048 tokens of 32 heads 13,658 and 2,040 (2,018 without the look at the values).
 namespace {
 constexpr int AF_ROWS = 32, AF_KEYS = 64, AF_HD = 128, AF_LD = AF_HD + 4, AF_LDP = AF_KEYS + 4, AF_TH = 128;
 struct AfItem {

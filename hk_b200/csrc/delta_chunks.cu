@@ -22,9 +22,10 @@
 // A value, key, gate or decay that is NaN or Inf reaches its own token and later ones, as in the walk: the products with triangular
 // matrices leave out what stands above the diagonal (`triangle_rows`), which a zero there would not keep out.
 //
-// One request of 2,048 tokens at 64 heads of 64 x 64 (walk token by token -> here): generalised rule 994 -> 435 us, gated rule
-// 989 -> 405, matrix memory 1,089 -> 296, retention 607 -> 211; of 1,000 at 32 heads 392 -> 144, 390 -> 138, 428 -> 111,
-// 241 -> 68; of 64 tokens level (39 -> 38, 42 -> 35, 57 -> 52, 30 -> 30), of 128 61 -> 38, 61 -> 38, 78 -> 54, 42 -> 31.
+// One request of 2,048 tokens at 64 heads of 64 x 64 (walk token by token -> here, L2 cold): generalised rule 988 -> 433 us, gated
+// rule 978 -> 402, matrix memory 1,074 -> 284, retention 605 -> 206; of 1,000 at 32 heads 390 -> 140, 390 -> 138, 417 -> 103,
+// 241 -> 64; at 64 heads of 64 tokens level (42 -> 38, 46 -> 40, 54 -> 40, 32 -> 30), of 128 75 -> 48, 79 -> 48, 89 -> 46, 50 -> 36.
+// (With the triangular products whole: 429, 400, 284, 212 at 2,048 tokens.)
 // Relative error against 64 bits at 2,048 tokens: 5.3e-7 -> 5.1e-7, 5.5e-7 -> 5.3e-7, 7.1e-7 -> 7.0e-7, 5.2e-7 -> 1.9e-7.
 #include "common.cuh"
 
@@ -142,7 +143,7 @@ struct DeltaSmem {
 }  // namespace
 
 // ------------------------------------------------------------------ 1. local part with a removal term
-// Bound by its multiply-adds (1.05 M a block, of which a third of the rate goes to operands that no register keeps: 8 x 4
+// Bound by its multiply-adds (0.9 M a block, of which a third of the rate goes to operands that no register keeps: 8 x 4
 // outputs a thread from 16-byte loads of shared memory).  70 KB of shared memory and 128 threads: three blocks share an SM.
 template <bool GATED>
 __global__ void __launch_bounds__(NTH, 3)

@@ -3,8 +3,9 @@
 //
 // A step's batch is described by a segment table int32 [n_seg, 3] = (state slot, first row, rows): the rows
 // of a request are consecutive and in increasing position.  Every scan walks a segment's rows in order, one
-// token after the other, whatever the cut of the prompt was, so the state after a token (and every sum's
-// order) depends on the tokens before it alone: never on the portion sizes, the batch or the slot.  (Steps with a long
+// token after the other, whatever the cut of the prompt was, so the state after a token depends on the tokens before it alone,
+// never on the portion sizes or the slot; the number of requests decides how many lanes share a column (`dr_plan`), and with
+// it the order of a column's sum over the keys.  (Steps with a long
 // portion take `delta_chunks.cu` instead in bfloat16 models; these scans are the 32-bit path, decode and shorter portions.)
 //
 //   * generalised delta rule (per head a matrix state S [dk, dv]):
@@ -51,7 +52,8 @@ static dim3 prep_grid(long long items, const int* segs, int n_seg) {
 __global__ void delta_rule_prep_kernel(const float* __restrict__ r, const float* __restrict__ k, const float* __restrict__ v,
                                        const float* __restrict__ al, long long ld, const float* __restrict__ wl, long long ldw,
                                        const float* __restrict__ a_bias, const float* __restrict__ w_bias, float* __restrict__ rec,
-                                       const int* __restrict__ psegs, int rec_rows, long long items, int H, int dk, int dv, int L, int RPT, float decay_scale, float key_eps) {
+                                       const int* __restrict__ psegs, int rec_rows, long long items, int H, int dk, int dv, int L, int RPT,
+                                       float decay_scale, float key_eps) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long at;
   const int lane = threadIdx.x & 31;
@@ -362,8 +364,8 @@ static int dr_scan_records(const float* rec, const int* segs, int n_seg, float* 
 // `most_rows` > 0: the segments do not hold all of the step's rows, and none holds more than so many; only theirs are prepared.
 // With `rec_rows` (0, or at least most_rows) > 0 `rec` holds so many rows per segment instead, n_seg * rec_rows.
 HK_API int hk_delta_rule_scan(const float* r, const float* k, const float* v, const float* al, long long ld, const float* wl,
-                              long long ldw, const float* a_bias, const float* w_bias, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows,
-                              float* rec, float* state, float* out, int H, int dk, int dv, float decay_scale, float key_eps,
+                              long long ldw, const float* a_bias, const float* w_bias, const int* segs, int n_seg, int n_rows,
+                              int most_rows, int rec_rows, float* rec, float* state, float* out, int H, int dk, int dv, float decay_scale, float key_eps,
                               void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
   if (H < 1 || dk < 1 || dv < 1 || dk > 2048 || ((uintptr_t)rec & 15)) return HK_ERR_UNSUPPORTED;
@@ -483,8 +485,8 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log
 __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                         long long ld, const float* __restrict__ bl, const float* __restrict__ al, long long ldg,
                                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ rec,
-                                        const int* __restrict__ psegs, int rec_rows, long long items, int H, int G, int dk, int dv, int L, int RPT, float q_scale,
-                                        float unit_eps) {
+                                        const int* __restrict__ psegs, int rec_rows, long long items, int H, int G, int dk, int dv, int L, int RPT,
+                                        float q_scale, float unit_eps) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long at;
   const int lane = threadIdx.x & 31;
@@ -528,8 +530,8 @@ __global__ void gated_delta_prep_kernel(const float* __restrict__ q, const float
 // q, k [n, G*dk] and v [n, H*dv] are column slices of one float32 matrix (row stride ld), already convolved and
 // activated; b_logit and a_logit [n, H] slices of one (row stride ldg).  `rec` as for hk_delta_rule_scan.
 HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, long long ld, const float* bl, const float* al,
-                               long long ldg, const float* a_log, const float* dt_bias, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows,
-                               float* rec, float* state, float* out, int H, int G, int dk, int dv, float q_scale, float unit_eps,
+                               long long ldg, const float* a_log, const float* dt_bias, const int* segs, int n_seg, int n_rows,
+                               int most_rows, int rec_rows, float* rec, float* state, float* out, int H, int G, int dk, int dv, float q_scale, float unit_eps,
                                void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
   if (H < 1 || G < 1 || H % G || dk < 1 || dv < 1 || dk > 2048 || ((uintptr_t)rec & 15)) return HK_ERR_UNSUPPORTED;
@@ -556,7 +558,8 @@ HK_API int hk_gated_delta_scan(const float* q, const float* k, const float* v, l
 __global__ void retention_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                                       long long ld, const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot,
                                       const int* __restrict__ positions, const float* __restrict__ decay, float* __restrict__ rec,
-                                      const int* __restrict__ psegs, int rec_rows, long long items, int H, int dk, int dv, int L, int RPT, float k_scale, int lean) {
+                                      const int* __restrict__ psegs, int rec_rows, long long items, int H, int dk, int dv, int L, int RPT,
+                                      float k_scale, int lean) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long at;
   const int lane = threadIdx.x & 31;
@@ -739,8 +742,8 @@ static int ret_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s
 // q, k [n, H*dk] and v [n, H*dv] are column slices of one float32 matrix (row stride ld); decay float32 [H]; `rec` as for
 // hk_delta_rule_scan.  Blocks, columns a block and columns a lane group are chosen as for the delta rule's scan.
 HK_API int hk_retention_scan(const float* q, const float* k, const float* v, long long ld, const float* cos_t, const float* sin_t,
-                             int rot, const int* positions, const float* decay, const int* segs, int n_seg, int n_rows, int most_rows, int rec_rows, float* rec,
-                             float* state, float* out, int H, int dk, int dv, float k_scale, void* stream) {
+                             int rot, const int* positions, const float* decay, const int* segs, int n_seg, int n_rows,
+                             int most_rows, int rec_rows, float* rec, float* state, float* out, int H, int dk, int dv, float k_scale, void* stream) {
   if (n_seg <= 0 || n_rows <= 0) return 0;
   if (H < 1 || dk < 1 || dv < 1 || dk > 2048 || rot < 0 || rot > dk || (rot & 1) || ((uintptr_t)rec & 15)) return HK_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
@@ -843,8 +846,8 @@ HK_API int hk_mlstm_gates(const float* il, const float* fl, long long ld, const 
 }
 
 __global__ void mlstm_prep_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                  long long ld, const float* __restrict__ gates, float* __restrict__ rec, const int* __restrict__ psegs, int rec_rows, long long items, int H,
-                                  int dk, int dv, int dvp, int L, int RPT, float q_scale) {
+                                  long long ld, const float* __restrict__ gates, float* __restrict__ rec, const int* __restrict__ psegs, int rec_rows,
+                                  long long items, int H, int dk, int dv, int dvp, int L, int RPT, float q_scale) {
   long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long at;
   const int lane = threadIdx.x & 31;

@@ -3,7 +3,8 @@
 Both keep their state in float32 in the request's state slot (`StateSpec`) and find the rows of every request
 of a step through one host-built table, `segments` int32 [requests of the step, 3] = (slot, first row, rows),
 shared by all recurrent mixers of a model.  The scans (`csrc/recurrent.cu`) walk a request's rows in order, so
-what a position computes does not depend on how the prompt was cut, on the batch or on the slot.  In bfloat16 steps
+what a position computes does not depend on how the prompt was cut or on the slot, and on the batch only in how many lanes share
+a column's sum.  In bfloat16 steps
 with a long portion take it in chunks instead: the delta rules, the matrix memory and retention with the same float32 sums
 grouped by chunk (`csrc/delta_chunks.cu`), the state-space and the key-gated recurrence with kernels of their own.  There a
 prompt's cut, and through the choice the step's other requests, move a result by float32 rounding.  Projections
@@ -109,8 +110,8 @@ class _ChunkedScan(_SegmentScan):
     takes chunks when its longest request brings `LONGEST_FROM` tokens (half that with many heads: tokens times heads at least
     `ROWS_FROM`) and all rows to be chunked times the heads are at most
     `BESIDE` times the longest; then every request of `CHUNKS_FROM` tokens or more goes that way.  Scan kernels of the delta
-    rule with 64 heads, us in chunks and walked: one request of 2,048 tokens 423 and 988, one of 512 120 and 249, four of 512
-    423 and 576, nine of 227 474 and 373 (over the limit: walked); with 32 heads one of 512 76 and 193, nine of 100 137 and 121.
+    rule with 64 heads, us in chunks and walked: one request of 2,048 tokens 433 and 988, one of 512 130 and 257, four of 512
+    433 and 587, nine of 227 484 and 384 (over the limit: walked); with 32 heads one of 512 85 and 206, nine of 100 146 and 132.
     Below, the kernels still gain (one request of 512 tokens over 32 heads, see above), but the launches and tables of the longer
     route cost the host as much: requests of 34 and 471 tokens took 288 us walked and 309 with the longer one in chunks."""
     CHUNKS_FROM = 64
