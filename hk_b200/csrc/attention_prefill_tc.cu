@@ -380,7 +380,7 @@ attention_prefill_tc_kernel(const bf16* __restrict__ q, const bf16* __restrict__
     else if (alive && n > 0) mbar_arrive(&sm.v_full[(n - 1) % VSTAGES]);
   } else if (warp == 8) {
     // ================================================================= MMA issuer (one lane)
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = mbar_wait(&sm.q_full, 0, abort_flag);
       const uint32_t qs = smem_u32(sm.q);
       // scores of tile t into S buffer (t - t_begin) & 1
@@ -817,7 +817,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
     }
   } else if (warp == 8) {
     // ================================================================= MMA issuer (one lane)
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = mbar_wait(&sm.q_full, 0, abort_flag);
       const int nq = two ? 2 : 1;
       auto issue_s = [&](int qt, int n) {

@@ -79,7 +79,7 @@ def libraries_for(bfloat16: bool, model=None) -> List[str]:
 
 
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
-HEADERS: List[str] = ["common.cuh", "attention_noalloc.h"]
+HEADERS: List[str] = ["common.cuh", "gemm_tc.cuh", "attention_noalloc.h"]
 
 _loaded: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()

@@ -377,7 +377,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   if (warp == CONSUMERS) {
     // ---- producer ----
-    if (lane == 0) {
+    if (elect_one()) {
       int tile = ns > 0 ? (int)(u0 / kc) : own_first, c = ns > 0 ? (int)(u0 % kc) : 0;
       uint32_t i = 0;
       for (; i < (uint32_t)n_local; ++i) {
