@@ -37,6 +37,7 @@ LIBRARIES: Dict[str, str] = {
     "sampling": "sampling.cu",
     "random_init": "random_init.cu",
     "gemm_tc": "gemm_tc.cu",
+    "gemm_pair": "gemm_pair.cu",       # the tcgen05 product on pairs of SMs
     "gemm_smallm": "gemm_smallm.cu",
     "gemm_stream": "gemm_stream.cu",
     "attention_flash": "attention_flash.cu",
@@ -61,7 +62,7 @@ def libraries_for(bfloat16: bool, model=None) -> List[str]:
     name in their `kernel_libraries` (a recurrent mixer's scans, a routed feed-forward's kernels)."""
     needed = ["elementwise", "gemm_generic", "attention_generic"]
     if bfloat16:
-        needed += ["gemm_smallm", "gemm_stream", "gemm_tc"]
+        needed += ["gemm_smallm", "gemm_stream", "gemm_tc", "gemm_pair"]
         if model is None:
             needed += ["attention_flash", "attention_prefill_tc"]
 

@@ -4,7 +4,9 @@
     weights (gate/up, down, the output head), the weight-streaming mma.sync kernel (`gemm_smallm.cu`) for the
     smaller ones (q/k/v, o);
   * 9 to 16 rows: the streaming kernel at every shape;
-  * more rows (larger decode batches, prefill, mixed batches): the persistent tcgen05 kernel (`gemm_tc.cu`) with
+  * more than 128 rows (prefill, mixed batches): the tcgen05 kernel on pairs of SMs (`gemm_pair.cu`), unless the output has few
+    columns (`pair_config`);
+  * the rows between (larger decode batches) and those few columns: the persistent tcgen05 kernel (`gemm_tc.cu`) with
     the tile width that fills whole waves of SMs (`tc_config`), cutting K into slices when the output has fewer
     tiles than the GPU has SMs; up to 128 rows and from three slices on, the slices are added inside a cluster
     (`cluster_config`).
@@ -106,8 +108,9 @@ def tc_config(M: int, N: int, K: int, sms: int, swiglu: bool = False):
     """Tile width (a multiple of 16, of 32 with the SwiGLU epilogue) and number of K slices for the tcgen05 kernel.
     Very many tiles (prefill): the width, from 256 down to 192, whose tiles leave the least of the last wave of SMs
     empty, a tile costing its width plus a fixed part.  Several row tiles but few waves: `_tc_ragged_config`.  One row tile
-    (decode batches): with the SwiGLU epilogue the widest tile that gives every SM one (no slices: the epilogue cannot run on
-    partial sums without a second kernel); else 128- or 256-wide tiles with K cut into slices so that every SM streams a
+    (decode batches): with the SwiGLU epilogue, and from 48 columns an SM on, the narrowest tile that needs one wave (no slices: the
+    epilogue cannot run on partial sums without a second kernel; 64 rows by 20,544 x 4,096 39.6 us with 81 tiles of 256, 32.4 with
+    143 of 144); else 128- or 256-wide tiles with K cut into slices so that every SM streams a
     share of the weights.  (A finer cost model that also weighed wave tails chose more slices there and measured slower:
     the second kernel that adds the slices has a fixed cost.)"""
     m_tiles = -(-M // 128)
@@ -126,8 +129,8 @@ def tc_config(M: int, N: int, K: int, sms: int, swiglu: bool = False):
             if best is None or cost < best[0]:
                 best = (cost, cand)
         bn = best[1]
-    elif swiglu and m_tiles == 1:
-        bn = min(256, max(32, -(-N // sms + step - 1) // step * step))       # the narrowest tile width that needs one wave
+    elif m_tiles == 1 and (swiglu or N > 48 * sms) and N <= 256 * sms:
+        bn = min(256, max(32 if swiglu else 64, -(-N // sms + step - 1) // step * step))       # the narrowest tile width that needs one wave
         while bn < 256 and -(-N // bn) > sms:
             bn += step
     else:
@@ -263,6 +266,70 @@ def run_cluster(a, w, out, accumulate: bool, bn: int, slices: int) -> bool:
     return True
 
 
+PAIR_M = 128            # from here on the rows' padding to 32 instead of 128 and the pairs' larger tiles pay
+PAIR_K = 1024           # below, a tile's start and end weigh more than its loop: 4,096 x 512 by 527 rows 7.9 us, on pairs 8.7
+
+
+def _tc_time(M: int, N: int, K: int, bn: int, splits: int, sms: int) -> float:
+    """The time in us of the kernel of one SM a tile, fitted to 2,000 measured (shape, width, slices) as `pair_config`'s."""
+    tiles, k_blocks, last = -(-M // 128) * -(-N // bn), -(-K // 64), 0.0208 * bn
+    loop = k_blocks / splits * max(0.234, 0.024 + 0.00157 * bn)
+    slices = 1.7 + 1.4e-6 * M * N * splits if splits > 1 else 0.0
+    return max(-(-tiles * splits // sms) * max(loop, last), N * K / 2.92e6) + 0.5 * last + slices + 2.6
+
+
+@functools.lru_cache(maxsize=4096)
+def pair_config(M: int, N: int, K: int, sms: int, gated: bool = False):
+    """(tiles along the rows, K slices) of the product on pairs of SMs, or None where the kernel of one SM a tile stays: up to
+    128 rows, short K, and where two row tiles of that kernel fill one wave of SMs better (10,304 x 2,048 by 256 rows 15.5 us, on
+    pairs 17.6; 2,048 x 6,144 by 256 14.1 and 17.5, by 1,000 24.9 and 22.2).
+    Both times come from models that were fitted to measured ones, 130 to 2,048 rows by the products of layers 2,048 and 4,096
+    wide; what they pick is within 1 % of the best of the measured choices on average."""
+    pairs, units, k_blocks, f_tiles = sms // 2, -(-M // 32), -(-K // 64), -(-N // 256)
+    if M <= PAIR_M or K < PAIR_K:
+        return None
+    best = None
+    for tiles_m in range(-(-units // 8), min(units, -(-units // 8) + 7) + 1):
+        width, tiles = 32 * units / tiles_m, f_tiles * tiles_m
+        for slices in (1, 2, 3, 4):
+            if slices > 1 and (tiles * slices > pairs or k_blocks < 16 * slices):
+                break
+            loop, last = k_blocks / slices * max(0.184, 0.084 + 0.0012 * width), 0.0235 * width         # `last`: a tile's epilogue
+            waves = -(-tiles * slices // pairs)
+            cost = waves * max(loop, last) + 0.8 * (waves - 1) + 0.5 * last + (4.0 * slices - 1.0 if slices > 1 else 0.0)
+            if best is None or cost < best[0]:
+                best = (cost, tiles_m, slices)
+    if best[0] + 3.0 > 1.08 * _tc_time(M, N, K, *tc_config(M, N, K, sms, gated), sms):
+        return None
+    return best[1:]
+
+
+def run_pair(a, w, out, epilogue: int, ldo: int, tiles_m: int, slices: int, limit: float = 0.0, slope: float = 1.0) -> bool:
+    """The product on pairs of SMs; `epilogue` and its numbers as `hk_gemm_pair` takes them.  False when the kernel refuses."""
+    from . import ops
+    M, K = a.shape
+    N = w.shape[0]
+    lib = build.load("gemm_pair")
+    partial = None
+    if slices > 1:
+        lib.hk_gemm_pair_partial_floats.restype = ctypes.c_longlong
+        partial = torch.empty(int(lib.hk_gemm_pair_partial_floats(M, N, tiles_m, slices)), dtype=torch.float32, device=a.device)
+    code = lib.hk_gemm_pair(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(ldo), epilogue, tiles_m, slices, _sms(a.device) // 2,
+                            _ptr(partial) if slices > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)), ctypes.c_float(limit),
+                            ctypes.c_float(slope), _stream())
+    if code == _UNSUPPORTED:
+        return False
+    ops._check(code, "gemm (tcgen05, pairs)")
+    return True
+
+
+def _run_pair_where_chosen(a, w, out, epilogue: int, ldo: int, limit: float = 0.0, slope: float = 1.0) -> bool:
+    if _tc_bn or _tc_splits:
+        return False
+    chosen = pair_config(a.shape[0], w.shape[0], a.shape[1], _sms(a.device), epilogue in (2, 3, 4))
+    return chosen is not None and run_pair(a, w, out, epilogue, ldo, *chosen, limit, slope)
+
+
 def _tc_partial(lib, M: int, N: int, splits: int, device):
     """Scratch for the partial sums of `splits` K slices (None without slices)."""
     if splits <= 1:
@@ -292,6 +359,8 @@ def run(a, w, out, accumulate: bool, choice: Optional[str]) -> bool:
         if code == _UNSUPPORTED:
             return False
         ops._check(code, "gemm (small-M)")
+        return True
+    if _run_pair_where_chosen(a, w, out, 1 if accumulate else 0, N):
         return True
     clusters = None if _tc_bn or _tc_splits else cluster_config(M, N, K, _sms(a.device))
     if clusters is not None and run_cluster(a, w, out, accumulate, *clusters):
@@ -326,6 +395,8 @@ def run_swiglu(a, w_gate_up, out, choice: Optional[str] = None, act: int = 0, li
             return False
     if choice is None and M <= SMALL_M_AUTO:
         return False             # few rows, small weights: the small-M product and the swiglu kernel
+    if _run_pair_where_chosen(a, w_gate_up, out, epilogue, out.shape[1], limit, slope):
+        return True
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device), swiglu=True)
     partial = _tc_partial(lib, M, N, splits, a.device)
@@ -365,6 +436,8 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
             return False
         ops._check(code, "gemm+squared relu (small-M)")
         return True
+    if _run_pair_where_chosen(a, w, out, 5, N, slope=factor):
+        return True
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)
@@ -384,6 +457,8 @@ def run_narrow(a, w, out) -> bool:
     N = w.shape[0]
     if not _aligned(a, w):
         return False
+    if _run_pair_where_chosen(a, w, out, 6, N):
+        return True
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)

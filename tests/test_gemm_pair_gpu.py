@@ -1,0 +1,80 @@
+"""The product on pairs of SMs: rows, columns and K off every tile's edge, several tiles a pair, K slices, every epilogue; and the
+rule that chooses it."""
+import ctypes
+
+import pytest
+import torch
+
+
+def test_rule_gives_what_the_kernel_takes():
+    from hk_b200.csrc import gemm_fast
+    for refused in ((128, 24576, 4096), (527, 4096, 512), (256, 2048, 6144), (256, 10304, 2048)):
+        assert gemm_fast.pair_config(*refused, 148) is None
+    for m in (129, 200, 257, 384, 527, 1000, 2048, 4096, 8192):
+        for n, k in ((4096, 4096), (4096, 12288), (6144, 4096), (20544, 4096), (10304, 2048), (2048, 6144), (72, 512), (151936, 4096)):
+            for gated in (False, True):
+                got = gemm_fast.pair_config(m, n, k, 148, gated)
+                if got is None:
+                    assert k < 1024 or m < 600 or n < 4096          # what many rows by long rows of weights never get
+                    continue
+                tiles_m, slices = got
+                units = -(-m // 32)
+                assert 1 <= tiles_m <= units and -(-units // tiles_m) <= 8 and 1 <= slices <= -(-k // 64)
+
+
+def _reference(a, w, epilogue, start, limit, slope):
+    z = a.double() @ w.double().T
+    if epilogue in (2, 3, 4):
+        g, u = z.chunk(2, dim=1)
+        if epilogue == 4:
+            g, u = g.clamp(max=limit), u.clamp(-limit, limit) + 1
+            return g * torch.sigmoid(slope * g) * u
+        return (torch.nn.functional.silu(g) if epilogue == 2 else torch.nn.functional.gelu(g, approximate="tanh")) * u
+    return {0: z, 1: start.double() + z, 5: slope * z.clamp(min=0) ** 2, 6: z}[epilogue]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,tiles_m,slices,pairs", [
+    (1, 256, 64, 1, 1, 74), (33, 256, 72, 1, 1, 74), (100, 300, 200, 1, 1, 74), (129, 770, 1000, 1, 4, 74), (256, 512, 256, 1, 1, 1),
+    (250, 4098, 192, 1, 3, 2), (700, 514, 328, 4, 2, 5), (300, 1000, 520, 2, 1, 3), (527, 1030, 1024, 3, 1, 74), (2048, 1536, 136, 9, 1, 74)])
+@pytest.mark.parametrize("epilogue", range(7))
+def test_pair_product(M, N, K, tiles_m, slices, pairs, epilogue):
+    from hk_b200.csrc import build, gemm_fast, ops
+    gen = torch.Generator().manual_seed(M * 7 + K + epilogue)
+    a, w = torch.randn(M, K, generator=gen).bfloat16(), (torch.randn(N, K, generator=gen) / K ** 0.5).bfloat16()
+    columns, kind = (N // 2 if epilogue in (2, 3, 4) else N), (torch.float32 if epilogue < 2 else torch.bfloat16)
+    guard = torch.full((M + 40, columns), 5.0, dtype=kind, device="cuda")
+    start = torch.randn(M, columns, generator=gen).to(kind)
+    guard[:M] = start.cuda()
+    lib = build.load("gemm_pair")
+    lib.hk_gemm_pair_partial_floats.restype = ctypes.c_longlong
+    partial = torch.full((int(lib.hk_gemm_pair_partial_floats(M, N, tiles_m, slices)),), float("nan"), device="cuda")
+    da, dw = a.cuda(), w.cuda()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())      # noqa: E731
+    limit, slope = 0.8, 1.702
+    assert lib.hk_gemm_pair(p(da), p(dw), p(guard), M, N, K, ctypes.c_longlong(columns), epilogue, tiles_m, slices, pairs, p(partial),
+                            p(gemm_fast.status_flag(guard.device)), ctypes.c_float(limit), ctypes.c_float(slope), ops._stream()) == 0
+    gemm_fast.check_status(guard.device)
+    want, got = _reference(a, w, epilogue, start, limit, slope), guard[:M].double().cpu()
+    # 32-bit sums of exact products: each of at most K + slices additions rounds by 2^-24 of the sum of magnitudes; the tensor
+    # core may cut instead of round within a step of 16, which doubles that.  A narrowed result is rounded by 2^-9 of itself, and an
+    # activation's slope is at most 1.2 (a squared relu's 2 |z|): the sums are of order 1, so their error vanishes beside that
+    sums = (a.double().abs() @ w.double().abs().T) * (K + slices) * 2 ** -23
+    if epilogue < 2:
+        bound = sums + (start.double().abs() * 2 ** -23 if epilogue else 0)
+    else:
+        bound = want.abs() * 2 ** -8 + 16 * sums.max() + 1e-6
+    assert bool(((got - want).abs() <= bound).all())
+    assert bool((guard[M:] == 5.0).all())
+    assert float((got - want).norm() / want.norm()) < (1e-5 if epilogue < 2 else 3e-3)       # a dropped K block would be 1e-1
+
+
+@pytest.mark.gpu
+def test_pair_refusals():
+    from hk_b200.csrc import gemm_fast
+    a, w = torch.zeros(300, 512, dtype=torch.bfloat16, device="cuda"), torch.zeros(4096, 512, dtype=torch.bfloat16, device="cuda")
+    out = torch.full((300, 4096), 3.0, device="cuda")
+    for tiles_m, slices in ((0, 1), (1, 1), (11, 1), (2, 0), (2, 9)):
+        assert not gemm_fast.run_pair(a, w, out, 0, 4096, tiles_m, slices)
+    assert not gemm_fast.run_pair(a, w[:4095], out, 2, 4096, 2, 1)
+    assert bool((out == 3.0).all())
