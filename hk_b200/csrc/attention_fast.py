@@ -10,7 +10,6 @@ positions), never on values.
 """
 from __future__ import annotations
 
-import ctypes
 import math
 from dataclasses import dataclass
 from typing import Callable, Optional
@@ -18,7 +17,7 @@ from typing import Callable, Optional
 import numpy as np
 import torch
 
-from . import build
+from . import build, gemm_fast, ops
 
 _UNSUPPORTED = 100001
 TILE_N = 64
@@ -198,7 +197,7 @@ def build_plan(slots, q_starts, q_lens, start_positions, n_tokens: int, window: 
 
 
 def _ptr(t):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def tma_decode_supported(hd: int, group: int, page_tokens: int) -> bool:
@@ -214,14 +213,13 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
     """Runs the step on the flash kernels.  Returns False when they refuse it, True when `out` holds the attention, and
     GATED when it holds the attention times gate_scale * sigmoid(gate) (the tcgen05 prompt kernels apply a gate whose
     rows are 16-byte aligned in their epilogue; after any other kernel the caller applies it)."""
-    from . import gemm_fast, ops
     if not supported(hd, H // G) or plan is None:
         return False
     sk = 1 if sink else 0
-    extra = (_ptr(sinks), ctypes.c_float(softcap), int(chunk))
+    extra = (_ptr(sinks), softcap, int(chunk))
     bias = (_ptr(dist), int(dist.shape[1]) if dist is not None else 0)      # per query head and distance, in the base-2 domain
     fused_gate = gate is not None and gate.data_ptr() % 16 == 0 and gate.stride(0) % 4 == 0 and gate.stride(1) == 1
-    gate_args = (_ptr(gate if fused_gate else None), ctypes.c_longlong(gate.stride(0) if fused_gate else 0), ctypes.c_float(gate_scale))
+    gate_args = (_ptr(gate if fused_gate else None), gate.stride(0) if fused_gate else 0, gate_scale)
     done = GATED if fused_gate else True
     lib = build.load("attention_flash")
     stream = ops._stream()
@@ -235,9 +233,9 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
             return False
         lib_tc = build.load("attention_prefill_tc")
         code = lib_tc.hk_attention_prefill_tc2(
-            _ptr(q), _ptr(k_pages), _ptr(v_pages), ctypes.c_longlong(k_pages.shape[0]), _ptr(block_table),
+            _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
             int(block_table.shape[1]), _ptr(plan.items), plan.n_items, _ptr(out), H, G, hd, int(page_tokens), int(window),
-            ctypes.c_float(scale * math.log2(math.e)), plan.max_keys // int(page_tokens) + 2,
+            scale * math.log2(math.e), plan.max_keys // int(page_tokens) + 2,
             _ptr(gemm_fast.status_flag(q.device)), sk, *extra, *gate_args, *bias, stream)
         if code == _UNSUPPORTED:
             return False
@@ -249,7 +247,7 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
         lib_tc = build.load("attention_prefill_tc")
         code = lib_tc.hk_attention_prefill_tc(
             _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), int(block_table.shape[1]), _ptr(plan.items),
-            plan.n_items, _ptr(out), H, G, hd, int(page_tokens), int(window), ctypes.c_float(scale * math.log2(math.e)),
+            plan.n_items, _ptr(out), H, G, hd, int(page_tokens), int(window), scale * math.log2(math.e),
             plan.max_keys // int(page_tokens) + 2, _ptr(gemm_fast.status_flag(q.device)), sk, *extra, *gate_args, *bias, stream)
         if code == _UNSUPPORTED:
             return False
@@ -258,14 +256,14 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
     code = _UNSUPPORTED
     if plan.nw == 1 and allow_tma and tma_decode_supported(hd, H // G, int(page_tokens)):
         code = lib.hk_attention_decode_tma(
-            _ptr(q), _ptr(k_pages), _ptr(v_pages), ctypes.c_longlong(k_pages.shape[0]), _ptr(block_table),
+            _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
             int(block_table.shape[1]), _ptr(plan.items), plan.n_items, _ptr(out), _ptr(part_o), _ptr(part_ml), H, G, hd,
-            int(page_tokens), int(window), ctypes.c_float(scale * math.log2(math.e)), sk, plan.max_keys // int(page_tokens) + 2,
+            int(page_tokens), int(window), scale * math.log2(math.e), sk, plan.max_keys // int(page_tokens) + 2,
             _ptr(gemm_fast.status_flag(q.device)), *extra, *bias, stream)
     if code == _UNSUPPORTED:
         code = lib.hk_attention_flash(_ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(block_table), int(block_table.shape[1]),
                                       _ptr(plan.items), plan.n_items, plan.nw, _ptr(out), _ptr(part_o), _ptr(part_ml), H, G, hd,
-                                      int(page_tokens), int(window), ctypes.c_float(scale * math.log2(math.e)), sk,
+                                      int(page_tokens), int(window), scale * math.log2(math.e), sk,
                                       plan.max_keys // int(page_tokens) + 2, *extra, *bias, stream)
     if code == _UNSUPPORTED:
         return False
@@ -292,7 +290,6 @@ def run_latent(q, pages, block_table, out, H: int, dk: int, dv: int, page_tokens
     """out bf16 [n, H * dv] from q bf16 [n, H * dk] over the cache rows `pages` [pages, 1, page_tokens, dk]; the plan's
     items hold at most 64 / H tokens each (a plan made with `plan_arrays(..., H, 1, ...)`).  `single_tokens`: every item
     holds one token (a decode step), which the kernel's decode variant takes."""
-    from . import ops
     if not latent_supported(H, dk, dv) or plan is None:
         return False
     lib = build.load("attention_latent")
@@ -303,7 +300,7 @@ def run_latent(q, pages, block_table, out, H: int, dk: int, dv: int, page_tokens
         part_ml = torch.empty((plan.n_parts, LATENT_ROWS, 2), dtype=torch.float32, device=q.device)
     code = lib.hk_attention_latent(_ptr(q), _ptr(pages), _ptr(block_table), int(block_table.shape[1]), _ptr(plan.items),
                                    plan.n_items, _ptr(out), _ptr(part_o), _ptr(part_ml), H, dk, dv, int(page_tokens), int(window),
-                                   ctypes.c_float(scale * math.log2(math.e)), 1 if single_tokens else 0, stream)
+                                   scale * math.log2(math.e), 1 if single_tokens else 0, stream)
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "latent attention")
@@ -354,12 +351,11 @@ def run_made(q, kv, rope, items, out, H: int, window: int, scale: float, c, w_uv
     """out bf16 [n, H * 128] of the items' rows, from q bf16 [n, H * (128 + 64)] (128 without `rope`), kv bf16 [rows, H * 256] =
     per head 128 key dims and 128 value dims, and rope bf16 [rows, 64], the key dims that all heads share (or None).  c bf16
     [rows, r] and w_uv bf16 [H, 128, r]: what the values were made of, for the rows of `firsts`."""
-    from . import gemm_fast, ops
     stream = ops._stream()
-    gated = (_ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), 1 if gate_per_head else 0, ctypes.c_float(gate_scale))
-    scale_log2 = ctypes.c_float(scale * math.log2(math.e))
+    gated = (_ptr(gate), gate.stride(0) if gate is not None else 0, 1 if gate_per_head else 0, gate_scale)
+    scale_log2 = scale * math.log2(math.e)
     lib = build.load("attention_prefill_tc")
-    code = lib.hk_attention_prefill_made(_ptr(q), _ptr(kv), _ptr(rope), ctypes.c_longlong(kv.shape[0]), _ptr(items), int(items.shape[0]),
+    code = lib.hk_attention_prefill_made(_ptr(q), _ptr(kv), _ptr(rope), kv.shape[0], _ptr(items), int(items.shape[0]),
                                          _ptr(out), H, int(window), scale_log2, _ptr(gemm_fast.status_flag(q.device)), *gated, stream)
     ops._check(code, "latent attention (made keys and values)")
     if not firsts.shape[0]:

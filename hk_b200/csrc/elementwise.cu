@@ -1426,3 +1426,24 @@ HK_API int hk_diff_heads_out(const void* a, int a_dtype, const float* gate, long
                      lambda, eps, out_scale);
   return HK_ERR_UNSUPPORTED;
 }
+
+// One request's slot of every state of a cache: table [states, 2] = (address, bytes a slot).  Bound by its launch: a slot is a few
+// MB at most, and a launch for each state was what opening a request cost.
+__global__ void __launch_bounds__(256)
+zero_slot_kernel(const long long* __restrict__ table, int slot) {
+  const long long bytes = table[2 * blockIdx.y + 1];
+  uint8_t* p = reinterpret_cast<uint8_t*>(table[2 * blockIdx.y]) + slot * bytes;
+  const long long head = min(bytes, (long long)(-(uintptr_t)p & 15)), wide = (bytes - head) >> 4, tail = head + (wide << 4);
+  const long long i0 = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+  for (long long i = i0; i < wide; i += step) reinterpret_cast<uint4*>(p + head)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (i0 < head) p[i0] = 0;
+  if (i0 < bytes - tail) p[tail + i0] = 0;
+}
+
+HK_API int hk_zero_slot(const long long* table, int n_states, int slot, long long most_bytes, void* stream) {
+  if (n_states <= 0 || most_bytes <= 0) return 0;
+  if (slot < 0 || n_states > 65535) return HK_ERR_UNSUPPORTED;
+  const long long blocks = (most_bytes + 16 * 1024 - 1) / (16 * 1024);
+  return hk_launch(zero_slot_kernel, dim3((unsigned)(blocks < 148 ? blocks : 148), (unsigned)n_states), dim3(256), 0, (cudaStream_t)stream,
+                   table, slot);
+}

@@ -15,13 +15,12 @@ Shapes all of them refuse (K not a multiple of 8, unaligned operands) go to the 
 """
 from __future__ import annotations
 
-import ctypes
 import functools
 from typing import Optional
 
 import torch
 
-from . import build
+from . import build, ops
 
 _UNSUPPORTED = 100001
 SMALL_M = 64          # the most rows the weight-streaming kernel takes
@@ -53,13 +52,12 @@ def _sms(device: torch.device) -> int:
     return _sm_count[key]
 
 
-def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+def _ptr(t) -> int:
+    return t.data_ptr()
 
 
-def _stream():
-    from .ops import _stream as current
-    return current()
+def _stream() -> int:
+    return ops._stream()
 
 
 def _aligned(a, w) -> bool:
@@ -164,7 +162,6 @@ def _stream_buffers(device: torch.device, lib):
     if key not in _stream_scratch:
         if torch.cuda.is_current_stream_capturing():
             return None
-        lib.hk_gemm_stream_workspace.restype = ctypes.c_longlong
         ws = torch.empty(int(lib.hk_gemm_stream_workspace(STREAM_M, 8)), dtype=torch.float32, device=device)
         ct = torch.zeros(STREAM_MAX_N // 16 + 2, dtype=torch.int32, device=device)
         _stream_scratch[key] = (ws, ct)
@@ -195,7 +192,6 @@ def stream_wanted(M: int, N: int, K: int) -> bool:
 def run_stream(a, w, out, epilogue: int, ldo: int, limit: float = 0.0, slope: float = 1.0) -> bool:
     """The persistent streaming kernel; epilogue 0 store, 1 add, 2 silu(gate) * up (3: tanh gelu; 4: the clamped form with
     its limit and slope) over w = [gate rows | up rows], 5 slope * max(z, 0)^2 in bf16."""
-    from . import ops
     M, K = a.shape
     N = w.shape[0]
     if M > STREAM_M or N > STREAM_MAX_N:
@@ -206,15 +202,15 @@ def run_stream(a, w, out, epilogue: int, ldo: int, limit: float = 0.0, slope: fl
         return False
     ws, ct = scratch
     if epilogue == 4:
-        code = lib.hk_gemm_stream_clamped(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(ldo),
+        code = lib.hk_gemm_stream_clamped(_ptr(a), _ptr(w), _ptr(out), M, N, K, ldo,
                                           stream_row_warps(N, _sms(a.device)), _ptr(ws), _ptr(ct), _ptr(status_flag(a.device)),
-                                          _stream_ctas, ctypes.c_float(limit), ctypes.c_float(slope), _stream())
+                                          _stream_ctas, limit, slope, _stream())
     elif epilogue == 5:
-        code = lib.hk_gemm_stream_sqrelu(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(ldo),
+        code = lib.hk_gemm_stream_sqrelu(_ptr(a), _ptr(w), _ptr(out), M, N, K, ldo,
                                          stream_row_warps(N, _sms(a.device)), _ptr(ws), _ptr(ct), _ptr(status_flag(a.device)),
-                                         _stream_ctas, ctypes.c_float(slope), _stream())
+                                         _stream_ctas, slope, _stream())
     else:
-        code = lib.hk_gemm_stream(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(ldo), epilogue,
+        code = lib.hk_gemm_stream(_ptr(a), _ptr(w), _ptr(out), M, N, K, ldo, epilogue,
                                   stream_row_warps(N, _sms(a.device)),
                                   _ptr(ws), _ptr(ct), _ptr(status_flag(a.device)), _stream_ctas, _stream())
     if code == _UNSUPPORTED:
@@ -255,10 +251,9 @@ def cluster_config(M: int, N: int, K: int, sms: int):
 
 def run_cluster(a, w, out, accumulate: bool, bn: int, slices: int) -> bool:
     """out (fp32) = a w^T (+ out) with the K slices added inside clusters.  False when the kernel refuses."""
-    from . import ops
     M, K = a.shape
     N = w.shape[0]
-    code = build.load("gemm_tc").hk_gemm_tc_cluster(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), 1 if accumulate else 0,
+    code = build.load("gemm_tc").hk_gemm_tc_cluster(_ptr(a), _ptr(w), _ptr(out), M, N, K, N, 1 if accumulate else 0,
                                                     bn, slices, _ptr(status_flag(a.device)), _stream())
     if code == _UNSUPPORTED:
         return False
@@ -306,17 +301,15 @@ def pair_config(M: int, N: int, K: int, sms: int, gated: bool = False):
 
 def run_pair(a, w, out, epilogue: int, ldo: int, tiles_m: int, slices: int, limit: float = 0.0, slope: float = 1.0) -> bool:
     """The product on pairs of SMs; `epilogue` and its numbers as `hk_gemm_pair` takes them.  False when the kernel refuses."""
-    from . import ops
     M, K = a.shape
     N = w.shape[0]
     lib = build.load("gemm_pair")
     partial = None
     if slices > 1:
-        lib.hk_gemm_pair_partial_floats.restype = ctypes.c_longlong
         partial = torch.empty(int(lib.hk_gemm_pair_partial_floats(M, N, tiles_m, slices)), dtype=torch.float32, device=a.device)
-    code = lib.hk_gemm_pair(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(ldo), epilogue, tiles_m, slices, _sms(a.device) // 2,
-                            _ptr(partial) if slices > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)), ctypes.c_float(limit),
-                            ctypes.c_float(slope), _stream())
+    code = lib.hk_gemm_pair(_ptr(a), _ptr(w), _ptr(out), M, N, K, ldo, epilogue, tiles_m, slices, _sms(a.device) // 2,
+                            _ptr(partial) if slices > 1 else 0, _ptr(status_flag(a.device)), limit,
+                            slope, _stream())
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "gemm (tcgen05, pairs)")
@@ -334,13 +327,11 @@ def _tc_partial(lib, M: int, N: int, splits: int, device):
     """Scratch for the partial sums of `splits` K slices (None without slices)."""
     if splits <= 1:
         return None
-    lib.hk_gemm_tc_partial_floats.restype = ctypes.c_longlong
     return torch.empty(int(lib.hk_gemm_tc_partial_floats(M, N, splits)), dtype=torch.float32, device=device)
 
 
 def run(a, w, out, accumulate: bool, choice: Optional[str]) -> bool:
     """out (fp32) = a w^T (+ out).  Returns False when no tensor-core kernel takes the shape."""
-    from . import ops
     M, K = a.shape
     N = w.shape[0]
     if not _aligned(a, w):
@@ -354,7 +345,7 @@ def run(a, w, out, accumulate: bool, choice: Optional[str]) -> bool:
         if M > SMALL_M:
             return False
         lib = build.load("gemm_smallm")
-        code = lib.hk_gemm_smallm(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), 1 if accumulate else 0,
+        code = lib.hk_gemm_smallm(_ptr(a), _ptr(w), _ptr(out), M, N, K, N, 1 if accumulate else 0,
                                   row_tiles(M, N, a.device), _stream())
         if code == _UNSUPPORTED:
             return False
@@ -368,8 +359,8 @@ def run(a, w, out, accumulate: bool, choice: Optional[str]) -> bool:
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)
-    code = lib.hk_gemm_tc(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), 1 if accumulate else 0, bn,
-                          splits, _ptr(partial) if splits > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)), _stream())
+    code = lib.hk_gemm_tc(_ptr(a), _ptr(w), _ptr(out), M, N, K, N, 1 if accumulate else 0, bn,
+                          splits, _ptr(partial) if splits > 1 else 0, _ptr(status_flag(a.device)), _stream())
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "gemm (tcgen05)")
@@ -383,7 +374,6 @@ def run_swiglu(a, w_gate_up, out, choice: Optional[str] = None, act: int = 0, li
     if act not in (0, 1, 2):
         return False
     epilogue = 2 + int(act)
-    from . import ops
     M, K = a.shape
     N = w_gate_up.shape[0]
     if not _aligned(a, w_gate_up) or N % 2:
@@ -401,12 +391,12 @@ def run_swiglu(a, w_gate_up, out, choice: Optional[str] = None, act: int = 0, li
     bn, splits = tc_config(M, N, K, _sms(a.device), swiglu=True)
     partial = _tc_partial(lib, M, N, splits, a.device)
     if epilogue == 4:
-        code = lib.hk_gemm_tc_clamped(_ptr(a), _ptr(w_gate_up), _ptr(out), M, N, K, ctypes.c_longlong(out.shape[1]), bn, splits,
-                                      _ptr(partial) if splits > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)),
-                                      ctypes.c_float(limit), ctypes.c_float(slope), _stream())
+        code = lib.hk_gemm_tc_clamped(_ptr(a), _ptr(w_gate_up), _ptr(out), M, N, K, out.shape[1], bn, splits,
+                                      _ptr(partial) if splits > 1 else 0, _ptr(status_flag(a.device)),
+                                      limit, slope, _stream())
     else:
-        code = lib.hk_gemm_tc(_ptr(a), _ptr(w_gate_up), _ptr(out), M, N, K, ctypes.c_longlong(out.shape[1]), epilogue, bn,
-                              splits, _ptr(partial) if splits > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)), _stream())
+        code = lib.hk_gemm_tc(_ptr(a), _ptr(w_gate_up), _ptr(out), M, N, K, out.shape[1], epilogue, bn,
+                              splits, _ptr(partial) if splits > 1 else 0, _ptr(status_flag(a.device)), _stream())
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "gemm+swiglu (tcgen05)")
@@ -416,7 +406,6 @@ def run_swiglu(a, w_gate_up, out, choice: Optional[str] = None, act: int = 0, li
 def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> bool:
     """out (bf16 [M, N]) = factor * max(a w^T, 0)^2 in the epilogue of the product that `run` would take for the shape.
     False when no tensor-core kernel takes it."""
-    from . import ops
     M, K = a.shape
     N = w.shape[0]
     if not _aligned(a, w):
@@ -430,8 +419,8 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
         if M > SMALL_M:
             return False
         lib = build.load("gemm_smallm")
-        code = lib.hk_gemm_smallm_sqrelu(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), row_tiles(M, N, a.device),
-                                         ctypes.c_float(factor), _stream())
+        code = lib.hk_gemm_smallm_sqrelu(_ptr(a), _ptr(w), _ptr(out), M, N, K, N, row_tiles(M, N, a.device),
+                                         factor, _stream())
         if code == _UNSUPPORTED:
             return False
         ops._check(code, "gemm+squared relu (small-M)")
@@ -441,9 +430,9 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)
-    code = lib.hk_gemm_tc_sqrelu(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), bn, splits,
-                                 _ptr(partial) if splits > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)),
-                                 ctypes.c_float(factor), _stream())
+    code = lib.hk_gemm_tc_sqrelu(_ptr(a), _ptr(w), _ptr(out), M, N, K, N, bn, splits,
+                                 _ptr(partial) if splits > 1 else 0, _ptr(status_flag(a.device)),
+                                 factor, _stream())
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "gemm+squared relu (tcgen05)")
@@ -452,7 +441,6 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
 
 def run_narrow(a, w, out) -> bool:
     """out (bf16 [M, N]) = a w^T on the tcgen05 kernel.  False when it refuses the shape."""
-    from . import ops
     M, K = a.shape
     N = w.shape[0]
     if not _aligned(a, w):
@@ -462,8 +450,8 @@ def run_narrow(a, w, out) -> bool:
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)
-    code = lib.hk_gemm_tc_narrow(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(N), bn, splits,
-                                 _ptr(partial) if splits > 1 else ctypes.c_void_p(0), _ptr(status_flag(a.device)), _stream())
+    code = lib.hk_gemm_tc_narrow(_ptr(a), _ptr(w), _ptr(out), M, N, K, N, bn, splits,
+                                 _ptr(partial) if splits > 1 else 0, _ptr(status_flag(a.device)), _stream())
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "gemm, narrowed (tcgen05)")
@@ -478,7 +466,6 @@ def run_grouped(a, w, out, groups, gated: bool, act: int = 0, limit: float = 0.0
     2 (the clamped form) of the two halves."""
     if gated and act not in (0, 2):
         return False
-    from . import ops
     M, K = a.shape
     E, N = int(w.shape[0]), int(w.shape[1])
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or K % 8 or M % GROUPED_ROWS or not _aligned(a, w) \
@@ -486,8 +473,8 @@ def run_grouped(a, w, out, groups, gated: bool, act: int = 0, limit: float = 0.0
         return False
     bn = min(256, -(-N // 32) * 32)
     lib = build.load("gemm_tc")
-    code = lib.hk_gemm_tc_grouped(_ptr(a), _ptr(w), _ptr(out), M, N, K, ctypes.c_longlong(out.shape[1]), 2 + act if gated else 0, bn, E,
-                                  _ptr(groups), _ptr(status_flag(a.device)), ctypes.c_float(limit), ctypes.c_float(slope), _stream())
+    code = lib.hk_gemm_tc_grouped(_ptr(a), _ptr(w), _ptr(out), M, N, K, out.shape[1], 2 + act if gated else 0, bn, E,
+                                  _ptr(groups), _ptr(status_flag(a.device)), limit, slope, _stream())
     if code == _UNSUPPORTED:
         return False
     ops._check(code, "grouped gemm (tcgen05)")

@@ -10,7 +10,6 @@ can be pinned with `force()` by tests.
 from __future__ import annotations
 
 import contextlib
-import ctypes
 from typing import Optional
 
 import numpy as np
@@ -34,16 +33,19 @@ def _dt(t: torch.Tensor) -> int:
     raise KernelError(f"kernels take float32 or bfloat16 tensors, not {t.dtype}")
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def _stream():
     """The current device's current stream, as its handle (an object around it would cost two microseconds a launch)."""
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, dims: Optional[int] = None) -> None:
+    if isinstance(t, torch.Tensor) and t.is_cuda and (dtype is None or t.dtype is dtype) and (dims is None or t.dim() == dims) \
+            and t.is_contiguous():
+        return
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor")
     if dtype is not None and t.dtype != dtype:
@@ -130,7 +132,7 @@ def embedding(table: torch.Tensor, token_ids: torch.Tensor, out: torch.Tensor, s
         raise KernelError(f"embedding: out {tuple(out.shape)} does not fit ids {tuple(token_ids.shape)} and table {tuple(table.shape)}")
     lib = build.load("elementwise")
     _check(lib.hk_embedding(_ptr(table), _dt(table), _ptr(token_ids), _ptr(out), n, d, table.shape[0],
-                            ctypes.c_float(scale), _ptr(narrow), _stream()),
+                            scale, _ptr(narrow), _stream()),
            "embedding")
 
 
@@ -156,7 +158,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tenso
             raise KernelError("rms_norm: fewer row indices than output rows")
     lib = build.load("elementwise")
     _check(lib.hk_rms_norm(_ptr(x), _ptr(weight), _ptr(rows), _ptr(out), _dt(out), n_out, d,
-                           ctypes.c_longlong(ldx), ctypes.c_float(eps), _stream()), "rms_norm")
+                           ldx, eps, _stream()), "rms_norm")
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float, out: torch.Tensor,
@@ -177,7 +179,7 @@ def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: f
         if rows.shape[0] < n_out:
             raise KernelError("layer_norm: fewer row indices than output rows")
     lib = build.load("norms")
-    _check(lib.hk_layer_norm(_ptr(x), _ptr(weight), _ptr(bias), _ptr(rows), _ptr(out), _dt(out), n_out, d, ctypes.c_float(eps),
+    _check(lib.hk_layer_norm(_ptr(x), _ptr(weight), _ptr(bias), _ptr(rows), _ptr(out), _dt(out), n_out, d, eps,
                              _stream()), "layer_norm")
 
 
@@ -206,9 +208,9 @@ def pair_norm_add(a, wa, eps_a: float, scale_a: float, b, wb, eps_b: float, scal
         if lw.shape[0] != d or lb.shape[0] != d or next_out.shape != residual.shape:
             raise KernelError("pair_norm_add: the next norm does not fit")
     lib = build.load("norms")
-    _check(lib.hk_pair_norm_add(_ptr(a), _ptr(a_bias), _ptr(wa), ctypes.c_float(eps_a), ctypes.c_float(scale_a), _ptr(b), _ptr(wb),
-                                ctypes.c_float(eps_b), ctypes.c_float(scale_b), _ptr(residual), 1 if accumulate else 0, _ptr(lw),
-                                _ptr(lb), ctypes.c_float(leps), _ptr(next_out if lw is not None else None),
+    _check(lib.hk_pair_norm_add(_ptr(a), _ptr(a_bias), _ptr(wa), eps_a, scale_a, _ptr(b), _ptr(wb),
+                                eps_b, scale_b, _ptr(residual), 1 if accumulate else 0, _ptr(lw),
+                                _ptr(lb), leps, _ptr(next_out if lw is not None else None),
                                 _dt(next_out) if lw is not None else F32, n, d, _stream()), "pair_norm_add")
 
 
@@ -232,8 +234,8 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, block: int = 0, act: str = 
     if gate_up.shape[0] != n or gate_up.shape[1] != 2 * f or f % block:
         raise KernelError("swiglu: gate_up must be [n, 2F] for out [n, F], and the block must divide F")
     lib = build.load("elementwise")
-    _check(lib.hk_swiglu(_ptr(gate_up), _ptr(out), _dt(out), n, f, int(block), GLU_ACTS[act], ctypes.c_float(limit),
-                         ctypes.c_float(slope), _stream()), "swiglu")
+    _check(lib.hk_swiglu(_ptr(gate_up), _ptr(out), _dt(out), n, f, int(block), GLU_ACTS[act], limit,
+                         slope, _stream()), "swiglu")
 
 
 def _as_weights(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
@@ -264,7 +266,6 @@ def gemm_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, act
     if a.shape[0] != M or w_gate_up.shape != (2 * F, a.shape[1]):
         raise KernelError("gemm_swiglu: shapes do not fit")
     if a.dtype == torch.bfloat16 and _forced["gemm"] in (None, "tc", "stream"):
-        from . import gemm_fast
         if gemm_fast.run_swiglu(a, w_gate_up, out, _forced["gemm"], act=GLU_ACTS[act], limit=limit, slope=slope):
             return
     gu = torch.empty((M, 2 * F), dtype=torch.float32, device=a.device)
@@ -279,7 +280,7 @@ def squared_relu(z: torch.Tensor, out: torch.Tensor, factor: float = 1.0) -> Non
     if z.shape != out.shape:
         raise KernelError("squared_relu: shapes differ")
     lib = build.load("elementwise")
-    _check(lib.hk_squared_relu(_ptr(z), _ptr(out), _dt(out), ctypes.c_longlong(z.numel()), ctypes.c_float(factor), _stream()),
+    _check(lib.hk_squared_relu(_ptr(z), _ptr(out), _dt(out), z.numel(), factor, _stream()),
            "squared_relu")
 
 
@@ -297,7 +298,6 @@ def gemm_squared_relu(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, facto
     if a.shape[1] != w.shape[1] or tuple(out.shape) != (a.shape[0], w.shape[0]):
         raise KernelError("gemm_squared_relu: shapes do not fit")
     if a.dtype == torch.bfloat16 and _forced["gemm"] != "generic":
-        from . import gemm_fast
         if gemm_fast.run_squared_relu(a, w, out, factor, _forced["gemm"]):
             return
     z = torch.empty(out.shape, dtype=torch.float32, device=a.device)
@@ -362,12 +362,12 @@ def qk_norm_rope_kv_write(qkv, q_out, q_weight, k_weight, eps, cos, sin, rotary_
             raise KernelError("cache pages must be [pages, G, page_tokens, head_dim] (values: their own width)")
     lib = build.load("elementwise")
     _check(lib.hk_qk_norm_rope_kv_write(
-        _ptr(qkv), _ptr(q_out), _dt(q_out), _ptr(q_weight), _ptr(k_weight), ctypes.c_float(eps),
+        _ptr(qkv), _ptr(q_out), _dt(q_out), _ptr(q_weight), _ptr(k_weight), eps,
         _ptr(cos if rotary_dim > 0 else None), _ptr(sin if rotary_dim > 0 else None), int(rotary_dim),
         _ptr(positions), _ptr(slot_of_token), _ptr(block_table if write_kv else None),
         int(block_table.shape[1]) if write_kv else 0, _ptr(k_pages if write_kv else None),
         _ptr(v_pages if write_kv else None), n, H, G, hd, int(page_tokens), 1 if write_kv else 0, _ptr(bias),
-        PAIRINGS[pairing], 1 if norm_after else 0, 1 if tied_v else 0, vd, ctypes.c_longlong(qkv.stride(0)),
+        PAIRINGS[pairing], 1 if norm_after else 0, 1 if tied_v else 0, vd, qkv.stride(0),
         *_query_factor(q_factor), _stream()),
         "qk_norm_rope_kv_write")
 
@@ -376,7 +376,7 @@ def _query_factor(q_factor):
     coef, every = q_factor if q_factor is not None else (0.0, 0)
     if q_factor is not None and int(every) < 1:
         raise KernelError("the queries' factor needs a positive number of positions per step")
-    return ctypes.c_float(coef), int(every)
+    return coef, int(every)
 
 
 def qk_row_norm_kv_write(qkv, q_out, q_weight, k_weight, q_count: int, k_count: int, eps: float, positions, slot_of_token, block_table,
@@ -410,8 +410,8 @@ def qk_row_norm_kv_write(qkv, q_out, q_weight, k_weight, q_count: int, k_count: 
         raise KernelError("cache pages must be [pages, G, page_tokens, head_dim] (values: their own width)")
     lib = build.load("elementwise")
     _check(lib.hk_qk_row_norm_kv_write(
-        _ptr(qkv), ctypes.c_longlong(ld), _ptr(bias), _ptr(q_out), _dt(q_out), _ptr(q_weight), _ptr(k_weight), ctypes.c_float(q_count),
-        ctypes.c_float(k_count), ctypes.c_float(eps), _ptr(positions), _ptr(slot_of_token), _ptr(block_table), int(block_table.shape[1]),
+        _ptr(qkv), ld, _ptr(bias), _ptr(q_out), _dt(q_out), _ptr(q_weight), _ptr(k_weight), q_count,
+        k_count, eps, _ptr(positions), _ptr(slot_of_token), _ptr(block_table), int(block_table.shape[1]),
         _ptr(k_pages), _ptr(v_pages), n, H, G, hd, vd, int(page_tokens), 1 if write_kv else 0, *_query_factor(q_factor), _stream()),
         "qk_row_norm_kv_write")
 
@@ -443,7 +443,7 @@ def maps_rope_kv_write(x, q_out, cos, sin, rotary_dim: int, positions, slot_of_t
     _need(block_table, "block_table", torch.int32, 2)
     lib = build.load("elementwise")
     _check(lib.hk_maps_rope_kv_write(
-        _ptr(x), ctypes.c_longlong(ld), _ptr(q_out), _dt(q_out), _ptr(cos if rotary_dim > 0 else None),
+        _ptr(x), ld, _ptr(q_out), _dt(q_out), _ptr(cos if rotary_dim > 0 else None),
         _ptr(sin if rotary_dim > 0 else None), int(rotary_dim), _ptr(positions), _ptr(slot_of_token), _ptr(block_table),
         int(block_table.shape[1]), _ptr(k_pages), _ptr(v_pages), n, H, G, M, dk, vd, int(page_tokens), 1 if write_kv else 0,
         _stream()), "maps_rope_kv_write")
@@ -464,8 +464,8 @@ def diff_heads_out(a, gate, out, n_heads: int, value_dim: int, lam: float, eps: 
             or (a.dtype != torch.float32 and a.dtype != out.dtype):
         raise KernelError("diff_heads_out: shapes or types do not fit")
     lib = build.load("elementwise")
-    _check(lib.hk_diff_heads_out(_ptr(a), _dt(a), _ptr(gate), ctypes.c_longlong(ldg), _ptr(out), _dt(out), n, H, vd,
-                                 ctypes.c_float(lam), ctypes.c_float(eps), ctypes.c_float(out_scale), _stream()), "diff_heads_out")
+    _check(lib.hk_diff_heads_out(_ptr(a), _dt(a), _ptr(gate), ldg, _ptr(out), _dt(out), n, H, vd,
+                                 lam, eps, out_scale, _stream()), "diff_heads_out")
 
 
 # ---- matrix product -------------------------------------------------------------------
@@ -499,14 +499,13 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool =
         raise KernelError(f"gemm: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} do not fit")
     choice = _forced["gemm"]
     if a.dtype == torch.bfloat16 and choice != "generic":
-        from . import gemm_fast
         if gemm_fast.run(a, w, out, accumulate, choice):
             return
         if choice is not None:
             raise KernelError(f"gemm: the '{choice}' kernel refuses M={M} N={N} K={K}")
     lib = build.load("gemm_generic")
-    _check(lib.hk_gemm_generic(_ptr(a), _ptr(w), _dt(a), _ptr(out), M, N, K, ctypes.c_longlong(K),
-                               ctypes.c_longlong(K), ctypes.c_longlong(N), 1 if accumulate else 0, _stream()),
+    _check(lib.hk_gemm_generic(_ptr(a), _ptr(w), _dt(a), _ptr(out), M, N, K, K,
+                               K, N, 1 if accumulate else 0, _stream()),
            "gemm")
 
 
@@ -581,7 +580,6 @@ def paged_attention(q, k_pages, v_pages, block_table, positions, slot_of_token, 
     choice = _forced["attention"]
     if q.dtype == torch.bfloat16 and choice != "generic" and plan is not None and v_pages is not None and vd == hd \
             and (dist is None or dist_log2 is not None):
-        from . import attention_fast
         done = attention_fast.run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, scale, plan,
                                   allow_tma=choice != "flash_cp", sink=sink, sinks=sinks, softcap=softcap, chunk=chunk,
                                   gate=gate, gate_scale=gate_scale, dist=dist_log2 if dist is not None else None)
@@ -596,17 +594,17 @@ def paged_attention(q, k_pages, v_pages, block_table, positions, slot_of_token, 
         _need(runs, "runs", torch.int32, 2)
         code = lib.hk_attention_f32(
             _ptr(q), _ptr(k_pages), _ptr(v_pages if v_pages is not None else k_pages), _ptr(block_table), int(block_table.shape[1]), _ptr(runs),
-            int(runs.shape[0]), _ptr(out), H, G, hd, int(page_tokens), int(window), ctypes.c_float(scale), vd, 1 if sink else 0, _ptr(sinks),
-            ctypes.c_float(softcap), int(chunk), vd if v_pages is not None else hd, _ptr(gate), ctypes.c_longlong(gate_ld),
-            ctypes.c_float(gate_scale), _ptr(dist), int(dist.shape[1]) if dist is not None else 0, _stream())
+            int(runs.shape[0]), _ptr(out), H, G, hd, int(page_tokens), int(window), scale, vd, 1 if sink else 0, _ptr(sinks),
+            softcap, int(chunk), vd if v_pages is not None else hd, _ptr(gate), gate_ld,
+            gate_scale, _ptr(dist), int(dist.shape[1]) if dist is not None else 0, _stream())
         if code != _ERR_UNSUPPORTED:
             _check(code, "paged_attention (float32 runs)")
             return
     _check(lib.hk_attention_generic(
         _ptr(q), _ptr(k_pages), _ptr(v_pages if v_pages is not None else k_pages), _dt(q), _ptr(block_table),
         int(block_table.shape[1]), _ptr(positions), _ptr(slot_of_token), _ptr(out), n, H, G, hd, int(page_tokens), int(window),
-        ctypes.c_float(scale), vd, 1 if sink else 0, _ptr(sinks), ctypes.c_float(softcap), int(chunk),
-        vd if v_pages is not None else hd, _ptr(gate), ctypes.c_longlong(gate_ld), ctypes.c_float(gate_scale), _ptr(dist),
+        scale, vd, 1 if sink else 0, _ptr(sinks), softcap, int(chunk),
+        vd if v_pages is not None else hd, _ptr(gate), gate_ld, gate_scale, _ptr(dist),
         int(dist.shape[1]) if dist is not None else 0, _stream()), "paged_attention")
 
 
@@ -620,7 +618,7 @@ def sigmoid_gate(x: torch.Tensor, gate: torch.Tensor, out: torch.Tensor, scale: 
     if x.shape != out.shape or gate.shape[0] != n or (x.dtype != torch.float32 and x.dtype != out.dtype):
         raise KernelError("sigmoid_gate: shapes or types do not fit")
     lib = build.load("elementwise")
-    _check(lib.hk_sigmoid_gate(_ptr(x), _dt(x), _ptr(gate), ctypes.c_longlong(ld), _ptr(out), _dt(out), n, W, ctypes.c_float(scale),
+    _check(lib.hk_sigmoid_gate(_ptr(x), _dt(x), _ptr(gate), ld, _ptr(out), _dt(out), n, W, scale,
                                _stream()), "sigmoid_gate")
 
 
@@ -667,9 +665,9 @@ def latent_prep(q, kv, q_plain, q_full, c_weight, eps, cos, sin, rotary_dim, pai
             raise KernelError("latent_prep: cache pages must be [pages, 1, page_tokens, rank + rot_dim]")
     lib = build.load("elementwise")
     _check(lib.hk_latent_prep(
-        _ptr(q), ctypes.c_longlong(ldq), _ptr(kv), ctypes.c_longlong(ldkv), _ptr(q_plain), int(plain_head),
-        ctypes.c_void_p(rot_out), int(rot_head), _dt(q_plain), _ptr(c_weight),
-        ctypes.c_float(eps), _ptr(cos if rotary_dim > 0 else None), _ptr(sin if rotary_dim > 0 else None), int(rotary_dim),
+        _ptr(q), ldq, _ptr(kv), ldkv, _ptr(q_plain), int(plain_head),
+        rot_out, int(rot_head), _dt(q_plain), _ptr(c_weight),
+        eps, _ptr(cos if rotary_dim > 0 else None), _ptr(sin if rotary_dim > 0 else None), int(rotary_dim),
         PAIRINGS[pairing], _ptr(positions), _ptr(slot_of_token), _ptr(block_table if write_kv else None),
         int(block_table.shape[1]) if write_kv else 0, _ptr(pages if write_kv else None), n, H, dn, dr, r, int(page_tokens),
         1 if write_kv else 0, _stream()), "latent_prep")
@@ -702,7 +700,6 @@ def gemm_narrow(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _need(out, "out", torch.bfloat16, 2)
     if a.shape[1] != w.shape[1] or tuple(out.shape) != (a.shape[0], w.shape[0]):
         raise KernelError("gemm_narrow: shapes do not fit")
-    from . import gemm_fast
     if not gemm_fast.run_narrow(a, w, out):
         raise KernelError("gemm_narrow: the tcgen05 kernel refuses this shape")
 
@@ -730,17 +727,17 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n_heads: int
             raise KernelError("gemm_heads: one row of gate logits per row")
     if a.dtype == torch.bfloat16 and _forced["gemm"] != "generic":
         lib = build.load("gemm_heads")
-        code = lib.hk_gemm_heads_mma(_ptr(a), _ptr(w), _ptr(out), _dt(out), n, N, K, H, ctypes.c_longlong(a.stride(0)),
-                                     ctypes.c_longlong(a.stride(1)), ctypes.c_longlong(out.stride(0)),
-                                     ctypes.c_longlong(out.stride(1)), _ptr(gate), ctypes.c_longlong(gate_ld),
-                                     1 if gate_per_head else 0, ctypes.c_float(gate_scale), _stream())
+        code = lib.hk_gemm_heads_mma(_ptr(a), _ptr(w), _ptr(out), _dt(out), n, N, K, H, a.stride(0),
+                                     a.stride(1), out.stride(0),
+                                     out.stride(1), _ptr(gate), gate_ld,
+                                     1 if gate_per_head else 0, gate_scale, _stream())
         if code != _ERR_UNSUPPORTED:
             _check(code, "gemm_heads (mma)")
             return
     lib = build.load("gemm_generic")
-    _check(lib.hk_gemm_heads(_ptr(a), _ptr(w), _dt(a), _ptr(out), _dt(out), n, N, K, H, ctypes.c_longlong(a.stride(0)),
-                             ctypes.c_longlong(a.stride(1)), ctypes.c_longlong(out.stride(0)), ctypes.c_longlong(out.stride(1)),
-                             _ptr(gate), ctypes.c_longlong(gate_ld), 1 if gate_per_head else 0, ctypes.c_float(gate_scale),
+    _check(lib.hk_gemm_heads(_ptr(a), _ptr(w), _dt(a), _ptr(out), _dt(out), n, N, K, H, a.stride(0),
+                             a.stride(1), out.stride(0), out.stride(1),
+                             _ptr(gate), gate_ld, 1 if gate_per_head else 0, gate_scale,
                              _stream()), "gemm_heads")
 
 
@@ -807,7 +804,7 @@ def rms_norm_add(y: torch.Tensor, weight: torch.Tensor, eps: float, residual: to
     if y.shape != residual.shape or weight.shape[0] != y.shape[1]:
         raise KernelError("rms_norm_add: y, residual and weight do not fit")
     lib = build.load("elementwise")
-    _check(lib.hk_rms_norm_add(_ptr(y), _ptr(weight), _ptr(residual), y.shape[0], y.shape[1], ctypes.c_float(eps), _ptr(narrow),
+    _check(lib.hk_rms_norm_add(_ptr(y), _ptr(weight), _ptr(residual), y.shape[0], y.shape[1], eps, _ptr(narrow),
                                _stream()), "rms_norm_add")
 
 
@@ -820,7 +817,7 @@ def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor)
     if out.shape != z.shape or coef.shape[0] != 4:
         raise KernelError("polynorm: out must have z's shape and coef four entries")
     lib = build.load("elementwise")
-    _check(lib.hk_polynorm(_ptr(z), _ptr(coef), _ptr(out), _dt(out), z.shape[0], z.shape[1], ctypes.c_float(eps), _stream()),
+    _check(lib.hk_polynorm(_ptr(z), _ptr(coef), _ptr(out), _dt(out), z.shape[0], z.shape[1], eps, _stream()),
            "polynorm")
 
 
@@ -841,7 +838,7 @@ def tanh_cols(x: torch.Tensor, out: torch.Tensor) -> None:
     if x.shape[0] != out.shape[0]:
         raise KernelError("tanh_cols: rows differ")
     lib = build.load("elementwise")
-    _check(lib.hk_tanh_cols(_ptr(x), ctypes.c_longlong(ld), _ptr(out), _dt(out), out.shape[0], out.shape[1], _stream()), "tanh_cols")
+    _check(lib.hk_tanh_cols(_ptr(x), ld, _ptr(out), _dt(out), out.shape[0], out.shape[1], _stream()), "tanh_cols")
 
 
 # ---- recurrent mixers ---------------------------------------------------------------------
@@ -882,7 +879,6 @@ def _walk_record(n: int, segments, most_rows: int, H: int, dk: int, dv: int, dev
 
 
 def _chunk_scratch(lib, chunks, H: int, dk: int, dvp: int, removal: bool, device):
-    lib.hk_delta_chunks_scratch.restype = ctypes.c_longlong
     return torch.empty(int(lib.hk_delta_chunks_scratch(int(chunks.shape[0]), H, dk, dvp, 1 if removal else 0)), dtype=torch.float32,
                        device=device)
 
@@ -915,17 +911,17 @@ def delta_rule_scan(r, k, v, a_logit, w_logit, a_bias, w_bias, segments, state, 
     if chunks is not None and chunks.shape[0]:
         lib = build.load("delta_chunks")
         scratch = _chunk_scratch(lib, chunks, H, dk, dv, True, out.device)
-        _check(lib.hk_delta_rule_chunks(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ctypes.c_longlong(ld), _ptr(w_logit),
-                                        ctypes.c_longlong(ldw), _ptr(a_bias), _ptr(w_bias), *_chunk_tables(chunks, requests, "delta_rule_scan"),
-                                        _ptr(scratch), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
-                                        ctypes.c_float(key_eps), _stream()), "delta_rule_scan (chunks)", launches=2)
+        _check(lib.hk_delta_rule_chunks(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ld, _ptr(w_logit),
+                                        ldw, _ptr(a_bias), _ptr(w_bias), *_chunk_tables(chunks, requests, "delta_rule_scan"),
+                                        _ptr(scratch), _ptr(state), _ptr(out), H, dk, dv, decay_scale,
+                                        key_eps, _stream()), "delta_rule_scan (chunks)", launches=2)
     if rec is None:
         return
     lib = build.load("recurrent")
-    _check(lib.hk_delta_rule_scan(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ctypes.c_longlong(ld), _ptr(w_logit),
-                                  ctypes.c_longlong(ldw), _ptr(a_bias), _ptr(w_bias), _ptr(segments), int(segments.shape[0]), n,
-                                  int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(decay_scale),
-                                  ctypes.c_float(key_eps), _stream()), "delta_rule_scan", launches=2)
+    _check(lib.hk_delta_rule_scan(_ptr(r), _ptr(k), _ptr(v), _ptr(a_logit), ld, _ptr(w_logit),
+                                  ldw, _ptr(a_bias), _ptr(w_bias), _ptr(segments), int(segments.shape[0]), n,
+                                  int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, decay_scale,
+                                  key_eps, _stream()), "delta_rule_scan", launches=2)
 
 
 def head_norm_gate(o, gate_logit, weight, eps: float, out, n_heads: int, value_dim: int) -> None:
@@ -938,8 +934,8 @@ def head_norm_gate(o, gate_logit, weight, eps: float, out, n_heads: int, value_d
     if tuple(o.shape) != (out.shape[0], H * dv) or out.shape != o.shape or weight.shape[0] != H * dv:
         raise KernelError("head_norm_gate: shapes do not fit")
     lib = build.load("recurrent")
-    _check(lib.hk_head_norm_gate(_ptr(o), _ptr(gate_logit), ctypes.c_longlong(ldg), _ptr(weight), _ptr(out), _dt(out),
-                                 o.shape[0], H, dv, ctypes.c_float(eps), _stream()), "head_norm_gate")
+    _check(lib.hk_head_norm_gate(_ptr(o), _ptr(gate_logit), ldg, _ptr(weight), _ptr(out), _dt(out),
+                                 o.shape[0], H, dv, eps, _stream()), "head_norm_gate")
 
 
 def mingru_scan(proj, z_bias, x_bias, segments, state, out) -> None:
@@ -959,7 +955,7 @@ def mingru_scan(proj, z_bias, x_bias, segments, state, out) -> None:
     if proj.shape[1] != 3 * W or tuple(out.shape) != (proj.shape[0], W) or segments.shape[1] != 3:
         raise KernelError("mingru_scan: shapes do not fit")
     lib = build.load("recurrent")
-    _check(lib.hk_mingru_scan(_ptr(proj), ctypes.c_longlong(3 * W), _ptr(z_bias), _ptr(x_bias), _ptr(segments),
+    _check(lib.hk_mingru_scan(_ptr(proj), 3 * W, _ptr(z_bias), _ptr(x_bias), _ptr(segments),
                               int(segments.shape[0]), _ptr(state), _ptr(out), _dt(out), W, _stream()), "mingru_scan")
 
 
@@ -982,8 +978,8 @@ def short_conv(x, weight, segments, tail, out, act: str = "silu", bias=None) -> 
             or act not in ("silu", "none"):
         raise KernelError("short_conv: shapes do not fit")
     lib = build.load("short_conv")
-    _check(lib.hk_short_conv(_ptr(x), ctypes.c_longlong(ldx), _ptr(weight), _ptr(bias), _ptr(segments), int(segments.shape[0]),
-                             int(x.shape[0]), _ptr(tail), _ptr(out), _dt(out), ctypes.c_longlong(ldy), C, taps, 1 if act == "silu" else 0, _stream()),
+    _check(lib.hk_short_conv(_ptr(x), ldx, _ptr(weight), _ptr(bias), _ptr(segments), int(segments.shape[0]),
+                             int(x.shape[0]), _ptr(tail), _ptr(out), _dt(out), ldy, C, taps, 1 if act == "silu" else 0, _stream()),
            "short_conv")
 
 
@@ -1016,18 +1012,18 @@ def gated_delta_scan(q, k, v, b_logit, a_logit, a_log, dt_bias, segments, state,
     if chunks is not None and chunks.shape[0]:
         lib = build.load("delta_chunks")
         scratch = _chunk_scratch(lib, chunks, H, dk, dv, True, out.device)
-        _check(lib.hk_gated_delta_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(b_logit), _ptr(a_logit),
-                                         ctypes.c_longlong(ldg), _ptr(a_log), _ptr(dt_bias),
+        _check(lib.hk_gated_delta_chunks(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(b_logit), _ptr(a_logit),
+                                         ldg, _ptr(a_log), _ptr(dt_bias),
                                          *_chunk_tables(chunks, requests, "gated_delta_scan"), _ptr(scratch), _ptr(state), _ptr(out), H, G, dk,
-                                         dv, ctypes.c_float(q_scale), ctypes.c_float(unit_eps), _stream()), "gated_delta_scan (chunks)",
+                                         dv, q_scale, unit_eps, _stream()), "gated_delta_scan (chunks)",
                launches=2)
     if rec is None:
         return
     lib = build.load("recurrent")
-    _check(lib.hk_gated_delta_scan(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(b_logit), _ptr(a_logit),
-                                   ctypes.c_longlong(ldg), _ptr(a_log), _ptr(dt_bias), _ptr(segments), int(segments.shape[0]), n,
-                                   int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, G, dk, dv, ctypes.c_float(q_scale),
-                                   ctypes.c_float(unit_eps), _stream()), "gated_delta_scan", launches=2)
+    _check(lib.hk_gated_delta_scan(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(b_logit), _ptr(a_logit),
+                                   ldg, _ptr(a_log), _ptr(dt_bias), _ptr(segments), int(segments.shape[0]), n,
+                                   int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, G, dk, dv, q_scale,
+                                   unit_eps, _stream()), "gated_delta_scan", launches=2)
 
 
 def retention_scan(q, k, v, cos, sin, rotary_dim: int, positions, decay, segments, state, out, n_heads: int, key_dim: int,
@@ -1060,16 +1056,16 @@ def retention_scan(q, k, v, cos, sin, rotary_dim: int, positions, decay, segment
     if chunks is not None and chunks.shape[0]:
         lib = build.load("delta_chunks")
         scratch = _chunk_scratch(lib, chunks, H, dk, dv, False, out.device)
-        _check(lib.hk_retention_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(cos if rotary_dim > 0 else None),
+        _check(lib.hk_retention_chunks(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(cos if rotary_dim > 0 else None),
                                        _ptr(sin if rotary_dim > 0 else None), int(rotary_dim), _ptr(positions), _ptr(decay),
                                        *_chunk_tables(chunks, requests, "retention_scan"), _ptr(scratch), _ptr(state), _ptr(out), H, dk, dv,
-                                       ctypes.c_float(k_scale), _stream()), "retention_scan (chunks)", launches=3)
+                                       k_scale, _stream()), "retention_scan (chunks)", launches=3)
     if rec is None:
         return
     lib = build.load("recurrent")
-    _check(lib.hk_retention_scan(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(cos if rotary_dim > 0 else None),
+    _check(lib.hk_retention_scan(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(cos if rotary_dim > 0 else None),
                                  _ptr(sin if rotary_dim > 0 else None), int(rotary_dim), _ptr(positions), _ptr(decay), _ptr(segments),
-                                 int(segments.shape[0]), n, int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(k_scale),
+                                 int(segments.shape[0]), n, int(most_rows), rec_rows, _ptr(rec), _ptr(state), _ptr(out), H, dk, dv, k_scale,
                                  _stream()), "retention_scan", launches=2)
 
 
@@ -1106,11 +1102,11 @@ def state_space_scan(xbc, dt_logit, dt_bias, a_log, skip, segments, state, out, 
         _need(long_segments, "long_segments", torch.int32, 2)
         if xbc.dtype != torch.bfloat16 or long_segments.shape[1] != 3:
             raise KernelError("state_space_scan: long segments [n_long, 3] need bfloat16 rows")
-        _check(lib.hk_state_space_chunks(_ptr(xbc), ctypes.c_longlong(ldx), _ptr(dt_logit), ctypes.c_longlong(ldt), _ptr(dt_bias),
+        _check(lib.hk_state_space_chunks(_ptr(xbc), ldx, _ptr(dt_logit), ldt, _ptr(dt_bias),
                                          _ptr(a_log), _ptr(skip), _ptr(long_segments), int(long_segments.shape[0]), n, _ptr(state),
                                          _ptr(out), H, G, N, dv, _stream()), "state_space_scan (chunks)")
     if segments.shape[0]:
-        _check(lib.hk_state_space_walk(_ptr(xbc), _dt(xbc), ctypes.c_longlong(ldx), _ptr(dt_logit), ctypes.c_longlong(ldt), _ptr(dt_bias),
+        _check(lib.hk_state_space_walk(_ptr(xbc), _dt(xbc), ldx, _ptr(dt_logit), ldt, _ptr(dt_bias),
                                        _ptr(a_log), _ptr(skip), _ptr(segments), int(segments.shape[0]), n, _ptr(state), _ptr(out), H, G,
                                        N, dv, 1 if segments.shape[0] == n else 0, _stream()), "state_space_scan")
 
@@ -1126,8 +1122,8 @@ def gla_decay(hid, w2, bias, tau: float, out) -> None:
     if tuple(out.shape) != (hid.shape[0], K) or bias.shape[0] != K or not tau > 0:
         raise KernelError("gla_decay: shapes do not fit, or tau is not positive")
     lib = build.load("gated_linear")
-    _check(lib.hk_gla_decay(_ptr(hid), ctypes.c_longlong(ldh), int(R), _ptr(w2), _ptr(bias), _ptr(out), out.shape[0], int(K),
-                            ctypes.c_float(tau), _stream()), "gla_decay")
+    _check(lib.hk_gla_decay(_ptr(hid), ldh, int(R), _ptr(w2), _ptr(bias), _ptr(out), out.shape[0], int(K),
+                            tau, _stream()), "gla_decay")
 
 
 GLA_CHUNK = 64      # tokens of a chunk of `gla_scan`'s chunked form
@@ -1167,14 +1163,14 @@ def gla_scan(q, k, v, la, segments, state, out, n_heads: int, key_dim: int, valu
         u = torch.empty(nc * H * dv * dk, dtype=torch.float32, device=out.device)
         decay = torch.empty(nc * H * dk, dtype=torch.float32, device=out.device)
         lib = build.load("gated_linear_chunks")
-        _check(lib.hk_gla_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(la), _ptr(chunks), nc, _ptr(requests),
-                                 int(requests.shape[0]), _ptr(u), _ptr(decay), _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(q_scale),
+        _check(lib.hk_gla_chunks(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(la), _ptr(chunks), nc, _ptr(requests),
+                                 int(requests.shape[0]), _ptr(u), _ptr(decay), _ptr(state), _ptr(out), H, dk, dv, q_scale,
                                  _stream()), "gla_scan (chunks)", launches=3)
     if not segments.shape[0]:
         return
     lib = build.load("gated_linear")
-    _check(lib.hk_gla_walk(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(la), _ptr(segments), int(segments.shape[0]),
-                           _ptr(state), _ptr(out), H, dk, dv, ctypes.c_float(q_scale), 1 if segments.shape[0] == n else 0, _stream()),
+    _check(lib.hk_gla_walk(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(la), _ptr(segments), int(segments.shape[0]),
+                           _ptr(state), _ptr(out), H, dk, dv, q_scale, 1 if segments.shape[0] == n else 0, _stream()),
            "gla_scan")
 
 
@@ -1189,8 +1185,8 @@ def gated_part_norm(y, z, weight, eps: float, out, parts: int) -> None:
     if tuple(out.shape) != (n, W) or z.shape[0] != n or weight.shape[0] != W or W % parts:
         raise KernelError("gated_part_norm: shapes do not fit")
     lib = build.load("state_space")
-    _check(lib.hk_gated_part_norm(_ptr(y), _ptr(z), ctypes.c_longlong(ldz), _ptr(weight), _ptr(out), _dt(out), n, W, int(parts),
-                                  ctypes.c_float(eps), _stream()), "gated_part_norm")
+    _check(lib.hk_gated_part_norm(_ptr(y), _ptr(z), ldz, _ptr(weight), _ptr(out), _dt(out), n, W, int(parts),
+                                  eps, _stream()), "gated_part_norm")
 
 
 def mlstm_padded(value_dim: int) -> int:
@@ -1233,16 +1229,16 @@ def mlstm_scan(q, k, v, i_logit, f_logit, i_bias, f_bias, segments, state, m_sta
         tables = _chunk_tables(chunks, requests, "mlstm_scan")
         wide = build.load("delta_chunks")
         scratch = _chunk_scratch(wide, chunks, H, dk, dvp, False, out.device)
-        _check(lib.hk_mlstm_gates(_ptr(i_logit), _ptr(f_logit), ctypes.c_longlong(ld), _ptr(i_bias), _ptr(f_bias), _ptr(long_segments),
-                                  int(long_segments.shape[0]), _ptr(gates), _ptr(m_state), H, ctypes.c_float(cap), _stream()),
+        _check(lib.hk_mlstm_gates(_ptr(i_logit), _ptr(f_logit), ld, _ptr(i_bias), _ptr(f_bias), _ptr(long_segments),
+                                  int(long_segments.shape[0]), _ptr(gates), _ptr(m_state), H, cap, _stream()),
                "mlstm_scan (gates)")
-        _check(wide.hk_mlstm_chunks(_ptr(q), _ptr(k), _ptr(v), ctypes.c_longlong(ld), _ptr(gates), *tables, _ptr(scratch), _ptr(state),
-                                    _ptr(out), H, dk, dv, ctypes.c_float(q_scale), _stream()), "mlstm_scan (chunks)", launches=3)
+        _check(wide.hk_mlstm_chunks(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(gates), *tables, _ptr(scratch), _ptr(state),
+                                    _ptr(out), H, dk, dv, q_scale, _stream()), "mlstm_scan (chunks)", launches=3)
     if rec is None:
         return
-    _check(lib.hk_mlstm_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(i_logit), _ptr(f_logit), ctypes.c_longlong(ld), _ptr(i_bias),
+    _check(lib.hk_mlstm_scan(_ptr(q), _ptr(k), _ptr(v), _ptr(i_logit), _ptr(f_logit), ld, _ptr(i_bias),
                              _ptr(f_bias), _ptr(segments), int(segments.shape[0]), n, int(most_rows), rec_rows, _ptr(rec), _ptr(gates), _ptr(state),
-                             _ptr(m_state), _ptr(out), H, dk, dv, ctypes.c_float(cap), ctypes.c_float(q_scale), _stream()),
+                             _ptr(m_state), _ptr(out), H, dk, dv, cap, q_scale, _stream()),
            "mlstm_scan", launches=3)
 
 
@@ -1269,9 +1265,9 @@ def head_out_gate(o, gate_logit, weight, eps: float, out, n_heads: int, value_di
             raise KernelError("head_out_gate: gates must be [n, H, 3]")
     shared = 1 if (weight is not None and weight.shape[0] == dv and H > 1) else 0
     lib = build.load("recurrent")
-    _check(lib.hk_head_out_gate(_ptr(o), int(ldo), _ptr(gate_logit), ctypes.c_longlong(ldg), _ptr(weight), shared,
-                                0 if act == "sigmoid" else 1, _ptr(gates), ctypes.c_float(den_eps), _ptr(out), _dt(out), n, H, dv,
-                                ctypes.c_float(eps), _stream()), "head_out_gate")
+    _check(lib.hk_head_out_gate(_ptr(o), int(ldo), _ptr(gate_logit), ldg, _ptr(weight), shared,
+                                0 if act == "sigmoid" else 1, _ptr(gates), den_eps, _ptr(out), _dt(out), n, H, dv,
+                                eps, _stream()), "head_out_gate")
 
 
 # ---- small element-wise kernels of layers with several streams -------------------------------
@@ -1287,8 +1283,8 @@ def scaled_sum(out, a, alpha: float, b=None, beta: float = 0.0, accumulate: bool
     if a.shape != out.shape or (b is not None and b.shape != out.shape):
         raise KernelError("scaled_sum: shapes differ")
     lib = build.load("elementwise")
-    _check(lib.hk_scaled_sum(_ptr(out), _ptr(a), ctypes.c_float(alpha), _ptr(b), ctypes.c_float(beta),
-                             ctypes.c_longlong(out.numel()), 1 if accumulate else 0, _stream()), "scaled_sum")
+    _check(lib.hk_scaled_sum(_ptr(out), _ptr(a), alpha, _ptr(b), beta,
+                             out.numel(), 1 if accumulate else 0, _stream()), "scaled_sum")
 
 
 def soft_cap(x: torch.Tensor, cap: float) -> None:
@@ -1297,7 +1293,7 @@ def soft_cap(x: torch.Tensor, cap: float) -> None:
     if not cap > 0:
         raise KernelError("soft_cap: the cap must be positive")
     lib = build.load("elementwise")
-    _check(lib.hk_soft_cap(_ptr(x), ctypes.c_longlong(x.numel()), ctypes.c_float(cap), _stream()), "soft_cap")
+    _check(lib.hk_soft_cap(_ptr(x), x.numel(), cap, _stream()), "soft_cap")
 
 
 def narrow(x, out) -> None:
@@ -1307,7 +1303,7 @@ def narrow(x, out) -> None:
     if x.shape != out.shape:
         raise KernelError("narrow: shapes differ")
     lib = build.load("elementwise")
-    _check(lib.hk_narrow(_ptr(x), _ptr(out), _dt(out), ctypes.c_longlong(x.numel()), _stream()), "narrow")
+    _check(lib.hk_narrow(_ptr(x), _ptr(out), _dt(out), x.numel(), _stream()), "narrow")
 
 
 def token_gate(z, table, col0: int, token_ids, out, act: str = "gelu_tanh") -> None:
@@ -1321,7 +1317,7 @@ def token_gate(z, table, col0: int, token_ids, out, act: str = "gelu_tanh") -> N
     if z.shape[0] != n or token_ids.shape[0] != n or act not in ("gelu_tanh", "silu"):
         raise KernelError("token_gate: shapes do not fit")
     lib = build.load("elementwise")
-    _check(lib.hk_token_gate(_ptr(z), ctypes.c_longlong(ld), _ptr(table), _dt(table), ctypes.c_longlong(table.shape[1]), int(col0),
+    _check(lib.hk_token_gate(_ptr(z), ld, _ptr(table), _dt(table), table.shape[1], int(col0),
                              _ptr(token_ids), _ptr(out), _dt(out), n, W, 0 if act == "gelu_tanh" else 1, _stream()), "token_gate")
 
 
@@ -1370,8 +1366,8 @@ def route_topk(x, w_router, ids, weights, scores: str = "softmax", correction=No
             raise KernelError("route_topk: one bias per row of the router")
     lib = build.load("routed")
     _check(lib.hk_route_topk(_ptr(x), _dt(x), _ptr(w_router), _ptr(ids), _ptr(weights), n, d, E, ids.shape[1],
-                             ROUTE_SCORES[scores], _ptr(correction), int(groups), int(keep), ctypes.c_float(scale),
-                             ctypes.c_float(norm_eps), extra, _ptr(extra_out), _ptr(bias), _stream()), "route_topk")
+                             ROUTE_SCORES[scores], _ptr(correction), int(groups), int(keep), scale,
+                             norm_eps, extra, _ptr(extra_out), _ptr(bias), _stream()), "route_topk")
 
 
 def route_sort(ids, n_experts: int, offsets, perm, inv, tiles) -> None:
@@ -1405,7 +1401,7 @@ def grouped_gemm(a, w, out, tiles, offsets, perm, top: int, gather: bool, gated:
     lib = build.load("routed")
     _check(lib.hk_grouped_gemm(_ptr(a), _ptr(w), _dt(a), _ptr(out), _ptr(tiles), tiles.shape[0], _ptr(offsets), _ptr(perm),
                                int(top), 1 if gather else 0, N, K, 1 if gated else 0, 1 if act == "swish_clamped" else 0,
-                               ctypes.c_float(limit), ctypes.c_float(slope), _stream()), "grouped_gemm")
+                               limit, slope, _stream()), "grouped_gemm")
 
 
 def route_combine(ys, inv, weights, y, accumulate: bool = False, shared=None, shared_gate=None, x=None, factor: float = 1.0) -> None:
@@ -1431,7 +1427,7 @@ def route_combine(ys, inv, weights, y, accumulate: bool = False, shared=None, sh
     lib = build.load("routed")
     _check(lib.hk_route_combine(_ptr(ys), _ptr(inv), _ptr(weights), _ptr(y), n, y.shape[1], top, 1 if accumulate else 0,
                                 _ptr(shared), _ptr(shared_gate if shared is not None else None), _ptr(x),
-                                _dt(x) if x is not None else F32, ctypes.c_float(factor), _stream()), "route_combine")
+                                _dt(x) if x is not None else F32, factor, _stream()), "route_combine")
 
 
 def route_sort_padded(ids, n_experts: int, pad: int, perm, inv, groups) -> None:
@@ -1463,5 +1459,14 @@ def grouped_gemm_tc(a, w, out, groups, gated: bool, act: str = "silu", limit: fl
     """The grouped product on the tcgen05 kernel: a bf16 [M, K] in tiles of 128 rows, tile t belonging to expert groups[t]
     (-1: skipped); w bf16 [E, N, K] (gated: [E, 2N, K]); out float32 [M, N], or bf16 silu(gate) * up (or the clamped form) when gated.  False when
     the kernel refuses the shape."""
-    from . import gemm_fast
     return gemm_fast.run_grouped(a, w, out, groups, gated, GLU_ACTS[act], limit, slope)
+
+
+def zero_slot(table: torch.Tensor, slot: int, most_bytes: int) -> None:
+    """Zeroes one request's slot in every state of a cache: `table` int64 [states, 2] = (address, bytes a slot), of tensors that the
+    caller keeps; `most_bytes`: the most that a state has to a slot."""
+    _need(table, "table", torch.int64, 2)
+    _check(build.load("elementwise").hk_zero_slot(_ptr(table), int(table.shape[0]), slot, most_bytes, _stream()), "zero_slot")
+
+
+from . import attention_fast, gemm_fast  # noqa: E402  (they use this module; looked up once, not on each call)

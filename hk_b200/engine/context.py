@@ -2,6 +2,7 @@
 host-built tables the parts asked for."""
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass, field
 from typing import Callable, Dict, Hashable, List, Optional, Sequence, Tuple
 
@@ -104,6 +105,6 @@ def bind_step(ctx: StepContext, packed: PackedStep, device_buffer: torch.Tensor)
     for key, arrs in packed.layout.items():
         views = {}
         for name, (off, shape) in arrs.items():
-            size = int(np.prod(shape)) if len(shape) else 1
+            size = math.prod(shape)
             views[name] = device_buffer[off:off + size].view(shape)
         ctx.tables[key] = (views, packed.infos[key])
