@@ -458,24 +458,32 @@ def run_narrow(a, w, out) -> bool:
     return True
 
 
-GROUPED_ROWS = 128      # rows of a tile of the grouped tcgen05 product: an expert's rows start on a multiple of it
+def grouped_tile_rows(pairs: int, experts: int) -> int:
+    """Rows of a tile of the grouped product for so many (row, choice) pairs: a tile's width follows its rows in steps of 32, but what
+    it loads, and how deep its ring is, follows the most it may have.  Both products, us (8 experts, width 4,096; rows a tile 64 / 128 /
+    256): 128 pairs 71.1 / 71.3 / 72.0, 600 87.0 / 77.5 / 78.4, 1,400 115 / 101 / 90, 4,096 263 / 196 / 187."""
+    each = pairs / experts
+    return 64 if each <= 32 else 128 if each <= 100 else 256
 
 
-def run_grouped(a, w, out, groups, gated: bool, act: int = 0, limit: float = 0.0, slope: float = 1.0) -> bool:
-    """out[tile rows] = a[tile rows] w[groups[tile]]^T over tiles of 128 rows (`hk_gemm_tc_grouped`); gated: act 0 (silu) or
-    2 (the clamped form) of the two halves."""
+def run_pair_grouped(a, w, out, tiles, offsets, tile_rows: int, gated: bool, act: int = 0, limit: float = 0.0, slope: float = 1.0) -> bool:
+    """out[p] = a[p] w[group of p]^T for the rows p that `tiles` and `offsets` name (`hk_gemm_pair_grouped`); gated: act 0 (silu) or 2
+    (the clamped form) of the two halves.  False when the kernel refuses."""
     if gated and act not in (0, 2):
         return False
     M, K = a.shape
     E, N = int(w.shape[0]), int(w.shape[1])
-    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or K % 8 or M % GROUPED_ROWS or not _aligned(a, w) \
-            or not w.is_contiguous() or (gated and N % 2):
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or K % 8 or not _aligned(a, w) or not w.is_contiguous() or (gated and N % 2):
         return False
-    bn = min(256, -(-N // 32) * 32)
-    lib = build.load("gemm_tc")
-    code = lib.hk_gemm_tc_grouped(_ptr(a), _ptr(w), _ptr(out), M, N, K, out.shape[1], 2 + act if gated else 0, bn, E,
-                                  _ptr(groups), _ptr(status_flag(a.device)), limit, slope, _stream())
+    code = build.load("gemm_pair").hk_gemm_pair_grouped(
+        _ptr(a), _ptr(w), _ptr(out), M, N, K, out.shape[1], 2 + act if gated else 0, E, _ptr(tiles), tiles.shape[0], _ptr(offsets), tile_rows,
+        _sms(a.device) // 2, _ptr(status_flag(a.device)), limit, slope, _stream())
     if code == _UNSUPPORTED:
         return False
-    ops._check(code, "grouped gemm (tcgen05)")
+    ops._check(code, "grouped gemm (tcgen05, pairs)")
     return True
+
+
+def run_grouped(*args, **kwargs) -> bool:
+    """`run_pair_grouped` for prompt-sized steps, whose rows are in the experts' order already."""
+    return run_pair_grouped(*args, **kwargs)

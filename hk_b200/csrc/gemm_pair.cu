@@ -50,18 +50,46 @@ struct PairShape {
 
 __host__ __device__ inline int widest(const PairShape& s) { return 32 * ((s.units + s.tiles_m - 1) / s.tiles_m); }
 
-// One item: weight rows from 256 tf on, `width` rows of a from t0 on, K blocks [k0, k1).
+// The grouped form (a feed-forward of experts): a's rows are sorted by group, tile g = tiles[2 g] (its group; -1 from the first
+// unused one on) has up to `rows` of them from tiles[2 g + 1] on, none past offsets[group + 1], and group e's weights are the N rows
+// from e N on.
+struct PairGroups {
+  const int *tiles, *offsets;
+  int max_tiles, rows;
+};
+
+// One item: weight rows from w_row on (the tile's column `tf` of N), `width` rows of a from t0 on of which those below `end` count,
+// K blocks [k0, k1).
 struct PairItem {
-  int tile, slice, tf, t0, width, k0, k1;
-  __device__ PairItem(const PairShape& s, int item) {
-    slice = item / s.tiles;
-    tile = item - slice * s.tiles;
-    tf = tile / s.tiles_m;
-    const int tm = tile - tf * s.tiles_m, lo = tm * s.units / s.tiles_m, hi = (tm + 1) * s.units / s.tiles_m;
-    t0 = 32 * lo;
-    width = 32 * (hi - lo);
-    k0 = (int)((long long)s.kb * slice / s.slices);
-    k1 = (int)((long long)s.kb * (slice + 1) / s.slices);
+  int tile, tf, w_row, t0, width, end, k0, k1;
+  template <bool GLU>
+  static __device__ __forceinline__ PairItem plain(const PairShape& s, int item) {
+    PairItem it;
+    const int slice = item / s.tiles;
+    it.tile = item - slice * s.tiles;
+    it.tf = it.tile / s.tiles_m;
+    const int tm = it.tile - it.tf * s.tiles_m, lo = tm * s.units / s.tiles_m, hi = (tm + 1) * s.units / s.tiles_m;
+    it.t0 = 32 * lo;
+    it.width = 32 * (hi - lo);
+    it.end = min(s.M, 32 * hi);
+    it.w_row = it.tf * (GLU ? FT / 2 : FT);
+    it.k0 = (int)((long long)s.kb * slice / s.slices);
+    it.k1 = (int)((long long)s.kb * (slice + 1) / s.slices);
+    return it;
+  }
+  template <bool GLU>
+  static __device__ __forceinline__ PairItem grouped(const PairShape& s, const PairGroups& g, int used, int item) {
+    PairItem it;
+    it.tf = item / used;
+    it.tile = item - it.tf * used;
+    const int e = g.tiles[2 * it.tile];
+    it.t0 = g.tiles[2 * it.tile + 1];
+    it.end = min(it.t0 + g.rows, g.offsets[e + 1]);
+    it.width = (it.end - it.t0 + 31) & ~31;
+    it.w_row = e * s.N + it.tf * (GLU ? FT / 2 : FT);
+    it.k0 = 0;
+    it.k1 = s.kb;
+    return it;
   }
 };
 // Floats of one item's sums in `partial`: [CTA][quarter of its rows][row of a][lane]
@@ -219,10 +247,11 @@ __device__ __forceinline__ void emit(const float (&v)[32], void* out, long long 
 }
 
 // map_a: boxes of half the widest tile's rows; map_w: 128 weight rows, gated 64 of [K, 2, F] so that gate and up rows alternate.
-template <int EPI>
+template <int EPI, bool GROUPED>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, void* __restrict__ out,
-                 const PairShape s, long long ldo, int stages, float* __restrict__ partial, int* __restrict__ status, GluParams gp) {
+                 const PairShape s, const PairGroups g, long long ldo, int stages, float* __restrict__ partial, int* __restrict__ status,
+                 GluParams gp) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   PairControl& sm = *reinterpret_cast<PairControl*>(base);
@@ -230,7 +259,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   volatile int* abort_flag = &sm.abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = blockIdx.x & 1, other = rank ^ 1;
-  const int max_w = widest(s);
+  const int max_w = GROUPED ? g.rows : widest(s);
   const uint32_t stage_bytes = W_BYTES + (uint32_t)max_w * BK;           // (max_w / 2 rows of 128 bytes)
 
   if (threadIdx.x == 0) {
@@ -256,22 +285,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const uint32_t tmem_base = sm.tmem_base;
   pdl_wait();
 
-  const int first_item = blockIdx.x >> 1, pairs = gridDim.x >> 1, items = s.tiles * s.slices;
+  int used = 0;                 // tiles that have rows
+  if (GROUPED) {
+    for (int t = lane; t < g.max_tiles; t += 32) used += g.tiles[2 * t] >= 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) used += __shfl_xor_sync(0xffffffffu, used, o);
+  }
+  const int first_item = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int items = GROUPED ? used * s.tiles : s.tiles * s.slices;
+  auto item_of = [&](int i) {
+    if constexpr (GROUPED) return PairItem::grouped<IS_GLU(EPI)>(s, g, used, i);
+    else return PairItem::plain<IS_GLU(EPI)>(s, i);
+  };
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0, issued = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int i = first_item; i < items && ok; i += pairs) {
-        const PairItem it(s, i);
+        const PairItem it = item_of(i);
         const int row = it.t0 + (int)rank * (it.width >> 1);
         for (int kb = it.k0; kb < it.k1; ++kb) {
           if (!pair_wait(&sm.empty[stage], phase ^ 1u, abort_flag, other)) { ok = false; break; }
           const uint32_t st = smem_u32(ring) + (uint32_t)stage * stage_bytes;
           if (rank == 0) mbar_expect_tx(&sm.full[stage], 2 * stage_bytes);
           const uint32_t bar = in_cta(smem_u32(&sm.full[stage]), 0);
-          if (IS_GLU(EPI)) pair_load_3d(st, &map_w, bar, kb * BK, 0, it.tf * (FT / 2) + (int)rank * 64);
-          else pair_load_2d(st, &map_w, bar, kb * BK, it.tf * FT + (int)rank * 128);
+          if (IS_GLU(EPI)) pair_load_3d(st, &map_w, bar, kb * BK, 0, it.w_row + (int)rank * 64);
+          else pair_load_2d(st, &map_w, bar, kb * BK, it.w_row + (int)rank * 128);
           pair_load_2d(st + W_BYTES, &map_a, bar, kb * BK, row);
           ++issued;
           if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -290,7 +330,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       uint32_t phase = 0;
       bool ok = true;
       for (int i = first_item; i < items && ok; i += pairs) {
-        const PairItem it(s, i);
+        const PairItem it = item_of(i);
         // fp32 accumulate, bf16 x bf16, both K-major, N = width, M = 256
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(it.width >> 3) << 17) | ((uint32_t)(FT >> 4) << 24);
         const int buf = local & 1;
@@ -317,16 +357,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int first = (warp - 2) >> 2 ? 32 : 0;       // its chunks of 32 rows of a: every other one
     int local = 0;
     for (int i = first_item; i < items; i += pairs) {
-      const PairItem it(s, i);
+      const PairItem it = item_of(i);
       const int buf = local & 1;
       const uint32_t use = (uint32_t)(local >> 1) & 1u;
       ++local;
-      const int f = lane_row<EPI>(it.tf, (int)rank, quarter, lane), end = it.t0 + it.width;
+      const int f = lane_row<EPI>(it.tf, (int)rank, quarter, lane);
       const bool whole = s.slices == 1;
       // what a whole tile is added onto does not depend on the product: asked for a chunk ahead
       float y[32];
       const float* onto = reinterpret_cast<const float*>(out);
-      if (EPI == EPI_ADD && whole) load_onto(onto, ldo, f, it.t0 + first, min(s.M, end), s.N, y);
+      if (EPI == EPI_ADD && whole) load_onto(onto, ldo, f, it.t0 + first, it.end, s.N, y);
       if (!__all_sync(0xffffffffu, pair_wait(&sm.tmem_full[buf], use, abort_flag, other))) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MAX_W);
@@ -344,13 +384,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           float sum[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) sum[j] = y[j] + __uint_as_float(v[j]);
-          if (c + 64 < it.width) load_onto(onto, ldo, f, it.t0 + c + 64, s.M, s.N, y);
-          store_rows(sum, reinterpret_cast<float*>(out), ldo, f, it.t0 + c, s.M, s.N);
+          if (c + 64 < it.width) load_onto(onto, ldo, f, it.t0 + c + 64, it.end, s.N, y);
+          store_rows(sum, reinterpret_cast<float*>(out), ldo, f, it.t0 + c, it.end, s.N);
         } else {
           float sum[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) sum[j] = __uint_as_float(v[j]);
-          emit<EPI>(sum, out, ldo, f, it.t0 + c, s.M, s.N, gp);
+          emit<EPI>(sum, out, ldo, f, it.t0 + c, it.end, s.N, gp);
         }
       }
       tc_fence_before();
@@ -376,7 +416,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 template <int EPI>
 __global__ void __launch_bounds__(128)
 gemm_pair_add_kernel(const float* __restrict__ partial, void* __restrict__ out, const PairShape s, long long ldo, GluParams gp) {
-  const PairItem it(s, (int)blockIdx.x >> 1);
+  const PairItem it = PairItem::plain<IS_GLU(EPI)>(s, (int)blockIdx.x >> 1);
   const int rank = blockIdx.x & 1, c = blockIdx.y * 32, quarter = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int max_w = widest(s), f = lane_row<EPI>(it.tf, rank, quarter, lane);
   const float* p = partial + it.tile * item_floats(max_w) + ((size_t)(rank * 4 + quarter) * max_w + c) * 32 + lane;
@@ -398,11 +438,11 @@ gemm_pair_add_kernel(const float* __restrict__ partial, void* __restrict__ out, 
   emit<EPI>(sum, out, ldo, f, it.t0 + c, s.M, s.N, gp);
 }
 
-// [2][F][K] seen as [F][2][K]: 64 pairs of a gate row and its up row
-bool make_gated_map(CUtensorMap* map, const void* ptr, int F, int cols) {
+// [groups][2][F][K], row f of a group's gates beside row f of its ups: 64 such pairs from row 2 F group + f on
+bool make_gated_map(CUtensorMap* map, const void* ptr, int F, int cols, int groups) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[3] = {(cuuint64_t)cols, 2, (cuuint64_t)F};
+  cuuint64_t dims[3] = {(cuuint64_t)cols, 2, (cuuint64_t)F * (2 * groups - 1)};
   cuuint64_t strides[2] = {(cuuint64_t)F * cols * 2, (cuuint64_t)cols * 2};
   cuuint32_t box[3] = {(cuuint32_t)BK, 2, 64};
   cuuint32_t estr[3] = {1, 1, 1};
@@ -411,16 +451,17 @@ bool make_gated_map(CUtensorMap* map, const void* ptr, int F, int cols) {
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int EPI>
-int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* out, const PairShape& s, long long ldo, int pairs, float* partial,
-                int* status, GluParams gp, cudaStream_t stream) {
+template <int EPI, bool GROUPED>
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* out, const PairShape& s, const PairGroups& g, long long ldo, int pairs,
+                float* partial, int* status, GluParams gp, cudaStream_t stream) {
   static HkSmemCache allowed = {};
-  const int stage_bytes = W_BYTES + widest(s) * BK;
+  const int stage_bytes = W_BYTES + (GROUPED ? g.rows : widest(s)) * BK;
   const int stages = min(PAIR_STAGES, PAIR_RING / stage_bytes);
   const size_t smem = (size_t)stages * stage_bytes + PAIR_CONTROL + 1024;
-  if (int e = hk_allow_smem(gemm_pair_kernel<EPI>, smem, allowed)) return e;
+  if (int e = hk_allow_smem(gemm_pair_kernel<EPI, GROUPED>, smem, allowed)) return e;
+  const long long items = (long long)s.tiles * (GROUPED ? g.max_tiles : s.slices);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(2 * min(pairs, s.tiles * s.slices)));
+  cfg.gridDim = dim3((unsigned)(2 * (items < pairs ? (int)items : pairs)));
   cfg.blockDim = dim3(PAIR_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
@@ -432,8 +473,8 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* out, const P
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  if (int e = (int)cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI>, ma, mw, out, s, ldo, stages, partial, status, gp)) return e;
-  if (s.slices == 1) return 0;
+  if (int e = (int)cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI, GROUPED>, ma, mw, out, s, g, ldo, stages, partial, status, gp)) return e;
+  if (GROUPED || s.slices == 1) return 0;
   return hk_launch_pdl(gemm_pair_add_kernel<EPI>, dim3((unsigned)(2 * s.tiles), (unsigned)(widest(s) / 32)), dim3(128), 0, stream,
                        (const float*)partial, out, s, ldo, gp);
 }
@@ -467,16 +508,45 @@ HK_API int hk_gemm_pair(const void* a, const void* w, void* out, int M, int N, i
   s.tiles = (int)tiles;
   CUtensorMap ma, mw;
   if (!make_map(&ma, a, M, K, widest(s) / 2)) return HK_ERR_UNSUPPORTED;
-  if (!(IS_GLU(epilogue) ? make_gated_map(&mw, w, N / 2, K) : make_map(&mw, w, N, K, 128))) return HK_ERR_UNSUPPORTED;
+  if (!(IS_GLU(epilogue) ? make_gated_map(&mw, w, N / 2, K, 1) : make_map(&mw, w, N, K, 128))) return HK_ERR_UNSUPPORTED;
   const GluParams gp = {limit, slope};
+  const PairGroups none = {};
   cudaStream_t st = (cudaStream_t)stream;
   switch (epilogue) {
-    case EPI_STORE: return launch_pair<EPI_STORE>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
-    case EPI_ADD: return launch_pair<EPI_ADD>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
-    case EPI_SWIGLU: return launch_pair<EPI_SWIGLU>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
-    case EPI_GEGLU: return launch_pair<EPI_GEGLU>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
-    case EPI_CLAMPGLU: return launch_pair<EPI_CLAMPGLU>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
-    case EPI_SQRELU: return launch_pair<EPI_SQRELU>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
-    default: return launch_pair<EPI_NARROW>(ma, mw, out, s, ldo, pairs, partial, status, gp, st);
+    case EPI_STORE: return launch_pair<EPI_STORE, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
+    case EPI_ADD: return launch_pair<EPI_ADD, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
+    case EPI_SWIGLU: return launch_pair<EPI_SWIGLU, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
+    case EPI_GEGLU: return launch_pair<EPI_GEGLU, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
+    case EPI_CLAMPGLU: return launch_pair<EPI_CLAMPGLU, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
+    case EPI_SQRELU: return launch_pair<EPI_SQRELU, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
+    default: return launch_pair<EPI_NARROW, false>(ma, mw, out, s, none, ldo, pairs, partial, status, gp, st);
   }
+}
+
+// The grouped form: a has M rows sorted by group, w is [n_groups][N][K], out has a's rows: out[p] = a[p] w[group of p]^T for the rows that
+// tiles int32 [max_tiles, 2] = (group, first row; group -1 from the first unused tile on) name, at most tile_rows (a multiple of 32 up
+// to 256) of each and none past offsets[group + 1].  Epilogue 0 (fp32 store), 2 or 4 (gated, w[group] = [N/2 gate rows | N/2 up rows]).
+HK_API int hk_gemm_pair_grouped(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, int epilogue, int n_groups,
+                                const int* tiles, int max_tiles, const int* offsets, int tile_rows, int pairs, int* status, float limit,
+                                float slope, void* stream) {
+  if (M <= 0 || N <= 0 || n_groups <= 0 || max_tiles <= 0) return 0;
+  if (K <= 0 || (K & 7) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || pairs < 1) return HK_ERR_UNSUPPORTED;
+  if ((epilogue != EPI_STORE && epilogue != EPI_SWIGLU && epilogue != EPI_CLAMPGLU) || (IS_GLU(epilogue) && (N & 1))) return HK_ERR_UNSUPPORTED;
+  if (tile_rows < 32 || tile_rows > MAX_W || (tile_rows & 31)) return HK_ERR_UNSUPPORTED;
+  if ((long long)n_groups * N > 0x7fffffffLL) return HK_ERR_UNSUPPORTED;
+  PairShape s = {};
+  s.M = M, s.N = N, s.K = K;
+  s.kb = (K + BK - 1) / BK;
+  s.slices = 1;
+  s.tiles = (N + FT - 1) / FT;          // (of one tile of rows)
+  if ((long long)s.tiles * max_tiles > 0x3fffffffLL) return HK_ERR_UNSUPPORTED;
+  const PairGroups g = {tiles, offsets, max_tiles, tile_rows};
+  CUtensorMap ma, mw;
+  if (!make_map(&ma, a, M, K, tile_rows / 2)) return HK_ERR_UNSUPPORTED;
+  if (!(IS_GLU(epilogue) ? make_gated_map(&mw, w, N / 2, K, n_groups) : make_map(&mw, w, n_groups * N, K, 128))) return HK_ERR_UNSUPPORTED;
+  const GluParams gp = {limit, slope};
+  cudaStream_t st = (cudaStream_t)stream;
+  if (epilogue == EPI_STORE) return launch_pair<EPI_STORE, true>(ma, mw, out, s, g, ldo, pairs, nullptr, status, gp, st);
+  if (epilogue == EPI_SWIGLU) return launch_pair<EPI_SWIGLU, true>(ma, mw, out, s, g, ldo, pairs, nullptr, status, gp, st);
+  return launch_pair<EPI_CLAMPGLU, true>(ma, mw, out, s, g, ldo, pairs, nullptr, status, gp, st);
 }

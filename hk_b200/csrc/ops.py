@@ -10,6 +10,7 @@ can be pinned with `force()` by tests.
 from __future__ import annotations
 
 import contextlib
+import ctypes
 from typing import Optional
 
 import numpy as np
@@ -1370,25 +1371,26 @@ def route_topk(x, w_router, ids, weights, scores: str = "softmax", correction=No
                              norm_eps, extra, _ptr(extra_out), _ptr(bias), _stream()), "route_topk")
 
 
-def route_sort(ids, n_experts: int, offsets, perm, inv, tiles) -> None:
+def route_sort(ids, n_experts: int, offsets, perm, inv, tiles, tile_rows: int = 0) -> None:
     """Lays the (row, choice) pairs out by expert: offsets int32 [E+1], perm [pairs] (sorted place -> pair), inv [pairs]
     (pair -> sorted place, -1 for an id of n_experts or more: an identity), tiles int32 [max_tiles, 2] = (expert, first sorted place) of every tile of
-    `route_tile_rows()` rows, -1 for unused tiles."""
+    `tile_rows` (0: `route_tile_rows()`) rows, -1 for unused tiles."""
     for name, t in (("ids", ids), ("offsets", offsets), ("perm", perm), ("inv", inv), ("tiles", tiles)):
         _need(t, name, torch.int32)
     pairs = ids.numel()
     if offsets.numel() != n_experts + 1 or perm.numel() != pairs or inv.numel() != pairs or tiles.dim() != 2 or tiles.shape[1] != 2:
         raise KernelError("route_sort: shapes do not fit")
     lib = build.load("routed")
-    _check(lib.hk_route_sort(_ptr(ids), pairs, n_experts, _ptr(offsets), _ptr(perm), _ptr(inv), _ptr(tiles), tiles.shape[0],
+    _check(lib.hk_route_sort(_ptr(ids), pairs, n_experts, tile_rows or route_tile_rows(), _ptr(offsets), _ptr(perm), _ptr(inv), _ptr(tiles), tiles.shape[0],
                              _stream()), "route_sort")
 
 
 def grouped_gemm(a, w, out, tiles, offsets, perm, top: int, gather: bool, gated: bool, act: str = "silu", limit: float = 0.0,
-                 slope: float = 1.0) -> None:
+                 slope: float = 1.0, tile_rows: int = 0) -> None:
     """A product per expert over the sorted rows.  w [E, N, K] (gated: [E, 2N, K] = N gate rows then N up rows);
     row p of the product reads a[perm[p] // top] (gather) or a[p]; out[p, :N] = a . w[e]^T in float32, or
-    silu(gate) * up (or the clamped form of `swiglu`) in a's type when gated."""
+    silu(gate) * up (or the clamped form of `swiglu`) in a's type when gated.  bfloat16 with K a multiple of 8 takes the tensor cores, in
+    tiles of `tile_rows` rows (0: `route_tile_rows()`); else FMAs, in tiles of `route_tile_rows()`."""
     if act not in ("silu", "swish_clamped"):
         raise KernelError(f"grouped_gemm: activation {act!r} is neither 'silu' nor 'swish_clamped'")
     _need(a, "a", dims=2)
@@ -1398,6 +1400,15 @@ def grouped_gemm(a, w, out, tiles, offsets, perm, top: int, gather: bool, gated:
     N = out.shape[1]
     if w.shape[2] != K or w.shape[1] != (2 * N if gated else N) or out.dtype != (a.dtype if gated else torch.float32):
         raise KernelError("grouped_gemm: shapes or types do not fit")
+    if a.dtype == torch.bfloat16 and K % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0:
+        rows = a
+        if gather:
+            rows = torch.empty((perm.shape[0], K), dtype=a.dtype, device=a.device)
+            route_gather(a, perm, offsets, top, rows)
+        if gemm_fast.run_pair_grouped(rows, w, out, tiles, offsets, tile_rows or route_tile_rows(), gated, GLU_ACTS[act], limit, slope):
+            return
+    if tile_rows not in (0, route_tile_rows()):
+        raise KernelError(f"grouped_gemm: tiles of {tile_rows} rows for the product without tensor cores")
     lib = build.load("routed")
     _check(lib.hk_grouped_gemm(_ptr(a), _ptr(w), _dt(a), _ptr(out), _ptr(tiles), tiles.shape[0], _ptr(offsets), _ptr(perm),
                                int(top), 1 if gather else 0, N, K, 1 if gated else 0, 1 if act == "swish_clamped" else 0,
@@ -1430,36 +1441,64 @@ def route_combine(ys, inv, weights, y, accumulate: bool = False, shared=None, sh
                                 _dt(x) if x is not None else F32, factor, _stream()), "route_combine")
 
 
-def route_sort_padded(ids, n_experts: int, pad: int, perm, inv, groups) -> None:
-    """The layout for the tcgen05 grouped product: every expert's rows start on a multiple of `pad`.  perm int32 [M_max]
-    (sorted place -> pair, -1 for padding), inv [pairs], groups [M_max / pad] (tile -> expert or -1);
-    M_max >= pairs + E * (pad - 1) and a multiple of pad."""
-    for name, t in (("ids", ids), ("perm", perm), ("inv", inv), ("groups", groups)):
-        _need(t, name, torch.int32)
-    pairs, m_max = ids.numel(), perm.numel()
-    if inv.numel() != pairs or groups.numel() * pad != m_max:
-        raise KernelError("route_sort_padded: shapes do not fit")
-    lib = build.load("routed")
-    _check(lib.hk_route_sort_padded(_ptr(ids), pairs, n_experts, int(pad), _ptr(perm), _ptr(inv), _ptr(groups), m_max, _stream()),
-           "route_sort_padded")
-
-
-def route_gather(x, perm, top: int, xs) -> None:
-    """xs[p, :] = x[perm[p] // top, :] (zeros where perm[p] < 0), bfloat16 rows of a multiple of 8 elements."""
+def route_gather(x, perm, offsets, top: int, xs) -> None:
+    """xs[p, :] = x[perm[p] // top, :] for the sorted places p below offsets[-1], bfloat16 rows of a multiple of 8 elements."""
     _need(x, "x", torch.bfloat16, 2)
     _need(xs, "xs", torch.bfloat16, 2)
     _need(perm, "perm", torch.int32, 1)
+    _need(offsets, "offsets", torch.int32, 1)
     if xs.shape[0] != perm.shape[0] or xs.shape[1] != x.shape[1]:
         raise KernelError("route_gather: shapes do not fit")
     lib = build.load("routed")
-    _check(lib.hk_route_gather(_ptr(x), _ptr(perm), int(top), _ptr(xs), xs.shape[0], xs.shape[1], _stream()), "route_gather")
+    _check(lib.hk_route_gather(_ptr(x), _ptr(perm), _ptr(offsets) + 4 * (offsets.shape[0] - 1), int(top), _ptr(xs), xs.shape[0], xs.shape[1],
+                               _stream()), "route_gather")
 
 
-def grouped_gemm_tc(a, w, out, groups, gated: bool, act: str = "silu", limit: float = 0.0, slope: float = 1.0) -> bool:
-    """The grouped product on the tcgen05 kernel: a bf16 [M, K] in tiles of 128 rows, tile t belonging to expert groups[t]
-    (-1: skipped); w bf16 [E, N, K] (gated: [E, 2N, K]); out float32 [M, N], or bf16 silu(gate) * up (or the clamped form) when gated.  False when
-    the kernel refuses the shape."""
-    return gemm_fast.run_grouped(a, w, out, groups, gated, GLU_ACTS[act], limit, slope)
+def grouped_gemm_tc(a, w, out, tiles, offsets, tile_rows: int, gated: bool, act: str = "silu", limit: float = 0.0, slope: float = 1.0) -> bool:
+    """The grouped product on the tensor cores for rows that are in the experts' order: a bf16 [pairs, K], `tiles` and `offsets` of
+    `route_sort` with `tile_rows`; w bf16 [E, N, K] (gated: [E, 2N, K]); out float32 [pairs, N], or bf16 silu(gate) * up (or the
+    clamped form) when gated.  False when the kernel refuses the shape."""
+    return gemm_fast.run_grouped(a, w, out, tiles, offsets, tile_rows, gated, GLU_ACTS[act], limit, slope)
+
+
+_grouped_product = None
+
+
+def routed_experts(x, ids, weights, w_gate_up, w_down, y, act: str = "silu", limit: float = 0.0, slope: float = 1.0, accumulate: bool = False,
+                   shared=None, shared_gate=None, identities: bool = False, factor: float = 1.0) -> None:
+    """What follows `route_topk` in a step of few pairs, in bfloat16: x [n, d] by expert, `w_gate_up` [E, 2F, d] with the gated activation,
+    `w_down` [E, d, F], and the choices put together in y as `route_combine` does (`identities`: ids of E and more give x back).
+    d and F are multiples of 8."""
+    global _grouped_product
+    _need(x, "x", torch.bfloat16, 2)
+    _need(ids, "ids", torch.int32, 2)
+    _need(weights, "weights", torch.float32, 2)
+    _need(w_gate_up, "w_gate_up", torch.bfloat16, 3)
+    _need(w_down, "w_down", torch.bfloat16, 3)
+    _need(y, "y", torch.float32, 2)
+    n, d = x.shape
+    E, _, F = w_down.shape
+    top = ids.shape[1]
+    if w_gate_up.shape != (E, 2 * F, d) or w_down.shape[1] != d or ids.shape[0] != n or weights.shape != ids.shape or y.shape != x.shape \
+            or act not in ("silu", "swish_clamped"):
+        raise KernelError("routed_experts: shapes do not fit")
+    if shared is not None:
+        _need(shared, "shared", torch.float32, 2)
+        if shared.shape != y.shape:
+            raise KernelError("routed_experts: the shared result must have y's shape")
+        if shared_gate is not None:
+            _need(shared_gate, "shared_gate", torch.float32)
+            if shared_gate.numel() != n:
+                raise KernelError("routed_experts: one shared gate per row")
+    lib = build.load("routed")
+    if _grouped_product is None:
+        _grouped_product = ctypes.cast(build.load("gemm_pair").hk_gemm_pair_grouped, ctypes.c_void_p).value
+    rows = gemm_fast.grouped_tile_rows(n * top, E)
+    scratch = torch.empty(lib.hk_routed_experts_scratch(n * top, E, d, F, rows), dtype=torch.uint8, device=x.device)
+    _check(lib.hk_routed_experts(_grouped_product, _ptr(x), _ptr(ids), _ptr(weights), _ptr(w_gate_up), _ptr(w_down), _ptr(y), _ptr(scratch),
+                                 n, d, F, E, top, rows, 2 + 2 * (act == "swish_clamped"), limit, slope, 1 if accumulate else 0, _ptr(shared),
+                                 _ptr(shared_gate if shared is not None else None), 1 if identities else 0, factor,
+                                 gemm_fast._sms(x.device) // 2, _ptr(gemm_fast.status_flag(x.device)), _stream()), "routed_experts", launches=4)
 
 
 def zero_slot(table: torch.Tensor, slot: int, most_bytes: int) -> None:

@@ -18,12 +18,13 @@
 //               back the token's vector); the sort leaves their pairs out and the combine adds the vector itself.
 //   2. sort:    one CTA counts the (token, choice) pairs per expert, lays the experts' rows out one after
 //               the other (`perm`: sorted place -> pair, `inv`: pair -> sorted place) and cuts every
-//               expert's rows into tiles of RT_BM rows (`tiles`: expert and first row, -1 for unused).
-//   3. experts: a grouped product over those tiles: tile rows are gathered through `perm`, the weights are
+//               expert's rows into tiles of so many rows (`tiles`: expert and first row, -1 for unused).
+//   3. experts: a grouped product over those tiles: tile rows are gathered through `perm` (in bfloat16 by a kernel
+//               of its own, before the tensor-core product of gemm_pair.cu), the weights are
 //               the tile's expert's; first gate and up with silu(gate) * up (or the clamped
 //               activation) in the epilogue, then down.
 //               A row's result does not depend on its place in a tile: every output element is one chain of
-//               k = 0..K-1 (the FMA kernel) or a fixed tree (the tensor-core kernel).
+//               k = 0..K-1 (the FMA kernel) or one of steps of 16 k (the tensor cores).
 //   4. combine: y[t] = sum over the token's choices, in the order of the choices, of weight * expert output.
 #include <math_constants.h>
 
@@ -273,77 +274,87 @@ route_sort_kernel(const int* __restrict__ ids, int pairs, int E, int bm, int* __
   }
 }
 
-HK_API int hk_route_sort(const int* ids, int pairs, int E, int* offsets, int* perm, int* inv, int* tiles, int max_tiles,
+HK_API int hk_route_sort(const int* ids, int pairs, int E, int tile_rows, int* offsets, int* perm, int* inv, int* tiles, int max_tiles,
                          void* stream) {
   if (pairs <= 0) return 0;
-  if (E > 4096) return HK_ERR_UNSUPPORTED;
+  if (E > 4096 || tile_rows < 1) return HK_ERR_UNSUPPORTED;
   return hk_launch(route_sort_kernel, dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), (cudaStream_t)stream, ids, pairs, E,
-                   RT_BM, offsets, perm, inv, tiles, max_tiles);
+                   tile_rows, offsets, perm, inv, tiles, max_tiles);
 }
 
 HK_API int hk_route_tile_rows() { return RT_BM; }
 
-// The padded layout for the tcgen05 grouped product: every expert's rows start on a multiple of `pad` (the product's
-// 128-row tile), so a tile's rows all belong to one expert.  perm[M_max] (sorted place -> pair, -1 for padding),
-// inv[pairs] (pair -> sorted place), groups[M_max / pad] (tile -> expert, -1 for tiles past the last expert).
-__global__ void __launch_bounds__(1024)
-route_sort_padded_kernel(const int* __restrict__ ids, int pairs, int E, int pad, int* __restrict__ perm, int* __restrict__ inv,
-                         int* __restrict__ groups, int m_max) {
-  extern __shared__ int smi[];                // counts[E], cursor[E]
-  int* counts = smi;
-  int* cursor = smi + E;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = 0;
-  for (int p = threadIdx.x; p < m_max; p += blockDim.x) perm[p] = -1;
-  __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x)
-    if (ids[p] < E) atomicAdd(&counts[ids[p]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int e = 0; e < E; ++e) {
-      cursor[e] = at;
-      const int span = (counts[e] + pad - 1) / pad * pad;
-      for (int r = 0; r < span && at + r < m_max; r += pad) groups[(at + r) / pad] = e;
-      at += span;
-    }
-    for (int t = at / pad; t < m_max / pad; ++t) groups[t] = -1;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    if (ids[p] >= E) {
-      inv[p] = -1;
-      continue;
-    }
-    const int at = atomicAdd(&cursor[ids[p]], 1);
-    perm[at] = p;
-    inv[p] = at;
-  }
-}
-
-HK_API int hk_route_sort_padded(const int* ids, int pairs, int E, int pad, int* perm, int* inv, int* groups, int m_max, void* stream) {
-  if (pairs <= 0) return 0;
-  if (E > 4096 || pad < 1 || m_max % pad || m_max < pairs + E * (pad - 1)) return HK_ERR_UNSUPPORTED;
-  return hk_launch(route_sort_padded_kernel, dim3(1), dim3(1024), (size_t)2 * E * sizeof(int), (cudaStream_t)stream, ids, pairs, E, pad,
-                   perm, inv, groups, m_max);
-}
-
-// xs[p, :] = x[perm[p] / top, :], or zeros where perm[p] < 0: the tokens' vectors in the padded sorted order (bf16, d % 8 == 0).
-__global__ void route_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ perm, int top, bf16* __restrict__ xs, int d) {
+// xs[p, :] = x[perm[p] / top, :] for the sorted places p < *placed: the tokens' vectors in the experts' order (bf16, d % 8 == 0).
+__global__ void route_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ perm, const int* __restrict__ placed, int top,
+                                    bf16* __restrict__ xs, int d) {
   const int p = blockIdx.x;
-  const int src = perm[p];
+  pdl_launch_dependents();
+  pdl_wait();
+  if (p >= *placed) return;             // (identities have no place)
   uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)p * d);
-  const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)(src < 0 ? 0 : src / top) * d);
-  for (int i = threadIdx.x; i < d / 8; i += blockDim.x) dst[i] = src < 0 ? make_uint4(0, 0, 0, 0) : from[i];
+  const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)(perm[p] / top) * d);
+  for (int i = threadIdx.x; i < d / 8; i += blockDim.x) dst[i] = from[i];
 }
 
-HK_API int hk_route_gather(const void* x, const int* perm, int top, void* xs, int m_max, int d, void* stream) {
-  if (m_max <= 0) return 0;
+HK_API int hk_route_gather(const void* x, const int* perm, const int* placed, int top, void* xs, int pairs, int d, void* stream) {
+  if (pairs <= 0) return 0;
   if ((d & 7) || (((uintptr_t)x | (uintptr_t)xs) & 15)) return HK_ERR_UNSUPPORTED;
-  return hk_launch(route_gather_kernel, dim3((unsigned)m_max), dim3(d >= 2048 ? 256 : 128), 0, (cudaStream_t)stream, (const bf16*)x, perm,
-                   top, (bf16*)xs, d);
+  return hk_launch_pdl(route_gather_kernel, dim3((unsigned)pairs), dim3(d >= 2048 ? 256 : 128), 0, (cudaStream_t)stream, (const bf16*)x, perm,
+                       placed, top, (bf16*)xs, d);
 }
 
-
+// Sort and gather at once for steps of few pairs: a block per pair finds its place by counting the pairs before it (lower expert, or
+// the same and earlier) and brings the token's vector there; one more block lays out `offsets` and `tiles`.  Bound by its launch: the
+// counting is pairs / 256 loads a thread.
+__global__ void __launch_bounds__(256)
+route_place_kernel(const bf16* __restrict__ x, const int* __restrict__ ids, int pairs, int E, int top, int bm, int* __restrict__ offsets,
+                   int* __restrict__ inv, int* __restrict__ tiles, int max_tiles, bf16* __restrict__ xs, int d) {
+  extern __shared__ int smi[];                // the last block: counts[E]
+  __shared__ int before;
+  const int p = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (p == pairs) {
+    for (int e = threadIdx.x; e < E; e += 256) smi[e] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < pairs; i += 256)
+      if (ids[i] < E) atomicAdd(&smi[ids[i]], 1);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    int at = 0, tile = 0;
+    for (int e = 0; e < E; ++e) {
+      offsets[e] = at;
+      for (int r = 0; r < smi[e] && tile < max_tiles; r += bm, ++tile) {
+        tiles[2 * tile] = e;
+        tiles[2 * tile + 1] = at + r;
+      }
+      at += smi[e];
+    }
+    offsets[E] = at;
+    for (; tile < max_tiles; ++tile) {
+      tiles[2 * tile] = -1;
+      tiles[2 * tile + 1] = 0;
+    }
+    return;
+  }
+  const int e = ids[p];
+  if (e >= E) {                               // an identity: it has no place
+    if (threadIdx.x == 0) inv[p] = -1;
+    return;
+  }
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  int mine = 0;
+  for (int i = threadIdx.x; i < pairs; i += 256) mine += ids[i] < e || (ids[i] == e && i < p);
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&before, mine);
+  __syncthreads();
+  const int place = before;
+  if (threadIdx.x == 0) inv[p] = place;
+  uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)place * d);
+  const uint4* from = reinterpret_cast<const uint4*>(x + (size_t)(p / top) * d);
+  for (int i = threadIdx.x; i < d / 8; i += 256) dst[i] = from[i];
+}
 
 // ------------------------------------------------------------------------------------ 3. experts
 struct GluAct {
@@ -436,156 +447,6 @@ grouped_gemm_kernel(const T* __restrict__ a, const T* __restrict__ w, TO* __rest
   }
 }
 
-// The same on the tensor cores (bf16 operands, fp32 accumulation; K a multiple of 8): a CTA takes a tile of RT_BM
-// sorted rows and 128 weight rows: plain, 128 output columns; gated, 64 gate rows and the 64 up rows that match
-// them, so that the gated activation is taken in the epilogue.  Operands come through a three-stage cp.async ring in
-// slices of 32 k (A rows gathered through `rows`), fragments by ldmatrix, products by mma.sync m16n8k16: eight
-// warps as 2 (rows) x 4 (columns), a warp 32 rows x 32 weight rows.  An output element's sum runs over k in an
-// order that does not depend on the row's place in its tile, so a token's result does not depend on the batch.
-#define GM_BN 128
-#define GM_BK 32
-#define GM_LD (GM_BK + 8)
-
-__device__ __forceinline__ uint32_t gm_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void gm_cp_async16(void* dst, const void* src, bool valid) {
-  const int bytes = valid ? 16 : 0;   // 0 source bytes: the 16 destination bytes are zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(gm_smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void gm_ldmatrix_x4(uint32_t* r, const void* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(gm_smem_u32(p)));
-}
-__device__ __forceinline__ void gm_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-// GM_STAGES: slices in the ring (dynamic shared memory): all but one on their way while one is multiplied.
-template <bool GATED, int GM_STAGES>
-__global__ void __launch_bounds__(256)
-grouped_gemm_mma_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, void* __restrict__ out_, const int* __restrict__ tiles,
-                        const int* __restrict__ offsets, const int* __restrict__ perm, int top, int gather, int N, int K, GluAct act) {
-  extern __shared__ __align__(16) uint8_t gm_smem[];
-  typedef bf16 (*ATile)[RT_BM][GM_LD];
-  typedef bf16 (*WTile)[GM_BN][GM_LD];
-  ATile As = reinterpret_cast<ATile>(gm_smem);                                               // [GM_STAGES][RT_BM][GM_LD]
-  WTile Ws = reinterpret_cast<WTile>(gm_smem + sizeof(bf16) * GM_STAGES * RT_BM * GM_LD);    // [GM_STAGES][GM_BN][GM_LD]
-  __shared__ int rows[RT_BM];
-  const int e = tiles[2 * blockIdx.y];
-  if (e < 0) return;
-  const int p0 = tiles[2 * blockIdx.y + 1];
-  const int p_end = min(p0 + RT_BM, offsets[e + 1]);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < RT_BM) {
-    const int p = p0 + tid;
-    rows[tid] = p < p_end ? (gather ? perm[p] / top : p) : -1;
-  }
-  __syncthreads();
-  constexpr int COLS = GATED ? 64 : 128;            // output columns of a tile
-  const int n0 = blockIdx.x * COLS;
-  const bf16* we = w + (size_t)e * (GATED ? 2 : 1) * N * K;
-  // what this thread copies per stage: one 16-byte piece of A, two of W
-  const int a_row = tid >> 2, a_k = (tid & 3) * 8;
-  const int a_src = rows[a_row];
-  const bf16* a_ptr = a + (size_t)max(a_src, 0) * K + a_k;
-  const bf16* w_ptr[2];
-  bool w_ok[2];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int r = (tid + j * 256) >> 2;              // row of the W tile
-    const int col = GATED ? (r & 63) : r;
-    const int gn = n0 + col;
-    w_ok[j] = gn < N;
-    const size_t wrow = GATED ? (size_t)(r >> 6) * N + min(gn, N - 1) : (size_t)min(gn, N - 1);
-    w_ptr[j] = we + wrow * K + a_k;
-  }
-  auto load = [&](int stage, int k0) {
-    const bool kin = k0 + a_k < K;
-    gm_cp_async16(&As[stage][a_row][a_k], a_ptr + k0, kin && a_src >= 0);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) gm_cp_async16(&Ws[stage][(tid + j * 256) >> 2][a_k], w_ptr[j] + k0, kin && w_ok[j]);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  const int wr = warp >> 2, wc = warp & 3;           // warp row (32 rows each), warp column
-  // the W-tile row of this warp's n8 tile nt: gated, tiles 0 and 1 are gate rows and 2 and 3 the up rows that match them
-  auto wn = [&](int nt) { return GATED ? ((nt >> 1) * 64 + wc * 16 + (nt & 1) * 8) : (wc * 32 + nt * 8); };
-  float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.f;
-  const int ksteps = (K + GM_BK - 1) / GM_BK;
-#pragma unroll
-  for (int pre = 0; pre < GM_STAGES - 1; ++pre) {      // one group per slice, also past the end: the counting below relies on it
-    if (pre < ksteps) load(pre, pre * GM_BK); else asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  for (int ks = 0; ks < ksteps; ++ks) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(GM_STAGES - 2) : "memory");
-    __syncthreads();                                  // stage ks has landed; stage ks - 1 is free for everyone
-    if (ks + GM_STAGES - 1 < ksteps) load((ks + GM_STAGES - 1) % GM_STAGES, (ks + GM_STAGES - 1) * GM_BK);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    const int st = ks % GM_STAGES;
-#pragma unroll
-    for (int kk = 0; kk < GM_BK; kk += 16) {
-      uint32_t af[2][4], bfr[2][4];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-        gm_ldmatrix_x4(af[mt], &As[st][wr * 32 + mt * 16 + (lane & 15)][kk + (lane >> 4) * 8]);
-#pragma unroll
-      for (int np = 0; np < 2; ++np)                 // two n8 tiles per ldmatrix: (tile, k half) = (lane / 16, (lane / 8) & 1)
-        gm_ldmatrix_x4(bfr[np], &Ws[st][wn(np * 2 + (lane >> 4)) + (lane & 7)][kk + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) gm_mma(acc[mt][nt], af[mt], bfr[nt >> 1][(nt & 1) * 2], bfr[nt >> 1][(nt & 1) * 2 + 1]);
-    }
-  }
-  const int g = lane >> 2, t2 = (lane & 3) * 2;
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int p = p0 + wr * 32 + mt * 16 + g + half * 8;
-      if (p >= p_end) continue;
-      if (GATED) {
-        bf16* out = reinterpret_cast<bf16*>(out_);
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int gn = n0 + wc * 16 + nt * 8 + t2 + c;
-            if (gn >= N) continue;
-            const float gate = acc[mt][nt][half * 2 + c], up = acc[mt][nt + 2][half * 2 + c];
-            out[(size_t)p * N + gn] = __float2bfloat16_rn(glu_value(gate, up, act));
-          }
-      } else {
-        float* out = reinterpret_cast<float*>(out_);
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const int gn = n0 + wc * 32 + nt * 8 + t2 + c;
-            if (gn < N) out[(size_t)p * N + gn] = acc[mt][nt][half * 2 + c];
-          }
-      }
-    }
-}
-
-template <bool GATED, int STAGES>
-static int gm_launch(const void* a, const void* w, void* out, const int* tiles, int max_tiles, const int* offsets, const int* perm,
-                     int top, int gather, int N, int K, GluAct act, cudaStream_t s) {
-  const size_t smem = sizeof(bf16) * STAGES * (RT_BM + GM_BN) * GM_LD;
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(grouped_gemm_mma_kernel<GATED, STAGES>, smem, cache)) return e;
-  dim3 grid((unsigned)((N + (GATED ? 63 : GM_BN - 1)) / (GATED ? 64 : GM_BN)), (unsigned)max_tiles);
-  return hk_launch(grouped_gemm_mma_kernel<GATED, STAGES>, grid, dim3(256), smem, s, (const bf16*)a, (const bf16*)w, out, tiles, offsets,
-                   perm, top, gather, N, K, act);
-}
-
 HK_API int hk_grouped_gemm(const void* a, const void* w, int dtype, void* out, const int* tiles, int max_tiles, const int* offsets,
                            const int* perm, int top, int gather, int N, int K, int gated, int clamped, float limit, float slope,
                            void* stream) {
@@ -600,16 +461,6 @@ HK_API int hk_grouped_gemm(const void* a, const void* w, int dtype, void* out, c
                        tiles, offsets, perm, top, gather, N, K, act);
     return hk_launch(grouped_gemm_kernel<float, float, false>, grid, dim3(256), 0, s, (const float*)a, (const float*)w, (float*)out,
                      tiles, offsets, perm, top, gather, N, K, act);
-  }
-  if (dtype == HK_BF16 && (K & 7) == 0 && ((((uintptr_t)a | (uintptr_t)w) & 15) == 0)) {
-    // few rows (decode steps): the products are bound by the experts' weight bytes, and a ring of six slices keeps more of
-    // them on their way (width 4,096, 128 pairs: 88 and 45 us against 97 and 57 with three); many rows: three slices leave
-    // room for four CTAs an SM (4,096 pairs: 546 and 297 us against 653 and 307 with six)
-    const bool deep = max_tiles <= 40;       // tiles = pairs / 64 + experts: a few hundred pairs at most
-    if (gated) return deep ? gm_launch<true, 6>(a, w, out, tiles, max_tiles, offsets, perm, top, gather, N, K, act, s)
-                           : gm_launch<true, 3>(a, w, out, tiles, max_tiles, offsets, perm, top, gather, N, K, act, s);
-    return deep ? gm_launch<false, 6>(a, w, out, tiles, max_tiles, offsets, perm, top, gather, N, K, act, s)
-                : gm_launch<false, 3>(a, w, out, tiles, max_tiles, offsets, perm, top, gather, N, K, act, s);
   }
   if (dtype == HK_BF16) {
     if (gated)
@@ -630,6 +481,7 @@ __global__ void route_combine_kernel(const float* __restrict__ ys, const int* __
                                      float* __restrict__ y, int d, int top, int accumulate, const float* __restrict__ shared,
                                      const float* __restrict__ shared_gate, const T* __restrict__ x, float factor) {
   const int t = blockIdx.x;
+  pdl_wait();
   const float sg = shared != nullptr ? (shared_gate != nullptr ? shared_gate[t] : 1.0f) : 0.f;
   for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < d; i += gridDim.y * blockDim.x) {
     float acc = 0.f;
@@ -654,10 +506,66 @@ HK_API int hk_route_combine(const float* ys, const int* inv, const float* weight
   const dim3 grid((unsigned)n, (unsigned)split);
   cudaStream_t s = (cudaStream_t)stream;
   if (x_dtype == HK_F32)
-    return hk_launch(route_combine_kernel<float>, grid, dim3(threads), 0, s, ys, inv, weights, y, d, top, accumulate, shared, shared_gate,
+    return hk_launch_pdl(route_combine_kernel<float>, grid, dim3(threads), 0, s, ys, inv, weights, y, d, top, accumulate, shared, shared_gate,
                      (const float*)x, factor);
   if (x_dtype == HK_BF16)
-    return hk_launch(route_combine_kernel<bf16>, grid, dim3(threads), 0, s, ys, inv, weights, y, d, top, accumulate, shared, shared_gate,
+    return hk_launch_pdl(route_combine_kernel<bf16>, grid, dim3(threads), 0, s, ys, inv, weights, y, d, top, accumulate, shared, shared_gate,
                      (const bf16*)x, factor);
   return HK_ERR_UNSUPPORTED;
+}
+
+// ------------------------------------------------------------------------------------ 2 to 4 at once
+// Everything behind the choice for a step of few (token, choice) pairs in bf16: sort and gather, the two grouped products
+// (`grouped`: hk_gemm_pair_grouped of the library beside this one), combine.  One call, because such a step waits for the host: 64
+// tokens of 4,096 by eight experts of 2,048 take the GPU 90 us, and a wrapper around each launch made the pass 171.
+// w_gate_up [E][2 F][d], w_down [E][d][F]; scratch: hk_routed_experts_scratch bytes, 16-byte aligned; the rest as hk_route_combine.
+typedef int (*GroupedProduct)(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, int epilogue, int n_groups,
+                              const int* tiles, int max_tiles, const int* offsets, int tile_rows, int pairs, int* status, float limit,
+                              float slope, void* stream);
+namespace {
+struct ExpertsScratch {
+  size_t offsets, inv, tiles, xs, h, ys, bytes;
+  int max_tiles;
+  ExpertsScratch(int pairs, int E, int d, int F, int tile_rows) {
+    size_t at = 0;
+    auto take = [&](size_t n) { const size_t r = at; at += (n + 255) & ~(size_t)255; return r; };
+    max_tiles = pairs / tile_rows + (E < pairs ? E : pairs);
+    offsets = take((size_t)(E + 1) * 4);
+    inv = take((size_t)pairs * 4);
+    tiles = take((size_t)max_tiles * 8);
+    xs = take((size_t)pairs * d * 2);
+    h = take((size_t)pairs * F * 2);
+    ys = take((size_t)pairs * d * 4);
+    bytes = at;
+  }
+};
+}  // namespace
+
+HK_API long long hk_routed_experts_scratch(int pairs, int E, int d, int F, int tile_rows) {
+  return (long long)ExpertsScratch(pairs, E, d, F, tile_rows).bytes;
+}
+
+HK_API int hk_routed_experts(const void* grouped, const void* x, const int* ids, const float* weights, const void* w_gate_up,
+                             const void* w_down, float* y, void* scratch, int n, int d, int F, int E, int top, int tile_rows, int epilogue,
+                             float limit, float slope, int accumulate, const float* shared, const float* shared_gate, int identities,
+                             float factor, int sm_pairs, int* status, void* stream) {
+  if (n <= 0) return 0;
+  if (grouped == nullptr || E < 1 || E > 4096 || top < 1 || (d & 7) || (F & 7) || tile_rows < 32 || (((uintptr_t)x | (uintptr_t)scratch) & 15))
+    return HK_ERR_UNSUPPORTED;
+  const int pairs = n * top;
+  const ExpertsScratch sc(pairs, E, d, F, tile_rows);
+  char* base = reinterpret_cast<char*>(scratch);
+  int *offsets = (int*)(base + sc.offsets), *inv = (int*)(base + sc.inv), *tiles = (int*)(base + sc.tiles);
+  const GroupedProduct product = (GroupedProduct)grouped;
+  if (int e = hk_launch_pdl(route_place_kernel, dim3((unsigned)pairs + 1), dim3(256), (size_t)E * sizeof(int), (cudaStream_t)stream, (const bf16*)x,
+                            ids, pairs, E, top, tile_rows, offsets, inv, tiles, sc.max_tiles, (bf16*)(base + sc.xs), d))
+    return e;
+  if (int e = product(base + sc.xs, w_gate_up, base + sc.h, pairs, 2 * F, d, F, epilogue, E, tiles, sc.max_tiles, offsets, tile_rows, sm_pairs,
+                      status, limit, slope, stream))
+    return e;
+  if (int e = product(base + sc.h, w_down, base + sc.ys, pairs, d, F, d, 0, E, tiles, sc.max_tiles, offsets, tile_rows, sm_pairs, status, limit,
+                      slope, stream))
+    return e;
+  return hk_route_combine((const float*)(base + sc.ys), inv, weights, y, n, d, top, accumulate, shared, shared_gate, identities ? x : nullptr,
+                          HK_BF16, factor, stream);
 }

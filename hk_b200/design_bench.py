@@ -217,46 +217,29 @@ def kernel_points(width: int, n: int, peaks: dict) -> dict:
     us = _time_kernel(lambda: ops.route_topk(xb, wr, ids, wts))
     note("route_topk", us, n * width * 2 + E * width * 4, 2.0 * n * E * width, FP32_TFLOPS * 1e12)
     pairs = n * top
-    tile_rows = ops.route_tile_rows()
+    from .csrc import gemm_fast
+    tile_rows = gemm_fast.grouped_tile_rows(pairs, E)
     max_tiles = pairs // tile_rows + min(E, pairs)
     offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
     perm = torch.empty(pairs, dtype=torch.int32, device=dev)
     inv = torch.empty(pairs, dtype=torch.int32, device=dev)
     tiles = torch.empty(max_tiles, 2, dtype=torch.int32, device=dev)
-    us = _time_kernel(lambda: ops.route_sort(ids, E, offsets, perm, inv, tiles))
+    us = _time_kernel(lambda: ops.route_sort(ids, E, offsets, perm, inv, tiles, tile_rows))
     note("route_sort", us, pairs * 16, 0, 0)
+    xs = torch.empty(pairs, width, dtype=torch.bfloat16, device=dev)
+    us = _time_kernel(lambda: ops.route_gather(xb, perm, offsets, top, xs))
+    note("route_gather", us, (n + pairs) * width * 2, 0, 0)
     wgu = (torch.randn(E, 2 * Fe, width, device=dev) * 0.02).bfloat16()
     wd = (torch.randn(E, width, Fe, device=dev) * 0.02).bfloat16()
     h = torch.empty(pairs, Fe, dtype=torch.bfloat16, device=dev)
     ys = torch.empty(pairs, width, device=dev)
     used = min(E, pairs)
-    us = _time_kernel(lambda: ops.grouped_gemm(xb, wgu, h, tiles, offsets, perm, top, gather=True, gated=True))
-    note("grouped gate/up product + SwiGLU (mma.sync)", us, used * 2 * Fe * width * 2 + n * width * 2 + pairs * Fe * 2, 2.0 * pairs * 2 * Fe * width, tc,
+    us = _time_kernel(lambda: ops.grouped_gemm_tc(xs, wgu, h, tiles, offsets, tile_rows, gated=True))
+    note("grouped gate/up product + SwiGLU (tcgen05)", us, used * 2 * Fe * width * 2 + pairs * (width + Fe) * 2, 2.0 * pairs * 2 * Fe * width, tc,
          like="gate/up product with SwiGLU epilogue (same FLOPs)")
-    us = _time_kernel(lambda: ops.grouped_gemm(h, wd, ys, tiles, offsets, perm, top, gather=False, gated=False))
-    note("grouped down product (mma.sync)", us, used * Fe * width * 2 + pairs * (Fe * 2 + width * 4), 2.0 * pairs * Fe * width, tc,
+    us = _time_kernel(lambda: ops.grouped_gemm_tc(h, wd, ys, tiles, offsets, tile_rows, gated=False))
+    note("grouped down product (tcgen05)", us, used * Fe * width * 2 + pairs * (Fe * 2 + width * 4), 2.0 * pairs * Fe * width, tc,
          like="down product (same FLOPs)")
-    if pairs >= 1024:
-        # the form that prompt-sized steps take: rows gathered into padded expert order, both products on the tcgen05 kernel
-        from .csrc import gemm_fast
-        pad = gemm_fast.GROUPED_ROWS
-        m_max = -(-(pairs + E * (pad - 1)) // pad) * pad
-        perm_p = torch.empty(m_max, dtype=torch.int32, device=dev)
-        inv_p = torch.empty(pairs, dtype=torch.int32, device=dev)
-        groups = torch.empty(m_max // pad, dtype=torch.int32, device=dev)
-        us = _time_kernel(lambda: ops.route_sort_padded(ids, E, pad, perm_p, inv_p, groups))
-        note("route_sort_padded", us, pairs * 16, 0, 0)
-        xs = torch.empty(m_max, width, dtype=torch.bfloat16, device=dev)
-        us = _time_kernel(lambda: ops.route_gather(xb, perm_p, top, xs))
-        note("route_gather", us, (n + m_max) * width * 2, 0, 0)
-        hp = torch.empty(m_max, Fe, dtype=torch.bfloat16, device=dev)
-        ysp = torch.empty(m_max, width, device=dev)
-        us = _time_kernel(lambda: ops.grouped_gemm_tc(xs, wgu, hp, groups, gated=True))
-        note("grouped gate/up product + SwiGLU (tcgen05)", us, used * 2 * Fe * width * 2 + pairs * (width + Fe) * 2, 2.0 * pairs * 2 * Fe * width, tc,
-             like="gate/up product with SwiGLU epilogue (same FLOPs)")
-        us = _time_kernel(lambda: ops.grouped_gemm_tc(hp, wd, ysp, groups, gated=False))
-        note("grouped down product (tcgen05)", us, used * Fe * width * 2 + pairs * (Fe * 2 + width * 4), 2.0 * pairs * Fe * width, tc,
-             like="down product (same FLOPs)")
     y = torch.empty(n, width, device=dev)
     us = _time_kernel(lambda: ops.route_combine(ys, inv, wts, y))
     note("route_combine", us, pairs * width * 4 + n * width * 4, 0, 0)
@@ -923,28 +906,17 @@ def gezavik_kernel_points(width: int, n: int, decode: bool, peaks: dict) -> dict
     wgu = (torch.randn(E, 2 * Fe, width, device=dev) * 0.02).bfloat16()
     used = min(E, pairs)
     nbytes, flops = used * 2 * Fe * width * 2 + real * (width + Fe) * 2, 2.0 * real * 2 * Fe * width
-    if pairs >= 1024:
-        pad = gemm_fast.GROUPED_ROWS
-        m_max = -(-(pairs + E * (pad - 1)) // pad) * pad
-        perm = torch.empty(m_max, dtype=torch.int32, device=dev)
-        inv = torch.empty(pairs, dtype=torch.int32, device=dev)
-        tiles = torch.empty(m_max // pad, dtype=torch.int32, device=dev)
-        ops.route_sort_padded(ids, E, pad, perm, inv, tiles)
-        xs = torch.empty(m_max, width, dtype=bf, device=dev)
-        ops.route_gather(xb, perm, top, xs)
-        h = torch.empty(m_max, Fe, dtype=bf, device=dev)
-        ys = torch.randn(m_max, width, device=dev)
-        grouped = lambda act: ops.grouped_gemm_tc(xs, wgu, h, tiles, gated=True, act=act, limit=7.0, slope=1.702)
-    else:
-        max_tiles = pairs // ops.route_tile_rows() + min(E, pairs)
-        offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
-        perm = torch.empty(pairs, dtype=torch.int32, device=dev)
-        inv = torch.empty(pairs, dtype=torch.int32, device=dev)
-        tiles = torch.empty(max_tiles, 2, dtype=torch.int32, device=dev)
-        ops.route_sort(ids, E, offsets, perm, inv, tiles)
-        h = torch.empty(pairs, Fe, dtype=bf, device=dev)
-        ys = torch.randn(pairs, width, device=dev)
-        grouped = lambda act: ops.grouped_gemm(xb, wgu, h, tiles, offsets, perm, top, gather=True, gated=True, act=act, limit=7.0, slope=1.702)
+    tile_rows = gemm_fast.grouped_tile_rows(pairs, E)
+    offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
+    perm = torch.empty(pairs, dtype=torch.int32, device=dev)
+    inv = torch.empty(pairs, dtype=torch.int32, device=dev)
+    tiles = torch.empty(pairs // tile_rows + min(E, pairs), 2, dtype=torch.int32, device=dev)
+    ops.route_sort(ids, E, offsets, perm, inv, tiles, tile_rows)
+    xs = torch.empty(pairs, width, dtype=bf, device=dev)
+    ops.route_gather(xb, perm, offsets, top, xs)
+    h = torch.empty(pairs, Fe, dtype=bf, device=dev)
+    ys = torch.randn(pairs, width, device=dev)
+    grouped = lambda act: ops.grouped_gemm_tc(xs, wgu, h, tiles, offsets, tile_rows, gated=True, act=act, limit=7.0, slope=1.702)
     us = _time_kernel(lambda: grouped("swish_clamped"))
     note("grouped gate/up product, clamped activation", us, nbytes, flops, tc, like="grouped gate/up product, silu (Zazulix)")
     us = _time_kernel(lambda: grouped("silu"))

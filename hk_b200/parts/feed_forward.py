@@ -11,7 +11,7 @@ from typing import Dict
 
 import torch
 
-from ..csrc import ops
+from ..csrc import gemm_fast, ops
 from .base import MATRIX, VECTOR, ParamSpec, Part, Precision, register_part
 
 
@@ -209,33 +209,7 @@ class RoutedFeedForward(Part):
         self.w_down = torch.stack([tensors[self._expert(e, "down")].to(dt) for e in range(self.E)]).contiguous()
         self._tile_rows = ops.route_tile_rows()
 
-    TC_MIN_PAIRS = 1024     # from this many (row, choice) pairs on, a bfloat16 step takes the tcgen05 grouped product
-
-    def _forward_tc(self, xb, residual, ids, weights, accumulate: bool, shared_y=None, shared_gate=None) -> bool:
-        """Prompt-sized steps in bfloat16: the rows are gathered into expert order with every expert's rows padded to whole
-        128-row tiles, and both products run on the tcgen05 kernel with a tile's expert choosing its weights."""
-        from ..csrc import gemm_fast
-        n, dev = xb.shape[0], xb.device
-        pairs, pad = n * self.top, gemm_fast.GROUPED_ROWS
-        m_max = -(-(pairs + self.E * (pad - 1)) // pad) * pad
-        perm = torch.empty(m_max, dtype=torch.int32, device=dev)
-        inv = torch.empty(pairs, dtype=torch.int32, device=dev)
-        groups = torch.empty(m_max // pad, dtype=torch.int32, device=dev)
-        ops.route_sort_padded(ids, self.E, pad, perm, inv, groups)
-        xs = torch.empty((m_max, self.hidden), dtype=xb.dtype, device=dev)
-        ops.route_gather(xb, perm, self.top, xs)
-        h = torch.empty((m_max, self.F), dtype=xb.dtype, device=dev)
-        if not ops.grouped_gemm_tc(xs, self.w_gate_up, h, groups, gated=True, act=self.act, limit=self.limit, slope=self.slope):
-            return False
-        ys = torch.empty((m_max, self.hidden), dtype=torch.float32, device=dev)
-        if not ops.grouped_gemm_tc(h, self.w_down, ys, groups, gated=False):
-            return False
-        self._combine(ys, inv, weights, xb, residual, accumulate, shared_y, shared_gate)
-        return True
-
-    def _combine(self, ys, inv, weights, xb, residual, accumulate: bool, shared_y, shared_gate) -> None:
-        ops.route_combine(ys, inv, weights, residual, accumulate=accumulate, shared=shared_y, shared_gate=shared_gate,
-                          x=xb if self.identity else None, factor=self.out_scale)
+    TC_MIN_PAIRS = 1024     # up to here one call issues all launches of a bfloat16 step, which would wait for the host; above, the GPU sets the time
 
     def forward(self, xb: torch.Tensor, residual: torch.Tensor, ctx, accumulate: bool = True) -> None:
         n, dev = xb.shape[0], xb.device
@@ -251,21 +225,32 @@ class RoutedFeedForward(Part):
         if self.shared is not None:
             shared_y = torch.empty((n, self.hidden), dtype=torch.float32, device=dev)
             self.shared.forward(xb, shared_y, ctx, accumulate=False)
-        if xb.dtype == torch.bfloat16 and pairs >= self.TC_MIN_PAIRS and self.hidden % 8 == 0 and self.F % 8 == 0 \
-                and self._forward_tc(xb, residual, ids, weights, accumulate, shared_y, shared_gate):
+        glu = {"act": self.act, "limit": self.limit, "slope": self.slope}
+        fast = xb.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.F % 8 == 0
+        if fast and pairs < self.TC_MIN_PAIRS:
+            ops.routed_experts(xb, ids, weights, self.w_gate_up, self.w_down, residual, accumulate=accumulate, shared=shared_y,
+                               shared_gate=shared_gate, identities=bool(self.identity), factor=self.out_scale, **glu)
             return
-        max_tiles = pairs // self._tile_rows + min(self.E, pairs)
+        rows = gemm_fast.grouped_tile_rows(pairs, self.E) if fast else self._tile_rows
+        max_tiles = pairs // rows + min(self.E, pairs)
         offsets = torch.empty(self.E + 1, dtype=torch.int32, device=dev)
         perm = torch.empty(pairs, dtype=torch.int32, device=dev)
         inv = torch.empty(pairs, dtype=torch.int32, device=dev)
         tiles = torch.empty((max_tiles, 2), dtype=torch.int32, device=dev)
-        ops.route_sort(ids, self.E, offsets, perm, inv, tiles)
+        ops.route_sort(ids, self.E, offsets, perm, inv, tiles, rows)
         h = torch.empty((pairs, self.F), dtype=xb.dtype, device=dev)
-        ops.grouped_gemm(xb, self.w_gate_up, h, tiles, offsets, perm, self.top, gather=True, gated=True, act=self.act,
-                         limit=self.limit, slope=self.slope)
         ys = torch.empty((pairs, self.hidden), dtype=torch.float32, device=dev)
-        ops.grouped_gemm(h, self.w_down, ys, tiles, offsets, perm, self.top, gather=False, gated=False)
-        self._combine(ys, inv, weights, xb, residual, accumulate, shared_y, shared_gate)
+        if fast:
+            xs = torch.empty((pairs, self.hidden), dtype=xb.dtype, device=dev)
+            ops.route_gather(xb, perm, offsets, self.top, xs)
+            if not (ops.grouped_gemm_tc(xs, self.w_gate_up, h, tiles, offsets, rows, gated=True, **glu)
+                    and ops.grouped_gemm_tc(h, self.w_down, ys, tiles, offsets, rows, gated=False)):
+                raise ops.KernelError("the grouped product refuses the experts' weights")
+        else:
+            ops.grouped_gemm(xb, self.w_gate_up, h, tiles, offsets, perm, self.top, gather=True, gated=True, **glu)
+            ops.grouped_gemm(h, self.w_down, ys, tiles, offsets, perm, self.top, gather=False, gated=False)
+        ops.route_combine(ys, inv, weights, residual, accumulate=accumulate, shared=shared_y, shared_gate=shared_gate,
+                          x=xb if self.identity else None, factor=self.out_scale)
 
 
 register_part("feed_forward", "squared_relu", SquaredReLUFeedForward)

@@ -78,3 +78,34 @@ def test_pair_refusals():
         assert not gemm_fast.run_pair(a, w, out, 0, 4096, tiles_m, slices)
     assert not gemm_fast.run_pair(a, w[:4095], out, 2, 4096, 2, 1)
     assert bool((out == 3.0).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("counts,N,K,tile_rows", [([1, 0, 3], 256, 64, 32), ([70, 1, 33, 0, 64], 300, 136, 64), ([257, 5, 128], 514, 200, 128),
+                                                  ([300, 0, 31, 513], 1030, 72, 256), ([0, 0, 9], 4096, 520, 64)])
+@pytest.mark.parametrize("epilogue", [0, 2, 4])
+def test_pair_product_by_group(counts, N, K, tile_rows, epilogue):
+    from hk_b200.csrc import gemm_fast
+    gen = torch.Generator().manual_seed(N + K)
+    E, M = len(counts), sum(counts)
+    a, w = torch.randn(M, K, generator=gen).bfloat16(), (torch.randn(E, N, K, generator=gen) / K ** 0.5).bfloat16()
+    offsets, tiles, want = [0], [], []
+    limit, slope = 0.8, 1.702
+    for e, count in enumerate(counts):
+        tiles += [(e, offsets[-1] + r) for r in range(0, count, tile_rows)]
+        want.append(_reference(a[offsets[-1]:offsets[-1] + count], w[e], epilogue, torch.zeros(()), limit, slope))
+        offsets.append(offsets[-1] + count)
+    tiles += [(-1, 0)] * 3
+    columns, kind = (N if epilogue == 0 else N // 2), (torch.float32 if epilogue == 0 else torch.bfloat16)
+    guard = torch.full((M + 40, columns), 5.0, dtype=kind, device="cuda")
+    table = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")      # noqa: E731
+    assert gemm_fast.run_pair_grouped(a.cuda(), w.cuda(), guard[:M], table(tiles), table(offsets), tile_rows, epilogue != 0,
+                                      2 if epilogue == 4 else 0, limit, slope)
+    gemm_fast.check_status(guard.device)
+    want, got = torch.cat(want), guard[:M].double().cpu()
+    # as in test_pair_product; the sums are of order 1
+    sums = K * 2 ** -23 * float((a.double().abs().max() * w.double().abs().max()) * K)
+    bound = torch.full_like(want, sums) if epilogue == 0 else want.abs() * 2 ** -8 + 16 * sums + 1e-6
+    assert bool(((got - want).abs() <= bound).all())
+    assert bool((guard[M:] == 5.0).all())
+    assert float((got - want).norm() / want.norm()) < (1e-5 if epilogue == 0 else 3e-3)
