@@ -9,24 +9,28 @@
 //   1. local:  a block per (chunk, head) solves the unit triangular system for [U~ | Auk V] and writes
 //              P [dk], M [dk, dk], B [dk, dv] with S = P S_0 + (M S_0 + B), Rq [32, dk] and Ov [32, dv] (to `out`) with
 //              O = Rq S_0 + Ov;
-//   2. walk:   a block per (request, head, 16 or 32 value columns) goes through the request's chunks, S in shared memory.
+//   2. walk:   a block per (request, head, 16 or 32 value columns) goes through the request's chunks, S in registers.
 // Without a removal term (retention, matrix memory) there is no M and no system to solve, and P is one number: see below.
 // P S_0 is added last: what is summed before it is small where decays are weak, and rounds less.
 //
-// All arithmetic is float32 multiply-adds, decays are products of the tokens' decays (never differences of logarithms): an
+// Products run on mma.sync with float32 factors in three bf16 pieces each, sums, decays and everything else are float32 (one number per
+// token: 64 bits), decays are products of the tokens' decays (never differences of logarithms): an
 // entry of the four matrices carries the rounding of the decays between its two tokens, as the walk token by token does.
 // Where the decay is one number per token the products between every two tokens are made one by one; where it is one per
 // channel (generalised delta rule) rows are scaled by P_t and 1 / P_s, which holds while a chunk's decay stays above 2^-64
 // (the launcher's condition on decay_scale).
 //
-// A value, key, gate or decay that is NaN or Inf reaches its own token and later ones, as in the walk: the products with triangular
-// matrices leave out what stands above the diagonal (`triangle_rows`), which a zero there would not keep out.
+// A value, key, gate or decay that is NaN or Inf reaches its own token and later ones, as in the walk: a product with zeros above the
+// diagonal would not keep it out, so a chunk with such a factor of a triangular matrix takes multiply-adds that leave them out.  (An Inf
+// may come out as NaN: its pieces do not add up.)
 //
-// One request of 2,048 tokens at 64 heads of 64 x 64 (walk token by token -> here, L2 cold): generalised rule 988 -> 433 us, gated
-// rule 978 -> 402, matrix memory 1,074 -> 284, retention 605 -> 206; of 1,000 at 32 heads 390 -> 140, 390 -> 138, 417 -> 103,
-// 241 -> 64; at 64 heads of 64 tokens level (42 -> 38, 46 -> 40, 54 -> 40, 32 -> 30), of 128 75 -> 48, 79 -> 48, 89 -> 46, 50 -> 36.
-// (With the triangular products whole: 429, 400, 284, 212 at 2,048 tokens.)
-// Relative error against 64 bits at 2,048 tokens: 5.3e-7 -> 5.1e-7, 5.5e-7 -> 5.3e-7, 7.1e-7 -> 7.0e-7, 5.2e-7 -> 1.9e-7.
+// One request of 2,048 tokens at 64 heads of 64 x 64 (walk token by token -> chunks on float32 multiply-adds -> here, L2 cold): generalised
+// rule 988 -> 430 -> 364 us, gated rule 978 -> 397 -> 323, matrix memory 1,074 -> 287 -> 240, retention 605 -> 201 -> 193; of 512 tokens
+// 257 -> 128 -> 112, 257 -> 122 -> 98, 288 -> 91 -> 81, 161 -> 69 -> 65.
+// Relative error against 64 bits at 1,000 tokens, generalised and gated rule: walk 1.5e-7 and 1.4e-7, multiply-adds 2.0e-7 and 1.8e-7, here
+// 1.5e-7 and 1.3e-7.
+#include <math_constants.h>
+
 #include "common.cuh"
 
 namespace {
@@ -44,27 +48,14 @@ struct Request {
   int slot, chunk0, chunks;
 };
 
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
+// (the division without the branch for unusual operands: the denominator is 1 or more, and above 2^126 the result 0)
+__device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.0f, 1.0f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ float4 mul4(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
-__device__ __forceinline__ float at4(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c))));
-}
-// two multiply-adds at once, each rounded as fmaf rounds
-__device__ __forceinline__ ulonglong2 ld_pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
-__device__ __forceinline__ void fma_pairs(unsigned long long& c, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float pair_sum(unsigned long long c) {
-  return __uint_as_float((uint32_t)c) + __uint_as_float((uint32_t)(c >> 32));
-}
-// the same as dot4 in two sums
-__device__ __forceinline__ void dot4_by_two(float4 a, float4 b, float* c) {
-  c[0] = fmaf(a.z, b.z, fmaf(a.x, b.x, c[0]));
-  c[1] = fmaf(a.w, b.w, fmaf(a.y, b.y, c[1]));
 }
 __device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0)
@@ -77,46 +68,33 @@ __device__ __forceinline__ void fma4(float4& c, float a, float4 b) {
   c.w = fmaf(a, b.w, c.w);
 }
 
-// acc[i] (N rows, row i's token ty + 8 (i & 3)) += sign * a[row i, s] * b[s, :] over the tokens s below limit(i), a row's own at most:
-// `a` row ty + 8 i with ROWS floats between rows, `b` four columns with LD between tokens.  The two values of ty in a warp lie
-// in one group of four tokens, so a warp skips the groups above the diagonal as one, half of all.
-template <int N, int ROWS, int SIGN, int NB, typename Limit>
-__device__ __forceinline__ void triangle_rows(float4 (&acc)[NB][N], const float* a, const float* (&b)[NB], int ty, Limit limit) {
-#pragma unroll 2
-  for (int s = 0; s < CQ; s += 4) {
-    float4 x[NB][4];
+// The products of a chunk's decays, one number g per token, in 64 bits: the same decay in every token (retention) would round the
+// same way in every product, chunk after chunk.  A lane per token: `win` [5][CQ], the products of 1, 2, 4, 8 and 16 tokens up to its
+// own; `from` [CQ] = g[0] .. g[t], and what `from` of the last token is short of the product.  (Each product as a chain of its own, 32
+// long, took a warp 5,600 clocks that the block waited for.)
+__device__ __forceinline__ void decay_windows(float g, double* win, float* from, float* rest, int lane) {
+  double x = g;
 #pragma unroll
-    for (int n = 0; n < NB; ++n)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) x[n][j] = ld4(b[n] + (s + j) * LD);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const int end = limit(i);
-      if (s >= (end + 3 & ~3)) continue;
-      const float4 w = ld4(a + (ty + 8 * i) * ROWS + s);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (s + j < end)
-#pragma unroll
-          for (int n = 0; n < NB; ++n) fma4(acc[n][i], SIGN * at4(w, j), x[n][j]);
-    }
+  for (int j = 0; j < 5; ++j) {
+    win[j * CQ + lane] = x;
+    const double y = __shfl_up_sync(0xffffffffu, x, 1 << j);
+    if (lane >= 1 << j) x *= y;
   }
+  from[lane] = (float)x;
+  if (lane == CQ - 1) *rest = (float)(x - (double)(float)x);
 }
-
-// The products of a chunk's decays, one number g[t] per token: gam[t][s] = g[s + 1] .. g[t] for s <= t (0 above), `from` [CQ]
-// = g[0] .. g[t], and what `from` of the last token is short of the product.  One warp, a lane per s, in 64 bits: the same
-// decay in every token (retention) would round the same way in every product, chunk after chunk.
-__device__ __forceinline__ void decay_products(const float* g, float* gam, int ldg, float* from, float* rest, int lane) {
-  double run = 0., all = 1.;
+// g[s + 1] .. g[t] for s <= t, 0 above: the windows that make up t - s
+__device__ __forceinline__ float decay_between(const double* win, int t, int s) {
+  if (s > t) return 0.f;
+  double x = 1.;
+  int at = t;
 #pragma unroll
-  for (int t = 0; t < CQ; ++t) {
-    const double x = g[t];
-    run = t == lane ? 1. : run * x;
-    all *= x;
-    gam[t * ldg + lane] = (float)run;
-    if (lane == 0) from[t] = (float)all;
-  }
-  if (lane == 0) *rest = (float)(all - (double)(float)all);
+  for (int j = 0; j < 5; ++j)
+    if ((t - s) >> j & 1) {
+      x *= win[j * CQ + at];
+      at -= 1 << j;
+    }
+  return (float)x;
 }
 
 // What a rule reads: columns slices of one matrix of row stride ld, and the rule's own.
@@ -138,13 +116,91 @@ struct DeltaSmem {
   float w[CQ * LD];             // the decays' products, then Auk V, then W
   float pc[NT];                 // the chunk's decay per channel
   float g[CQ], gb[CQ], from[CQ], rest[4];
+  double win[5 * CQ];
 };
 
 }  // namespace
 
+// ------------------------------------------------------------------ products on the tensor cores
+// mma.sync (16 x 8 x 16, bf16, float32 sums): a float32 factor is cut into three bf16 numbers whose sum it is, and of the nine products
+// of two such factors the six of the largest pieces are taken, the first in a sum of its own.
+namespace {
+__device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, const uint32_t* b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// two float32 numbers as three pairs of bf16 whose sums they are, `step` words apart
+__device__ __forceinline__ void split3(float2 x, uint32_t* out, int step) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    out[p * step] = pack_bf16(x.x, x.y);
+    x.x -= __uint_as_float(out[p * step] << 16);
+    x.y -= __uint_as_float(out[p * step] & 0xffff0000u);
+  }
+}
+// big += the product of the largest pieces, small += the five next
+__device__ __forceinline__ void mma_split(float* big, float* small, const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+  mma_bf16(small, a[2], b[0]);
+  mma_bf16(small, a[1], b[1]);
+  mma_bf16(small, a[0], b[2]);
+  mma_bf16(small, a[1], b[0]);
+  mma_bf16(small, a[0], b[1]);
+  mma_bf16(big, a[0], b[0]);
+}
+
+// Fragments of a float32 matrix in shared memory, cut into pieces; g = lane / 4, q = lane % 4.
+// A operand, 16 rows by 16 k, rows side by side: `a` at (row g, k 2 q); the rows times f0 (g) and f1 (g + 8)
+__device__ __forceinline__ void frag_rows(const float* a, int ld, float f0, float f1, uint32_t (&out)[3][4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    float2 x = *reinterpret_cast<const float2*>(a + 8 * (e & 1) * ld + 8 * (e >> 1));
+    x.x *= e & 1 ? f1 : f0;
+    x.y *= e & 1 ? f1 : f0;
+    split3(x, &out[0][e], 4);
+  }
+}
+// A operand from a matrix that lies the other way round, k by k: `a` at (k 2 q, row g); all times f, or the k times their own (f at 2 q)
+__device__ __forceinline__ void frag_turned(const float* a, int ld, float f, uint32_t (&out)[3][4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float* p = a + 8 * (e >> 1) * ld + 8 * (e & 1);
+    split3(make_float2(p[0] * f, p[ld] * f), &out[0][e], 4);
+  }
+}
+__device__ __forceinline__ void frag_turned(const float* a, int ld, const float* f, uint32_t (&out)[3][4]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int k = 8 * (e >> 1);
+    const float* p = a + k * ld + 8 * (e & 1);
+    split3(make_float2(p[0] * f[k], p[ld] * f[k + 1]), &out[0][e], 4);
+  }
+}
+__device__ __forceinline__ bool finite4(float4 v) {
+  return fabsf(v.x) < CUDART_INF_F && fabsf(v.y) < CUDART_INF_F && fabsf(v.z) < CUDART_INF_F && fabsf(v.w) < CUDART_INF_F;
+}
+// B operand, 16 k by 8 columns: `b` at (column g, k 2 q) of a matrix column by column ...
+__device__ __forceinline__ void frag_columns(const float* b, uint32_t (&out)[3][2]) {
+#pragma unroll
+  for (int e = 0; e < 2; ++e) split3(*reinterpret_cast<const float2*>(b + 8 * e), &out[0][e], 2);
+}
+// ... or at (k 2 q, column g) of one k by k
+__device__ __forceinline__ void frag_k(const float* b, int ld, uint32_t (&out)[3][2]) {
+#pragma unroll
+  for (int e = 0; e < 2; ++e) split3(make_float2(b[8 * e * ld], b[(8 * e + 1) * ld]), &out[0][e], 2);
+}
+
+}  // namespace
+
 // ------------------------------------------------------------------ 1. local part with a removal term
-// Bound by its multiply-adds (0.9 M a block, of which a third of the rate goes to operands that no register keeps: 8 x 4
-// outputs a thread from 16-byte loads of shared memory).  70 KB of shared memory and 128 threads: three blocks share an SM.
+// Bound by the instructions that bring and cut the products' operands (IPC 2.1 of 4, tensor pipe 26 %, shared memory 60 %): 0.9 M
+// multiply-adds a block, the records' two sigmoids and two exponentials an entry, the triangular system.  70 KB of shared memory and 128
+// threads: three blocks share an SM; with 256 threads 396 us instead of 364 (2,048 tokens, 64 heads, with the walk).
 template <bool GATED>
 __global__ void __launch_bounds__(NTH, 3)
 delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __restrict__ mm, float* __restrict__ rq,
@@ -154,7 +210,7 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
   const int H = in.H, dk = in.dk, dv = in.dv;
   const int c = blockIdx.x / H, h = blockIdx.x % H;
   const Chunk ch = chunks[c];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 
   // ---- the tokens' records; a token's row in four threads
@@ -230,7 +286,9 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
   }
   __syncthreads();
   if (GATED) {
-    if (tid < 32) decay_products(sm.g, sm.w, LD, sm.from, sm.rest, tid);
+    if (tid < CQ) decay_windows(sm.g[tid], sm.win, sm.from, sm.rest, tid);
+    __syncthreads();
+    for (int e = tid; e < CQ * CQ; e += NTH) sm.w[(e / CQ) * LD + e % CQ] = decay_between(sm.win, e / CQ, e % CQ);
   } else {
     // a channel's decays in two threads: rows of u and r are decayed from the start, those of k and a*u back to it
     const int i = tid & 63;
@@ -256,48 +314,49 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
   }
   __syncthreads();
 
-  // ---- the four matrices: rows u, r against columns k, a*u (gated: a*u is a number times k)
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  // ---- the four matrices: rows u, r against columns k, a*u (gated: a*u is a number times k).  A warp has 16 rows: tokens
+  // 16 (warp & 1) .. of u (warps 0 and 1) or r; columns of tokens above its own it leaves out
   {
-    constexpr int NC = GATED ? 2 : 4;
-    unsigned long long acc[8][NC];
+    constexpr int NC = GATED ? 4 : 8;           // column tiles: 32 tokens of k, then of a*u
+    const int t0 = (warp & 1) * 16;
+    const bool read = warp >= 2;
+    float big[NC][4] = {}, small[NC][4] = {};
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int k = 0; k < NT / 16; ++k) {
+      uint32_t a[3][4];
+      frag_rows(sm.ur + (warp * 16 + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a);
 #pragma unroll
-      for (int j = 0; j < NC; ++j) acc[i][j] = 0ull;
-#pragma unroll 2
-    for (int e = 0; e < NT; e += 4) {
-      ulonglong2 b[NC];
-#pragma unroll
-      for (int j = 0; j < NC; ++j) b[j] = ld_pairs(sm.ka + (tx + 16 * j) * LD + e);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const ulonglong2 a = ld_pairs(sm.ur + (ty + 8 * i) * LD + e);
-#pragma unroll
-        for (int j = 0; j < NC; ++j) {
-          fma_pairs(acc[i][j], a.x, b[j].x);
-          fma_pairs(acc[i][j], a.y, b[j].y);
+      for (int n = 0; n < NC; ++n)
+        if ((n & 3) * 8 <= t0 + 15) {
+          uint32_t b[3][2];
+          frag_columns(sm.ka + (8 * n + g) * LD + k * 16 + 2 * q, b);
+          mma_split(big[n], small[n], a, b);
         }
-      }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int t = ty + 8 * (i & 3);
-      const bool read = i >= 4;
+    for (int n = 0; n < NC; ++n)
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        const int s = tx + 16 * (j & 1);
+      for (int e = 0; e < 4; ++e) {
+        const int t = t0 + g + 8 * (e >> 1), s = (n & 3) * 8 + 2 * q + (e & 1);
         const bool in_tri = (read ? s <= t : s < t) && t < ch.count;
-        float x = in_tri ? pair_sum(acc[i][j]) : 0.f;
-        float* dst = sm.a + (ty + 8 * i) * LD + tx + 16 * j;
+        float x = in_tri ? big[n][e] + small[n][e] : 0.f;
+        float* dst = sm.a + (warp * 16 + g + 8 * (e >> 1)) * LD + 8 * n + 2 * q + (e & 1);
         if (GATED) {
           x *= in_tri ? sm.w[(read ? t : t - 1) * LD + s] : 0.f;
           dst[CQ] = in_tri ? x * sm.gb[s] : 0.f;
         }
         *dst = x;
       }
-    }
   }
-  __syncthreads();
+  // (what is not finite would spread through products with zeros: such a chunk takes FMAs that leave out what is above the diagonal)
+  bool ordinary = true;
+#pragma unroll
+  for (int j = 0; j < CQ * NT / 4 / NTH; ++j) {
+    const int e = tid + j * NTH;
+    ordinary = ordinary && finite4(ld4(sm.vs + (e / (NT / 4)) * LD + (e % (NT / 4)) * 4));
+  }
+  ordinary = __syncthreads_and(ordinary);
   if (GATED) {
     // rows decayed from the chunk's start and to its end (the products' last row), which the matrices did not want
     for (int e = tid; e < CQ * (NT / 4); e += NTH) {
@@ -312,20 +371,44 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
     __syncthreads();
   }
 
-  // ---- [Auk ; Ark] V
+  // ---- [Auk ; Ark] V: into w, and over the k columns of the matrices (Ark V's columns 32 and up where Ark was)
   {
-    float4 acc[1][8];
+    const int t0 = (warp & 1) * 16;
+    const bool read = warp >= 2;
+    float big[8][4] = {}, small[8][4] = {};
+    if (ordinary) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[0][i] = zero;
-    const float* v[1] = {sm.vs + 4 * tx};
-    triangle_rows<8, LD, 1>(acc, sm.a, v, ty, [&](int i) { return ty + 8 * (i & 3) + (i >= 4 ? 1 : 0); });
+      for (int k = 0; k < CQ / 16; ++k) {
+        if (16 * k > t0) break;
+        uint32_t a[3][4];
+        frag_rows(sm.a + (warp * 16 + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a);
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+          uint32_t b[3][2];
+          frag_k(sm.vs + (k * 16 + 2 * q) * LD + 8 * n + g, LD, b);
+          mma_split(big[n], small[n], a, b);
+        }
+      }
+    } else {
+      for (int s = 0; s < t0 + 16; ++s)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = t0 + g + 8 * (e >> 1);
+          if (read ? s > t : s >= t) continue;
+          const float x = sm.a[(warp * 16 + g + 8 * (e >> 1)) * LD + s];
+#pragma unroll
+          for (int n = 0; n < 8; ++n) big[n][e] = fmaf(x, sm.vs[s * LD + 8 * n + 2 * q + (e & 1)], big[n][e]);
+        }
+    }
     __syncthreads();            // everyone has read the k columns of the matrices
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = ty + 8 * i;
-      st4(sm.w + t * LD + 4 * tx, acc[0][i]);
-      st4(sm.a + (t + (tx >= 8 ? CQ : 0)) * LD + 4 * (tx & 7), acc[0][4 + i]);
-    }
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = t0 + g + 8 * i, d = 8 * n + 2 * q;
+        float* dst = read ? sm.a + (t + (d >= CQ ? CQ : 0)) * LD + (d & (CQ - 1)) : sm.w + t * LD + d;
+        *reinterpret_cast<float2*>(dst) = make_float2(big[n][2 * i] + small[n][2 * i], big[n][2 * i + 1] + small[n][2 * i + 1]);
+      }
   }
   __syncthreads();
 
@@ -351,63 +434,96 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
     }
 #pragma unroll
     for (int t = 1; t < CQ; ++t) col[t * LD] = x[t];
+#pragma unroll
+    for (int t = 0; t < CQ; ++t) ordinary = ordinary && fabsf(x[t]) < CUDART_INF_F;
   }
-  __syncthreads();
+  ordinary = __syncthreads_and(ordinary);
 
   const size_t item = (size_t)c * H + h;
   const int col0 = blockIdx.y * NT, ncols = min(NT, dv - col0);
-  // ---- Rq = R~ - Aru X,  Ov = Ark V - Aru W
+  // ---- Rq = R~ - Aru X,  Ov = Ark V - Aru W: a warp has 16 tokens of one of the two
   {
-    float4 ro[2][4];
+    const int t0 = (warp & 1) * 16;
+    const bool offset = warp >= 2;
+    const float* xw = offset ? sm.w : sm.ur;
+    float big[8][4] = {}, small[8][4] = {};
+    if (ordinary) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = ty + 8 * i;
-      ro[0][i] = ld4(sm.ur + (CQ + t) * LD + 4 * tx);
-      ro[1][i] = ld4(sm.a + (t + (tx >= 8 ? CQ : 0)) * LD + 4 * (tx & 7));
-    }
-    const float* xw[2] = {sm.ur + 4 * tx, sm.w + 4 * tx};
-    triangle_rows<4, LD, -1>(ro, sm.a + CQ * LD + CQ, xw, ty, [&](int i) { return ty + 8 * i + 1; });
+      for (int k = 0; k < CQ / 16; ++k) {
+        if (16 * k > t0) break;
+        uint32_t a[3][4];
+        frag_rows(sm.a + (CQ + t0 + g) * LD + CQ + k * 16 + 2 * q, LD, -1.f, -1.f, a);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int t = ty + 8 * i;
-      if (blockIdx.y == 0) st4(rq + (item * CQ + t) * NT + 4 * tx, ro[0][i]);
-      if (t < ch.count && 4 * tx < ncols) st4(out + ((size_t)(ch.row0 + t) * H + h) * dv + col0 + 4 * tx, ro[1][i]);
-    }
-  }
-  // ---- M = -AU'^T X and P,  B = K'^T V - AU'^T W
-  {
-    float4 m[8], b[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m[i] = b[i] = zero;
-#pragma unroll 2
-    for (int s = 0; s < CQ; ++s) {
-      const float4 x = ld4(sm.ur + s * LD + 4 * tx), w = ld4(sm.w + s * LD + 4 * tx), v = ld4(sm.vs + s * LD + 4 * tx);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const float4 k = ld4(sm.ka + s * LD + 8 * ty + 4 * half), au = ld4(sm.ka + (CQ + s) * LD + 8 * ty + 4 * half);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          fma4(m[4 * half + j], -at4(au, j), x);
-          fma4(b[4 * half + j], at4(k, j), v);
-          fma4(b[4 * half + j], -at4(au, j), w);
+        for (int n = 0; n < 8; ++n) {
+          uint32_t b[3][2];
+          frag_k(xw + (k * 16 + 2 * q) * LD + 8 * n + g, LD, b);
+          mma_split(big[n], small[n], a, b);
         }
       }
+    } else {
+      for (int s = 0; s < t0 + 16; ++s)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = t0 + g + 8 * (e >> 1);
+          if (s > t) continue;
+          const float x = -sm.a[(CQ + t) * LD + CQ + s];
+#pragma unroll
+          for (int n = 0; n < 8; ++n) big[n][e] = fmaf(x, xw[s * LD + 8 * n + 2 * q + (e & 1)], big[n][e]);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = 8 * ty + i;
-      const float p = GATED ? sm.from[CQ - 1] : sm.pc[row];
-      float4 x = m[i];
-      float4 y = b[i];
-      if (!GATED) {
-        x = mul4(x, p);
-        y = mul4(y, p);
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = t0 + g + 8 * i, d = 8 * n + 2 * q;
+        const float2 onto = *reinterpret_cast<const float2*>(offset ? sm.a + (t + (d >= CQ ? CQ : 0)) * LD + (d & (CQ - 1)) : sm.ur + (CQ + t) * LD + d);
+        const float2 y = make_float2(onto.x + (big[n][2 * i] + small[n][2 * i]), onto.y + (big[n][2 * i + 1] + small[n][2 * i + 1]));
+        if (!offset) {
+          if (blockIdx.y == 0) *reinterpret_cast<float2*>(rq + (item * CQ + t) * NT + d) = y;
+        } else if (t < ch.count && d < ncols) {
+          *reinterpret_cast<float2*>(out + ((size_t)(ch.row0 + t) * H + h) * dv + col0 + d) = y;
+        }
       }
-      if (blockIdx.y == 0) {
-        st4(mm + item * MFLOATS + row * NT + 4 * tx, x);
-        if (tx == 0) mm[item * MFLOATS + NT * NT + row] = p;
+  }
+  // ---- M = -AU'^T X and P,  B = K'^T V - AU'^T W: a warp has 16 rows
+  {
+    const int row = warp * 16 + g;
+    uint32_t kk[CQ / 16][3][4], au[CQ / 16][3][4];
+#pragma unroll
+    for (int k = 0; k < CQ / 16; ++k) {
+      frag_turned(sm.ka + (k * 16 + 2 * q) * LD + row, LD, 1.f, kk[k]);
+      frag_turned(sm.ka + (CQ + k * 16 + 2 * q) * LD + row, LD, -1.f, au[k]);
+    }
+    const float p0 = GATED ? sm.from[CQ - 1] : sm.pc[row], p1 = GATED ? sm.from[CQ - 1] : sm.pc[row + 8];
+#pragma unroll 2
+    for (int n = 0; n < 8; ++n) {
+      float mb[4] = {}, ms[4] = {}, vb[4] = {}, vsm[4] = {};
+#pragma unroll
+      for (int k = 0; k < CQ / 16; ++k) {
+        const int at = (k * 16 + 2 * q) * LD + 8 * n + g;
+        uint32_t b[3][2];
+        frag_k(sm.ur + at, LD, b);
+        mma_split(mb, ms, au[k], b);
+        frag_k(sm.vs + at, LD, b);
+        mma_split(vb, vsm, kk[k], b);
+        frag_k(sm.w + at, LD, b);
+        mma_split(vb, vsm, au[k], b);
       }
-      if (row < dk && 4 * tx < ncols) st4(bb + (item * dk + row) * dv + col0 + 4 * tx, y);
+      const int d = 8 * n + 2 * q;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float f = GATED ? 1.f : i ? p1 : p0;
+        if (blockIdx.y == 0)
+          *reinterpret_cast<float2*>(mm + item * MFLOATS + (row + 8 * i) * NT + d) =
+              make_float2((mb[2 * i] + ms[2 * i]) * f, (mb[2 * i + 1] + ms[2 * i + 1]) * f);
+        if (row + 8 * i < dk && d < ncols)
+          *reinterpret_cast<float2*>(bb + (item * dk + row + 8 * i) * dv + col0 + d) =
+              make_float2((vb[2 * i] + vsm[2 * i]) * f, (vb[2 * i + 1] + vsm[2 * i + 1]) * f);
+      }
+    }
+    if (blockIdx.y == 0 && q == 0) {
+      mm[item * MFLOATS + NT * NT + row] = p0;
+      mm[item * MFLOATS + NT * NT + row + 8] = p1;
     }
   }
 }
@@ -420,7 +536,8 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
 //   2. carry:   a thread per four state entries goes through a request's chunks and leaves every chunk's start state in B's place;
 //   3. outputs: a block per (chunk, head) makes A V + R~ S_0.
 // (As two kernels, the second walking the chunks with the outputs' products, one request of 2,048 tokens at 64 heads of 64 took
-// 103 + 141 us, the walk bound by the latency of a chain that these three do not have.)
+// 103 + 141 us, the walk bound by the latency of a chain that these three do not have.)  A block of the outputs waits for memory and for
+// its decays (17,000 of its 24,600 clocks before the windows of `decay_windows`, the products 6,700).
 struct DecayIn {
   const float *q, *k, *v;
   long long ld;
@@ -437,14 +554,18 @@ namespace {
 constexpr int LA = CQ + 4;
 struct StatesSmem {
   float k[CQ * LD], vs[CQ * LD];
-  float gam[CQ * LA], g[CQ], from[CQ], rest[4];
+  float from[CQ], rest[4];
+  double win[5 * CQ];
 };
 struct OutSmem {
-  float q[CQ * LD], k[CQ * LD], vs[CQ * LD], a[CQ * LA], st[NT * LD];
-  float gam[CQ * LA], g[CQ], from[CQ], rest[4];
+  float q[CQ * LD], k[CQ * LD], vs[CQ * LD], a[CQ * LA], st[NT * LD];     // (behind a row's NT numbers four more columns fit)
+  float from[CQ], rest[4];
+  double win[5 * CQ];
 };
+// The columns of a pass from col0 on: the last ones go along if they fit into the rows of shared memory.
+__device__ __forceinline__ int pass_columns(int left) { return left <= LD ? left : NT; }
 
-// A chunk's q (or none), k and first 64 value columns, and the products of its decays.  Ends behind a barrier.
+// A chunk's q (or none), k and first value columns, and the windows of its decays.  Ends behind a barrier.
 template <bool MEMORY, bool WITH_Q, typename S>
 __device__ __forceinline__ void decay_rows(const DecayIn& in, const Chunk& ch, int h, S& sm, float* sq) {
   const int H = in.H, dk = in.dk, dv = in.dv, tid = threadIdx.x;
@@ -464,7 +585,31 @@ __device__ __forceinline__ void decay_rows(const DecayIn& in, const Chunk& ch, i
     if (WITH_Q) qr[j] = row_in && i < dk ? ld4(qp + i) : zero;
     vr[j] = row_in && i < min(NT, dv) ? ld4(vp + i) : zero;
   }
-  if ((tid & 3) == 0) sm.g[t] = !row_in ? 1.f : MEMORY ? in.gates[(row * H + h) * 3] : in.decay[h];
+  // turned below, a pair of dims (i, i + rot / 2) a thread: the angles are asked for here
+  constexpr int PAIRS = CQ * (NT / 2) / NTH;
+  const int half = MEMORY ? 0 : in.rot >> 1;
+  float cs[PAIRS], sn[PAIRS];
+  if (!MEMORY)
+#pragma unroll
+    for (int j = 0; j < PAIRS; ++j) {
+      const int e = tid + j * NTH, r = half ? e / half : CQ;
+      const bool turned = r < ch.count;
+      const size_t at = turned ? (size_t)in.positions[ch.row0 + r] * half + (e - r * half) : 0;
+      cs[j] = turned ? in.cos_t[at] : 1.f;
+      sn[j] = turned ? in.sin_t[at] : 0.f;
+    }
+  if (tid < CQ) {
+    const bool has = tid < ch.count;
+    decay_windows(!has ? 1.f : MEMORY ? in.gates[((size_t)(ch.row0 + tid) * H + h) * 3] : in.decay[h], sm.win, sm.from, sm.rest, tid);
+  } else if (tid < 2 * CQ) {    // columns NT and up, where they go along with the first pass (the matrix memory's first one past dv: 1)
+    const int r = tid - CQ;
+    float4 x = zero;
+    if (r < ch.count) {
+      if (dv > NT) x = ld4(in.v + (size_t)(ch.row0 + r) * in.ld + (size_t)h * dv + NT);
+      else if (MEMORY && dv == NT) x.x = 1.f;
+    }
+    st4(sm.vs + r * LD + NT, x);
+  }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int i = i0 + 4 * j;
@@ -473,26 +618,23 @@ __device__ __forceinline__ void decay_rows(const DecayIn& in, const Chunk& ch, i
     st4(sm.vs + t * LD + i, vr[j]);
   }
   __syncthreads();
-  if (tid < 32) decay_products(sm.g, sm.gam, LA, sm.from, sm.rest, tid);
   if (MEMORY && dv < NT)
     for (int r = tid; r < ch.count; r += NTH) sm.vs[r * LD + dv] = 1.f;
   if (!MEMORY) {
-    // turned in place, a pair of dims (i, i + rot / 2) a thread, then k times its factor
-    const int half = in.rot >> 1;
-    for (int e = tid; e < CQ * half; e += NTH) {
-      const int r = e / half, i = e % half;
-      if (r >= ch.count) continue;
-      const size_t at = (size_t)in.positions[ch.row0 + r] * half + i;
-      const float cs = in.cos_t[at], sn = in.sin_t[at];
-      float* k = sm.k + r * LD + i;
+    // in place, k times its factor
+#pragma unroll
+    for (int j = 0; j < PAIRS; ++j) {
+      const int e = tid + j * NTH, r = half ? e / half : CQ;
+      if (r >= ch.count) break;
+      float* k = sm.k + r * LD + e - r * half;
       const float k0 = k[0], k1 = k[half];
-      k[0] = (k0 * cs - k1 * sn) * kf;
-      k[half] = (k1 * cs + k0 * sn) * kf;
+      k[0] = (k0 * cs[j] - k1 * sn[j]) * kf;
+      k[half] = (k1 * cs[j] + k0 * sn[j]) * kf;
       if (WITH_Q) {
-        float* q = sq + r * LD + i;
+        float* q = sq + r * LD + e - r * half;
         const float q0 = q[0], q1 = q[half];
-        q[0] = q0 * cs - q1 * sn;
-        q[half] = q1 * cs + q0 * sn;
+        q[0] = q0 * cs[j] - q1 * sn[j];
+        q[half] = q1 * cs[j] + q0 * sn[j];
       }
     }
     const int plain = dk - in.rot;
@@ -501,14 +643,14 @@ __device__ __forceinline__ void decay_rows(const DecayIn& in, const Chunk& ch, i
   __syncthreads();
 }
 
-// The next 64 value columns from col0 on (and the matrix memory's column of ones).
+// The value columns from col0 on (and the matrix memory's column of ones); zeros up to LD.
 template <bool MEMORY>
 __device__ __forceinline__ void next_columns(const DecayIn& in, const Chunk& ch, int h, int col0, float* vs) {
-  for (int e = threadIdx.x; e < CQ * NT; e += NTH) {
-    const int t = e / NT, d = col0 + e % NT;
+  for (int e = threadIdx.x; e < CQ * LD; e += NTH) {
+    const int t = e / LD, d = col0 + e % LD;
     float x = 0.f;
     if (t < ch.count) x = d < in.dv ? in.v[(size_t)(ch.row0 + t) * in.ld + (size_t)h * in.dv + d] : MEMORY && d == in.dv ? 1.f : 0.f;
-    vs[t * LD + e % NT] = x;
+    vs[e] = x;
   }
 }
 }  // namespace
@@ -520,48 +662,45 @@ decay_states_kernel(const DecayIn in, const Chunk* __restrict__ chunks, float2* 
   const int H = in.H, dk = in.dk, dvp = in.dvp;
   const int c = blockIdx.x / H, h = blockIdx.x % H;
   const Chunk ch = chunks[c];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
   const size_t item = (size_t)c * H + h;
   decay_rows<MEMORY, false>(in, ch, h, sm, nullptr);
-  for (int e = tid; e < CQ * (NT / 4); e += NTH) {
-    const int t = e / (NT / 4), i = (e % (NT / 4)) * 4;
-    st4(sm.k + t * LD + i, mul4(ld4(sm.k + t * LD + i), sm.gam[(CQ - 1) * LA + t]));
-  }
   if (tid == 0) pp[item] = make_float2(sm.from[CQ - 1], sm.rest[0]);
-  for (int col0 = 0; col0 < dvp; col0 += NT) {
-    const int ncols = min(NT, dvp - col0);
+  // a warp has 16 rows of the state, all columns
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  uint32_t a[CQ / 16][3][4];
+#pragma unroll
+  for (int k = 0; k < CQ / 16; ++k) {
+    float to[10];               // the decays from the lane's tokens to the chunk's end
+#pragma unroll
+    for (int e = 0; e < 4; ++e) to[8 * (e >> 1) + (e & 1)] = decay_between(sm.win, CQ - 1, k * 16 + 2 * q + 8 * (e >> 1) + (e & 1));
+    frag_turned(sm.k + (k * 16 + 2 * q) * LD + warp * 16 + g, LD, to, a[k]);
+  }
+  for (int col0 = 0, ncols; col0 < dvp; col0 += ncols) {
+    ncols = pass_columns(dvp - col0);
     if (col0) {
       __syncthreads();
       next_columns<MEMORY>(in, ch, h, col0, sm.vs);
+      __syncthreads();
     }
-    __syncthreads();
-    if (ncols <= 8) {           // a few columns
-      for (int e = tid; e < dk * ncols; e += NTH) {
-        const int i = e / ncols, d = e % ncols;
-        float x = 0.f;
-#pragma unroll 8
-        for (int s = 0; s < CQ; ++s) x = fmaf(sm.k[s * LD + i], sm.vs[s * LD + d], x);
-        bb[(item * dk + i) * dvp + col0 + d] = x;
+#pragma unroll 2
+    for (int n = 0; n < (ncols + 7) / 8; ++n) {
+      float big[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < CQ / 16; ++k) {
+        uint32_t v[3][2];
+        frag_k(sm.vs + (k * 16 + 2 * q) * LD + 8 * n + g, LD, v);
+        mma_split(big, small, a[k], v);
       }
-      continue;
+      const int d = 8 * n + 2 * q;
+      if (d < ncols)            // (dvp is a multiple of 4)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int row = warp * 16 + g + 8 * i;
+          if (row < dk)
+            *reinterpret_cast<float2*>(bb + (item * dk + row) * dvp + col0 + d) = make_float2(big[2 * i] + small[2 * i], big[2 * i + 1] + small[2 * i + 1]);
+        }
     }
-    float4 b[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) b[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (int s = 0; s < CQ; ++s) {
-      const float4 v = ld4(sm.vs + s * LD + 4 * tx);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const float4 k = ld4(sm.k + s * LD + 8 * ty + 4 * half);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) fma4(b[4 * half + i], at4(k, i), v);
-      }
-    }
-    if (4 * tx < ncols)
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (8 * ty + i < dk) st4(bb + (item * dk + 8 * ty + i) * dvp + col0 + 4 * tx, b[i]);
   }
 }
 
@@ -606,11 +745,11 @@ decay_out_kernel(const DecayIn in, const Chunk* __restrict__ chunks, const float
   const int H = in.H, dk = in.dk, dvp = in.dvp;
   const int c = blockIdx.x / H, h = blockIdx.x % H;
   const Chunk ch = chunks[c];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
   const float* sp = start + ((size_t)c * H + h) * dk * dvp;
-  auto fetch_state = [&](int col0) {            // its 64 columns from col0 on; what does not exist as zeros
-    for (int e = tid; e < NT * (NT / 4); e += NTH) {
-      const int i = e / (NT / 4), d = (e % (NT / 4)) * 4;
+  auto fetch_state = [&](int col0) {            // its columns from col0 on; what does not exist as zeros
+    for (int e = tid; e < NT * (LD / 4); e += NTH) {
+      const int i = e / (LD / 4), d = (e % (LD / 4)) * 4;
       const bool ok = i < dk && col0 + d < dvp;
       cp_async16_or_zero(sm.st + i * LD + d, ok ? sp + (size_t)i * dvp + col0 + d : sp, ok);
     }
@@ -618,133 +757,147 @@ decay_out_kernel(const DecayIn in, const Chunk* __restrict__ chunks, const float
   };
   fetch_state(0);
   decay_rows<MEMORY, true>(in, ch, h, sm, sm.q);
-  // ---- A = (q k^T) times the decays between the tokens
-  {
-    float acc[4][2][2];
+  // a warp has 16 tokens, and half of the keys (columns)
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, t0 = (warp & 1) * 16, side = warp >> 1;
+  const float f0 = sm.from[t0 + g], f1 = sm.from[t0 + g + 8];
+  // ---- A = (q k^T) times the decays between the tokens (keys 16 and up concern no token below them)
+  if (side == 0 || t0) {
+    float big[2][4] = {}, small[2][4] = {};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.f;
-#pragma unroll 4
-    for (int e = 0; e < NT; e += 4) {
-      const float4 b0 = ld4(sm.k + tx * LD + e), b1 = ld4(sm.k + (tx + 16) * LD + e);
+    for (int k = 0; k < NT / 16; ++k) {
+      uint32_t a[3][4];
+      frag_rows(sm.q + (t0 + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 a = ld4(sm.q + (ty + 8 * i) * LD + e);
-        dot4_by_two(a, b0, acc[i][0]);
-        dot4_by_two(a, b1, acc[i][1]);
+      for (int n = 0; n < 2; ++n) {
+        uint32_t b[3][2];
+        frag_columns(sm.k + (side * 16 + 8 * n + g) * LD + k * 16 + 2 * q, b);
+        mma_split(big[n], small[n], a, b);
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int t = ty + 8 * i, s = tx + 16 * j;
-        sm.a[t * LA + s] = s <= t ? (acc[i][j][0] + acc[i][j][1]) * sm.gam[t * LA + s] : 0.f;
+      for (int e = 0; e < 4; ++e) {
+        const int t = t0 + g + 8 * (e >> 1), s = side * 16 + 8 * n + 2 * q + (e & 1);
+        sm.a[t * LA + s] = s <= t ? (big[n][e] + small[n][e]) * decay_between(sm.win, t, s) : 0.f;
       }
+  } else {
+    for (int e = lane; e < 16 * 16; e += 32) sm.a[(e >> 4) * LA + 16 + (e & 15)] = 0.f;
   }
-  __syncthreads();
-  for (int e = tid; e < CQ * (NT / 4); e += NTH) {
-    float* q = sm.q + (e / (NT / 4)) * LD + (e % (NT / 4)) * 4;
-    st4(q, mul4(ld4(q), sm.from[e / (NT / 4)]));
-  }
-  for (int col0 = 0; col0 < dvp; col0 += NT) {
-    const int ncols = min(NT, dvp - col0);
+  for (int col0 = 0, ncols; col0 < dvp; col0 += ncols) {
+    ncols = pass_columns(dvp - col0);
     if (col0) {
       __syncthreads();
       fetch_state(col0);
       next_columns<MEMORY>(in, ch, h, col0, sm.vs);
+      __syncthreads();
     }
+    // a product with zeros above the diagonal would bring a value that is not finite to earlier tokens: such a chunk takes FMAs
+    bool ordinary = true;
+    for (int e = tid; e < CQ * LD / 4; e += NTH) ordinary = ordinary && finite4(ld4(sm.vs + 4 * e));
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    if (ncols <= 8) {           // a few columns
-      for (int e = tid; e < CQ * ncols; e += NTH) {
-        const int t = e / ncols, d = e % ncols;
-        float x = 0.f, y = 0.f;
-        for (int s = 0; s <= t; ++s) x = fmaf(sm.a[t * LA + s], sm.vs[s * LD + d], x);
-#pragma unroll 8
-        for (int i = 0; i < NT; ++i) y = fmaf(sm.q[t * LD + i], sm.st[i * LD + d], y);
-        if (t < ch.count) out[((size_t)(ch.row0 + t) * H + h) * dvp + col0 + d] = x + y;
+    const bool all = __syncthreads_and(ordinary);          // and the state and A are there
+    if (all) {
+      const int tiles = (ncols + 7) / 8;
+      constexpr int NJ = (LD / 8 + 2) / 2;                  // column tiles side, side + 2, ..
+      float big[NJ][4] = {}, small[NJ][4] = {};
+#pragma unroll
+      for (int k = 0; k < CQ / 16; ++k) {
+        if (16 * k > t0) break;
+        uint32_t a[3][4];
+        frag_rows(sm.a + (t0 + g) * LA + k * 16 + 2 * q, LA, 1.f, 1.f, a);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+          if (side + 2 * j < tiles) {
+            uint32_t b[3][2];
+            frag_k(sm.vs + (k * 16 + 2 * q) * LD + (side + 2 * j) * 8 + g, LD, b);
+            mma_split(big[j], small[j], a, b);
+          }
+      }
+#pragma unroll
+      for (int k = 0; k < NT / 16; ++k) {
+        uint32_t a[3][4];
+        frag_rows(sm.q + (t0 + g) * LD + k * 16 + 2 * q, LD, f0, f1, a);
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+          if (side + 2 * j < tiles) {
+            uint32_t b[3][2];
+            frag_k(sm.st + (k * 16 + 2 * q) * LD + (side + 2 * j) * 8 + g, LD, b);
+            mma_split(big[j], small[j], a, b);
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int d = (side + 2 * j) * 8 + 2 * q;
+        if (d < ncols)          // (dvp is a multiple of 4)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int t = t0 + g + 8 * i;
+            if (t < ch.count)
+              *reinterpret_cast<float2*>(out + ((size_t)(ch.row0 + t) * H + h) * dvp + col0 + d) =
+                  make_float2(big[j][2 * i] + small[j][2 * i], big[j][2 * i + 1] + small[j][2 * i + 1]);
+          }
       }
       continue;
     }
-    float4 o[1][4], y[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) o[0][i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float* values[1] = {sm.vs + 4 * tx};
-    triangle_rows<4, LA, 1>(o, sm.a, values, ty, [&](int i) { return ty + 8 * i + 1; });
-#pragma unroll 2
-    for (int s = 0; s < NT; s += 4) {
-      float4 v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = ld4(sm.st + (s + j) * LD + 4 * tx);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 x = ld4(sm.q + (ty + 8 * i) * LD + s);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) fma4(y[i], at4(x, j), v[j]);
-      }
+    for (int e = tid; e < CQ * ncols; e += NTH) {
+      const int t = e / ncols, d = e % ncols;
+      float x = 0.f, y = 0.f;
+      for (int s = 0; s <= t; ++s) x = fmaf(sm.a[t * LA + s], sm.vs[s * LD + d], x);
+#pragma unroll 8
+      for (int i = 0; i < NT; ++i) y = fmaf(sm.q[t * LD + i] * sm.from[t], sm.st[i * LD + d], y);
+      if (t < ch.count) out[((size_t)(ch.row0 + t) * H + h) * dvp + col0 + d] = x + y;
     }
-    if (4 * tx < ncols)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = ty + 8 * i;
-        if (t < ch.count)
-          st4(out + ((size_t)(ch.row0 + t) * H + h) * dvp + col0 + 4 * tx,
-              make_float4(o[0][i].x + y[i].x, o[0][i].y + y[i].y, o[0][i].z + y[i].z, o[0][i].w + y[i].w));
-      }
   }
 }
 
 // ------------------------------------------------------------------ 2. walk
-// S <- P S + (M S + B) and O = Rq S + Ov over a request's chunks.  A block owns DVS value columns of a head: S lies in shared
-// memory (column by column, two copies in turn), and what a chunk brings comes through a ring of three stages, two chunks
-// ahead.  A thread makes four columns of three rows (two of M, one of Rq) from 16-byte loads along the inner dimension, in
-// sums over even and odd places.  Bound by the bytes that its loads bring from shared memory (128 a clock and SM, also where
-// lanes read the same place): 7 loads for 12 outputs.
-// A chunk takes 2.7 us (64 heads, 256 blocks of 128 threads), with 3 x 2 outputs a thread as long, with 6 x 4 and two warps a
-// block 3.1.
+// S <- P S + (M S + B) and O = Rq S + Ov over a request's chunks.  A block owns DVS value columns of a head and has a warp per 16 rows
+// of [M ; Rq].  The four warps of M keep S in float32 registers (the tensor core's result layout) and leave its pieces in shared memory, two copies in
+// turn, for all six; what a chunk brings comes through a ring, a chunk ahead.
+// One request of 2,048 tokens at 64 heads of 64 x 64: 173 us with multiply-adds (7 wide loads of shared memory for 24 pairs of them were
+// the bound), 117 here (issue slots 53 %, tensor pipe 32 %: the pieces again).
 namespace {
 template <int DVS>
 struct WalkShape {
   static constexpr int ROWS = NT + CQ;                                 // rows of [M ; Rq]
-  static constexpr int OFF = ROWS * LD, P = OFF + ROWS * DVS;          // [B ; Ov] and P behind them
+  static constexpr int LM = NT + 8, LO = DVS + 8, LS = NT + 8;         // numbers between rows: neighbouring rows in other banks
+  static constexpr int OFF = ROWS * LM, P = OFF + ROWS * LO;           // [B ; Ov] and P behind them
   static constexpr int STAGE = P + NT;
-  static constexpr int STAGES = 3, THREADS = DVS * 8;
-  static constexpr size_t SMEM = (size_t)(STAGES * STAGE + 2 * DVS * LD) * sizeof(float);
+  static constexpr int STAGES = 2, THREADS = ROWS / 16 * 32;           // (two blocks an SM; three stages would leave one)
+  static constexpr int PLANE = DVS * LS;                               // bf16 of one piece of S, column by column
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE * sizeof(float) + (size_t)2 * 3 * PLANE * sizeof(bf16);
 };
 }  // namespace
 
 template <int DVS>
-__global__ void __launch_bounds__(DVS * 8)
+__global__ void __launch_bounds__(WalkShape<DVS>::THREADS, 2)
 chunk_walk_kernel(const Request* __restrict__ requests, const Chunk* __restrict__ chunks, const float* __restrict__ mm,
                   const float* __restrict__ rq, const float* __restrict__ bb, float* __restrict__ state, float* __restrict__ out,
                   int H, int dk, int dv) {
   using K = WalkShape<DVS>;
+  constexpr int NN = DVS / 8;                   // column tiles
   extern __shared__ __align__(16) float ws[];
-  float* sbuf = ws + K::STAGES * K::STAGE;
+  bf16* planes = reinterpret_cast<bf16*>(ws + K::STAGES * K::STAGE);
   const Request r = requests[blockIdx.x / H];
   const int h = blockIdx.x % H, col0 = blockIdx.y * DVS;
-  const int tid = threadIdx.x, tx = tid % (DVS / 4), ty = tid / (DVS / 4);      // ty in 0 .. 31
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   float* sp = state + ((size_t)r.slot * H + h) * dk * dv;
   const int row0 = chunks[r.chunk0].row0, rows = CQ * (r.chunks - 1) + chunks[r.chunk0 + r.chunks - 1].count;
-  // a thread's pieces of a chunk: the same places every time, a chunk further on
-  constexpr int NP = K::ROWS * (NT / 4) / K::THREADS, NO = K::ROWS * (DVS / 4) / K::THREADS;
-  static_assert(K::ROWS * (NT / 4) % K::THREADS == 0 && K::ROWS * (DVS / 4) % K::THREADS == 0, "whole pieces a thread");
   auto fetch = [&](int c) {
     float* st = ws + (c % K::STAGES) * K::STAGE;
     const size_t item = (size_t)(r.chunk0 + c) * H + h;
-    const float *m = mm + item * MFLOATS, *q = rq + item * CQ * NT;
-#pragma unroll
-    for (int j = 0; j < NP; ++j) {
-      const int e = tid + j * K::THREADS, row = e / (NT / 4), i = (e % (NT / 4)) * 4;
-      cp_async16_or_zero(st + row * LD + i, row < NT ? m + e * 4 : q + e * 4 - NT * NT, true);
+    const float *m = mm + item * MFLOATS, *rqp = rq + item * CQ * NT;
+    for (int e = tid; e < K::ROWS * (NT / 4); e += K::THREADS) {
+      const int row = e / (NT / 4), i = (e % (NT / 4)) * 4;
+      cp_async16_or_zero(st + row * K::LM + i, row < NT ? m + e * 4 : rqp + e * 4 - NT * NT, true);
     }
     if (tid < NT / 4) cp_async16_or_zero(st + K::P + 4 * tid, m + NT * NT + 4 * tid, true);
-#pragma unroll
-    for (int j = 0; j < NO; ++j) {
-      const int e = tid + j * K::THREADS, row = e / (DVS / 4), d = (e % (DVS / 4)) * 4, t = c * CQ + row - NT;
+    for (int e = tid; e < K::ROWS * (DVS / 4); e += K::THREADS) {
+      const int row = e / (DVS / 4), d = (e % (DVS / 4)) * 4, t = c * CQ + row - NT;
       const bool in = col0 + d < dv && (row < NT ? row < dk : t < rows);
       const float* src = row < NT ? bb + (item * dk + row) * dv : out + ((size_t)(row0 + t) * H + h) * dv;
-      cp_async16_or_zero(st + K::OFF + row * DVS + d, in ? src + col0 + d : bb, in);
+      cp_async16_or_zero(st + K::OFF + row * K::LO + d, in ? src + col0 + d : bb, in);
     }
   };
 #pragma unroll
@@ -752,68 +905,100 @@ chunk_walk_kernel(const Request* __restrict__ requests, const Chunk* __restrict_
     if (c < r.chunks) fetch(c);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  for (int e = tid; e < NT * DVS; e += K::THREADS) {
-    const int i = e / DVS, d = e % DVS;
-    sbuf[d * LD + i] = i < dk && col0 + d < dv ? sp[(size_t)i * dv + col0 + d] : 0.f;
+  // a lane's entries of S: rows mrow and mrow + 8, columns 8 n + 2 q and the next
+  const bool moves = warp < NT / 16;
+  const int mrow = warp * 16 + g;
+  float S[NN][4];
+  auto publish = [&](int copy) {
+    bf16* p = planes + (size_t)copy * 3 * K::PLANE;
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float x = S[n][e];
+        bf16* at = p + (8 * n + 2 * q + (e & 1)) * K::LS + mrow + 8 * (e >> 1);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const bf16 piece = __float2bfloat16_rn(x);
+          at[k * K::PLANE] = piece;
+          x -= __bfloat162float(piece);
+        }
+      }
+  };
+  if (moves) {
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = mrow + 8 * (e >> 1), d = col0 + 8 * n + 2 * q + (e & 1);
+        S[n][e] = i < dk && d < dv ? sp[(size_t)i * dv + d] : 0.f;
+      }
+    publish(0);
   }
   for (int c = 0; c < r.chunks; ++c) {
     asm volatile("cp.async.wait_group %0;" ::"n"(K::STAGES - 2) : "memory");
-    __syncthreads();            // chunk c is there, S is written, and the stage of chunk c - 1 may be filled again
+    __syncthreads();            // chunk c is there, S's pieces are written, and the stage of chunk c - 1 may be filled again
     if (c + K::STAGES - 1 < r.chunks) fetch(c + K::STAGES - 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const float* st = ws + (c % K::STAGES) * K::STAGE;
-    const float* off = st + K::OFF;
-    const float* s = sbuf + (c & 1) * DVS * LD;
-    float* sn = sbuf + ((c + 1) & 1) * DVS * LD;
-    constexpr int DQ = DVS / 4;
-    unsigned long long acc[3][4];
+    const bf16* sb = planes + (size_t)(c & 1) * 3 * K::PLANE + g * K::LS + 2 * q;
+    float big[NN][4], small[NN][4];
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+    for (int n = 0; n < NN; ++n)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-#pragma unroll 4
-    for (int e = 0; e < NT; e += 4) {
-      ulonglong2 x[4];
+      for (int e = 0; e < 4; ++e) big[n][e] = small[n][e] = 0.f;
+    const float* ap = st + mrow * K::LM + 2 * q;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) x[j] = ld_pairs(s + (tx + DQ * j) * LD + e);
+    for (int k = 0; k < NT / 16; ++k) {
+      uint32_t a[3][4];
+      frag_rows(ap + k * 16, K::LM, 1.f, 1.f, a);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const ulonglong2 a = ld_pairs(st + (ty + 32 * i) * LD + e);
+      for (int n = 0; n < NN; ++n) {
+        uint32_t b[3][2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          fma_pairs(acc[i][j], a.x, x[j].x);
-          fma_pairs(acc[i][j], a.y, x[j].y);
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            b[p][e] = *reinterpret_cast<const uint32_t*>(sb + p * K::PLANE + n * 8 * K::LS + k * 16 + 8 * e);
+        mma_split(big[n], small[n], a, b);
+      }
+    }
+    const float* off = st + K::OFF + mrow * K::LO + 2 * q;
+    if (moves) {
+      const float p0 = st[K::P + mrow], p1 = st[K::P + mrow + 8];
+#pragma unroll
+      for (int n = 0; n < NN; ++n)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 o = *reinterpret_cast<const float2*>(off + 8 * i * K::LO + 8 * n);
+          S[n][2 * i] = fmaf(i ? p1 : p0, S[n][2 * i], big[n][2 * i] + small[n][2 * i] + o.x);
+          S[n][2 * i + 1] = fmaf(i ? p1 : p0, S[n][2 * i + 1], big[n][2 * i + 1] + small[n][2 * i + 1] + o.y);
         }
-      }
-    }
+      publish((c + 1) & 1);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int row = ty + 32 * i;
-      const float p = st[K::P + row];
+      for (int i = 0; i < 2; ++i) {
+        const int t = c * CQ + mrow + 8 * i - NT;
+        if (t >= rows) continue;
+        float* o = out + ((size_t)(row0 + t) * H + h) * dv + col0 + 2 * q;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int d = tx + DQ * j;
-        sn[d * LD + row] = fmaf(p, s[d * LD + row], pair_sum(acc[i][j]) + off[row * DVS + d]);
-      }
-    }
-#pragma unroll
-    for (int i = 2; i < 3; ++i) {
-      const int row = ty + 32 * i, t = c * CQ + row - NT;
-      float* o = out + ((size_t)(row0 + t) * H + h) * dv + col0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int d = tx + DQ * j;
-        if (t < rows && col0 + d < dv) o[d] = pair_sum(acc[i][j]) + off[row * DVS + d];
+        for (int n = 0; n < NN; ++n) {
+          const float2 v = *reinterpret_cast<const float2*>(off + 8 * i * K::LO + 8 * n);
+          if (col0 + 8 * n + 2 * q < dv)        // (dv is a multiple of 4)
+            *reinterpret_cast<float2*>(o + 8 * n) = make_float2(big[n][2 * i] + small[n][2 * i] + v.x, big[n][2 * i + 1] + small[n][2 * i + 1] + v.y);
+        }
       }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-  const float* s = sbuf + (r.chunks & 1) * DVS * LD;
-  for (int e = tid; e < NT * DVS; e += K::THREADS) {
-    const int i = e / DVS, d = e % DVS;
-    if (i < dk && col0 + d < dv) sp[(size_t)i * dv + col0 + d] = s[d * LD + i];
-  }
+  if (moves)
+#pragma unroll
+    for (int n = 0; n < NN; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = mrow + 8 * (e >> 1), d = col0 + 8 * n + 2 * q + (e & 1);
+        if (i < dk && d < dv) sp[(size_t)i * dv + d] = S[n][e];
+      }
 }
 
 namespace {

@@ -121,3 +121,12 @@ def test_more_walked_requests_than_a_grid_is_high():
     lengths = [1] * 65536 + [64]
     t = inputs("general", 1, 4, 4, lengths, torch.Generator(DEV).manual_seed(3))
     same(scan("general", 1, 4, 4, lengths, t, 65536), scan("general", 1, 4, 4, lengths, t, len(lengths)))
+
+
+@pytest.mark.parametrize("kind", ["general", "gated", "retention", "memory"])
+@pytest.mark.parametrize("dk,dv", [(64, 68), (60, 64), (8, 72), (64, 128)])
+def test_value_columns_around_a_pass(kind, dk, dv):
+    """One, two and three passes over the value columns, the last of them with columns that a pass of 64 leaves over."""
+    lengths = [33, 100]
+    t = inputs(kind, 3, dk, dv, lengths, torch.Generator(DEV).manual_seed(dk * dv))
+    same(*(scan(kind, 3, dk, dv, lengths, t, first) for first in (0, len(lengths))))
