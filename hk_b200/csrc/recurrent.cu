@@ -932,16 +932,18 @@ __global__ void head_out_gate_kernel(const float* __restrict__ o, int ldo, const
 }
 
 // The same for heads of whole 16-byte pieces, up to 128 values: L lanes hold a head's values, four each, so a warp takes 32 / L
-// heads at once.  Bound by its bytes; one value a lane and load took 61 us for 2,048 tokens of 64 heads of 64, this 21 (4 TB/s).
+// heads at once.  Bound by its bytes; one value a lane and load took 61 us for 2,048 tokens of 64 heads of 64, this 18 (4.7 TB/s).
 template <typename T, int L>
 __global__ void __launch_bounds__(256)
 head_out_gate_vec_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, long long ldg, const float* __restrict__ weight,
-                         int shared_weight, int act, const float* __restrict__ gates, float den_eps, T* __restrict__ out, long long items,
+                         int shared_weight, int act, const float* __restrict__ gates, float den_eps, T* __restrict__ out, int items,
                          int H, int dv, float eps) {
-  const long long item = (long long)blockIdx.x * (256 / L) + threadIdx.x / L;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int item = blockIdx.x * (256 / L) + threadIdx.x / L;
   const int i = (threadIdx.x % L) * 4;
   const bool in = item < items, on = in && i < dv;
-  const size_t it = in ? (size_t)item : 0, t = it / (size_t)H;
+  const size_t it = in ? (size_t)item : 0, t = in ? (size_t)(item / H) : 0;       // (a 64-bit division would cost as much as a gate)
   const int h = (int)(it - t * (size_t)H);
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* src = o + it * ldo;
@@ -955,7 +957,9 @@ head_out_gate_vec_kernel(const float* __restrict__ o, int ldo, const float* __re
   for (int k = L >> 1; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
   if (!on) return;
   const float inv = scale / sqrtf(ss / (float)dv + eps);
-  auto gate = [&](float z) { return act == 0 ? sigmoid_f(z) : z * sigmoid_f(z); };
+  // (narrowed, by a division without the branch for unusual operands)
+  auto sigmoid = [](float z) { return sizeof(T) == 4 ? sigmoid_f(z) : __fdividef(1.0f, 1.0f + expf(-z)); };
+  auto gate = [&](float z) { return act == 0 ? sigmoid(z) : z * sigmoid(z); };
   const float4 y = make_float4(x.x * inv * w.x * gate(gl.x), x.y * inv * w.y * gate(gl.y), x.z * inv * w.z * gate(gl.z), x.w * inv * w.w * gate(gl.w));
   T* dst = out + it * dv + i;
   if (sizeof(T) == 4) {
@@ -969,11 +973,11 @@ head_out_gate_vec_kernel(const float* __restrict__ o, int ldo, const float* __re
 template <typename T>
 static int head_out_gate(const float* o, int ldo, const float* g, long long ldg, const float* weight, int shared_weight, int act,
                          const float* gates, float den_eps, T* out, long long items, int H, int dv, float eps, cudaStream_t s) {
-  const bool vec = dv <= 128 && !(dv & 3) && !(ldo & 3) && !(ldg & 3) &&
+  const bool vec = dv <= 128 && !(dv & 3) && !(ldo & 3) && !(ldg & 3) && items <= 0x7fffffffLL - 32 &&
                    (((uintptr_t)o | (uintptr_t)g | (uintptr_t)weight | (uintptr_t)out) & 15) == 0;
 #define HEAD_OUT_VEC(L)                                                                                                               \
-  return hk_launch(head_out_gate_vec_kernel<T, L>, dim3((unsigned)((items + 256 / L - 1) / (256 / L))), dim3(256), 0, s, o, ldo, g, ldg, \
-                   weight, shared_weight, act, gates, den_eps, out, items, H, dv, eps)
+  return hk_launch_pdl(head_out_gate_vec_kernel<T, L>, dim3((unsigned)((items + 256 / L - 1) / (256 / L))), dim3(256), 0, s, o, ldo, g, ldg, \
+                   weight, shared_weight, act, gates, den_eps, out, (int)items, H, dv, eps)
   if (vec && dv > 64) HEAD_OUT_VEC(32);
   if (vec && dv > 32) HEAD_OUT_VEC(16);
   if (vec) HEAD_OUT_VEC(8);

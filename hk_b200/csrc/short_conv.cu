@@ -17,6 +17,13 @@
 #define SC_GROUP 8
 #define SC_MAX_TAPS 16
 
+// silu in float32; where the result is narrowed, by a division without the branch for unusual operands
+template <typename T>
+__device__ __forceinline__ float conv_act(float z, int act) {
+  if (!act) return z;
+  return sizeof(T) == 4 ? z / (1.0f + expf(-z)) : __fdividef(z, 1.0f + expf(-z));
+}
+
 // The thread walks its tokens in groups of SC_GROUP: the group's inputs are loaded at once (each input is read once; the
 // taps - 1 before them stay in registers from the group before), then the group's outputs are summed, oldest tap first.
 // A segment of one row (a decoded token) takes a path of its own with the same sum.  TAPS: the most taps an instance holds.
@@ -53,7 +60,7 @@ short_conv_kernel(const float* __restrict__ x, long long ldx, const float* __res
     for (int s = TAPS - 1; s >= 1; --s)
       if (s <= back) acc = fmaf(wr[s], hist[s], acc);
     acc = fmaf(wr[0], now, acc);
-    y[(size_t)row0 * ldy + c] = from_f32<T>(act ? acc / (1.0f + expf(-acc)) : acc);
+    y[(size_t)row0 * ldy + c] = from_f32<T>(conv_act<T>(acc, act));
 #pragma unroll
     for (int s = TAPS - 1; s >= 2; --s)
       if (s <= back) tl[(size_t)(back - s) * C] = hist[s - 1];
@@ -77,7 +84,7 @@ short_conv_kernel(const float* __restrict__ x, long long ldx, const float* __res
     }
 #pragma unroll
     for (int u = 0; u < SC_GROUP; ++u)
-      if (tg + u < t1) y[(size_t)(row0 + tg + u) * ldy + c] = from_f32<T>(act ? acc[u] / (1.0f + expf(-acc[u])) : acc[u]);
+      if (tg + u < t1) y[(size_t)(row0 + tg + u) * ldy + c] = from_f32<T>(conv_act<T>(acc[u], act));
     float next[TAPS];
 #pragma unroll
     for (int s = 1; s < TAPS; ++s) next[s] = s <= SC_GROUP ? nw[s <= SC_GROUP ? SC_GROUP - s : 0] : hist[s <= SC_GROUP ? 0 : s - SC_GROUP];
@@ -95,9 +102,109 @@ short_conv_kernel(const float* __restrict__ x, long long ldx, const float* __res
   }
 }
 
+// The same for up to four taps and channels in whole 16-byte pieces: a thread makes four channels of eight tokens, everything it reads
+// asked for at once, with the sums in the same order.  A block's tokens are found by counting through the segments, so that no block is
+// launched for tokens that do not exist.  Bound by its bytes and the activations: four requests
+// of 512 tokens by 6,144 channels 31.3 -> 21.4 us (3.5 TB/s), by 4,352 23.0 -> 16.0; 64 requests of one token 13.1 -> 11.4.
+#define SCV_TOKENS 8
+template <typename T>
+__global__ void __launch_bounds__(128)
+short_conv_vec_kernel(const float* __restrict__ x, long long ldx, const float* __restrict__ w, const float* __restrict__ bias,
+                      const int* __restrict__ segs, int n_seg, float* __restrict__ tail, T* __restrict__ y, long long ldy, int C, int taps,
+                      int act) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, back = taps - 1;
+  int left = blockIdx.x, seg = -1, count = 0;
+  for (int base = 0; base < n_seg; base += 32) {
+    const int mine = base + lane < n_seg ? segs[(base + lane) * 3 + 2] : 0, chunks = (mine + SCV_TOKENS - 1) / SCV_TOKENS;
+    int upto = chunks;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, upto > left);
+    if (past) {
+      const int l = __ffs(past) - 1;
+      seg = base + l;
+      count = __shfl_sync(0xffffffffu, mine, l);
+      left -= __shfl_sync(0xffffffffu, upto - chunks, l);
+      break;
+    }
+    left -= __shfl_sync(0xffffffffu, upto, 31);
+  }
+  const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+  if (seg < 0 || c >= C) return;
+  const int slot = segs[seg * 3], row0 = segs[seg * 3 + 1], t0 = left * SCV_TOKENS;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float* tl = tail + (size_t)slot * back * C + c;
+  const float* xp = x + (size_t)row0 * ldx + c;
+  float in[SCV_TOKENS + 3][4], wr[4][4], b[4];
+#pragma unroll
+  for (int i = 0; i < SCV_TOKENS + 3; ++i) {
+    const int r = t0 - 3 + i;
+    float4 v = zero;
+    if (r >= 0) {
+      if (r < count && (i >= 3 || 3 - i <= back)) v = *reinterpret_cast<const float4*>(xp + (size_t)r * ldx);
+    } else if (-r <= back) {
+      v = *reinterpret_cast<const float4*>(tl + (size_t)(back + r) * C);
+    }
+    in[i][0] = v.x; in[i][1] = v.y; in[i][2] = v.z; in[i][3] = v.w;
+  }
+  const float4 bv = bias != nullptr ? *reinterpret_cast<const float4*>(bias + c) : zero;
+  b[0] = bv.x; b[1] = bv.y; b[2] = bv.z; b[3] = bv.w;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (taps == 4) {
+      const float4 v = *reinterpret_cast<const float4*>(w + (size_t)(c + e) * 4);
+      wr[0][e] = v.w; wr[1][e] = v.z; wr[2][e] = v.y; wr[3][e] = v.x;
+    } else {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) wr[s][e] = s <= back ? w[(size_t)(c + e) * taps + back - s] : 0.f;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < SCV_TOKENS; ++u) {
+    if (t0 + u >= count) break;
+    float acc[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      acc[e] = b[e];
+#pragma unroll
+      for (int s = 3; s >= 0; --s)
+        if (s <= back) acc[e] = fmaf(wr[s][e], in[3 + u - s][e], acc[e]);
+      acc[e] = conv_act<T>(acc[e], act);
+    }
+    T* dst = y + (size_t)(row0 + t0 + u) * ldy + c;
+    if (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(dst)) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[0], acc[1]), hi = __floats2bfloat162_rn(acc[2], acc[3]);
+      *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+  if (t0 == 0) {                // the first block of tokens has read the old tail: the last `back` inputs take its place
+    float4 keep[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int r = count - back + j;
+      const float* h = r == -1 ? in[2] : r == -2 ? in[1] : in[0];
+      if (j < back) keep[j] = r >= 0 ? *reinterpret_cast<const float4*>(xp + (size_t)r * ldx) : make_float4(h[0], h[1], h[2], h[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      if (j < back) *reinterpret_cast<float4*>(tl + (size_t)j * C) = keep[j];
+  }
+}
+
 template <typename T, int TAPS>
 static int short_conv(const float* x, long long ldx, const float* w, const float* bias, const int* segs, int n_seg, int n_rows, float* tail,
                       T* y, long long ldy, int C, int taps, int act, cudaStream_t s) {
+  if (taps <= 4 && !(C & 3) && !(ldx & 3) && !(ldy & 3) &&
+      !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)bias | (uintptr_t)tail | (uintptr_t)y) & 15))
+    return hk_launch_pdl(short_conv_vec_kernel<T>, dim3((unsigned)(n_rows / SCV_TOKENS + n_seg), (unsigned)((C + 511) / 512)), dim3(128), 0, s, x, ldx, w,
+                     bias, segs, n_seg, tail, y, ldy, C, taps, act);
   // a step of single rows needs no second block of tokens; else as many as the longest segment may have
   const int longest = n_rows - n_seg + 1;
   dim3 grid((unsigned)n_seg, (unsigned)((C + 127) / 128), (unsigned)((longest + SC_TOKENS - 1) / SC_TOKENS));

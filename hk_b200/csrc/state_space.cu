@@ -802,12 +802,65 @@ __global__ void gated_part_norm_kernel(const float* __restrict__ y, const float*
   }
 }
 
+// The same for many parts of up to 128 N numbers in whole 16-byte pieces: a warp per (token, part), the part's u in registers, everything
+// asked for at once, no barriers.  Bound by its bytes: 2,048 tokens of eight parts of 512 19.5 -> 11.2 us (7.5 TB/s, much of it from L2).
+template <typename T, int N>
+__global__ void __launch_bounds__(256)
+gated_part_norm_warp_kernel(const float* __restrict__ y, const float* __restrict__ z, long long ldz, const float* __restrict__ weight,
+                            T* __restrict__ out, int items, int parts, int W, int width, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= items) return;
+  const int t = item / parts, p0 = (item - t * parts) * width;
+  const float* yr = y + (size_t)t * W + p0;
+  const float* zr = z + (size_t)t * ldz + p0;
+  float4 u[N], zv[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int i = (j * 32 + lane) * 4;
+    u[j] = i < width ? *reinterpret_cast<const float4*>(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    zv[j] = i < width ? *reinterpret_cast<const float4*>(zr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  auto silu = [](float v) { return sizeof(T) == 4 ? v / (1.0f + expf(-v)) : __fdividef(v, 1.0f + expf(-v)); };
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    u[j] = make_float4(u[j].x * silu(zv[j].x), u[j].y * silu(zv[j].y), u[j].z * silu(zv[j].z), u[j].w * silu(zv[j].w));
+    ss = fmaf(u[j].x, u[j].x, fmaf(u[j].y, u[j].y, fmaf(u[j].z, u[j].z, fmaf(u[j].w, u[j].w, ss))));
+  }
+  const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)width + eps);
+  T* o = out + (size_t)t * W + p0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const int i = (j * 32 + lane) * 4;
+    if (i >= width) break;
+    const float4 w = *reinterpret_cast<const float4*>(weight + p0 + i);
+    const float4 r = make_float4(u[j].x * inv * w.x, u[j].y * inv * w.y, u[j].z * inv * w.z, u[j].w * inv * w.w);
+    if (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(o) + i) = r;
+    } else {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(r.x, r.y), hi = __floats2bfloat162_rn(r.z, r.w);
+      *reinterpret_cast<uint2*>(o + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+
 template <typename T>
 static int gated_part_norm(const float* y, const float* z, long long ldz, const float* weight, T* out, int n, int W, int parts, float eps,
                            cudaStream_t s) {
   const int width = W / parts;
   const bool vec = (width & 3) == 0 && (ldz & 3) == 0 &&
                    (((uintptr_t)y | (uintptr_t)z | (uintptr_t)weight | (uintptr_t)out) & 15) == 0;
+  // From 24 warps a SM on a warp a part is the faster: 3,200 parts of 512 4.8 us both ways, 4,000 5.6 against 5.0, 6,400 8.2 against
+  // 4.7; of 1,024 numbers 2,000 parts 5.2 against 5.9, 4,000 9.2 against 7.1; few parts leave most of the SMs idle (128 of 1,024 2.1 / 4.2).
+  const long long rows = (long long)n * parts;
+  if (vec && width <= 1024 && rows >= 24 * 148 && rows <= 0x7fffffffLL - 8) {
+    const dim3 grid((unsigned)((rows + 7) / 8));
+    if (width <= 256) return hk_launch_pdl(gated_part_norm_warp_kernel<T, 2>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
+    if (width <= 512) return hk_launch_pdl(gated_part_norm_warp_kernel<T, 4>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
+    return hk_launch_pdl(gated_part_norm_warp_kernel<T, 8>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
+  }
   const int items = vec ? width / 4 : width;
   const int threads = items >= 256 ? 256 : items > 64 ? 128 : items > 32 ? 64 : 32;
   const size_t smem = (size_t)width * sizeof(float);

@@ -333,6 +333,50 @@ def test_short_convolution_with_a_bias_across_the_edges_of_portions(taps, out):
     assert torch.all(tail[0] == 0.0)
 
 
+@pytest.mark.parametrize("taps,C,out", [(1, 4, torch.float32), (2, 132, torch.bfloat16), (3, 512, torch.float32), (4, 516, torch.bfloat16), (4, 1100, torch.float32)])
+def test_short_convolution_four_channels_a_thread(taps, C, out):
+    """Segments around a thread's eight tokens, empty ones, more than a warp counts at once, in slots of any order; cut in two passes."""
+    from hk_b200.csrc import ops
+    rng = np.random.default_rng(taps)
+    counts = [[8, 0, 1, 7, 9, 16, 17, 2, 3] + [1] * 30 + [70, 5], [1, 33, 8, 0, 3, 24, 1, 1, 9] + [2] * 31 + [40]]
+    slots = rng.permutation(len(counts[0])).tolist()
+    wt, bias = torch.randn(C, taps, device="cuda"), torch.randn(C, device="cuda")
+    tail = torch.zeros(len(slots), max(taps - 1, 1), C, device="cuda")
+    xs, got = [[] for _ in slots], [[] for _ in slots]
+    for part in counts:
+        n = sum(part)
+        x, y = torch.randn(n, C + 8, device="cuda"), torch.full((n + 1, C + 4), float("nan"), dtype=out, device="cuda")
+        starts = np.cumsum([0] + part[:-1]).tolist()
+        segs = torch.tensor([[s, r, c] for s, r, c in zip(slots, starts, part)], dtype=torch.int32, device="cuda")
+        ops.short_conv(x[:, 4:4 + C], wt, segs, tail, y[:n, :C], act="silu", bias=bias)
+        assert torch.isnan(y[:, C:]).all() and torch.isnan(y[n]).all()
+        for i, (r, c) in enumerate(zip(starts, part)):
+            xs[i].append(x[r:r + c, 4:4 + C].double().cpu().numpy())
+            got[i].append(y[r:r + c, :C].double().cpu().numpy())
+    tol = 1e-5 if out == torch.float32 else 5e-3          # half a unit of the last place, and five float32 roundings
+    for i, slot in enumerate(slots):
+        x = np.concatenate(xs[i])
+        want = P.silu(P.short_conv(x, wt.double().cpu().numpy(), bias.double().cpu().numpy()))
+        np.testing.assert_allclose(np.concatenate(got[i]), want, rtol=tol, atol=tol)
+        last = np.concatenate([np.zeros((taps - 1, C)), x])[len(x):]
+        assert np.array_equal(tail[slot][:taps - 1].double().cpu().numpy(), last)
+
+
+@pytest.mark.parametrize("n,parts,width", [(1, 1, 4), (7, 3, 1028), (4000, 1, 4), (1800, 2, 252), (1187, 3, 260), (900, 4, 512), (3600, 1, 516), (1800, 2, 1024)])
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16], ids=IDS)
+def test_gated_norm_of_parts_a_warp_each(n, parts, width, out):
+    from hk_b200.csrc import ops
+    W = parts * width
+    y, z, w = torch.randn(n, W, device="cuda"), torch.randn(n, W + 4, device="cuda") * 4, torch.randn(W, device="cuda")
+    got = torch.full((n + 1, W), float("nan"), dtype=out, device="cuda")
+    ops.gated_part_norm(y, z[:, 4:], w, 1e-5, got[:n], parts)
+    u = (y.double() * torch.nn.functional.silu(z[:, 4:].double())).view(n, parts, width)
+    want = (u / (u.square().mean(-1, keepdim=True) + 1e-5).sqrt()).view(n, W) * w.double()
+    tol = 1e-5 if out == torch.float32 else 5e-3
+    torch.testing.assert_close(got[:n].double(), want, rtol=tol, atol=tol)
+    assert torch.isnan(got[n].float()).all()
+
+
 # ------------------------------------------------------------------------------------ feed-forwards
 
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
