@@ -34,6 +34,7 @@ class FlashPlan:
     first: Optional[torch.Tensor] = None   # per token: first partial, number of partials, row within the item
     count: Optional[torch.Tensor] = None
     row0: Optional[torch.Tensor] = None
+    splits: int = 0              # every request has this many items side by side, one token each (0: as they come)
 
 
 def supported(hd: int, group: int) -> bool:
@@ -62,6 +63,7 @@ class PlanInfo:
     n_items: int
     n_parts: int
     max_keys: int
+    splits: int = 0
 
 
 def decode_splits(n_rows: int, n_kv_heads: int, sm_count: int) -> int:
@@ -174,11 +176,11 @@ def _decode_plan(slots, q_starts, start_positions, n_tokens, window, splits, max
     merge = np.zeros((3, n_tokens), dtype=np.int32)
     merge[0, qrow] = np.arange(B) * splits
     merge[1, qrow] = splits
-    return items.reshape(B * splits, 8), merge, PlanInfo(1, B * splits, B * splits, max_keys)
+    return items.reshape(B * splits, 8), merge, PlanInfo(1, B * splits, B * splits, max_keys, splits)
 
 
 def plan_on_device(info: PlanInfo, items: torch.Tensor, merge: Optional[torch.Tensor]) -> FlashPlan:
-    plan = FlashPlan(info.nw, info.n_items, items, info.n_parts, info.max_keys)
+    plan = FlashPlan(info.nw, info.n_items, items, info.n_parts, info.max_keys, splits=info.splits)
     if info.n_parts:
         plan.first, plan.count, plan.row0 = merge[0], merge[1], merge[2]
     return plan
@@ -224,6 +226,15 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
     lib = build.load("attention_flash")
     stream = ops._stream()
     rows = 16 * plan.nw
+    by_tma = plan.nw == 1 and allow_tma and tma_decode_supported(hd, H // G, int(page_tokens))
+    if by_tma and 2 <= plan.splits <= 8:
+        code = lib.hk_attention_decode_merged(
+            _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table), int(block_table.shape[1]), _ptr(plan.items),
+            plan.n_items, plan.splits, _ptr(out), H, G, hd, int(page_tokens), int(window), scale * math.log2(math.e), sk,
+            plan.max_keys // int(page_tokens) + 2, _ptr(gemm_fast.status_flag(q.device)), *extra, *bias, stream)
+        if code != _UNSUPPORTED:
+            ops._check(code, "paged_attention (decode, splits in a cluster)")
+            return True
     part_o = part_ml = None
     if plan.n_parts:
         part_o = torch.empty((plan.n_parts, G, rows, hd), dtype=torch.float32, device=q.device)
@@ -254,7 +265,7 @@ def run(q, k_pages, v_pages, block_table, out, H, G, hd, page_tokens, window, sc
         ops._check(code, "paged_attention (tcgen05 prefill)")
         return done
     code = _UNSUPPORTED
-    if plan.nw == 1 and allow_tma and tma_decode_supported(hd, H // G, int(page_tokens)):
+    if by_tma:
         code = lib.hk_attention_decode_tma(
             _ptr(q), _ptr(k_pages), _ptr(v_pages), k_pages.shape[0], _ptr(block_table),
             int(block_table.shape[1]), _ptr(plan.items), plan.n_items, _ptr(out), _ptr(part_o), _ptr(part_ml), H, G, hd,
