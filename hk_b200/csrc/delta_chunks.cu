@@ -61,6 +61,9 @@ __device__ __forceinline__ void cp_async16_or_zero(void* dst, const void* src, b
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0)
                : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void fma4(float4& c, float a, float4 b) {
   c.x = fmaf(a, b.x, c.x);
   c.y = fmaf(a, b.y, c.y);
@@ -200,7 +203,8 @@ __device__ __forceinline__ void frag_k(const float* b, int ld, uint32_t (&out)[3
 // ------------------------------------------------------------------ 1. local part with a removal term
 // Bound by the instructions that bring and cut the products' operands (IPC 2.1 of 4, tensor pipe 26 %, shared memory 60 %): 0.9 M
 // multiply-adds a block, the records' two sigmoids and two exponentials an entry, the triangular system.  70 KB of shared memory and 128
-// threads: three blocks share an SM; with 256 threads 396 us instead of 364 (2,048 tokens, 64 heads, with the walk).
+// threads: three blocks share an SM; with 256 threads 396 us instead of 364 (2,048 tokens, 64 heads, with the walk).  A warp has 32 rows
+// by 32 columns of most products, so that what it cuts serves two of them: 16 rows by 64 took 364 us, this 348 (gated: 325 and 316).
 template <bool GATED>
 __global__ void __launch_bounds__(NTH, 3)
 delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __restrict__ mm, float* __restrict__ rq,
@@ -315,39 +319,45 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
   __syncthreads();
 
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-  // ---- the four matrices: rows u, r against columns k, a*u (gated: a*u is a number times k).  A warp has 16 rows: tokens
-  // 16 (warp & 1) .. of u (warps 0 and 1) or r; columns of tokens above its own it leaves out
+  // ---- the four matrices: rows u, r against columns k, a*u (gated: a*u is a number times k).  A warp has the 32 tokens of u or of r
+  // against those of k or of a*u, so that a piece that was cut serves two products (gated: 16 tokens against all of k); columns of
+  // tokens above its own it leaves out
   {
-    constexpr int NC = GATED ? 4 : 8;           // column tiles: 32 tokens of k, then of a*u
-    const int t0 = (warp & 1) * 16;
+    constexpr int MT = GATED ? 1 : 2;           // row tiles of 16
     const bool read = warp >= 2;
-    float big[NC][4] = {}, small[NC][4] = {};
+    const int r0 = read ? CQ : 0, t0 = GATED ? (warp & 1) * 16 : 0, c0 = GATED ? 0 : (warp & 1) * CQ;
+    float big[MT][4][4] = {}, small[MT][4][4] = {};
 #pragma unroll
     for (int k = 0; k < NT / 16; ++k) {
-      uint32_t a[3][4];
-      frag_rows(sm.ur + (warp * 16 + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a);
+      uint32_t a[MT][3][4];
 #pragma unroll
-      for (int n = 0; n < NC; ++n)
-        if ((n & 3) * 8 <= t0 + 15) {
+      for (int m = 0; m < MT; ++m) frag_rows(sm.ur + (r0 + t0 + 16 * m + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a[m]);
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+        if (8 * n <= t0 + 16 * MT - 1) {
           uint32_t b[3][2];
-          frag_columns(sm.ka + (8 * n + g) * LD + k * 16 + 2 * q, b);
-          mma_split(big[n], small[n], a, b);
+          frag_columns(sm.ka + (c0 + 8 * n + g) * LD + k * 16 + 2 * q, b);
+#pragma unroll
+          for (int m = 0; m < MT; ++m)
+            if (8 * n <= t0 + 16 * m + 15) mma_split(big[m][n], small[m][n], a[m], b);
         }
     }
 #pragma unroll
-    for (int n = 0; n < NC; ++n)
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int t = t0 + g + 8 * (e >> 1), s = (n & 3) * 8 + 2 * q + (e & 1);
-        const bool in_tri = (read ? s <= t : s < t) && t < ch.count;
-        float x = in_tri ? big[n][e] + small[n][e] : 0.f;
-        float* dst = sm.a + (warp * 16 + g + 8 * (e >> 1)) * LD + 8 * n + 2 * q + (e & 1);
-        if (GATED) {
-          x *= in_tri ? sm.w[(read ? t : t - 1) * LD + s] : 0.f;
-          dst[CQ] = in_tri ? x * sm.gb[s] : 0.f;
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = t0 + 16 * m + g + 8 * (e >> 1), s = 8 * n + 2 * q + (e & 1);
+          const bool in_tri = (read ? s <= t : s < t) && t < ch.count;
+          float x = in_tri ? big[m][n][e] + small[m][n][e] : 0.f;
+          float* dst = sm.a + (r0 + t) * LD + c0 + s;
+          if (GATED) {
+            x *= in_tri ? sm.w[(read ? t : t - 1) * LD + s] : 0.f;
+            dst[CQ] = in_tri ? x * sm.gb[s] : 0.f;
+          }
+          *dst = x;
         }
-        *dst = x;
-      }
   }
   // (what is not finite would spread through products with zeros: such a chunk takes FMAs that leave out what is above the diagonal)
   bool ordinary = true;
@@ -371,44 +381,52 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
     __syncthreads();
   }
 
-  // ---- [Auk ; Ark] V: into w, and over the k columns of the matrices (Ark V's columns 32 and up where Ark was)
+  // ---- [Auk ; Ark] V: into w, and over the k columns of the matrices (Ark V's columns 32 and up where Ark was).  A warp has the 32
+  // rows of one of the two by half of the columns
+  const bool lower = warp >= 2;
+  const int d0 = (warp & 1) * (NT / 2);
   {
-    const int t0 = (warp & 1) * 16;
-    const bool read = warp >= 2;
-    float big[8][4] = {}, small[8][4] = {};
+    float big[2][4][4] = {}, small[2][4][4] = {};
+    const float* rows = sm.a + (lower ? CQ : 0) * LD;
     if (ordinary) {
 #pragma unroll
       for (int k = 0; k < CQ / 16; ++k) {
-        if (16 * k > t0) break;
-        uint32_t a[3][4];
-        frag_rows(sm.a + (warp * 16 + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a);
+        uint32_t a[2][3][4];
 #pragma unroll
-        for (int n = 0; n < 8; ++n) {
+        for (int m = k; m < 2; ++m) frag_rows(rows + (16 * m + g) * LD + k * 16 + 2 * q, LD, 1.f, 1.f, a[m]);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
           uint32_t b[3][2];
-          frag_k(sm.vs + (k * 16 + 2 * q) * LD + 8 * n + g, LD, b);
-          mma_split(big[n], small[n], a, b);
+          frag_k(sm.vs + (k * 16 + 2 * q) * LD + d0 + 8 * n + g, LD, b);
+#pragma unroll
+          for (int m = k; m < 2; ++m) mma_split(big[m][n], small[m][n], a[m], b);
         }
       }
     } else {
-      for (int s = 0; s < t0 + 16; ++s)
+      for (int s = 0; s < CQ; ++s)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = t0 + g + 8 * (e >> 1);
-          if (read ? s > t : s >= t) continue;
-          const float x = sm.a[(warp * 16 + g + 8 * (e >> 1)) * LD + s];
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int n = 0; n < 8; ++n) big[n][e] = fmaf(x, sm.vs[s * LD + 8 * n + 2 * q + (e & 1)], big[n][e]);
-        }
+          for (int e = 0; e < 4; ++e) {
+            const int t = 16 * m + g + 8 * (e >> 1);
+            if (lower ? s > t : s >= t) continue;
+            const float x = rows[t * LD + s];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) big[m][n][e] = fmaf(x, sm.vs[s * LD + d0 + 8 * n + 2 * q + (e & 1)], big[m][n][e]);
+          }
     }
     __syncthreads();            // everyone has read the k columns of the matrices
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int t = t0 + g + 8 * i, d = 8 * n + 2 * q;
-        float* dst = read ? sm.a + (t + (d >= CQ ? CQ : 0)) * LD + (d & (CQ - 1)) : sm.w + t * LD + d;
-        *reinterpret_cast<float2*>(dst) = make_float2(big[n][2 * i] + small[n][2 * i], big[n][2 * i + 1] + small[n][2 * i + 1]);
-      }
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int t = 16 * m + g + 8 * i, d = d0 + 8 * n + 2 * q;
+          float* dst = lower ? sm.a + (t + (d >= CQ ? CQ : 0)) * LD + (d & (CQ - 1)) : sm.w + t * LD + d;
+          *reinterpret_cast<float2*>(dst) =
+              make_float2(big[m][n][2 * i] + small[m][n][2 * i], big[m][n][2 * i + 1] + small[m][n][2 * i + 1]);
+        }
   }
   __syncthreads();
 
@@ -441,90 +459,98 @@ delta_local_kernel(const DeltaIn in, const Chunk* __restrict__ chunks, float* __
 
   const size_t item = (size_t)c * H + h;
   const int col0 = blockIdx.y * NT, ncols = min(NT, dv - col0);
-  // ---- Rq = R~ - Aru X,  Ov = Ark V - Aru W: a warp has 16 tokens of one of the two
+  // ---- Rq = R~ - Aru X,  Ov = Ark V - Aru W: a warp has the 32 tokens of one of the two by half of the columns
   {
-    const int t0 = (warp & 1) * 16;
-    const bool offset = warp >= 2;
-    const float* xw = offset ? sm.w : sm.ur;
-    float big[8][4] = {}, small[8][4] = {};
+    const float* xw = lower ? sm.w : sm.ur;
+    const float* rows = sm.a + CQ * LD + CQ;
+    float big[2][4][4] = {}, small[2][4][4] = {};
     if (ordinary) {
 #pragma unroll
       for (int k = 0; k < CQ / 16; ++k) {
-        if (16 * k > t0) break;
-        uint32_t a[3][4];
-        frag_rows(sm.a + (CQ + t0 + g) * LD + CQ + k * 16 + 2 * q, LD, -1.f, -1.f, a);
+        uint32_t a[2][3][4];
 #pragma unroll
-        for (int n = 0; n < 8; ++n) {
+        for (int m = k; m < 2; ++m) frag_rows(rows + (16 * m + g) * LD + k * 16 + 2 * q, LD, -1.f, -1.f, a[m]);
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
           uint32_t b[3][2];
-          frag_k(xw + (k * 16 + 2 * q) * LD + 8 * n + g, LD, b);
-          mma_split(big[n], small[n], a, b);
+          frag_k(xw + (k * 16 + 2 * q) * LD + d0 + 8 * n + g, LD, b);
+#pragma unroll
+          for (int m = k; m < 2; ++m) mma_split(big[m][n], small[m][n], a[m], b);
         }
       }
     } else {
-      for (int s = 0; s < t0 + 16; ++s)
+      for (int s = 0; s < CQ; ++s)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int t = t0 + g + 8 * (e >> 1);
-          if (s > t) continue;
-          const float x = -sm.a[(CQ + t) * LD + CQ + s];
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-          for (int n = 0; n < 8; ++n) big[n][e] = fmaf(x, xw[s * LD + 8 * n + 2 * q + (e & 1)], big[n][e]);
-        }
+          for (int e = 0; e < 4; ++e) {
+            const int t = 16 * m + g + 8 * (e >> 1);
+            if (s > t) continue;
+            const float x = -rows[t * LD + s];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) big[m][n][e] = fmaf(x, xw[s * LD + d0 + 8 * n + 2 * q + (e & 1)], big[m][n][e]);
+          }
     }
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int t = t0 + g + 8 * i, d = 8 * n + 2 * q;
-        const float2 onto = *reinterpret_cast<const float2*>(offset ? sm.a + (t + (d >= CQ ? CQ : 0)) * LD + (d & (CQ - 1)) : sm.ur + (CQ + t) * LD + d);
-        const float2 y = make_float2(onto.x + (big[n][2 * i] + small[n][2 * i]), onto.y + (big[n][2 * i + 1] + small[n][2 * i + 1]));
-        if (!offset) {
-          if (blockIdx.y == 0) *reinterpret_cast<float2*>(rq + (item * CQ + t) * NT + d) = y;
-        } else if (t < ch.count && d < ncols) {
-          *reinterpret_cast<float2*>(out + ((size_t)(ch.row0 + t) * H + h) * dv + col0 + d) = y;
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int t = 16 * m + g + 8 * i, d = d0 + 8 * n + 2 * q;
+          const float2 onto = *reinterpret_cast<const float2*>(lower ? sm.a + (t + (d >= CQ ? CQ : 0)) * LD + (d & (CQ - 1)) : sm.ur + (CQ + t) * LD + d);
+          const float2 y = make_float2(onto.x + (big[m][n][2 * i] + small[m][n][2 * i]), onto.y + (big[m][n][2 * i + 1] + small[m][n][2 * i + 1]));
+          if (!lower) {
+            if (blockIdx.y == 0) *reinterpret_cast<float2*>(rq + (item * CQ + t) * NT + d) = y;
+          } else if (t < ch.count && d < ncols) {
+            *reinterpret_cast<float2*>(out + ((size_t)(ch.row0 + t) * H + h) * dv + col0 + d) = y;
+          }
         }
-      }
   }
-  // ---- M = -AU'^T X and P,  B = K'^T V - AU'^T W: a warp has 16 rows
+  // ---- M = -AU'^T X and P,  B = K'^T V - AU'^T W: a warp has 32 rows by half of the columns
   {
-    const int row = warp * 16 + g;
-    uint32_t kk[CQ / 16][3][4], au[CQ / 16][3][4];
+    const int row0 = (warp >> 1) * 32 + g;
+    uint32_t kk[2][CQ / 16][3][4], au[2][CQ / 16][3][4];
 #pragma unroll
-    for (int k = 0; k < CQ / 16; ++k) {
-      frag_turned(sm.ka + (k * 16 + 2 * q) * LD + row, LD, 1.f, kk[k]);
-      frag_turned(sm.ka + (CQ + k * 16 + 2 * q) * LD + row, LD, -1.f, au[k]);
-    }
-    const float p0 = GATED ? sm.from[CQ - 1] : sm.pc[row], p1 = GATED ? sm.from[CQ - 1] : sm.pc[row + 8];
-#pragma unroll 2
-    for (int n = 0; n < 8; ++n) {
-      float mb[4] = {}, ms[4] = {}, vb[4] = {}, vsm[4] = {};
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
       for (int k = 0; k < CQ / 16; ++k) {
-        const int at = (k * 16 + 2 * q) * LD + 8 * n + g;
+        frag_turned(sm.ka + (k * 16 + 2 * q) * LD + row0 + 16 * m, LD, 1.f, kk[m][k]);
+        frag_turned(sm.ka + (CQ + k * 16 + 2 * q) * LD + row0 + 16 * m, LD, -1.f, au[m][k]);
+      }
+#pragma unroll 1
+    for (int n = 0; n < 4; ++n) {
+      float mb[2][4] = {}, ms[2][4] = {}, vb[2][4] = {}, vsm[2][4] = {};
+#pragma unroll
+      for (int k = 0; k < CQ / 16; ++k) {
+        const int at = (k * 16 + 2 * q) * LD + d0 + 8 * n + g;
         uint32_t b[3][2];
         frag_k(sm.ur + at, LD, b);
-        mma_split(mb, ms, au[k], b);
-        frag_k(sm.vs + at, LD, b);
-        mma_split(vb, vsm, kk[k], b);
-        frag_k(sm.w + at, LD, b);
-        mma_split(vb, vsm, au[k], b);
-      }
-      const int d = 8 * n + 2 * q;
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const float f = GATED ? 1.f : i ? p1 : p0;
-        if (blockIdx.y == 0)
-          *reinterpret_cast<float2*>(mm + item * MFLOATS + (row + 8 * i) * NT + d) =
-              make_float2((mb[2 * i] + ms[2 * i]) * f, (mb[2 * i + 1] + ms[2 * i + 1]) * f);
-        if (row + 8 * i < dk && d < ncols)
-          *reinterpret_cast<float2*>(bb + (item * dk + row + 8 * i) * dv + col0 + d) =
-              make_float2((vb[2 * i] + vsm[2 * i]) * f, (vb[2 * i + 1] + vsm[2 * i + 1]) * f);
+        for (int m = 0; m < 2; ++m) mma_split(mb[m], ms[m], au[m][k], b);
+        frag_k(sm.vs + at, LD, b);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) mma_split(vb[m], vsm[m], kk[m][k], b);
+        frag_k(sm.w + at, LD, b);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) mma_split(vb[m], vsm[m], au[m][k], b);
       }
+      const int d = d0 + 8 * n + 2 * q;
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int row = row0 + 16 * m + 8 * i;
+          const float f = GATED ? 1.f : sm.pc[row];
+          if (blockIdx.y == 0)
+            *reinterpret_cast<float2*>(mm + item * MFLOATS + row * NT + d) =
+                make_float2((mb[m][2 * i] + ms[m][2 * i]) * f, (mb[m][2 * i + 1] + ms[m][2 * i + 1]) * f);
+          if (row < dk && d < ncols)
+            *reinterpret_cast<float2*>(bb + (item * dk + row) * dv + col0 + d) =
+                make_float2((vb[m][2 * i] + vsm[m][2 * i]) * f, (vb[m][2 * i + 1] + vsm[m][2 * i + 1]) * f);
+        }
     }
-    if (blockIdx.y == 0 && q == 0) {
-      mm[item * MFLOATS + NT * NT + row] = p0;
-      mm[item * MFLOATS + NT * NT + row + 8] = p1;
-    }
+    if (blockIdx.y == 0 && tid < NT) mm[item * MFLOATS + NT * NT + tid] = GATED ? sm.from[CQ - 1] : sm.pc[tid];
   }
 }
 
@@ -856,7 +882,8 @@ decay_out_kernel(const DecayIn in, const Chunk* __restrict__ chunks, const float
 // of [M ; Rq].  The four warps of M keep S in float32 registers (the tensor core's result layout) and leave its pieces in shared memory, two copies in
 // turn, for all six; what a chunk brings comes through a ring, a chunk ahead.
 // One request of 2,048 tokens at 64 heads of 64 x 64: 173 us with multiply-adds (7 wide loads of shared memory for 24 pairs of them were
-// the bound), 117 here (issue slots 53 %, tensor pipe 32 %: the pieces again).
+// the bound), 117 with the pieces, 107 here, where a chunk's copies take one address a round of rows (issue slots 53 % before that,
+// tensor pipe 32 %: the pieces again).
 namespace {
 template <int DVS>
 struct WalkShape {
@@ -884,21 +911,31 @@ chunk_walk_kernel(const Request* __restrict__ requests, const Chunk* __restrict_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
   float* sp = state + ((size_t)r.slot * H + h) * dk * dv;
   const int row0 = chunks[r.chunk0].row0, rows = CQ * (r.chunks - 1) + chunks[r.chunk0 + r.chunks - 1].count;
+  // a chunk's copies, chunk after chunk: a thread has the same columns of rows that lie a fixed number apart
+  constexpr int RM = K::THREADS / (NT / 4), RB = K::THREADS / (DVS / 4);
+  static_assert(K::ROWS % RM == 0 && K::ROWS % RB == 0, "whole rounds of rows");
+  const int mr = tid / (NT / 4), br = tid / (DVS / 4), bd = (tid % (DVS / 4)) * 4;
+  const float* mp = mm + ((size_t)r.chunk0 * H + h) * MFLOATS + tid * 4;
+  const float* qp = rq + ((size_t)r.chunk0 * H + h) * CQ * NT + tid * 4;
+  const float* bp = bb + (((size_t)r.chunk0 * H + h) * dk + br) * dv + col0 + bd;
+  const float* op = out + ((size_t)row0 * H + h) * dv + col0 + bd;
+  const bool bcol = col0 + bd < dv;
   auto fetch = [&](int c) {
     float* st = ws + (c % K::STAGES) * K::STAGE;
-    const size_t item = (size_t)(r.chunk0 + c) * H + h;
-    const float *m = mm + item * MFLOATS, *rqp = rq + item * CQ * NT;
-    for (int e = tid; e < K::ROWS * (NT / 4); e += K::THREADS) {
-      const int row = e / (NT / 4), i = (e % (NT / 4)) * 4;
-      cp_async16_or_zero(st + row * K::LM + i, row < NT ? m + e * 4 : rqp + e * 4 - NT * NT, true);
+#pragma unroll
+    for (int j = 0; j < K::ROWS / RM; ++j)
+      cp_async16(st + (mr + j * RM) * K::LM + (tid % (NT / 4)) * 4, mr + j * RM < NT ? mp + j * K::THREADS * 4 : qp + j * K::THREADS * 4 - NT * NT);
+    if (tid < NT / 4) cp_async16(st + K::P + 4 * tid, mp + NT * NT);
+#pragma unroll
+    for (int j = 0; j < K::ROWS / RB; ++j) {
+      const int row = br + j * RB, t = c * CQ + row - NT;
+      const bool in = bcol && (row < NT ? row < dk : t < rows);
+      const float* src = row < NT ? bp + (size_t)(j * RB) * dv : op + (ptrdiff_t)t * H * dv;
+      cp_async16_or_zero(st + K::OFF + row * K::LO + bd, in ? src : bb, in);
     }
-    if (tid < NT / 4) cp_async16_or_zero(st + K::P + 4 * tid, m + NT * NT + 4 * tid, true);
-    for (int e = tid; e < K::ROWS * (DVS / 4); e += K::THREADS) {
-      const int row = e / (DVS / 4), d = (e % (DVS / 4)) * 4, t = c * CQ + row - NT;
-      const bool in = col0 + d < dv && (row < NT ? row < dk : t < rows);
-      const float* src = row < NT ? bb + (item * dk + row) * dv : out + ((size_t)(row0 + t) * H + h) * dv;
-      cp_async16_or_zero(st + K::OFF + row * K::LO + d, in ? src + col0 + d : bb, in);
-    }
+    mp += (size_t)H * MFLOATS;
+    qp += (size_t)H * CQ * NT;
+    bp += (size_t)H * dk * dv;
   };
 #pragma unroll
   for (int c = 0; c < K::STAGES - 1; ++c) {
