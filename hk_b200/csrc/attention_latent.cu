@@ -657,8 +657,10 @@ HK_API int hk_attention_latent_rows() { return ROWS; }
 // Where keys and values are made for a step, a value is rounded to bf16 before the attention's sum, not behind it.  The sums over
 // few keys are the largest (a prompt's first rows hold a third of its results' energy), so the first FIRST_ROWS positions of a
 // request are taken here again with values that are never rounded: out = W_uv,h (sum_j p_j c_j) [* gate], all in float32 behind
-// the scores.  A block per (head, request, 32 value dims), everything it reads staged in shared memory; 26 us at 32 heads.  Relative
-// error of a 2,048-token prompt through the mixer: 3.34e-3 in the latent space, 3.45e-3 without this, 3.19e-3 with it.
+// the scores.  A block per (head, request, 32 value dims), everything it reads asked for at once; bound by the latency of its four
+// steps, and starts under the attention's last blocks, whose rows it writes over once they are there: the pass of a 2,048-token prompt
+// at 32 heads 365 -> 346 us (27 of them were this kernel's, a row of weights a lane).  Relative error of a 2,048-token prompt through
+// the mixer: 3.34e-3 in the latent space, 3.45e-3 without this, 3.19e-3 with it.
 constexpr int FIRST_ROWS = 16;
 
 struct FirstRows {
@@ -673,6 +675,8 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
   constexpr int LDQ = 192 + 8;                          // 16-byte pieces of neighbouring rows lie in different banks
   __shared__ __align__(16) bf16 qs[FIRST_ROWS][LDQ], ks[FIRST_ROWS][LDQ];
   __shared__ float prob[FIRST_ROWS][FIRST_ROWS];
+  constexpr int WARPS = 8;
+  __shared__ float sums[WARPS][FIRST_ROWS][33];
   const int h = blockIdx.x, d0 = blockIdx.z * 32, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ldl = r + 4, ldc = r + 8;
   bf16* cs = reinterpret_cast<bf16*>(lat + FIRST_ROWS * ldl);
   const FirstRows f = firsts[blockIdx.y];
@@ -680,6 +684,12 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
   // would stand among the made rows another request stands, or nothing (row0 is then negative)
   const int wide = 128 + dr, last = f.pos0 + f.count, first = window > 0 ? max(0, f.pos0 - window + 1) : 0;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  // a lane's value dim, every WARPS-th piece of its weights: the first eight pieces come along with the rows
+  const int pieces = r / 8;
+  const uint4* wp = reinterpret_cast<const uint4*>(w_uv + ((size_t)h * 128 + d0 + lane) * r);
+  uint4 w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) w[j] = warp + WARPS * j < pieces ? wp[warp + WARPS * j] : zero;
   for (int e = tid; e < FIRST_ROWS * 24; e += 256) {
     const int i = e / 24, p = (e % 24) * 8;
     const bool q_in = i < f.count && p < wide;
@@ -746,25 +756,36 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
     *reinterpret_cast<float4*>(lat + i * ldl + p + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
   }
   __syncthreads();
-  const int d = d0 + lane, i0 = warp * 2;               // a lane per value dim, a warp per two rows
-  const uint4* wp = reinterpret_cast<const uint4*>(w_uv + ((size_t)h * 128 + d) * r);
-  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll 8
-  for (int k = 0; k < r; k += 8) {
-    float w[8];
-    halves(wp[k >> 3], w);
+  float acc[FIRST_ROWS] = {};
+  for (int p0 = warp; p0 < pieces; p0 += 8 * WARPS) {
+    if (p0 != warp)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float4 x = *reinterpret_cast<const float4*>(lat + (i0 + i) * ldl + k), y = *reinterpret_cast<const float4*>(lat + (i0 + i) * ldl + k + 4);
-      acc[i][0] = fmaf(w[6], y.z, fmaf(w[4], y.x, fmaf(w[2], x.z, fmaf(w[0], x.x, acc[i][0]))));
-      acc[i][1] = fmaf(w[7], y.w, fmaf(w[5], y.y, fmaf(w[3], x.w, fmaf(w[1], x.y, acc[i][1]))));
+      for (int j = 0; j < 8; ++j) w[j] = p0 + WARPS * j < pieces ? wp[p0 + WARPS * j] : zero;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = (p0 + WARPS * j) * 8;
+      if (k >= r) break;
+      float f[8];
+      halves(w[j], f);
+#pragma unroll
+      for (int i = 0; i < FIRST_ROWS; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(lat + i * ldl + k), y = *reinterpret_cast<const float4*>(lat + i * ldl + k + 4);
+        const float even = fmaf(f[6], y.z, fmaf(f[4], y.x, fmaf(f[2], x.z, f[0] * x.x)));
+        const float odd = fmaf(f[7], y.w, fmaf(f[5], y.y, fmaf(f[3], x.w, f[1] * x.y)));
+        acc[i] += even + odd;
+      }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    if (i0 + i >= f.count) continue;
-    const size_t row = (size_t)f.q_row + i0 + i;
-    float y = acc[i][0] + acc[i][1];
+  for (int i = 0; i < FIRST_ROWS; ++i) sums[warp][i][lane] = acc[i];
+  __syncthreads();
+  pdl_wait();                 // the attention's rows are written: these take their place
+  for (int i = warp; i < f.count; i += WARPS) {
+    const int d = d0 + lane;
+    const size_t row = (size_t)f.q_row + i;
+    float y = 0.f;
+#pragma unroll
+    for (int k = 0; k < WARPS; ++k) y += sums[k][i][lane];
     if (gate) y *= gate_scale / (1.0f + expf(-gate[row * gate_ld + (gate_heads ? h : h * 128 + d)]));
     out[(row * H + h) * 128 + d] = __float2bfloat16_rn(y);
   }
@@ -785,7 +806,7 @@ HK_API int hk_latent_first_rows(const void* q, const void* kv, const void* rope,
   if (smem > 200 * 1024) return HK_ERR_UNSUPPORTED;
   static HkSmemCache cache;
   if (int e = hk_allow_smem(latent_first_rows_kernel, smem, cache)) return e;
-  return hk_launch(latent_first_rows_kernel, dim3((unsigned)H, (unsigned)n_firsts, 4), dim3(256), smem, (cudaStream_t)stream, (const bf16*)q,
+  return hk_launch_pdl(latent_first_rows_kernel, dim3((unsigned)H, (unsigned)n_firsts, 4), dim3(256), smem, (cudaStream_t)stream, (const bf16*)q,
                    (const bf16*)kv, (const bf16*)rope, (const bf16*)c, (const bf16*)w_uv, (const FirstRows*)firsts, (bf16*)out, H, dr, r, window,
                    scale_log2, gate, gate_ld, gate_heads, gate_scale);
 }

@@ -697,6 +697,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   Smem2<HD, HDK>& sm = *reinterpret_cast<Smem2<HD, HDK>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   volatile int* abort_flag = &sm.abort_flag;
 
+  if (MADE) pdl_launch_dependents();     // the request's first rows are taken again beside this kernel's last blocks
   const Item it = items[blockIdx.x / G];
   const int g = blockIdx.x % G;
   const int group = H / G;

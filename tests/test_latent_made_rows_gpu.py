@@ -162,3 +162,14 @@ def test_sizes_that_the_host_shares_with_the_kernels():
     assert made.hk_attention_made_tile() == attention_fast.MADE_TILE and made.hk_attention_made_tokens() == attention_fast.MADE_TOKENS
     assert first.hk_latent_first_rows_count() == attention_fast.MADE_FIRST
     assert [runs.hk_attention_f32_tokens(g) for g in (1, 3, 32, 33)] == [ops.RUN_ROWS, ops.RUN_ROWS // 3, 1, 0]
+
+
+@pytest.mark.parametrize("rank", [8, 72, 520, 1000])
+def test_first_rows_of_any_rank(rank, monkeypatch):
+    """Fewer pieces of a latent row than the block has warps, a number that does not divide, more than come along with the rows."""
+    from hk_b200.csrc import attention_fast
+    monkeypatch.setitem(made_case.__globals__, "R", rank)
+    got, want, pos = made_case([(0, 70), (3, 40)], 0, tiled, tile=128)
+    scale, early = float(want.abs().max()), pos < attention_fast.MADE_FIRST
+    assert bool(torch.isfinite(got).all()) and float((got - want).abs().max()) <= 3e-2 * scale
+    assert bool(((got - want).abs()[early] <= 2.0 ** -8 * want.abs()[early] + 1e-4 * scale).all())
