@@ -104,20 +104,24 @@ class _SegmentScan(Part):
 class _ChunkedScan(_SegmentScan):
     """A recurrence that, when serving in bfloat16, walks the requests of a step in chunks of tokens (`csrc/delta_chunks.cu`)
     where a long one sets the time of the walk token by token; the lists of requests and chunks are host-built tables that the
-    mixers with as many heads share.
+    mixers of a kind with heads as many and as large share.
 
-    A walk's time grows with the longest request until requests times heads fill the SMs; the chunks' with all rows.  So a step
+    A walk's time grows with the longest request until requests times heads fill the SMs; the chunks' with all rows.  From
+    `CHUNKS_FROM` tokens on the chunks' kernels are the faster at every size (one request of 64 tokens 20 us against 26 to 34, one
+    of 512 over 64 heads 97 and 248, nine of 227 336 and 369, sixteen of 128 311 and 395), but their launches and tables cost the
+    host 10 to 25 us, and 3 more for each request, which a step that waits for the host anyway only loses.  So a step
     takes chunks when its longest request brings `LONGEST_FROM` tokens (half that with many heads: tokens times heads at least
-    `ROWS_FROM`) and all rows to be chunked times the heads are at most
-    `BESIDE` times the longest; then every request of `CHUNKS_FROM` tokens or more goes that way.  Scan kernels of the delta
-    rule with 64 heads, us in chunks and walked: one request of 2,048 tokens 433 and 988, one of 512 130 and 257, four of 512
-    433 and 587, nine of 227 484 and 384 (over the limit: walked); with 32 heads one of 512 85 and 206, nine of 100 146 and 132.
-    Below, the kernels still gain (one request of 512 tokens over 32 heads, see above), but the launches and tables of the longer
-    route cost the host as much: requests of 34 and 471 tokens took 288 us walked and 309 with the longer one in chunks."""
+    `ROWS_FROM`) and all rows to be chunked times the heads are at most `BESIDE` times the longest; or else when the walk is
+    estimated at more than 210 us less about one a head, with 6 more for each further request (by then the device has more to do than
+    the host), and at 20 more than the chunks.  Layers 4,096 and 2,048 wide, us walked and in chunks: delta rule, requests of 300,
+    120, 90 and 14 tokens 384 and 299 (64 heads), 316 and 298 (32); nine of 227 434 and 352 (32 heads); matrix memory 399 and 285,
+    423 and 331; the other way: sixteen of 128 over 16 heads 345 and 379, four of 300 to 14 over 16 255 and 291."""
     CHUNKS_FROM = 64
     LONGEST_FROM = 640
     ROWS_FROM = 320 * 64
     BESIDE = 256
+    WALK = 1.0                      # the walk's time in the delta rule's
+    CHUNK_NS = 2.4                  # a row's time in chunks, by head
     _chunks = False                 # set at bind: the chunked form takes this mixer's sizes
 
     def kernel_libraries(self, bfloat16: bool):
@@ -128,7 +132,24 @@ class _ChunkedScan(_SegmentScan):
         self._chunks = precision.compute == torch.bfloat16 and row % 4 == 0 and ops.delta_chunks_take(self.dk, self.dv, decay_scale)
 
     def step_tables_key(self):
-        return ("chunked_segments", self.H) if self._chunks else SEGMENTS_KEY
+        return ("chunked_segments", self.H, self.dk, self.dv, self.WALK) if self._chunks else SEGMENTS_KEY
+
+    def _chunks_pay(self, lengths) -> bool:
+        """Whether a step takes chunks for requests of these numbers of tokens, each `CHUNKS_FROM` or more."""
+        longest, rows, H = max(lengths), sum(lengths), self.H
+        worth = longest >= self.LONGEST_FROM or (2 * longest >= self.LONGEST_FROM and longest * H >= self.ROWS_FROM)
+        if worth and rows <= max(1, self.BESIDE // H) * longest:
+            return True
+        # the walk, while its requests end one after the other: us a token by how many pairs of a request and a head there are (from 74
+        # on a thread block has more than the fewest columns of a state), fitted at heads of 64 by 64; smaller ones are as long in chunks
+        # and shorter walked
+        heads = H * -(-self.dv // 64)
+        walk, done, pairs = 0.0, 0, len(lengths) * heads
+        for n in sorted(lengths):
+            walk += (n - done) * (0.3 + 0.0028 * pairs if pairs < 74 else max(1.06, 0.003 * pairs))
+            done, pairs = n, pairs - heads
+        walk *= self.WALK * min(self.dk, 64) * min(self.dv, 64) / 4096
+        return walk > 210 - 0.94 * min(heads, 64) + 6 * (len(lengths) - 1) and walk > 40 + self.CHUNK_NS * 1e-3 * rows * heads
 
     def step_tables(self, ctx):
         tables = segment_tables(ctx)
@@ -136,9 +157,8 @@ class _ChunkedScan(_SegmentScan):
             return tables
         seg = tables.arrays["segments"]
         long = seg[:, 2] >= self.CHUNKS_FROM
-        longest = int(seg[:, 2].max(initial=0))
-        worth = longest >= self.LONGEST_FROM or (2 * longest >= self.LONGEST_FROM and longest * self.H >= self.ROWS_FROM)
-        if not worth or int(seg[long, 2].sum()) > max(1, self.BESIDE // self.H) * longest:
+        lengths = seg[long, 2].tolist()
+        if not lengths or not self._chunks_pay(lengths):
             long[:] = False
         chunks, requests = [], []
         for slot, row, count in seg[long].tolist():
@@ -268,6 +288,8 @@ class GatedDeltaRule(_ChunkedScan):
     def kernel_libraries(self, bfloat16: bool):
         return super().kernel_libraries(bfloat16) + ("short_conv",)
 
+    CHUNK_NS = 2.1
+
     def __init__(self, hidden: int, n_heads: int, kv_heads: int, key_dim: int, value_dim: int, taps: int, prefix: str,
                  norm_eps: float, unit_eps: float = 1e-6, q_scale: Optional[float] = None, out_scale: float = 1.0,
                  names: Optional[Dict[str, str]] = None):
@@ -339,6 +361,8 @@ class GatedDeltaRule(_ChunkedScan):
 
 
 class Retention(_ChunkedScan):
+    WALK, CHUNK_NS = 0.55, 1.4
+
     def __init__(self, hidden: int, n_heads: int, key_dim: int, value_dim: int, decay, prefix: str, norm_eps: float,
                  position=None, k_scale: Optional[float] = None, names: Optional[Dict[str, str]] = None):
         decay = [float(x) for x in decay]
@@ -603,6 +627,8 @@ class GatedLinearAttention(_SegmentScan):
 
 
 class MLSTM(_ChunkedScan):
+    WALK, CHUNK_NS = 1.25, 1.4
+
     def __init__(self, hidden: int, n_heads: int, key_dim: int, value_dim: int, gate_cap: float, prefix: str, norm_eps: float,
                  den_eps: float = 1e-6, q_scale: Optional[float] = None, names: Optional[Dict[str, str]] = None):
         if not gate_cap > 0:
