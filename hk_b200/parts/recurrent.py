@@ -120,7 +120,7 @@ class _ChunkedScan(_SegmentScan):
     LONGEST_FROM = 640
     ROWS_FROM = 320 * 64
     BESIDE = 256
-    WALK = 1.0                      # the walk's time in the delta rule's
+    WALK = 0.0                      # a kind's walk time in the delta rule's (0: not measured; the first of the two lines alone)
     CHUNK_NS = 2.4                  # a row's time in chunks, by head
     _chunks = False                 # set at bind: the chunked form takes this mixer's sizes
 
@@ -140,6 +140,8 @@ class _ChunkedScan(_SegmentScan):
         worth = longest >= self.LONGEST_FROM or (2 * longest >= self.LONGEST_FROM and longest * H >= self.ROWS_FROM)
         if worth and rows <= max(1, self.BESIDE // H) * longest:
             return True
+        if not self.WALK:
+            return False
         # the walk, while its requests end one after the other: us a token by how many pairs of a request and a head there are (from 74
         # on a thread block has more than the fewest columns of a state), fitted at heads of 64 by 64; smaller ones are as long in chunks
         # and shorter walked
@@ -183,6 +185,8 @@ class _ChunkedScan(_SegmentScan):
 
 
 class GeneralDeltaRule(_ChunkedScan):
+    WALK = 1.0
+
     def __init__(self, hidden: int, n_heads: int, key_dim: int, prefix: str, norm_eps: float,
                  value_dim: Optional[int] = None, decay_rank: Optional[int] = None,
                  decay_scale: float = math.exp(-0.5), key_eps: float = 1e-6, names: Optional[Dict[str, str]] = None):
@@ -285,10 +289,10 @@ class MinGRU(_SegmentScan):
 
 
 class GatedDeltaRule(_ChunkedScan):
+    WALK, CHUNK_NS = 1.0, 2.1
+
     def kernel_libraries(self, bfloat16: bool):
         return super().kernel_libraries(bfloat16) + ("short_conv",)
-
-    CHUNK_NS = 2.1
 
     def __init__(self, hidden: int, n_heads: int, kv_heads: int, key_dim: int, value_dim: int, taps: int, prefix: str,
                  norm_eps: float, unit_eps: float = 1e-6, q_scale: Optional[float] = None, out_scale: float = 1.0,
