@@ -318,6 +318,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
       }
       pdl_launch_dependents();
+      // A stage's release is a signal of the tensor core to both CTAs that no thread orders: a CTA may not leave, nor its shared memory
+      // go to another block, before the last ones have come.
+      for (int i = issued > stages ? issued - stages : 0; i < issued && ok; ++i)
+        ok = pair_wait(&sm.empty[i % stages], (uint32_t)(i / stages) & 1u, abort_flag, other);
       if (*abort_flag && rank == 0) {       // giving up: let the copies that are still on their way land
         for (int i = issued > stages ? issued - stages : 0; i < issued; ++i)
           for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin)

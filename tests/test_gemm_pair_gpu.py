@@ -109,3 +109,26 @@ def test_pair_product_by_group(counts, N, K, tile_rows, epilogue):
     assert bool(((got - want).abs() <= bound).all())
     assert bool((guard[M:] == 5.0).all())
     assert float((got - want).norm() / want.norm()) < (1e-5 if epilogue == 0 else 3e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("blocks", [1, 6, 7, 8, 11, 12, 13, 25])
+def test_pair_products_one_after_the_other(blocks):
+    """K blocks below, at and beyond what the rings hold (12 stages at 32 rows, 7 at 256): the last releases of a launch must have come
+    before its blocks leave, or they would strike the barriers of the next one's, whose rings lie elsewhere."""
+    from hk_b200.csrc import gemm_fast
+    gen = torch.Generator("cuda").manual_seed(blocks)
+    w = torch.randn(74 * 256 + 256, blocks * 64, generator=gen, device="cuda").bfloat16()
+    cases = []
+    for rows, columns in ((256, 1024), (32, 256), (200, w.shape[0]), (96, 2048)):
+        a = torch.randn(rows, w.shape[1], generator=gen, device="cuda").bfloat16()
+        cases.append((a, w[:columns], torch.empty(rows, columns, device="cuda"), (a.double() @ w[:columns].double().T)))
+    for turn in range(40):
+        for a, wc, out, _ in cases:
+            assert gemm_fast.run_pair(a, wc, out, 0, out.shape[1], 1, 1)
+        if turn % 13 == 0:
+            for a, wc, out, want in cases:        # K exact products of bf16 summed in 32 bits, cut at most twice as far as rounded
+                bound = (a.double().abs() @ wc.double().abs().T) * (blocks * 64 + 1) * 2 ** -23
+                assert bool(((out.double() - want).abs() <= bound).all())
+                out.fill_(float("nan"))
+    gemm_fast.check_status(w.device)
