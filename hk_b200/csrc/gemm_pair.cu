@@ -100,6 +100,7 @@ struct PairControl {
   uint64_t tmem_full[2], tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
+  int filled_by_other;          // in the first CTA: how many stages the second one has filled in all (-1: it has not said)
 };
 static_assert(sizeof(PairControl) <= PAIR_CONTROL, "control block too large");
 
@@ -112,11 +113,28 @@ __device__ __forceinline__ void pair_sync() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
+__device__ __forceinline__ void put_in_cta(const volatile int* at, uint32_t rank, int value) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_u32((const void*)at), rank)), "r"(value) : "memory");
+}
 // A wait that gives up tells the other CTA too.
 __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t other) {
   if (mbar_wait(bar, parity, abort_flag)) return true;
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(in_cta(smem_u32((const void*)abort_flag), other)), "r"(1) : "memory");
+  put_in_cta(abort_flag, other, 1);
   return false;
+}
+// Giving up, in the first CTA, where all copies are counted: lets those that are still on their way land, in both CTAs.  The two may
+// have stopped at different stages: what the other one brought alone is still to be expected, what it did not bring counts as there.
+__device__ __forceinline__ void let_copies_land(PairControl& sm, int mine, int stages, uint32_t bytes) {
+  const volatile int* said = &sm.filled_by_other;
+  for (uint32_t spin = 0; spin < WAIT_LIMIT && *said < 0; ++spin) {}
+  const int others = max(*said, 0), most = max(mine, others);
+  for (int i = max(most - stages, 0); i < most; ++i) {
+    uint64_t* full = &sm.full[i % stages];
+    if (i >= mine) mbar_expect_tx(full, bytes);
+    if (i >= others) asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(full)), "r"(bytes) : "memory");
+    for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin)
+      if (mbar_try_wait(full, (uint32_t)(i / stages) & 1u)) break;
+  }
 }
 // Copies into this CTA that complete on a barrier of either CTA of the pair.
 __device__ __forceinline__ void pair_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
@@ -272,6 +290,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       mbar_init(&sm.tmem_empty[b], 16);
     }
     sm.abort_flag = 0;
+    sm.filled_by_other = -1;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -318,15 +337,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
       }
       pdl_launch_dependents();
+      if (rank == 1) put_in_cta(&sm.filled_by_other, 0, issued);
       // A stage's release is a signal of the tensor core to both CTAs that no thread orders: a CTA may not leave, nor its shared memory
       // go to another block, before the last ones have come.
       for (int i = issued > stages ? issued - stages : 0; i < issued && ok; ++i)
         ok = pair_wait(&sm.empty[i % stages], (uint32_t)(i / stages) & 1u, abort_flag, other);
-      if (*abort_flag && rank == 0) {       // giving up: let the copies that are still on their way land
-        for (int i = issued > stages ? issued - stages : 0; i < issued; ++i)
-          for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin)
-            if (mbar_try_wait(&sm.full[i % stages], (uint32_t)(i / stages) & 1u)) break;
-      }
+      if (*abort_flag && rank == 0) let_copies_land(sm, issued, stages, stage_bytes);
     }
   } else if (warp == 1) {
     if (rank == 0 && elect_one()) {
