@@ -886,15 +886,18 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     }
 #pragma unroll
     for (int s = 0; s < 8; ++s) mx = fmaxf(mx, pm[s]);
-    float acc = 0.f, lsum = 0.f;
+    float acc = 0.f;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
       const float f = pm[s] == -CUDART_INF_F ? 0.f : exp2f(pm[s] - mx);
-      acc = fmaf(po[s], f, acc);
-      lsum = fmaf(pl[s], f, lsum);
+      if (s < splits) acc = fmaf(po[s], f, acc);
+      pl[s] *= f;
     }
+    // (the sums in pairs, as attention_combine_kernel's lanes add them: both give the same bits)
+    float lsum = ((pl[0] + pl[4]) + (pl[2] + pl[6])) + ((pl[1] + pl[5]) + (pl[3] + pl[7]));
     if (so.sink && mx > -CUDART_INF_F) lsum += exp2f(sink_log2(so, g * group + r % group) - mx);
-    out[((size_t)(it.q_row0 + r / group) * H + g * group + r % group) * HD + d] = __float2bfloat16_rn(lsum > 0.f ? acc * (1.0f / lsum) : 0.f);
+    const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
+    out[((size_t)(it.q_row0 + r / group) * H + g * group + r % group) * HD + d] = __float2bfloat16_rn(acc * inv);
   }
   cluster_sync();      // nobody leaves while its shared memory is read
 }
