@@ -48,8 +48,7 @@ struct Request {
   int slot, chunk0, chunks;
 };
 
-// (the division without the branch for unusual operands: the denominator is 1 or more, and above 2^126 the result 0)
-__device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.0f, 1.0f + expf(-x)); }
+__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }

@@ -28,18 +28,21 @@ __device__ __forceinline__ bf16 squared_relu(float z, GluParams gp) {
   const float r = fmaxf(z, 0.f);
   return __float2bfloat16_rn(gp.slope * (r * r));
 }
-// (__fdividef: what a plain division adds is a branch for unusual operands, and a gate of 0, which every row that fills a tile up
-// has, is one: 100 rows by 12,288 x 2,048 took 20 us, 128 rows 15.  It gives 0 where the denominator is above 2^126, a result below
-// 1.1e-36 u.)
+// x / d, d at least 1, rounded as the plain division rounds.  A zero, which every row that fills a tile up has for a gate, would take
+// the division's branch for unusual operands: 100 rows by 12,288 x 2,048 took 20 us, 128 rows 15.
+__device__ __forceinline__ float over(float x, float d) {
+  const float y = (x == 0.f ? 1.f : x) / d;
+  return x == 0.f ? x * y : y;
+}
 template <int EPI>
 __device__ __forceinline__ float glu_pair(float g, float u, GluParams gp) {
   if (EPI == EPI_CLAMPGLU) {
     g = fminf(g, gp.limit);
     u = fminf(fmaxf(u, -gp.limit), gp.limit) + 1.0f;
-    return __fdividef(g, 1.0f + __expf(-gp.slope * g)) * u;
+    return over(g, 1.0f + __expf(-gp.slope * g)) * u;
   }
   const float z = EPI == EPI_GEGLU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : g;
-  return __fdividef(g, 1.0f + __expf(-z)) * u;
+  return over(g, 1.0f + __expf(-z)) * u;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -957,9 +957,7 @@ head_out_gate_vec_kernel(const float* __restrict__ o, int ldo, const float* __re
   for (int k = L >> 1; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
   if (!on) return;
   const float inv = scale / sqrtf(ss / (float)dv + eps);
-  // (narrowed, by a division without the branch for unusual operands)
-  auto sigmoid = [](float z) { return sizeof(T) == 4 ? sigmoid_f(z) : __fdividef(1.0f, 1.0f + expf(-z)); };
-  auto gate = [&](float z) { return act == 0 ? sigmoid(z) : z * sigmoid(z); };
+  auto gate = [&](float z) { return act == 0 ? sigmoid_f(z) : z * sigmoid_f(z); };
   const float4 y = make_float4(x.x * inv * w.x * gate(gl.x), x.y * inv * w.y * gate(gl.y), x.z * inv * w.z * gate(gl.z), x.w * inv * w.w * gate(gl.w));
   T* dst = out + it * dv + i;
   if (sizeof(T) == 4) {

@@ -17,12 +17,7 @@
 #define SC_GROUP 8
 #define SC_MAX_TAPS 16
 
-// silu in float32; where the result is narrowed, by a division without the branch for unusual operands
-template <typename T>
-__device__ __forceinline__ float conv_act(float z, int act) {
-  if (!act) return z;
-  return sizeof(T) == 4 ? z / (1.0f + expf(-z)) : __fdividef(z, 1.0f + expf(-z));
-}
+__device__ __forceinline__ float conv_act(float z, int act) { return act ? z / (1.0f + expf(-z)) : z; }
 
 // The thread walks its tokens in groups of SC_GROUP: the group's inputs are loaded at once (each input is read once; the
 // taps - 1 before them stay in registers from the group before), then the group's outputs are summed, oldest tap first.
@@ -60,7 +55,7 @@ short_conv_kernel(const float* __restrict__ x, long long ldx, const float* __res
     for (int s = TAPS - 1; s >= 1; --s)
       if (s <= back) acc = fmaf(wr[s], hist[s], acc);
     acc = fmaf(wr[0], now, acc);
-    y[(size_t)row0 * ldy + c] = from_f32<T>(conv_act<T>(acc, act));
+    y[(size_t)row0 * ldy + c] = from_f32<T>(conv_act(acc, act));
 #pragma unroll
     for (int s = TAPS - 1; s >= 2; --s)
       if (s <= back) tl[(size_t)(back - s) * C] = hist[s - 1];
@@ -84,7 +79,7 @@ short_conv_kernel(const float* __restrict__ x, long long ldx, const float* __res
     }
 #pragma unroll
     for (int u = 0; u < SC_GROUP; ++u)
-      if (tg + u < t1) y[(size_t)(row0 + tg + u) * ldy + c] = from_f32<T>(conv_act<T>(acc[u], act));
+      if (tg + u < t1) y[(size_t)(row0 + tg + u) * ldy + c] = from_f32<T>(conv_act(acc[u], act));
     float next[TAPS];
 #pragma unroll
     for (int s = 1; s < TAPS; ++s) next[s] = s <= SC_GROUP ? nw[s <= SC_GROUP ? SC_GROUP - s : 0] : hist[s <= SC_GROUP ? 0 : s - SC_GROUP];
@@ -174,7 +169,7 @@ short_conv_vec_kernel(const float* __restrict__ x, long long ldx, const float* _
 #pragma unroll
       for (int s = 3; s >= 0; --s)
         if (s <= back) acc[e] = fmaf(wr[s][e], in[3 + u - s][e], acc[e]);
-      acc[e] = conv_act<T>(acc[e], act);
+      acc[e] = conv_act(acc[e], act);
     }
     T* dst = y + (size_t)(row0 + t0 + u) * ldy + c;
     if (sizeof(T) == 4) {

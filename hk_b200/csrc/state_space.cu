@@ -822,7 +822,7 @@ gated_part_norm_warp_kernel(const float* __restrict__ y, const float* __restrict
     u[j] = i < width ? *reinterpret_cast<const float4*>(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     zv[j] = i < width ? *reinterpret_cast<const float4*>(zr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  auto silu = [](float v) { return sizeof(T) == 4 ? v / (1.0f + expf(-v)) : __fdividef(v, 1.0f + expf(-v)); };
+  auto silu = [](float v) { return v / (1.0f + expf(-v)); };
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
