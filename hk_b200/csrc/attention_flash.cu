@@ -970,8 +970,7 @@ template <int HD, int NW>
 int launch_flash(const void* q, const void* kp, const void* vp, const int* bt, int stride, const void* items, int n_items,
                  void* out, float* part_o, float* part_ml, int H, int G, int pt, int window, float scale_log2, ScoreOpts so, cudaStream_t s) {
   const size_t smem = (size_t)4 * TILE_N * (HD + 8) * sizeof(bf16) + 2 * TILE_N * sizeof(int);
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_flash_kernel<HD, NW>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<attention_flash_kernel<HD, NW>>(smem)) return e;
   dim3 grid((unsigned)n_items * (unsigned)G);
   attention_flash_kernel<HD, NW><<<grid, NW * 32, smem, s>>>((const bf16*)q, (const bf16*)kp, (const bf16*)vp, bt, stride,
                                                             (const Item*)items, (bf16*)out, part_o, part_ml, H, G, pt, window,
@@ -987,8 +986,7 @@ int launch_decode(const void* q, const void* kp, const void* vp, const int* bt, 
   const size_t merge = (size_t)DW * 16 * (HD + 2) * sizeof(float);
   const size_t smem = (tiles > merge ? tiles : merge) + (size_t)pages_cap * sizeof(int);
   if (smem > 200 * 1024) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_decode_kernel<HD>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<attention_decode_kernel<HD>>(smem)) return e;
   dim3 grid((unsigned)n_items, (unsigned)G);
   attention_decode_kernel<HD><<<grid, DW * 32, smem, s>>>((const bf16*)q, (const bf16*)kp, (const bf16*)vp, bt, stride,
                                                          (const Item*)items, (bf16*)out, part_o, part_ml, H, G, pt, window,
@@ -1123,8 +1121,7 @@ int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, const void* 
                       float scale_log2, ScoreOpts so, int pages_cap, int* status, cudaStream_t s) {
   const size_t smem = decode_tma_smem<HD>(TW * 16, pages_cap);
   if (smem > 110 * 1024) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_decode_tma_kernel<HD, DIST, TW>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<attention_decode_tma_kernel<HD, DIST, TW>>(smem)) return e;
   dim3 grid((unsigned)n_items, (unsigned)G);
   return hk_launch_pdl(attention_decode_tma_kernel<HD, DIST, TW>, grid, dim3((TW + 1) * 32), smem, s, mk, mv, (const bf16*)q, bt, stride,
                        (const Item*)items, (bf16*)out, part_o, part_ml, H, G, pt, box_rows, window, scale_log2, so, pages_cap, 0, status);
@@ -1139,8 +1136,7 @@ int launch_decode_merged(const CUtensorMap& mk, const CUtensorMap& mv, const voi
   constexpr int TW = 4, DEVICES = 64;
   const size_t smem = decode_tma_smem<HD>(TW * 16, pages_cap);
   if (decode_tma_slots(HD, TW) * (smem + 1024) > 228 * 1024) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_decode_tma_kernel<HD, DIST, TW>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<attention_decode_tma_kernel<HD, DIST, TW>>(smem)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)n_items, (unsigned)G);
   cfg.blockDim = dim3((TW + 1) * 32);

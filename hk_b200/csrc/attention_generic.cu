@@ -417,8 +417,7 @@ HK_API int hk_attention_f32(const float* q, const float* k_pages, const float* v
     return HK_ERR_UNSUPPORTED;
   if (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out) & 15) return HK_ERR_UNSUPPORTED;
   const AgOptions opt = {softcap, chunk, v_stride, sinks, gate, gate_ld, gate_scale, dist, dist_n};
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(attention_f32_kernel, sizeof(AfSmem), cache)) return e;
+  if (int e = hk_allow_smem<attention_f32_kernel>(sizeof(AfSmem))) return e;
   return hk_launch(attention_f32_kernel, dim3((unsigned)n_items * (unsigned)G), dim3(AF_TH), sizeof(AfSmem), (cudaStream_t)stream, q, k_pages,
                    v_pages, block_table, table_stride, (const AfItem*)items, out, H, G, hd, page_tokens, window, scale, vd, sink, opt);
 }

@@ -590,8 +590,7 @@ template <int DVW>
 int launch_latent(const void* q, const void* pages, const int* bt, int stride, const void* items, int n_items, void* out,
                   float* part_o, float* part_ml, int H, int DK, int DV, int pt, int window, float scale_log2, cudaStream_t s) {
   const size_t smem = latent_smem(DK);
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(latent_flash_kernel<DVW>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<latent_flash_kernel<DVW>>(smem)) return e;
   latent_flash_kernel<DVW><<<(unsigned)n_items, 256, smem, s>>>((const bf16*)q, (const bf16*)pages, bt, stride, (const Item*)items,
                                                                 (bf16*)out, part_o, part_ml, H, DK, DV, pt, window, scale_log2);
   return hk_launch_status();
@@ -601,8 +600,7 @@ template <int MT, int DVC>
 int launch_latent_decode(const void* q, const void* pages, const int* bt, int stride, const void* items, int n_items, void* out,
                          float* part_o, float* part_ml, int H, int DK, int DV, int pt, int window, float scale_log2, cudaStream_t s) {
   const size_t smem = latent_decode_smem(DK, MT);
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(latent_decode_kernel<MT, DVC>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<latent_decode_kernel<MT, DVC>>(smem)) return e;
   latent_decode_kernel<MT, DVC><<<(unsigned)n_items, 256, smem, s>>>((const bf16*)q, (const bf16*)pages, bt, stride, (const Item*)items,
                                                                      (bf16*)out, part_o, part_ml, H, DK, DV, pt, window, scale_log2);
   return hk_launch_status();
@@ -804,8 +802,7 @@ HK_API int hk_latent_first_rows(const void* q, const void* kv, const void* rope,
     return HK_ERR_UNSUPPORTED;
   const size_t smem = (size_t)FIRST_ROWS * ((r + 4) * sizeof(float) + (r + 8) * sizeof(bf16));
   if (smem > 200 * 1024) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(latent_first_rows_kernel, smem, cache)) return e;
+  if (int e = hk_allow_smem<latent_first_rows_kernel>(smem)) return e;
   return hk_launch_pdl(latent_first_rows_kernel, dim3((unsigned)H, (unsigned)n_firsts, 4), dim3(256), smem, (cudaStream_t)stream, (const bf16*)q,
                    (const bf16*)kv, (const bf16*)rope, (const bf16*)c, (const bf16*)w_uv, (const FirstRows*)firsts, (bf16*)out, H, dr, r, window,
                    scale_log2, gate, gate_ld, gate_heads, gate_scale);

@@ -565,8 +565,7 @@ int launch(const void* q, const void* kp, const void* vp, const int* bt, int str
            int H, int G, int pt, int window, float scale_log2, ScoreOpts so, int pages_cap, int* status, cudaStream_t s) {
   const size_t smem = sizeof(Smem<HD>) + 1024 + (size_t)pages_cap * sizeof(int);
   if (smem > 225 * 1024) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_prefill_tc_kernel<HD, DIST>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<attention_prefill_tc_kernel<HD, DIST>>(smem)) return e;
   dim3 grid((unsigned)n_items * (unsigned)G);
   attention_prefill_tc_kernel<HD, DIST><<<grid, NUM_THREADS, smem, s>>>((const bf16*)q, (const bf16*)kp, (const bf16*)vp, bt, stride,
                                                                  (const Item*)items, (bf16*)out, H, G, pt, window, scale_log2,
@@ -1063,8 +1062,7 @@ int launch2(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, const i
             const CUtensorMap* mr = nullptr, const void* made = nullptr, const void* made_rope = nullptr) {
   const size_t smem = sizeof(Smem2<HD, HDK>) + 1024 + (size_t)pages_cap * sizeof(int);
   if (smem > (MADE ? 227 : 225) * 1024) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>>(smem)) return e;
   dim3 grid((unsigned)n_items * (unsigned)G);
   return hk_launch(attention_prefill_tc2_kernel<HD, HDK, DIST, MADE>, grid, dim3(NT2), smem, s, mk, mv, mr ? *mr : mk, (const bf16*)q, bt, stride,
                    (const Item*)items, (bf16*)out, H, G, pt, window, scale_log2, so, pages_cap, status, (const bf16*)made, (const bf16*)made_rope);

@@ -9,6 +9,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #define HK_F32 0
 #define HK_BF16 1
 // Returned (instead of a cudaError_t) when an entry point refuses its arguments.
@@ -53,24 +56,32 @@ __device__ __forceinline__ bool elect_one() {
 
 static inline int hk_launch_status() { return (int)cudaGetLastError(); }
 
-// Dynamic shared memory above 48 KB has to be allowed per kernel on every device that runs it.  A launcher keeps a
-// `static HkSmemCache` per kernel: the largest size allowed so far on each device (devices beyond the table are
-// set on every launch).  Returns 0 or a cudaError_t.
+// A launch whose static and dynamic shared memory together pass 48 KB has to be allowed, per kernel and device.  The limit belongs to
+// the kernel, whichever launchers it has, and a lower one takes the place of a higher one: so what is remembered belongs to the kernel
+// too, and a limit is only ever raised.  Returns 0 or a cudaError_t.
 #define HK_MAX_DEVICES 64
-struct HkSmemCache {
-  size_t allowed[HK_MAX_DEVICES];
+struct HkSmemLimit {
+  std::atomic<size_t> known[HK_MAX_DEVICES];     // the dynamic bytes that a launch may surely ask for
+  std::mutex raising;
 };
-template <typename K>
-static inline int hk_allow_smem(K kernel, size_t smem, HkSmemCache& cache) {
-  if (smem <= 48 * 1024) return 0;
+template <auto KERNEL>
+static inline int hk_allow_smem(size_t dynamic) {
+  static HkSmemLimit limit;
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return (int)e;
-  const bool known = dev >= 0 && dev < HK_MAX_DEVICES;
-  if (known && smem <= cache.allowed[dev]) return 0;
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  if (known) cache.allowed[dev] = smem;
+  if (cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+  const bool in_table = dev >= 0 && dev < HK_MAX_DEVICES;
+  if (in_table && dynamic <= limit.known[dev].load(std::memory_order_acquire)) return 0;
+  std::lock_guard<std::mutex> one(limit.raising);
+  cudaFuncAttributes now;
+  if (cudaError_t e = cudaFuncGetAttributes(&now, KERNEL)) return (int)e;
+  constexpr size_t PLAIN = 48 * 1024;
+  size_t allowed = now.maxDynamicSharedSizeBytes > (int)PLAIN ? (size_t)now.maxDynamicSharedSizeBytes
+                   : now.sharedSizeBytes < PLAIN              ? PLAIN - now.sharedSizeBytes : 0;
+  if (dynamic > allowed) {
+    if (cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dynamic)) return (int)e;
+    allowed = dynamic;
+  }
+  if (in_table) limit.known[dev].store(allowed, std::memory_order_release);
   return 0;
 }
 

@@ -1043,8 +1043,7 @@ template <int DVS>
 int run_walk(const int* requests, int n_requests, const int* chunks, const float* mm, const float* rq, const float* bb, float* state,
              float* out, int H, int dk, int dv, cudaStream_t s) {
   using K = WalkShape<DVS>;
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(chunk_walk_kernel<DVS>, K::SMEM, cache)) return e;
+  if (int e = hk_allow_smem<chunk_walk_kernel<DVS>>(K::SMEM)) return e;
   return hk_launch(chunk_walk_kernel<DVS>, dim3((unsigned)(n_requests * H), (unsigned)((dv + DVS - 1) / DVS)), dim3(K::THREADS), K::SMEM,
                    s, (const Request*)requests, (const Chunk*)chunks, mm, rq, bb, state, out, H, dk, dv);
 }
@@ -1057,8 +1056,7 @@ int run_delta(const DeltaIn& in, const int* chunks, int n_chunks, const int* req
   float* rq = scratch;
   float* mm = rq + (size_t)n_chunks * in.H * CQ * NT;
   float* bb = mm + (size_t)n_chunks * in.H * MFLOATS;
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(delta_local_kernel<GATED>, sizeof(DeltaSmem), cache)) return e;
+  if (int e = hk_allow_smem<delta_local_kernel<GATED>>(sizeof(DeltaSmem))) return e;
   if (int e = hk_launch(delta_local_kernel<GATED>, dim3((unsigned)(n_chunks * in.H), (unsigned)((in.dv + NT - 1) / NT)), dim3(NTH), sizeof(DeltaSmem),
                         s, in, (const Chunk*)chunks, mm, rq, bb, out))
     return e;
@@ -1079,8 +1077,7 @@ int run_decay(const DecayIn& in, const int* chunks, int n_chunks, const int* req
   if (int e = hk_launch(decay_carry_kernel, dim3((unsigned)(n_requests * in.H), (unsigned)((entries / 4 + NTH - 1) / NTH)), dim3(NTH), 0, s,
                         (const Request*)requests, (const float2*)pp, bb, state, in.H, entries))
     return e;
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(decay_out_kernel<MEMORY>, sizeof(OutSmem), cache)) return e;
+  if (int e = hk_allow_smem<decay_out_kernel<MEMORY>>(sizeof(OutSmem))) return e;
   return hk_launch(decay_out_kernel<MEMORY>, grid, dim3(NTH), sizeof(OutSmem), s, in, (const Chunk*)chunks, (const float*)bb, out);
 }
 

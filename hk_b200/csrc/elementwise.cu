@@ -707,8 +707,7 @@ HK_API int hk_qk_row_norm_kv_write(const float* qkv, long long ld, const float* 
   cudaStream_t s = (cudaStream_t)stream;
 #define RNW_GO(T, V)                                                                                                             \
   do {                                                                                                                           \
-    static HkSmemCache cache;                                                                                                    \
-    if (int e = hk_allow_smem(qk_row_norm_kv_write_kernel<T, V>, smem, cache)) return e;                                         \
+    if (int e = hk_allow_smem<qk_row_norm_kv_write_kernel<T, V>>(smem)) return e;                                                \
     return hk_launch_pdl(qk_row_norm_kv_write_kernel<T, V>, dim3(n), dim3(RNW_THREADS), smem, s, qkv, ld, bias, (T*)q_out, q_w, k_w, \
                          q_count, k_count, eps, positions, slot_of_token, block_table, table_stride, (T*)k_pages, (T*)v_pages, H, G, hd, \
                          vd, page_tokens, write_kv, qt);                                                                         \

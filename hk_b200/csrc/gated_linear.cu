@@ -328,8 +328,7 @@ static int walk_launch(const float* q, const float* k, const float* v, long long
   int chunk = 16;
   while (chunk > 2 && (size_t)2 * chunk * R * sizeof(float) > 48 * 1024) chunk >>= 1;
   const size_t smem = (size_t)2 * chunk * R * sizeof(float);
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(gla_walk_kernel<L, RPT, CPT>, smem, cache)) return e;
+  if (int e = hk_allow_smem<gla_walk_kernel<L, RPT, CPT>>(smem)) return e;
   return hk_launch(gla_walk_kernel<L, RPT, CPT>, grid, dim3(128), smem, s, q, k, v, ld, la, segs, state, out, ldo, H, dk, dv, q_scale,
                    chunk, vec);
 }

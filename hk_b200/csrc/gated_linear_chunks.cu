@@ -432,9 +432,8 @@ int run_chunks(const float* q, const float* k, const float* v, long long ld, con
                const Request* requests, int n_requests, float* u, float* decay, float* state, float* out, int H, int dk, int dv,
                float q_scale, cudaStream_t s) {
   const dim3 grid((unsigned)(n_chunks * H), (unsigned)((dv + DVB - 1) / DVB));
-  static HkSmemCache c1, c3;
-  if (int e = hk_allow_smem(gla_states_kernel<NT, DVB>, StatesShape<NT, DVB>::SMEM, c1)) return e;
-  if (int e = hk_allow_smem(gla_out_kernel<NT, DVB>, OutShape<NT, DVB>::SMEM, c3)) return e;
+  if (int e = hk_allow_smem<gla_states_kernel<NT, DVB>>(StatesShape<NT, DVB>::SMEM)) return e;
+  if (int e = hk_allow_smem<gla_out_kernel<NT, DVB>>(OutShape<NT, DVB>::SMEM)) return e;
   if (int e = hk_launch(gla_states_kernel<NT, DVB>, grid, dim3(NTH), StatesShape<NT, DVB>::SMEM, s, k, v, ld, la, chunks, u, decay, H, dk, dv))
     return e;
   if (int e = hk_launch(gla_carry_kernel, dim3((unsigned)(n_requests * H), (unsigned)((dv * dk / 4 + NTH - 1) / NTH)), dim3(NTH), 0, s, requests, u,

@@ -128,8 +128,7 @@ static int gemm_f32_launch(const F32Product& p, int heads, cudaStream_t s) {
   using T = F32Tile<BM, BN, TM, TN, BK, STAGES>;
   const long long rows = ((long long)p.M + BM - 1) / BM;
   if (rows > 65535 || heads > 65535) return HK_ERR_UNSUPPORTED;
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(gemm_f32_kernel<BM, BN, TM, TN, BK, STAGES>, T::SMEM, cache)) return e;
+  if (int e = hk_allow_smem<gemm_f32_kernel<BM, BN, TM, TN, BK, STAGES>>(T::SMEM)) return e;
   return hk_launch(gemm_f32_kernel<BM, BN, TM, TN, BK, STAGES>, dim3((unsigned)((p.N + BN - 1) / BN), (unsigned)rows, (unsigned)heads),
                    dim3(T::THREADS), T::SMEM, s, p);
 }

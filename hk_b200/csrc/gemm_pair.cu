@@ -474,11 +474,10 @@ bool make_gated_map(CUtensorMap* map, const void* ptr, int F, int cols, int grou
 template <int EPI, bool GROUPED>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mw, void* out, const PairShape& s, const PairGroups& g, long long ldo, int pairs,
                 float* partial, int* status, GluParams gp, cudaStream_t stream) {
-  static HkSmemCache allowed = {};
   const int stage_bytes = W_BYTES + (GROUPED ? g.rows : widest(s)) * BK;
   const int stages = min(PAIR_STAGES, PAIR_RING / stage_bytes);
   const size_t smem = (size_t)stages * stage_bytes + PAIR_CONTROL + 1024;
-  if (int e = hk_allow_smem(gemm_pair_kernel<EPI, GROUPED>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<gemm_pair_kernel<EPI, GROUPED>>(smem)) return e;
   const long long items = (long long)s.tiles * (GROUPED ? g.max_tiles : s.slices);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * (items < pairs ? (int)items : pairs)));

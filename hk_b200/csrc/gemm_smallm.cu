@@ -162,8 +162,7 @@ gemm_smallm_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, void*
 template <int MT, int RT, int MODE>
 int launch_mode(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, float factor, cudaStream_t s) {
   const size_t smem = (size_t)SM_WARPS * RT * 16 * MT * 8 * sizeof(float);
-  static HkSmemCache allowed = {};
-  if (int e = hk_allow_smem(gemm_smallm_kernel<MT, RT, MODE>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<gemm_smallm_kernel<MT, RT, MODE>>(smem)) return e;
   const unsigned grid = (unsigned)((N + RT * 16 - 1) / (RT * 16));
   // launched so that it may start while the kernel before it drains: its first weights are on their way before it
   // waits for that kernel's output (0.8 microseconds a launch, measured over a decode step)

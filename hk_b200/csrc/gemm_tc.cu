@@ -561,12 +561,11 @@ __global__ void splitk_reduce_vec_kernel(const float* __restrict__ partial, floa
 template <int EPI>
 int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int M, int N, int K, long long ldo, int bn, int splits,
            float* partial, int* status, cudaStream_t s, GluParams gp = {0.f, 1.f}) {
-  static HkSmemCache allowed = {};
   const uint32_t stage_bytes = stage_bytes_of(bn);
   int stages = RING_BYTES / (int)stage_bytes;
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   const size_t smem = (size_t)stages * stage_bytes + CONTROL_BYTES + 1024;
-  if (int e = hk_allow_smem(gemm_tc_kernel<EPI>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<gemm_tc_kernel<EPI>>(smem)) return e;
   const int n_tiles = IS_GLU(EPI) ? (N / 2 + bn / 2 - 1) / (bn / 2) : (N + bn - 1) / bn;
   const int tiles = ((M + BM - 1) / BM) * n_tiles * splits;
   const int grid = tiles < sm_count() ? tiles : sm_count();
@@ -586,12 +585,11 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int M, int N
 template <bool ADD>
 int launch_cluster(const CUtensorMap& ma, const CUtensorMap& mw, float* out, int M, int N, int K, long long ldo, int bn, int slices,
                    int* status, cudaStream_t s) {
-  static HkSmemCache allowed = {};
   const uint32_t stage_bytes = cluster_stage_bytes(M, bn);
   int stages = (RING_BYTES - 16 * 1024) / (int)stage_bytes;       // 16 KB: what the tensor core may read past the last stage's a rows
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   const size_t smem = (size_t)RING_BYTES + CONTROL_BYTES + 1024;
-  if (int e = hk_allow_smem(gemm_tc_cluster_kernel<ADD>, smem, allowed)) return e;
+  if (int e = hk_allow_smem<gemm_tc_cluster_kernel<ADD>>(smem)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((N + bn - 1) / bn * slices));
   cfg.blockDim = dim3(NUM_THREADS);

@@ -296,8 +296,7 @@ static int dr_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s,
                      float* out, int H, int dk, int dv, int cols, int chunk, int rec_rows) {
 #define DR_LAUNCH(LL)                                                                                                       \
   do {                                                                                                                      \
-    static HkSmemCache cache;                                                                                               \
-    int e = hk_allow_smem(delta_rule_scan_kernel<RPT, LL, CPT>, smem, cache);                                               \
+    int e = hk_allow_smem<delta_rule_scan_kernel<RPT, LL, CPT>>(smem);                                                      \
     if (e) return e;                                                                                                        \
     return hk_launch(delta_rule_scan_kernel<RPT, LL, CPT>, grid, dim3(threads), smem, s, rec, segs, state, out, H, dk, dv, cols, \
                      chunk, rec_rows);                                                                                      \
@@ -331,8 +330,7 @@ static int dr_scan_records(const float* rec, const int* segs, int n_seg, float* 
     const int cols = max(1, min(dv, 128 / L));
     const int threads = ((cols * L + 31) / 32) * 32;      // whole warps: the lanes of a column meet by shuffle
     const size_t smem = (size_t)(threads * rpt + R) * sizeof(float);
-    static HkSmemCache cache;
-    int e = hk_allow_smem(delta_rule_scan_plain_kernel, smem, cache);
+    int e = hk_allow_smem<delta_rule_scan_plain_kernel>(smem);
     if (e) return e;
     return hk_launch(delta_rule_scan_plain_kernel, dim3((unsigned)(n_seg * H), (unsigned)((dv + cols - 1) / cols)), dim3(threads), smem, s,
                      rec, segs, state, out, H, dk, dv, L, rpt, cols, rec_rows);
@@ -722,8 +720,7 @@ static int ret_launch(int L, dim3 grid, int threads, size_t smem, cudaStream_t s
                       const float* decay, float* state, float* out, int H, int dk, int dv, int cols, int chunk, int rec_rows) {
 #define RET_LAUNCH(LL)                                                                                                      \
   do {                                                                                                                      \
-    static HkSmemCache cache;                                                                                               \
-    int e = hk_allow_smem(retention_scan_kernel<RPT, LL, CPT>, smem, cache);                                                \
+    int e = hk_allow_smem<retention_scan_kernel<RPT, LL, CPT>>(smem);                                                       \
     if (e) return e;                                                                                                        \
     return hk_launch(retention_scan_kernel<RPT, LL, CPT>, grid, dim3(threads), smem, s, rec, segs, decay, state, out, H, dk, dv, \
                      cols, chunk, rec_rows);                                                                                \

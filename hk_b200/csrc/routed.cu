@@ -218,13 +218,11 @@ HK_API int hk_route_topk(const void* x, int dtype, const float* w, int* ids, flo
   dim3 grid((unsigned)n);
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == HK_F32) {
-    static HkSmemCache cache;
-    if (int e = hk_allow_smem(route_topk_kernel<float>, smem, cache)) return e;
+    if (int e = hk_allow_smem<route_topk_kernel<float>>(smem)) return e;
     return hk_launch(route_topk_kernel<float>, grid, dim3(RK_WARPS * 32), smem, s, (const float*)x, w, ids, weights, n, d, E, top, opt);
   }
   if (dtype == HK_BF16) {
-    static HkSmemCache cache;
-    if (int e = hk_allow_smem(route_topk_kernel<bf16>, smem, cache)) return e;
+    if (int e = hk_allow_smem<route_topk_kernel<bf16>>(smem)) return e;
     return hk_launch(route_topk_kernel<bf16>, grid, dim3(RK_WARPS * 32), smem, s, (const bf16*)x, w, ids, weights, n, d, E, top, opt);
   }
   return HK_ERR_UNSUPPORTED;

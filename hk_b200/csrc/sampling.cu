@@ -387,9 +387,8 @@ HK_API int hk_sample(const float* logits, int rows, int V, const float* temperat
                      const float* top_p, const float* min_p, const unsigned long long* seeds,
                      const unsigned long long* counters, int* out, void* stream) {
   if (rows <= 0) return 0;
-  static HkSmemCache allowed = {};
   size_t smem = sizeof(SampleShared);
-  if (int e = hk_allow_smem(sample_kernel, smem, allowed)) return e;
+  if (int e = hk_allow_smem<sample_kernel>(smem)) return e;
   sample_kernel<<<rows, SMP_THREADS, smem, (cudaStream_t)stream>>>(logits, V, temperature, top_k, top_p, min_p, seeds,
                                                                  counters, out);
   return hk_launch_status();

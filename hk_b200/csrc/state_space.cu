@@ -290,8 +290,7 @@ static int walk_launch(const T* xbc, long long ldx, const float* dt, long long l
   auto bytes = [&](int c) { return (size_t)2 * c * R * sizeof(T) + 2 * c * sizeof(float) + c * sizeof(float2); };
   while (chunk > 2 && bytes(chunk) > 48 * 1024) chunk >>= 1;
   const size_t smem = bytes(chunk);
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(state_space_walk_kernel<T, L, RPT, CPT>, smem, cache)) return e;
+  if (int e = hk_allow_smem<state_space_walk_kernel<T, L, RPT, CPT>>(smem)) return e;
   return hk_launch(state_space_walk_kernel<T, L, RPT, CPT>, grid, dim3(128), smem, s, xbc, ldx, dt, ldt, dt_bias, a_log, skip, segs,
                    state, y, H, G, N, dv, chunk, vec);
 }
@@ -720,9 +719,8 @@ template <int NT, int DVB>
 static int chunks_launch(const bf16* xbc, long long ldx, const float* dt, long long ldt, const float* dt_bias, const float* a_log,
                          const float* skip, const int* segs, int n_seg, float* state, float* y, int H, int G, int N, int dv,
                          cudaStream_t s) {
-  static HkSmemCache cache;
   constexpr size_t smem = ChunkShape<NT, DVB>::SMEM;
-  if (int e = hk_allow_smem(state_space_chunks_kernel<NT, DVB>, smem, cache)) return e;
+  if (int e = hk_allow_smem<state_space_chunks_kernel<NT, DVB>>(smem)) return e;
   dim3 grid((unsigned)(n_seg * H), (unsigned)((dv + DVB - 1) / DVB));
   return hk_launch(state_space_chunks_kernel<NT, DVB>, grid, dim3(512), smem, s, xbc, ldx, dt, ldt, dt_bias, a_log, skip, segs, state, y, H,
                    G, N, dv);
@@ -866,12 +864,10 @@ static int gated_part_norm(const float* y, const float* z, long long ldz, const 
   const size_t smem = (size_t)width * sizeof(float);
   dim3 grid((unsigned)n, (unsigned)parts);
   if (vec) {
-    static HkSmemCache cache;
-    if (int e = hk_allow_smem(gated_part_norm_kernel<T, 4>, smem, cache)) return e;
+    if (int e = hk_allow_smem<gated_part_norm_kernel<T, 4>>(smem)) return e;
     return hk_launch_pdl(gated_part_norm_kernel<T, 4>, grid, dim3(threads), smem, s, y, z, ldz, weight, out, W, width, eps);
   }
-  static HkSmemCache cache;
-  if (int e = hk_allow_smem(gated_part_norm_kernel<T, 1>, smem, cache)) return e;
+  if (int e = hk_allow_smem<gated_part_norm_kernel<T, 1>>(smem)) return e;
   return hk_launch_pdl(gated_part_norm_kernel<T, 1>, grid, dim3(threads), smem, s, y, z, ldz, weight, out, W, width, eps);
 }
 
