@@ -660,6 +660,7 @@ HK_API int hk_attention_latent_rows() { return ROWS; }
 // at 32 heads 365 -> 346 us (27 of them were this kernel's, a row of weights a lane).  Relative error of a 2,048-token prompt through
 // the mixer: 3.34e-3 in the latent space, 3.45e-3 without this, 3.19e-3 with it.
 constexpr int FIRST_ROWS = 16;
+constexpr int FIRST_COLS = 512, FIRST_LDW = FIRST_COLS + 8;     // weights that are staged at once; neighbouring dims in other banks
 
 struct FirstRows {
   int q_row, row0, pos0, count;       // first of its rows of the step, the row of position 0 among the made rows
@@ -669,12 +670,11 @@ __global__ void __launch_bounds__(256)
 latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv, const bf16* __restrict__ rope, const bf16* __restrict__ c,
                          const bf16* __restrict__ w_uv, const FirstRows* __restrict__ firsts, bf16* __restrict__ out, int H, int dr, int r,
                          int window, float scale_log2, const float* __restrict__ gate, long long gate_ld, int gate_heads, float gate_scale) {
-  extern __shared__ __align__(16) float lat[];          // [FIRST_ROWS][r + 4], then bf16 [FIRST_ROWS][r + 8] of cache rows
+  extern __shared__ __align__(16) float lat[];          // [FIRST_ROWS][r + 4], then bf16 [FIRST_ROWS][r + 8] of cache rows, then of weights
   constexpr int LDQ = 192 + 8;                          // 16-byte pieces of neighbouring rows lie in different banks
   __shared__ __align__(16) bf16 qs[FIRST_ROWS][LDQ], ks[FIRST_ROWS][LDQ];
   __shared__ float prob[FIRST_ROWS][FIRST_ROWS];
   constexpr int WARPS = 8;
-  __shared__ float sums[WARPS][FIRST_ROWS][33];
   const int h = blockIdx.x, d0 = blockIdx.z * 32, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ldl = r + 4, ldc = r + 8;
   bf16* cs = reinterpret_cast<bf16*>(lat + FIRST_ROWS * ldl);
   const FirstRows f = firsts[blockIdx.y];
@@ -682,12 +682,17 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
   // would stand among the made rows another request stands, or nothing (row0 is then negative)
   const int wide = 128 + dr, last = f.pos0 + f.count, first = window > 0 ? max(0, f.pos0 - window + 1) : 0;
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  // a lane's value dim, every WARPS-th piece of its weights: the first eight pieces come along with the rows
+  // the block's weights, FIRST_COLS of a value dim's row at a time: a lane has a value dim and every WARPS-th piece of 16 bytes; the first
+  // ones come along with the rows
+  constexpr int EACH = FIRST_COLS / 8 / WARPS;
   const int pieces = r / 8;
   const uint4* wp = reinterpret_cast<const uint4*>(w_uv + ((size_t)h * 128 + d0 + lane) * r);
-  uint4 w[8];
+  uint4 w[EACH];
+  auto ask = [&](int p0) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) w[j] = warp + WARPS * j < pieces ? wp[warp + WARPS * j] : zero;
+    for (int j = 0; j < EACH; ++j) w[j] = p0 + warp + WARPS * j < pieces ? wp[p0 + warp + WARPS * j] : zero;
+  };
+  ask(0);
   for (int e = tid; e < FIRST_ROWS * 24; e += 256) {
     const int i = e / 24, p = (e % 24) * 8;
     const bool q_in = i < f.count && p < wide;
@@ -754,36 +759,38 @@ latent_first_rows_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kv
     *reinterpret_cast<float4*>(lat + i * ldl + p + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
   }
   __syncthreads();
-  float acc[FIRST_ROWS] = {};
-  for (int p0 = warp; p0 < pieces; p0 += 8 * WARPS) {
-    if (p0 != warp)
+  // a lane per value dim, a warp per two rows, an even and an odd sum each, in the order of k; the weights through shared memory, where
+  // the cache rows are no longer wanted
+  const int i0 = warp * 2;
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+  for (int p0 = 0; p0 < pieces; p0 += FIRST_COLS / 8) {
+    const int count = min(FIRST_COLS / 8, pieces - p0);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = p0 + WARPS * j < pieces ? wp[p0 + WARPS * j] : zero;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int k = (p0 + WARPS * j) * 8;
-      if (k >= r) break;
+    for (int j = 0; j < EACH; ++j)
+      if (warp + WARPS * j < count) *reinterpret_cast<uint4*>(cs + lane * FIRST_LDW + (warp + WARPS * j) * 8) = w[j];
+    __syncthreads();
+    if (p0 + FIRST_COLS / 8 < pieces) ask(p0 + FIRST_COLS / 8);
+#pragma unroll 4
+    for (int p = 0; p < count; ++p) {
       float f[8];
-      halves(w[j], f);
+      halves(*reinterpret_cast<const uint4*>(cs + lane * FIRST_LDW + p * 8), f);
 #pragma unroll
-      for (int i = 0; i < FIRST_ROWS; ++i) {
-        const float4 x = *reinterpret_cast<const float4*>(lat + i * ldl + k), y = *reinterpret_cast<const float4*>(lat + i * ldl + k + 4);
-        const float even = fmaf(f[6], y.z, fmaf(f[4], y.x, fmaf(f[2], x.z, f[0] * x.x)));
-        const float odd = fmaf(f[7], y.w, fmaf(f[5], y.y, fmaf(f[3], x.w, f[1] * x.y)));
-        acc[i] += even + odd;
+      for (int i = 0; i < 2; ++i) {
+        const float* l = lat + (i0 + i) * ldl + (p0 + p) * 8;
+        const float4 x = *reinterpret_cast<const float4*>(l), y = *reinterpret_cast<const float4*>(l + 4);
+        acc[i][0] = fmaf(f[6], y.z, fmaf(f[4], y.x, fmaf(f[2], x.z, fmaf(f[0], x.x, acc[i][0]))));
+        acc[i][1] = fmaf(f[7], y.w, fmaf(f[5], y.y, fmaf(f[3], x.w, fmaf(f[1], x.y, acc[i][1]))));
       }
     }
+    __syncthreads();
   }
-#pragma unroll
-  for (int i = 0; i < FIRST_ROWS; ++i) sums[warp][i][lane] = acc[i];
-  __syncthreads();
   pdl_wait();                 // the attention's rows are written: these take their place
-  for (int i = warp; i < f.count; i += WARPS) {
-    const int d = d0 + lane;
-    const size_t row = (size_t)f.q_row + i;
-    float y = 0.f;
 #pragma unroll
-    for (int k = 0; k < WARPS; ++k) y += sums[k][i][lane];
+  for (int i = 0; i < 2; ++i) {
+    if (i0 + i >= f.count) continue;
+    const int d = d0 + lane;
+    const size_t row = (size_t)f.q_row + i0 + i;
+    float y = acc[i][0] + acc[i][1];
     if (gate) y *= gate_scale / (1.0f + expf(-gate[row * gate_ld + (gate_heads ? h : h * 128 + d)]));
     out[(row * H + h) * 128 + d] = __float2bfloat16_rn(y);
   }
@@ -800,7 +807,8 @@ HK_API int hk_latent_first_rows(const void* q, const void* kv, const void* rope,
   if (H < 1 || n_firsts > 65535 || (dr != 0 && dr != 64) || (dr != 0) != (rope != nullptr) || r < 8 || (r & 7) ||
       (((uintptr_t)w_uv | (uintptr_t)q | (uintptr_t)kv | (uintptr_t)rope | (uintptr_t)c) & 15))
     return HK_ERR_UNSUPPORTED;
-  const size_t smem = (size_t)FIRST_ROWS * ((r + 4) * sizeof(float) + (r + 8) * sizeof(bf16));
+  const size_t rows = (size_t)FIRST_ROWS * (r + 8), weights = (size_t)32 * FIRST_LDW;
+  const size_t smem = (size_t)FIRST_ROWS * (r + 4) * sizeof(float) + (rows > weights ? rows : weights) * sizeof(bf16);
   if (smem > 200 * 1024) return HK_ERR_UNSUPPORTED;
   if (int e = hk_allow_smem<latent_first_rows_kernel>(smem)) return e;
   return hk_launch_pdl(latent_first_rows_kernel, dim3((unsigned)H, (unsigned)n_firsts, 4), dim3(256), smem, (cudaStream_t)stream, (const bf16*)q,

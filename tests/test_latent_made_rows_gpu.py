@@ -164,9 +164,10 @@ def test_sizes_that_the_host_shares_with_the_kernels():
     assert [runs.hk_attention_f32_tokens(g) for g in (1, 3, 32, 33)] == [ops.RUN_ROWS, ops.RUN_ROWS // 3, 1, 0]
 
 
-@pytest.mark.parametrize("rank", [8, 72, 520, 1000])
+@pytest.mark.parametrize("rank", [8, 72, 504, 512, 520, 1000, 1032])
 def test_first_rows_of_any_rank(rank, monkeypatch):
-    """Fewer pieces of a latent row than the block has warps, a number that does not divide, more than come along with the rows."""
+    """Fewer pieces of a latent row than the block has warps, a number that does not divide, one to three stagings of the
+    weights."""
     from hk_b200.csrc import attention_fast
     monkeypatch.setitem(made_case.__globals__, "R", rank)
     got, want, pos = made_case([(0, 70), (3, 40)], 0, tiled, tile=128)

@@ -81,10 +81,20 @@ def first_rows(rank):
     assert bool(((got - want).abs()[early] <= 2.0 ** -8 * want.abs()[early] + 1e-4 * scale).all())
 
 
+def most_ranks():
+    """The largest rank that the first rows' kernel takes runs, the next one is refused and not tried."""
+    import torch
+    from hk_b200.csrc import build
+    first_rows(2128)
+    lib, t = build.load("attention_latent"), torch.zeros(64, dtype=torch.int32, device="cuda")
+    p = t.data_ptr()
+    assert lib.hk_latent_first_rows(p, p, 0, p, p, p, 1, p, 1, 0, 2136, 0, 1.0, 0, 0, 0, 1.0, 0) == 100001
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", ["forms(8192, 8192, (24, 8, 32))", "forms(20000, 2048, (8, 24, 8))", "forms(2048, 8192, (32, 4, 32))",
                                   "forms(8192, 300, (1, 24, 1))", "engine()", "first_rows(8)", "first_rows(192)", "first_rows(256)", "first_rows(360)",
-                                  "first_rows(504)"])
+                                  "first_rows(504)", "most_ranks()"])
 def test_first_launches_of_a_process(case):
     ran = subprocess.run([sys.executable, "-c", f"import test_shared_memory_limits_gpu as t; t.{case}"], capture_output=True, text=True, timeout=300,
                          env=dict(os.environ, PYTHONPATH=os.pathsep.join([HERE, os.path.join(HERE, os.pardir)])))
