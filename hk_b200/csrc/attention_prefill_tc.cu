@@ -696,7 +696,10 @@ attention_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __
   Smem2<HD, HDK>& sm = *reinterpret_cast<Smem2<HD, HDK>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   volatile int* abort_flag = &sm.abort_flag;
 
-  if (MADE) pdl_launch_dependents();     // the request's first rows are taken again beside this kernel's last blocks
+  if (MADE) {                   // the request's first rows are taken again beside this kernel's last blocks, by a kernel that reads what this
+    pdl_wait();                 // one reads before it waits for this one's end: so this one lets it start only once all of that is there
+    pdl_launch_dependents();
+  }
   const Item it = items[blockIdx.x / G];
   const int g = blockIdx.x % G;
   const int group = H / G;

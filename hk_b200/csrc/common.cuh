@@ -92,7 +92,9 @@ static inline int hk_allow_smem(size_t dynamic) {
 // launch.  A kernel launched with `hk_launch_pdl` may start while the kernel before it
 // in the stream is still running; it must call `pdl_wait()` before it reads or writes anything that an
 // earlier kernel of the stream touches (what it may do before: set up shared memory, read weights and the
-// step's host-written tables).  `pdl_launch_dependents()` lets the NEXT kernel start its own prologue early.
+// step's host-written tables).  `pdl_launch_dependents()` lets the NEXT kernel start its own prologue early.  A kernel
+// that says so only behind its own `pdl_wait()` lets the next one also read what is older than itself
+// (`latent_first_rows_kernel`, behind the attention over made keys and values; no other pair of kernels does that).
 // Without the launch attribute both calls do nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
