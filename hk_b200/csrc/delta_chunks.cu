@@ -137,11 +137,18 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
+// The largest pieces, of finite numbers always finite: what would round up to an infinity, the last 0.2 % of float32's range, gives the
+// largest bf16 number, and zeros in the other factor still make zeros of it.
+__device__ __forceinline__ uint32_t pack_first(float lo, float hi) {
+  uint32_t v;
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
+}
 // two float32 numbers as three pairs of bf16 whose sums they are, `step` words apart
 __device__ __forceinline__ void split3(float2 x, uint32_t* out, int step) {
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
-    out[p * step] = pack_bf16(x.x, x.y);
+    out[p * step] = p == 0 ? pack_first(x.x, x.y) : pack_bf16(x.x, x.y);
     x.x -= __uint_as_float(out[p * step] << 16);
     x.y -= __uint_as_float(out[p * step] & 0xffff0000u);
   }
@@ -955,7 +962,7 @@ chunk_walk_kernel(const Request* __restrict__ requests, const Chunk* __restrict_
         bf16* at = p + (8 * n + 2 * q + (e & 1)) * K::LS + mrow + 8 * (e >> 1);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          const bf16 piece = __float2bfloat16_rn(x);
+          const bf16 piece = k == 0 ? __ushort_as_bfloat16((unsigned short)pack_first(x, 0.f)) : __float2bfloat16_rn(x);
           at[k * K::PLANE] = piece;
           x -= __bfloat162float(piece);
         }

@@ -130,3 +130,20 @@ def test_value_columns_around_a_pass(kind, dk, dv):
     lengths = [33, 100]
     t = inputs(kind, 3, dk, dv, lengths, torch.Generator(DEV).manual_seed(dk * dv))
     same(*(scan(kind, 3, dk, dv, lengths, t, first) for first in (0, len(lengths))))
+
+
+@pytest.mark.parametrize("kind", ["general", "gated", "retention", "memory"])
+@pytest.mark.parametrize("at", [0, 17, 40])
+def test_the_largest_finite_values_reach_no_earlier_token(kind, at):
+    """A value that bfloat16 would round to infinity, at a token with a small key: the bits of the tokens before it as without it, and
+    finite everywhere as in the walk (the generalised rule divides by a chunk's decays, which leaves it no room there)."""
+    H, d, lengths = 2, 64, [70]
+    t = inputs(kind, H, d, d, lengths, torch.Generator(DEV).manual_seed(at))
+    K = H * d
+    t["proj"][at, K:2 * K] *= 1e-2
+    clean, _ = scan(kind, H, d, d, lengths, t, 0)
+    t["proj"][at, 2 * K + 5] = 3.4e38
+    got, want = (scan(kind, H, d, d, lengths, t, first) for first in (0, len(lengths)))
+    assert torch.equal(got[0][:at], clean[:at]) and all(bool(torch.isfinite(x).all()) for x in want)
+    if kind != "general":
+        same(got, want)
