@@ -612,14 +612,15 @@ __device__ __forceinline__ uint32_t peer_u32(uint32_t addr, int rank) {
 }
 
 // DIST: with a bias by distance (an instance of its own, so that the steps of a model without one issues nothing for it).
-// splits: 0, or the CTAs of a cluster, whose items are the key splits of one request (2 to 8; their `part` is not looked at).
+// splits: 0, or the CTAs of a cluster, whose items are the key splits of one request (2 to 8; their `part` is not looked at).  early:
+// the next kernel may start under this one's end (see launch_decode_merged).
 template <int HD, bool DIST, int TW>
 __global__ void __launch_bounds__((TW + 1) * 32, decode_tma_slots(HD, TW))
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                             const bf16* __restrict__ q, const int* __restrict__ block_table, int table_stride,
                             const Item* __restrict__ items, bf16* __restrict__ out, float* __restrict__ part_o,
                             float* __restrict__ part_ml, int H, int G, int page_tokens, int box_rows, int window,
-                            float scale_log2, ScoreOpts so, int pages_cap, int splits, int* __restrict__ status) {
+                            float scale_log2, ScoreOpts so, int pages_cap, int splits, int early, int* __restrict__ status) {
   constexpr int ROWS = 16;
   constexpr int KSTEPS = HD / 16;
   constexpr int TT = TW * 16;                        // keys per tile
@@ -810,7 +811,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     }
   }
   __syncthreads();
-  pdl_launch_dependents();   // the keys are read: the next kernel may move in
+  if (early) pdl_launch_dependents();   // the keys are read: the next kernel may move in
   if (*abort_flag) {
     if (threadIdx.x == 0) atomicExch(status, 2);
     if (splits == 0) return;   // nothing is written (with splits: not by the others of the cluster either, who look at this flag)
@@ -866,8 +867,8 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
   }
   if (splits == 0) return;
   // ---- a cluster holds the splits of one request and kv head: each CTA merges its share of the numbers out of everyone's shared memory,
-  // in the order of the splits.  Bound by two cluster barriers and one round of reads: one request over 2,040 keys, 32 heads in 8
-  // groups, 2.3 us less a layer than partial results in memory and a kernel of their own for the merge (10,512 -> 10,290 us for 96).
+  // in the order of the splits.  Bound by two cluster barriers and one round of reads; against partial results in memory and a kernel of
+  // their own for the merge see launch_decode_merged.
   cluster_sync();
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -1124,11 +1125,24 @@ int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, const void* 
   if (int e = hk_allow_smem<attention_decode_tma_kernel<HD, DIST, TW>>(smem)) return e;
   dim3 grid((unsigned)n_items, (unsigned)G);
   return hk_launch_pdl(attention_decode_tma_kernel<HD, DIST, TW>, grid, dim3((TW + 1) * 32), smem, s, mk, mv, (const bf16*)q, bt, stride,
-                       (const Item*)items, (bf16*)out, part_o, part_ml, H, G, pt, box_rows, window, scale_log2, so, pages_cap, 0, status);
+                       (const Item*)items, (bf16*)out, part_o, part_ml, H, G, pt, box_rows, window, scale_log2, so, pages_cap, 0, 1, status);
 }
 
 // The same with the splits of a request in a cluster.  Refuses more clusters than the GPU holds at once: a second wave of them would
 // cost more than the merge's own kernel does.
+//
+// Dependent launches on both sides (`early`) gain the most, 3.5 us a layer of one request, but the next kernel's blocks then go to those
+// SMs that have room while clusters lie on the others.  The output projection of up to 8 rows is such a kernel, a block for 16 of its
+// columns: where it has more of them than the GPU has SMs, or clusters fill most of the GPU's shared memory, some SMs get far more of it
+// than others, and it takes up to 8 us longer.  There the launches are plain ones, and where a split may have more than 1,024 keys, fewer
+// CTAs than SMs, which clusters put in pairs on few of them, are refused (two requests over 8,000 tokens: 105.5 us where the other way takes
+// 104.0).  Whole layers, us, merged by a kernel of its own / in clusters, early / plain (contexts of 2,040; 300 and 8,000 alike):
+//     heads 32 in 8 of 128 (4,096 columns)        heads 16 in 4 of 128 (2,048 columns)        heads 32 in 8 of 64 (2,048 columns)
+//     requests  1    94.5 /  90.8 /  93.7         requests  1   48.2 / 44.6 / 47.4            requests  1   46.6 / 44.2 / 46.8
+//               2    95.5 / 101.3 /  95.2                   4   50.9 / 48.5 / 50.8                      4   50.4 / 47.9 / 49.6
+//               4    98.9 / 102.7 /  97.8                   7   54.4 / 54.1 / 53.0                      7   54.1 / 51.2 / 52.1
+//               8   104.9 / 110.2 / 103.4                   8   55.0 / 58.4 / 53.6                      8   55.4 / 52.6 / 53.1
+//              16   128.4 / 124.1 / 126.4                  16   78.3 / 73.9 / 75.6                     16   80.5 / 78.0 / 77.2
 template <int HD, bool DIST>
 int launch_decode_merged(const CUtensorMap& mk, const CUtensorMap& mv, const void* q, const int* bt, int stride, const void* items,
                          int n_items, int splits, void* out, int H, int G, int pt, int box_rows, int window, float scale_log2, ScoreOpts so,
@@ -1161,10 +1175,14 @@ int launch_decode_merged(const CUtensorMap& mk, const CUtensorMap& mv, const voi
     }
     most[dev][splits].store(++held);
   }
-  if ((long long)(n_items / splits) * G > held - 1) return HK_ERR_UNSUPPORTED;
-  cfg.numAttrs = 2;
+  const long long clusters = (long long)(n_items / splits) * G;
+  if (clusters > held - 1) return HK_ERR_UNSUPPORTED;
+  const long long ctas = clusters * splits, sms = sm_count();
+  const bool early = n_items / splits > 8 || (H * HD > 16 * sms ? 2 * ctas <= sms : 8 * ctas * (long long)(smem + 1024) <= 5 * sms * 228 * 1024);
+  if (!early && ctas <= sms && (long long)(pages_cap - 2) * pt > 1024) return HK_ERR_UNSUPPORTED;
+  cfg.numAttrs = early ? 2 : 1;
   return (int)cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<HD, DIST, TW>, mk, mv, (const bf16*)q, bt, stride, (const Item*)items, (bf16*)out,
-                                 (float*)nullptr, (float*)nullptr, H, G, pt, box_rows, window, scale_log2, so, pages_cap, splits, status);
+                                 (float*)nullptr, (float*)nullptr, H, G, pt, box_rows, window, scale_log2, so, pages_cap, splits, early ? 1 : 0, status);
 }
 
 }  // namespace
