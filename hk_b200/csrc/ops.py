@@ -1503,8 +1503,11 @@ def routed_experts(x, ids, weights, w_gate_up, w_down, y, act: str = "silu", lim
 
 def zero_slot(table: torch.Tensor, slot: int, most_bytes: int) -> None:
     """Zeroes one request's slot in every state of a cache: `table` int64 [states, 2] = (address, bytes a slot), of tensors that the
-    caller keeps; `most_bytes`: the most that a state has to a slot."""
+    caller keeps; `most_bytes`: the most that a state has to a slot.  On the table's device, whichever is current."""
     _need(table, "table", torch.int64, 2)
+    if table.device.index != torch._C._cuda_getDevice():
+        with torch.cuda.device(table.device.index):
+            return zero_slot(table, slot, most_bytes)
     _check(build.load("elementwise").hk_zero_slot(_ptr(table), int(table.shape[0]), slot, most_bytes, _stream()), "zero_slot")
 
 

@@ -139,3 +139,30 @@ def test_pages_passed_says_what_release_would_give_back():
     assert books.pages_passed(s) == [0, 5]
     assert books.release_passed(s) == 5 and books.pages_passed(s) == [0, 0]
     books.audit()
+
+
+def test_a_slot_is_zeroed_on_the_device_that_holds_it(monkeypatch):
+    """With another device current, the launch goes to the states' device and its stream (on the CPU: against stand-ins for both)."""
+    import contextlib
+    import types
+
+    import torch
+
+    from hk_b200.csrc import build, ops
+    current, launched = [1], []
+
+    @contextlib.contextmanager
+    def device(index):
+        old, current[0] = current[0], index
+        yield
+        current[0] = old
+    monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: current[0], raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 100 + index, raising=False)
+    monkeypatch.setattr(ops, "_need", lambda *a, **k: None)
+    lib = types.SimpleNamespace(hk_zero_slot=lambda table, n, slot, most, stream: launched.append((current[0], stream)) or 0)
+    monkeypatch.setattr(build, "load", lambda name: lib)
+    for index in (0, 1):
+        table = types.SimpleNamespace(device=types.SimpleNamespace(index=index), shape=(2, 2), data_ptr=lambda: 16)
+        ops.zero_slot(table, 3, 64)
+    assert launched == [(0, 100), (1, 101)] and current == [1]
