@@ -466,6 +466,13 @@ def grouped_tile_rows(pairs: int, experts: int) -> int:
     return 64 if each <= 32 else 128 if each <= 100 else 256
 
 
+def grouped_takes(x, *weights) -> bool:
+    """Whether the grouped product on the tensor cores takes rows x, as they lie, by each of the experts' weights [E, N, K]; what it does
+    not take goes to the product by FMAs."""
+    return x.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and \
+        all(w.data_ptr() % 16 == 0 and w.is_contiguous() and w.shape[0] * w.shape[1] < 2 ** 31 for w in weights)
+
+
 def run_pair_grouped(a, w, out, tiles, offsets, tile_rows: int, gated: bool, act: int = 0, limit: float = 0.0, slope: float = 1.0) -> bool:
     """out[p] = a[p] w[group of p]^T for the rows p that `tiles` and `offsets` name (`hk_gemm_pair_grouped`); gated: act 0 (silu) or 2
     (the clamped form) of the two halves.  False when the kernel refuses."""

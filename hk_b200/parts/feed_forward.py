@@ -226,7 +226,7 @@ class RoutedFeedForward(Part):
             shared_y = torch.empty((n, self.hidden), dtype=torch.float32, device=dev)
             self.shared.forward(xb, shared_y, ctx, accumulate=False)
         glu = {"act": self.act, "limit": self.limit, "slope": self.slope}
-        fast = xb.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.F % 8 == 0
+        fast = xb.dtype == torch.bfloat16 and self.F % 8 == 0 and gemm_fast.grouped_takes(xb, self.w_gate_up, self.w_down)
         if fast and pairs < self.TC_MIN_PAIRS:
             ops.routed_experts(xb, ids, weights, self.w_gate_up, self.w_down, residual, accumulate=accumulate, shared=shared_y,
                                shared_gate=shared_gate, identities=bool(self.identity), factor=self.out_scale, **glu)
@@ -245,7 +245,7 @@ class RoutedFeedForward(Part):
             ops.route_gather(xb, perm, offsets, self.top, xs)
             if not (ops.grouped_gemm_tc(xs, self.w_gate_up, h, tiles, offsets, rows, gated=True, **glu)
                     and ops.grouped_gemm_tc(h, self.w_down, ys, tiles, offsets, rows, gated=False)):
-                raise ops.KernelError("the grouped product refuses the experts' weights")
+                raise ops.KernelError("the grouped product refuses what `grouped_takes` lets through")
         else:
             ops.grouped_gemm(xb, self.w_gate_up, h, tiles, offsets, perm, self.top, gather=True, gated=True, **glu)
             ops.grouped_gemm(h, self.w_down, ys, tiles, offsets, perm, self.top, gather=False, gated=False)

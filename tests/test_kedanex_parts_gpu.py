@@ -332,6 +332,20 @@ def test_routed_feed_forward(dtype, d, F, E, top, n):
         close(y2.double().cpu().numpy(), y[some].double().cpu().numpy(), dtype)
 
 
+@pytest.mark.parametrize("n", [50, 700])
+def test_routed_feed_forward_of_rows_off_16_bytes(n):
+    from hk_b200.parts import RoutedFeedForward
+    d, F, E, top = 64, 48, 6, 2
+    part = RoutedFeedForward(d, F, E, top, "f.")
+    bind_random(part, torch.bfloat16, std=0.3)
+    wide = torch.randn(n * d + 1, device="cuda").bfloat16()
+    x = wide[1:].view(n, d)
+    got, want = (torch.empty(n, d, device="cuda") for _ in range(2))
+    part.forward(x, got, None, accumulate=False)
+    part.forward(x.clone(), want, None, accumulate=False)
+    close(got.double().cpu().numpy(), want.double().cpu().numpy(), torch.bfloat16)
+
+
 @pytest.mark.parametrize("dtype", DTYPES, ids=IDS)
 @pytest.mark.parametrize("with_ffn", [True, False])
 def test_sandwich_norm_block(dtype, with_ffn):
