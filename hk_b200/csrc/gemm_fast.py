@@ -316,10 +316,13 @@ def run_pair(a, w, out, epilogue: int, ldo: int, tiles_m: int, slices: int, limi
     return True
 
 
-def _run_pair_where_chosen(a, w, out, epilogue: int, ldo: int, limit: float = 0.0, slope: float = 1.0) -> bool:
-    if _tc_bn or _tc_splits:
+def _run_pair_where_chosen(a, w, out, choice: Optional[str], epilogue: int, ldo: int, limit: float = 0.0, slope: float = 1.0) -> bool:
+    """The product on pairs where `pair_config` picks it; everywhere when it is pinned, nowhere when the other tcgen05 kernel is."""
+    if choice == "tc" or _tc_bn or _tc_splits:
         return False
     chosen = pair_config(a.shape[0], w.shape[0], a.shape[1], _sms(a.device), epilogue in (2, 3, 4))
+    if chosen is None and choice == "pair":
+        chosen = (-(-a.shape[0] // 256), 1)
     return chosen is not None and run_pair(a, w, out, epilogue, ldo, *chosen, limit, slope)
 
 
@@ -351,8 +354,10 @@ def run(a, w, out, accumulate: bool, choice: Optional[str]) -> bool:
             return False
         ops._check(code, "gemm (small-M)")
         return True
-    if _run_pair_where_chosen(a, w, out, 1 if accumulate else 0, N):
+    if _run_pair_where_chosen(a, w, out, choice, 1 if accumulate else 0, N):
         return True
+    if choice == "pair":
+        return False
     clusters = None if _tc_bn or _tc_splits else cluster_config(M, N, K, _sms(a.device))
     if clusters is not None and run_cluster(a, w, out, accumulate, *clusters):
         return True
@@ -385,8 +390,10 @@ def run_swiglu(a, w_gate_up, out, choice: Optional[str] = None, act: int = 0, li
             return False
     if choice is None and M <= SMALL_M_AUTO:
         return False             # few rows, small weights: the small-M product and the swiglu kernel
-    if _run_pair_where_chosen(a, w_gate_up, out, epilogue, out.shape[1], limit, slope):
+    if _run_pair_where_chosen(a, w_gate_up, out, choice, epilogue, out.shape[1], limit, slope):
         return True
+    if choice == "pair":
+        return False
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device), swiglu=True)
     partial = _tc_partial(lib, M, N, splits, a.device)
@@ -425,8 +432,10 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
             return False
         ops._check(code, "gemm+squared relu (small-M)")
         return True
-    if _run_pair_where_chosen(a, w, out, 5, N, slope=factor):
+    if _run_pair_where_chosen(a, w, out, choice, 5, N, slope=factor):
         return True
+    if choice == "pair":
+        return False
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)
@@ -439,14 +448,16 @@ def run_squared_relu(a, w, out, factor: float, choice: Optional[str] = None) -> 
     return True
 
 
-def run_narrow(a, w, out) -> bool:
-    """out (bf16 [M, N]) = a w^T on the tcgen05 kernel.  False when it refuses the shape."""
+def run_narrow(a, w, out, choice: Optional[str] = None) -> bool:
+    """out (bf16 [M, N]) = a w^T on a tcgen05 kernel ('tc' and 'pair' pin one of them).  False when it refuses the shape."""
     M, K = a.shape
     N = w.shape[0]
     if not _aligned(a, w):
         return False
-    if _run_pair_where_chosen(a, w, out, 6, N):
+    if _run_pair_where_chosen(a, w, out, choice, 6, N):
         return True
+    if choice == "pair":
+        return False
     lib = build.load("gemm_tc")
     bn, splits = tc_config(M, N, K, _sms(a.device))
     partial = _tc_partial(lib, M, N, splits, a.device)

@@ -93,8 +93,8 @@ def forced(kind: str) -> Optional[str]:
 
 @contextlib.contextmanager
 def force(gemm: Optional[str] = None, attention: Optional[str] = None):
-    """Pins the kernel family inside the block: gemm in {'generic','tc','smallm','stream'},
-    attention in {'generic','flash','flash_cp'} ('flash_cp': the flash kernels without the TMA-fed decode
+    """Pins the kernel family inside the block: gemm in {'generic','tc','pair','smallm','stream'} ('tc': the tcgen05 product of
+    one SM a tile, 'pair': the one on pairs of SMs), attention in {'generic','flash','flash_cp'} ('flash_cp': the flash kernels without the TMA-fed decode
     variant).  A pinned kernel that refuses the shape raises."""
     old = dict(_forced)
     if gemm is not None:
@@ -266,7 +266,7 @@ def gemm_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, act
     M, F = out.shape
     if a.shape[0] != M or w_gate_up.shape != (2 * F, a.shape[1]):
         raise KernelError("gemm_swiglu: shapes do not fit")
-    if a.dtype == torch.bfloat16 and _forced["gemm"] in (None, "tc", "stream"):
+    if a.dtype == torch.bfloat16 and _forced["gemm"] in (None, "tc", "pair", "stream"):
         if gemm_fast.run_swiglu(a, w_gate_up, out, _forced["gemm"], act=GLU_ACTS[act], limit=limit, slope=slope):
             return
     gu = torch.empty((M, 2 * F), dtype=torch.float32, device=a.device)
@@ -701,7 +701,7 @@ def gemm_narrow(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     _need(out, "out", torch.bfloat16, 2)
     if a.shape[1] != w.shape[1] or tuple(out.shape) != (a.shape[0], w.shape[0]):
         raise KernelError("gemm_narrow: shapes do not fit")
-    if not gemm_fast.run_narrow(a, w, out):
+    if not gemm_fast.run_narrow(a, w, out, _forced["gemm"]):
         raise KernelError("gemm_narrow: the tcgen05 kernel refuses this shape")
 
 

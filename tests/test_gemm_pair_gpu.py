@@ -132,3 +132,28 @@ def test_pair_products_one_after_the_other(blocks):
                 assert bool(((out.double() - want).abs() <= bound).all())
                 out.fill_(float("nan"))
     gemm_fast.check_status(w.device)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [40, 300])
+def test_pinned_products(rows, monkeypatch):
+    """'tc' is the product of one SM a tile and 'pair' the one on pairs, through every epilogue and whatever the rule would take."""
+    from hk_b200.csrc import ops
+    gen = torch.Generator("cuda").manual_seed(rows)
+    a, w = (torch.randn(n, 1024, generator=gen, device="cuda").bfloat16() for n in (rows, 4096))
+    ran, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda code, what, **more: (ran.append(what), check(code, what, **more)))
+    results = {}
+    for kernel in ("tc", "pair"):
+        with ops.force(gemm=kernel):
+            outs = [torch.empty(rows, n, dtype=t, device="cuda") for n, t in ((4096, torch.float32), (2048, torch.bfloat16), (4096, torch.bfloat16),
+                                                                              (4096, torch.bfloat16))]
+            ops.gemm(a, w, outs[0])
+            ops.gemm_swiglu(a, w, outs[1])
+            ops.gemm_squared_relu(a, w, outs[2], 0.5)
+            ops.gemm_narrow(a, w, outs[3])
+        assert len(ran) == 4 and all(("pairs" in name) == (kernel == "pair") and "tcgen05" in name for name in ran), ran
+        ran.clear()
+        results[kernel] = outs
+    for x, y in zip(results["tc"], results["pair"]):        # float32 sums in another order, then at most one rounding to bfloat16
+        assert float((x.double() - y.double()).norm() / x.double().norm()) <= (2e-6 if x.dtype == torch.float32 else 1e-3)
