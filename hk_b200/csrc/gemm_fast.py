@@ -500,8 +500,3 @@ def run_pair_grouped(a, w, out, tiles, offsets, tile_rows: int, gated: bool, act
         return False
     ops._check(code, "grouped gemm (tcgen05, pairs)")
     return True
-
-
-def run_grouped(*args, **kwargs) -> bool:
-    """`run_pair_grouped` for prompt-sized steps, whose rows are in the experts' order already."""
-    return run_pair_grouped(*args, **kwargs)

@@ -1458,7 +1458,7 @@ def grouped_gemm_tc(a, w, out, tiles, offsets, tile_rows: int, gated: bool, act:
     """The grouped product on the tensor cores for rows that are in the experts' order: a bf16 [pairs, K], `tiles` and `offsets` of
     `route_sort` with `tile_rows`; w bf16 [E, N, K] (gated: [E, 2N, K]); out float32 [pairs, N], or bf16 silu(gate) * up (or the
     clamped form) when gated.  False when the kernel refuses the shape."""
-    return gemm_fast.run_grouped(a, w, out, tiles, offsets, tile_rows, gated, GLU_ACTS[act], limit, slope)
+    return gemm_fast.run_pair_grouped(a, w, out, tiles, offsets, tile_rows, gated, GLU_ACTS[act], limit, slope)
 
 
 _grouped_product = None

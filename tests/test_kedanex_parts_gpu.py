@@ -302,7 +302,7 @@ def test_polynorm_feed_forward(dtype, d, F):
                                          (40, 12, 3, 2, 33), (36, 20, 40, 4, 90), (128, 96, 1, 1, 70),
                                          # prompt-sized steps: in bfloat16 the tcgen05 grouped product takes them
                                          (64, 48, 6, 2, 700), (128, 96, 4, 3, 400), (256, 64, 8, 2, 1120), (72, 40, 3, 1, 1500)])
-def test_routed_feed_forward(dtype, d, F, E, top, n):
+def test_routed_feed_forward(dtype, d, F, E, top, n, monkeypatch):
     from hk_b200.parts import RoutedFeedForward
     part = RoutedFeedForward(d, F, E, top, "f.")
     prec, w = bind_random(part, dtype, std=0.3)
@@ -312,24 +312,23 @@ def test_routed_feed_forward(dtype, d, F, E, top, n):
     gap = logits[:, E - top] - logits[:, E - top - 1] if top < E else np.ones(n)
     assert gap.min() > 1e-4                          # no row rests on a close call
     y = torch.full((n, d), float("nan"), device="cuda")
-    from hk_b200.csrc import gemm_fast
-    taken, plain_run = [], gemm_fast.run_grouped
-    gemm_fast.run_grouped = lambda *a, **k: taken.append(plain_run(*a, **k)) or taken[-1]
-    try:
-        part.forward(x, y, None, accumulate=False)
-    finally:
-        gemm_fast.run_grouped = plain_run
-    # a prompt-sized bfloat16 step took the tcgen05 grouped product for both of its products, nothing else did
-    assert taken == ([True, True] if dtype == torch.bfloat16 and n * top >= part.TC_MIN_PAIRS else [])
+    from hk_b200.csrc import ops
+    ran, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda code, what, *more, **named: (ran.append(what), check(code, what, *more, **named)))
+    part.forward(x, y, None, accumulate=False)
+    products = [name for name in ran if "grouped" in name or "experts" in name]
+    if dtype == torch.float32:
+        assert products == ["grouped_gemm"] * 2                                         # FMAs
+    elif d % 8 == 0 and F % 8 == 0:     # tensor cores: in one call for a small step, one by one for a prompt
+        assert products == (["routed_experts"] if n * top < part.TC_MIN_PAIRS else ["grouped gemm (tcgen05, pairs)"] * 2)
+    else:                               # each product by its own K
+        assert products == ["grouped gemm (tcgen05, pairs)" if k % 8 == 0 else "grouped_gemm" for k in (d, F)]
     close(y.double().cpu().numpy(), K.routed_ff(xn, w, "f.", E, top), dtype)
     # a row's result does not depend on which rows share the batch
     some = [0, n // 2, n - 1]
     y2 = torch.empty((len(some), d), device="cuda")
     part.forward(x[some].contiguous(), y2, None, accumulate=False)
-    if dtype == torch.float32 or n * top < part.TC_MIN_PAIRS:
-        assert torch.equal(y2, y[some])
-    else:                       # a few rows take another kernel than a prompt does: equal to rounding
-        close(y2.double().cpu().numpy(), y[some].double().cpu().numpy(), dtype)
+    assert torch.equal(y2, y[some])
 
 
 @pytest.mark.parametrize("n", [50, 700])
