@@ -104,7 +104,7 @@ class _SegmentScan(Part):
 class _ChunkedScan(_SegmentScan):
     """A recurrence that, when serving in bfloat16, walks the requests of a step in chunks of tokens (`csrc/delta_chunks.cu`)
     where a long one sets the time of the walk token by token; the lists of requests and chunks are host-built tables that the
-    mixers of a kind with heads as many and as large share.
+    mixers with the same rule share: a kind, with heads as many and as large.
 
     A walk's time grows with the longest request until requests times heads fill the SMs; the chunks' with all rows.  From
     `CHUNKS_FROM` tokens on the chunks' kernels are the faster at every size (one request of 64 tokens 20 us against 26 to 34, one
@@ -120,7 +120,7 @@ class _ChunkedScan(_SegmentScan):
     LONGEST_FROM = 640
     ROWS_FROM = 320 * 64
     BESIDE = 256
-    WALK = 0.0                      # a kind's walk time in the delta rule's (0: not measured; the first of the two lines alone)
+    WALK = 0.0                      # a kind's walk time in the delta rule's; 0 for a kind that states none: the first of the two lines alone
     CHUNK_NS = 2.4                  # a row's time in chunks, by head
     _chunks = False                 # set at bind: the chunked form takes this mixer's sizes
 
@@ -132,7 +132,7 @@ class _ChunkedScan(_SegmentScan):
         self._chunks = precision.compute == torch.bfloat16 and row % 4 == 0 and ops.delta_chunks_take(self.dk, self.dv, decay_scale)
 
     def step_tables_key(self):
-        return ("chunked_segments", self.H, self.dk, self.dv, self.WALK) if self._chunks else SEGMENTS_KEY
+        return ("chunked_segments", self.H, self.dk, self.dv, self.WALK, self.CHUNK_NS) if self._chunks else SEGMENTS_KEY
 
     def _chunks_pay(self, lengths) -> bool:
         """Whether a step takes chunks for requests of these numbers of tokens, each `CHUNKS_FROM` or more."""

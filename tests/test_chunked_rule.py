@@ -23,3 +23,13 @@ def part_of(kind, heads, dim):
 ])
 def test_which_steps_go_in_chunks(kind, heads, dim, lengths, chunks):
     assert part_of(kind, heads, dim)._chunks_pay(lengths) is chunks
+
+
+def test_kinds_that_weigh_chunks_differently_share_no_tables():
+    """The choice follows from a kind's walk and its chunks' time; the tables of a step are shared by their key."""
+    parts = [part_of(kind, 64, 64) for kind in ("delta", "gated", "retention", "mlstm", "delta")]
+    for part in parts:
+        part._chunks = True
+    keys = [part.step_tables_key() for part in parts]
+    assert keys[0] == keys[4] and len(set(keys)) == 4
+    assert not parts[0]._chunks_pay([157] * 6) and parts[1]._chunks_pay([157] * 6)
