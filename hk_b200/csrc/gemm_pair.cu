@@ -509,7 +509,8 @@ HK_API long long hk_gemm_pair_partial_floats(int M, int N, int tiles_m, int slic
 // out = a w^T with the epilogues of hk_gemm_tc (0 store, 1 add, 2 to 4 gated, 5 squared relu, 6 narrowed; `limit` and `slope` as
 // there).  tiles_m: tiles along the rows of a, of at most 256 rows each; slices: how many slices K is cut into (above 1, `partial`
 // holds hk_gemm_pair_partial_floats of scratch); pairs: pairs of SMs at work.  `status`: a device int that a timed-out wait sets.
-// Refuses (HK_ERR_UNSUPPORTED) K that is no multiple of 8, a or w off a 16-byte boundary, gated products of odd N.
+// Refuses (HK_ERR_UNSUPPORTED) K that is no multiple of 8, a or w off a 16-byte boundary, gated products of odd N, and more rows than
+// 32-bit products of tiles and blocks of 32 rows hold (from about four million on).
 HK_API int hk_gemm_pair(const void* a, const void* w, void* out, int M, int N, int K, long long ldo, int epilogue, int tiles_m, int slices,
                         int pairs, float* partial, int* status, float limit, float slope, void* stream) {
   if (M <= 0 || N <= 0) return 0;
@@ -522,6 +523,7 @@ HK_API int hk_gemm_pair(const void* a, const void* w, void* out, int M, int N, i
   s.tiles_m = tiles_m;
   s.slices = slices;
   if (tiles_m < 1 || tiles_m > s.units || widest(s) > MAX_W || slices < 1 || slices > s.kb || pairs < 1) return HK_ERR_UNSUPPORTED;
+  if ((long long)tiles_m * s.units > 0x7fffffffLL) return HK_ERR_UNSUPPORTED;      // (a tile's rows are found with 32-bit products)
   const long long tiles = (long long)((N + FT - 1) / FT) * tiles_m;
   if (tiles * slices > 0x3fffffffLL || (slices > 1 && partial == nullptr)) return HK_ERR_UNSUPPORTED;
   s.tiles = (int)tiles;

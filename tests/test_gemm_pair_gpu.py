@@ -157,3 +157,13 @@ def test_pinned_products(rows, monkeypatch):
         results[kernel] = outs
     for x, y in zip(results["tc"], results["pair"]):        # float32 sums in another order, then at most one rounding to bfloat16
         assert float((x.double() - y.double()).norm() / x.double().norm()) <= (2e-6 if x.dtype == torch.float32 else 1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [4_200_000, 40_000_000, 2 ** 31 - 33])
+def test_more_rows_than_the_tiles_count_are_refused(rows):
+    """Before anything is launched: the addresses belong to nothing."""
+    from hk_b200.csrc import build
+    lib = build.load("gemm_pair")
+    for epilogue in (0, 2):
+        assert lib.hk_gemm_pair(1 << 20, 1 << 20, 1 << 20, rows, 4096, 4096, 4096, epilogue, -(-rows // 256), 1, 74, 0, 1 << 20, 0.0, 1.0, 0) == 100001
