@@ -15,6 +15,7 @@ Shapes all of them refuse (K not a multiple of 8, unaligned operands) go to the 
 """
 from __future__ import annotations
 
+import ctypes
 import functools
 from typing import Optional
 
@@ -265,38 +266,23 @@ PAIR_M = 128            # from here on the rows' padding to 32 instead of 128 an
 PAIR_K = 1024           # below, a tile's start and end weigh more than its loop: 4,096 x 512 by 527 rows 7.9 us, on pairs 8.7
 
 
-def _tc_time(M: int, N: int, K: int, bn: int, splits: int, sms: int) -> float:
-    """The time in us of the kernel of one SM a tile, fitted to 2,000 measured (shape, width, slices) as `pair_config`'s."""
-    tiles, k_blocks, last = -(-M // 128) * -(-N // bn), -(-K // 64), 0.0208 * bn
-    loop = k_blocks / splits * max(0.234, 0.024 + 0.00157 * bn)
-    slices = 1.7 + 1.4e-6 * M * N * splits if splits > 1 else 0.0
-    return max(-(-tiles * splits // sms) * max(loop, last), N * K / 2.92e6) + 0.5 * last + slices + 2.6
-
-
 @functools.lru_cache(maxsize=4096)
 def pair_config(M: int, N: int, K: int, sms: int, gated: bool = False):
     """(tiles along the rows, K slices) of the product on pairs of SMs, or None where the kernel of one SM a tile stays: up to
     128 rows, short K, and where two row tiles of that kernel fill one wave of SMs better (10,304 x 2,048 by 256 rows 15.5 us, on
     pairs 17.6; 2,048 x 6,144 by 256 14.1 and 17.5, by 1,000 24.9 and 22.2).
-    Both times come from models that were fitted to measured ones, 130 to 2,048 rows by the products of layers 2,048 and 4,096
-    wide; what they pick is within 1 % of the best of the measured choices on average."""
-    pairs, units, k_blocks, f_tiles = sms // 2, -(-M // 32), -(-K // 64), -(-N // 256)
+    The two times come from models in `runtime.cpp`."""
     if M <= PAIR_M or K < PAIR_K:
         return None
-    best = None
-    for tiles_m in range(-(-units // 8), min(units, -(-units // 8) + 7) + 1):
-        width, tiles = 32 * units / tiles_m, f_tiles * tiles_m
-        for slices in (1, 2, 3, 4):
-            if slices > 1 and (tiles * slices > pairs or k_blocks < 16 * slices):
-                break
-            loop, last = k_blocks / slices * max(0.184, 0.084 + 0.0012 * width), 0.0235 * width         # `last`: a tile's epilogue
-            waves = -(-tiles * slices // pairs)
-            cost = waves * max(loop, last) + 0.8 * (waves - 1) + 0.5 * last + (4.0 * slices - 1.0 if slices > 1 else 0.0)
-            if best is None or cost < best[0]:
-                best = (cost, tiles_m, slices)
-    if best[0] + 3.0 > 1.08 * _tc_time(M, N, K, *tc_config(M, N, K, sms, gated), sms):
-        return None
-    return best[1:]
+    found = _pair_choice()(M, N, K, sms, *tc_config(M, N, K, sms, gated))
+    return (found // 8, found % 8) if found else None
+
+
+@functools.lru_cache(maxsize=1)
+def _pair_choice():
+    choose = build.load("runtime").hk_pair_config
+    choose.argtypes, choose.restype = [ctypes.c_longlong] * 6, ctypes.c_longlong
+    return choose
 
 
 def run_pair(a, w, out, epilogue: int, ldo: int, tiles_m: int, slices: int, limit: float = 0.0, slope: float = 1.0) -> bool:

@@ -1,6 +1,6 @@
-// Host-side runtime of the paged cache, in C++ behind a C interface: page pools with ownership checks, block
-// tables for every layer group, request slots, window release, rewind and a full audit.  Nothing here touches
-// the GPU; the Python classes in hk_b200/cache/pages.py are thin views of these objects (tables and lengths are
+// Host-side runtime, in C++ behind a C interface.  The paged cache's books: page pools with ownership checks, block
+// tables for every layer group, request slots, window release, rewind and a full audit; and, at the end, the choice
+// between two matrix products.  Nothing here touches the GPU; the Python classes in hk_b200/cache/pages.py are thin views of these objects (tables and lengths are
 // read in place through numpy).
 //
 // Every call that can fail returns a negative code and leaves the books unchanged; hk_books_error() gives the
@@ -298,4 +298,43 @@ HK_API int hk_books_audit(void* h) {
       return b.fail(ERR_CACHE, "group " + std::to_string(gi) + ": " + std::to_string(g.pool.n - held - (int)g.pool.free_list.size()) + " pages lost");
   }
   return 0;
+}
+
+// ---- the choice between the two tcgen05 products -----------------------------------------------------------------------------------
+// Both times are models in us, fitted to 2,000 measured (shape, tiles, slices) of 130 to 2,048 rows by the products of layers 2,048 and
+// 4,096 wide; what they pick is within 1 % of the best of the measured choices on average.  Here and not in Python, because a mixed step
+// brings a new number of rows nearly every time: 15 us a shape there, 1 here.
+namespace {
+int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// The kernel of one SM a tile, with tiles of bn columns and K in `splits` slices.
+double one_sm_time(int64_t M, int64_t N, int64_t K, int64_t bn, int64_t splits, int64_t sms) {
+  const double last = 0.0208 * (double)bn;
+  const double loop = (double)ceil_div(K, 64) / (double)splits * std::max(0.234, 0.024 + 0.00157 * (double)bn);
+  const double slices = splits > 1 ? 1.7 + 1.4e-6 * (double)M * (double)N * (double)splits : 0.0;
+  const int64_t tiles = ceil_div(M, 128) * ceil_div(N, bn);
+  return std::max((double)ceil_div(tiles * splits, sms) * std::max(loop, last), (double)N * (double)K / 2.92e6) + 0.5 * last + slices + 2.6;
+}
+}  // namespace
+
+// The tiles along the rows and the K slices (tiles * 8 + slices) of the product on pairs of SMs, or 0 where the other kernel, at the
+// width and slices that it would get, is not 8 % slower.
+HK_API long long hk_pair_config(long long M, long long N, long long K, long long sms, long long bn, long long splits) {
+  const int64_t pairs = sms / 2, units = ceil_div(M, 32), k_blocks = ceil_div(K, 64), f_tiles = ceil_div(N, 256), fewest = ceil_div(units, 8);
+  double best = 0.0;
+  int64_t best_tiles = 0, best_slices = 0;
+  for (int64_t tiles_m = fewest; tiles_m <= std::min(units, fewest + 7); ++tiles_m) {
+    const double width = 32.0 * (double)units / (double)tiles_m, last = 0.0235 * width;         // `last`: a tile's epilogue
+    const int64_t tiles = f_tiles * tiles_m;
+    for (int64_t slices = 1; slices <= 4; ++slices) {
+      if (slices > 1 && (tiles * slices > pairs || k_blocks < 16 * slices)) break;
+      const double loop = (double)k_blocks / (double)slices * std::max(0.184, 0.084 + 0.0012 * width);
+      const int64_t waves = ceil_div(tiles * slices, pairs);
+      const double cost = (double)waves * std::max(loop, last) + 0.8 * (double)(waves - 1) + 0.5 * last +
+                          (slices > 1 ? 4.0 * (double)slices - 1.0 : 0.0);
+      if (best_tiles == 0 || cost < best) best = cost, best_tiles = tiles_m, best_slices = slices;
+    }
+  }
+  if (best + 3.0 > 1.08 * one_sm_time(M, N, K, bn, splits, sms)) return 0;
+  return best_tiles * 8 + best_slices;
 }

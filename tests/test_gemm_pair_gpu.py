@@ -22,6 +22,20 @@ def test_rule_gives_what_the_kernel_takes():
                 assert 1 <= tiles_m <= units and -(-units // tiles_m) <= 8 and 1 <= slices <= -(-k // 64)
 
 
+def test_rule_picks():
+    """Some of the choices (tiles along the rows, K slices), as the times that the models were fitted to have them."""
+    from hk_b200.csrc import gemm_fast
+    picks = {(527, 6144, 4096, False): (3, 1),
+             (527, 24576, 4096, True): (3, 1),
+             (527, 4096, 12288, False): (4, 1),
+             (2048, 24576, 4096, True): (9, 1),
+             (300, 4096, 4096, False): (4, 1),
+             (256, 8256, 2048, False): (2, 1),
+             (1000, 4096, 12288, False): (4, 1),
+             (200, 4096, 12288, False): (2, 2)}
+    assert {s: gemm_fast.pair_config(*s[:3], 148, s[3]) for s in picks} == picks
+
+
 def _reference(a, w, epilogue, start, limit, slope):
     z = a.double() @ w.double().T
     if epilogue in (2, 3, 4):
