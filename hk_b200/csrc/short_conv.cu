@@ -99,8 +99,7 @@ short_conv_kernel(const float* __restrict__ x, long long ldx, const float* __res
 
 // The same for up to four taps and channels in whole 16-byte pieces: a thread makes four channels of eight tokens, everything it reads
 // asked for at once, with the sums in the same order.  A block's tokens are found by counting through the segments, so that no block is
-// launched for tokens that do not exist.  Bound by its bytes and the activations: four requests
-// of 512 tokens by 6,144 channels 31.3 -> 21.4 us (3.5 TB/s), by 4,352 23.0 -> 16.0; 64 requests of one token 13.1 -> 11.4.
+// launched for tokens that do not exist.  Bound by its bytes and the activations (which steps take it, and both times: see short_conv).
 #define SCV_TOKENS 8
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -184,8 +183,8 @@ short_conv_vec_kernel(const float* __restrict__ x, long long ldx, const float* _
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const int r = count - back + j;
-      const float* h = r == -1 ? in[2] : r == -2 ? in[1] : in[0];
-      if (j < back) keep[j] = r >= 0 ? *reinterpret_cast<const float4*>(xp + (size_t)r * ldx) : make_float4(h[0], h[1], h[2], h[3]);
+      auto held = [&](int e) { return r == -1 ? in[2][e] : r == -2 ? in[1][e] : in[0][e]; };       // (selects: an address would cost local memory)
+      if (j < back) keep[j] = r >= 0 ? *reinterpret_cast<const float4*>(xp + (size_t)r * ldx) : make_float4(held(0), held(1), held(2), held(3));
     }
 #pragma unroll
     for (int j = 0; j < 3; ++j)
@@ -196,13 +195,21 @@ short_conv_vec_kernel(const float* __restrict__ x, long long ldx, const float* _
 template <typename T, int TAPS>
 static int short_conv(const float* x, long long ldx, const float* w, const float* bias, const int* segs, int n_seg, int n_rows, float* tail,
                       T* y, long long ldy, int C, int taps, int act, cudaStream_t s) {
-  if (taps <= 4 && !(C & 3) && !(ldx & 3) && !(ldy & 3) &&
+  // a step of single rows needs no second block of tokens; else as many as the longest segment may have
+  const int longest = n_rows - n_seg + 1, portions = (longest + SC_TOKENS - 1) / SC_TOKENS;
+  // Four channels a thread: the walk's threads go through up to 32 tokens one group of eight after the other and its blocks are counted for
+  // segments that are all as long as one may be, but finding a block's segment takes a look at all of them.  us, walk / four channels:
+  // one segment of 64, 512 and 2,048 tokens of 4,096 channels 6.7 / 5.3, 8.4 / 7.3, 20.0 / 17.3, four of 512 tokens of 6,144 29.0 / 25.5,
+  // 300 of 7 460 / 45, 16 single rows beside 512 tokens 16.0 / 10.6; 1,024 single rows beside 512 tokens 462 / 127, 4,096 beside 64 407 /
+  // 1,245 (so: at most 256 segments for each portion of tokens).  Portions of 8 tokens and less are one group to the walk as well: 64
+  // single rows beside 8 tokens of 2,048 channels 4.1 / 6.1.  Single rows alone, of 6,144 channels: 16 of them 2.9 / 3.4, 32 4.1 / 3.8,
+  // 128 9.2 / 8.5, 256 15.8 / 16.8; of 2,048 64 3.1 / 3.6, 96 4.3 / 4.1, 256 6.9 / 8.2.
+  const bool wide = longest == 1 ? n_seg <= 128 && (long long)n_seg * ((C + 127) / 128) >= 1536 : longest > 16 && n_seg <= 256LL * portions;
+  if (wide && taps <= 4 && !(C & 3) && !(ldx & 3) && !(ldy & 3) &&
       !(((uintptr_t)x | (uintptr_t)w | (uintptr_t)bias | (uintptr_t)tail | (uintptr_t)y) & 15))
     return hk_launch_pdl(short_conv_vec_kernel<T>, dim3((unsigned)(n_rows / SCV_TOKENS + n_seg), (unsigned)((C + 511) / 512)), dim3(128), 0, s, x, ldx, w,
                      bias, segs, n_seg, tail, y, ldy, C, taps, act);
-  // a step of single rows needs no second block of tokens; else as many as the longest segment may have
-  const int longest = n_rows - n_seg + 1;
-  dim3 grid((unsigned)n_seg, (unsigned)((C + 127) / 128), (unsigned)((longest + SC_TOKENS - 1) / SC_TOKENS));
+  dim3 grid((unsigned)n_seg, (unsigned)((C + 127) / 128), (unsigned)portions);
   return hk_launch(short_conv_kernel<T, TAPS>, grid, dim3(128), 0, s, x, ldx, w, bias, segs, tail, y, ldy, C, taps, act);
 }
 

@@ -362,6 +362,23 @@ def test_short_convolution_four_channels_a_thread(taps, C, out):
         assert np.array_equal(tail[slot][:taps - 1].double().cpu().numpy(), last)
 
 
+@pytest.mark.parametrize("segs,C", [([1] * 12, 16384), ([1] * 11, 16384), ([1] * 128, 1536), ([1] * 129, 1536), ([1] * 255 + [17], 132), ([1] * 256 + [17], 132),
+                                    ([1] * 511 + [33], 132), ([1] * 512 + [33], 132), ([3, 16], 64), ([1] * 3 + [14], 64)])
+def test_short_convolution_on_both_sides_of_its_lines(segs, C):
+    from hk_b200.csrc import ops
+    n, starts = sum(segs), np.cumsum([0] + segs[:-1]).tolist()
+    table = torch.tensor([[i, r, c] for i, (r, c) in enumerate(zip(starts, segs))], dtype=torch.int32, device="cuda")
+    x, wt = torch.randn(n, C, device="cuda"), torch.randn(C, 4, device="cuda")
+    tail, y = torch.randn(len(segs), 3, C, device="cuda"), torch.empty(n, C, device="cuda")
+    before = tail.clone()
+    ops.short_conv(x, wt, table, tail, y)
+    for i in {0, len(segs) // 2, len(segs) - 1}:
+        rows = torch.cat([before[i], x[starts[i]:starts[i] + segs[i]]]).double()
+        z = sum(rows[s:s + segs[i]] * wt[:, s].double() for s in range(4))
+        torch.testing.assert_close(y[starts[i]:starts[i] + segs[i]].double(), z * torch.sigmoid(z), rtol=1e-5, atol=1e-5)
+        assert torch.equal(tail[i].double(), rows[-3:])
+
+
 @pytest.mark.parametrize("n,parts,width", [(1, 1, 4), (7, 3, 1028), (4000, 1, 4), (1800, 2, 252), (1187, 3, 260), (900, 4, 512), (3600, 1, 516), (1800, 2, 1024)])
 @pytest.mark.parametrize("out", [torch.float32, torch.bfloat16], ids=IDS)
 def test_gated_norm_of_parts_a_warp_each(n, parts, width, out):
