@@ -801,7 +801,7 @@ __global__ void gated_part_norm_kernel(const float* __restrict__ y, const float*
 }
 
 // The same for many parts of up to 128 N numbers in whole 16-byte pieces: a warp per (token, part), the part's u in registers, everything
-// asked for at once, no barriers.  Bound by its bytes: 2,048 tokens of eight parts of 512 19.5 -> 11.2 us (7.5 TB/s, much of it from L2).
+// asked for at once, no barriers.  Bound by its bytes: 2,048 tokens of eight parts of 512 19.0 -> 12.5 us (6.7 TB/s, some of it from L2).
 template <typename T, int N>
 __global__ void __launch_bounds__(256)
 gated_part_norm_warp_kernel(const float* __restrict__ y, const float* __restrict__ z, long long ldz, const float* __restrict__ weight,
@@ -850,14 +850,15 @@ static int gated_part_norm(const float* y, const float* z, long long ldz, const 
   const int width = W / parts;
   const bool vec = (width & 3) == 0 && (ldz & 3) == 0 &&
                    (((uintptr_t)y | (uintptr_t)z | (uintptr_t)weight | (uintptr_t)out) & 15) == 0;
-  // From 24 warps a SM on a warp a part is the faster: 3,200 parts of 512 4.8 us both ways, 4,000 5.6 against 5.0, 6,400 8.2 against
-  // 4.7; of 1,024 numbers 2,000 parts 5.2 against 5.9, 4,000 9.2 against 7.1; few parts leave most of the SMs idle (128 of 1,024 2.1 / 4.2).
+  // From 24 warps an SM on a warp a part is the faster, from 34 on where half of its lanes and more would be idle.  us, a block / a warp a
+  // part: of 512 numbers 3,600 parts 5.5 / 5.5, 5,000 7.0 / 5.7, 12,000 14.2 / 9.8; of 256 3,600 4.4 / 3.7, 12,000 13.2 / 6.2; of 128 3,600 4.5 / 4.5;
+  // of 64 and less 3,600 4.5 / 5.7, 5,000 5.9 / 5.9, 12,000 13.2 / 9.5; few parts leave most of the SMs idle (2,000 of 512 3.8 / 3.9).  Of 1,024
+  // numbers a lane has 32 gates to divide: 3,600 parts 8.9 / 10.8, 12,000 27.7 / 28.6.
   const long long rows = (long long)n * parts;
-  if (vec && width <= 1024 && rows >= 24 * 148 && rows <= 0x7fffffffLL - 8) {
+  if (vec && width <= 512 && rows >= (width > 64 ? 24 : 34) * 148 && rows <= 0x7fffffffLL - 8) {
     const dim3 grid((unsigned)((rows + 7) / 8));
     if (width <= 256) return hk_launch_pdl(gated_part_norm_warp_kernel<T, 2>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
-    if (width <= 512) return hk_launch_pdl(gated_part_norm_warp_kernel<T, 4>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
-    return hk_launch_pdl(gated_part_norm_warp_kernel<T, 8>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
+    return hk_launch_pdl(gated_part_norm_warp_kernel<T, 4>, grid, dim3(256), 0, s, y, z, ldz, weight, out, (int)rows, parts, W, width, eps);
   }
   const int items = vec ? width / 4 : width;
   const int threads = items >= 256 ? 256 : items > 64 ? 128 : items > 32 ? 64 : 32;

@@ -379,7 +379,7 @@ def test_short_convolution_on_both_sides_of_its_lines(segs, C):
         assert torch.equal(tail[i].double(), rows[-3:])
 
 
-@pytest.mark.parametrize("n,parts,width", [(1, 1, 4), (7, 3, 1028), (4000, 1, 4), (1800, 2, 252), (1187, 3, 260), (900, 4, 512), (3600, 1, 516), (1800, 2, 1024)])
+@pytest.mark.parametrize("n,parts,width", [(1, 1, 4), (7, 3, 1028), (4000, 1, 4), (5031, 1, 4), (5040, 1, 4), (1184, 3, 68), (1800, 2, 252), (1187, 3, 260), (900, 4, 512), (3600, 1, 516), (1800, 2, 1024)])
 @pytest.mark.parametrize("out", [torch.float32, torch.bfloat16], ids=IDS)
 def test_gated_norm_of_parts_a_warp_each(n, parts, width, out):
     from hk_b200.csrc import ops
