@@ -109,7 +109,8 @@ def tc_config(M: int, N: int, K: int, sms: int, swiglu: bool = False):
     empty, a tile costing its width plus a fixed part.  Several row tiles but few waves: `_tc_ragged_config`.  One row tile
     (decode batches): with the SwiGLU epilogue, and from 48 columns an SM on, the narrowest tile that needs one wave (no slices: the
     epilogue cannot run on partial sums without a second kernel; 64 rows by 20,544 x 4,096 39.6 us with 81 tiles of 256, 32.4 with
-    143 of 144); else 128- or 256-wide tiles with K cut into slices so that every SM streams a
+    143 of 144; from 64 columns an SM on where the rows of a are less than 128 KB together, which every tile reads and which come
+    slower then: 24 rows by 8,256 x 2,048 15.0 us in one wave of tiles, 13.1 with slices, 32 rows 9.7 and 11.4); else 128- or 256-wide tiles with K cut into slices so that every SM streams a
     share of the weights.  (A finer cost model that also weighed wave tails chose more slices there and measured slower:
     the second kernel that adds the slices has a fixed cost.)"""
     m_tiles = -(-M // 128)
@@ -128,7 +129,7 @@ def tc_config(M: int, N: int, K: int, sms: int, swiglu: bool = False):
             if best is None or cost < best[0]:
                 best = (cost, cand)
         bn = best[1]
-    elif m_tiles == 1 and (swiglu or N > 48 * sms) and N <= 256 * sms:
+    elif m_tiles == 1 and (swiglu or N > (48 if M * K >= 1 << 16 else 64) * sms) and N <= 256 * sms:
         bn = min(256, max(32 if swiglu else 64, -(-N // sms + step - 1) // step * step))       # the narrowest tile width that needs one wave
         while bn < 256 and -(-N // bn) > sms:
             bn += step

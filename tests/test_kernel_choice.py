@@ -13,6 +13,14 @@ def test_tile_widths_the_tcgen05_product_chooses():
     assert bn in (128, 256) and splits > 1                               # narrow output: K slices
 
 
+def test_tile_widths_of_one_row_tile():
+    """Wide outputs in one wave of narrow tiles, unless the rows of a are few and short."""
+    from hk_b200.csrc import gemm_fast
+    cfg = gemm_fast.tc_config
+    assert cfg(31, 8256, 2048, 148) == (128, 2) and cfg(32, 8256, 2048, 148) == (64, 1) and cfg(17, 8256, 4096, 148) == (64, 1)
+    assert cfg(17, 12288, 2048, 148)[1] == 1 and cfg(24, 10304, 2048, 148) == (80, 1)
+
+
 def test_tile_widths_of_a_few_hundred_rows():
     """Several row tiles, few waves: every choice is one that the kernel takes, and none leaves half of the SMs idle."""
     from hk_b200.csrc import gemm_fast
