@@ -1159,8 +1159,8 @@ latent_prep_kernel(const float* __restrict__ q, long long ldq, const float* __re
   for (int i = lane; i < half; i += 32) {
     const int ia = pairing ? 2 * i : i, ib = pairing ? 2 * i + 1 : i + half;
     const float a = src[ia], b = src[ib];
-    dst[ia] = from_f32<T>(a * c[i] - b * s[i]);
-    dst[ib] = from_f32<T>(a * s[i] + b * c[i]);
+    dst[ia] = from_f32<T>(fmaf(a, c[i], -(b * s[i])));      // (said outright, so that both kernels round alike)
+    dst[ib] = from_f32<T>(fmaf(a, s[i], b * c[i]));
   }
   for (int i = rot + lane; i < dr; i += 32) dst[i] = from_f32<T>(src[i]);
 }
@@ -1199,8 +1199,8 @@ latent_prep_heads_kernel(const float* __restrict__ q, long long ldq, const float
   const int d = lane * 4, e0 = rot + lane, e1 = e0 + 32;      // a lane's plain dims, and what lies behind the turned ones
   auto turn = [&](T* dst, float a, float b, float x, float y) {
     if (turns) {
-      dst[ia] = from_f32<T>(a * c - b * s);
-      dst[ib] = from_f32<T>(a * s + b * c);
+      dst[ia] = from_f32<T>(fmaf(a, c, -(b * s)));
+      dst[ib] = from_f32<T>(fmaf(a, s, b * c));
     }
     if (e0 < dr) dst[e0] = from_f32<T>(x);
     if (e1 < dr) dst[e1] = from_f32<T>(y);
@@ -1231,12 +1231,9 @@ latent_prep_heads_kernel(const float* __restrict__ q, long long ldq, const float
   if (page < 0) return;   // the host never schedules this; keeps a stale table from writing out of bounds
   const float* cp = kv + (size_t)t * ldkv;
   T* out = pages + ((size_t)page * page_tokens + (pos % page_tokens)) * (r + dr);
-  float ss = 0.f;
-#pragma unroll 4
-  for (int i = d; i < r; i += 128) {
-    const float4 v = *reinterpret_cast<const float4*>(cp + i);
-    ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
-  }
+  float ss = 0.f;             // (in the order of the general kernel: a row of the cache is the same by either)
+#pragma unroll 8
+  for (int i = lane; i < r; i += 32) ss = fmaf(cp[i], cp[i], ss);
   ss = warp_sum(ss);
   const float inv = 1.0f / sqrtf(ss / (float)r + eps);
 #pragma unroll 4

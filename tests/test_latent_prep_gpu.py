@@ -48,3 +48,26 @@ def test_latent_prep(dtype, H, dn, dr, rot, r, pairing, packed, shift, write):
     if write:
         assert bool(((at.double() - cache).abs() <= tol * (cache.abs() + 2)).all())
     assert int(torch.isfinite(pages).any(-1).sum()) == (n if write else 0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("r,rot,pairing", [(512, 64, "half"), (132, 32, "adjacent"), (4, 0, "half")])
+def test_both_ways_give_the_same_bits(dtype, r, rot, pairing):
+    """Rows that begin on a 16-byte boundary and rows that do not."""
+    from hk_b200.csrc import ops
+    g = torch.Generator(DEV).manual_seed(r)
+    n, H, dn, dr, pt = 37, 5, 128, 64, 8
+    values, w, angle = torch.randn(n, H * (dn + dr) + r + dr, generator=g, device=DEV), torch.rand(r, generator=g, device=DEV), \
+        torch.rand(64, max(rot // 2, 1), generator=g, device=DEV) * 6
+    pos, slots = (torch.arange(n, device=DEV) * 7 % 64).int(), torch.arange(n, device=DEV, dtype=torch.int32)
+    table = torch.arange(n * 8, device=DEV, dtype=torch.int32).view(n, 8)
+    got = []
+    for shift in (0, 1):
+        wide = torch.zeros(n, values.shape[1] + 4, device=DEV)
+        wide[:, shift:shift + values.shape[1]] = values
+        q, kv = wide[:, shift:shift + H * (dn + dr)], wide[:, shift + H * (dn + dr):shift + values.shape[1]]
+        plain, full, both = (torch.zeros(n, H * x, dtype=dtype, device=DEV) for x in (dn, r + dr, dn + dr))
+        pages = torch.zeros(n * 8, 1, pt, r + dr, dtype=dtype, device=DEV)
+        ops.latent_prep(q, kv, plain, full, w, 1e-5, angle.cos(), angle.sin(), rot, pairing, pos, slots, table, pages, H, dn, dr, r, pt, q_packed=both)
+        got.append((both, pages))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and all(bool(x.any()) for x in got[0])
