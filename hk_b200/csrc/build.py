@@ -53,7 +53,7 @@ LIBRARIES: Dict[str, str] = {
     "gated_linear_chunks": "gated_linear_chunks.cu",   # the same for prompt portions, chunks of tokens on the tensor cores
     "norms": "norms.cu",               # layer norm; two mixers' results normed onto the residual stream
     "routed": "routed.cu",             # a feed-forward of experts: route, sort, grouped products, combine
-    "runtime": "runtime.cpp",          # host only: the cache's books (no GPU code, no CUDA headers)
+    "runtime": "runtime.cpp",          # host only: the cache's books, a choice between products (no GPU code, no CUDA headers)
 }
 
 

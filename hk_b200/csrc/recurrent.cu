@@ -929,7 +929,7 @@ __global__ void head_out_gate_kernel(const float* __restrict__ o, int ldo, const
 }
 
 // The same for heads of whole 16-byte pieces, up to 128 values: L lanes hold a head's values, four each, so a warp takes 32 / L
-// heads at once.  Bound by its bytes; one value a lane and load took 61 us for 2,048 tokens of 64 heads of 64, this 18 (4.7 TB/s).
+// heads at once.  Bound by its bytes; one value a lane and load took 61 us for 2,048 tokens of 64 heads of 64, this 19 (4.3 TB/s).
 template <typename T, int L>
 __global__ void __launch_bounds__(256)
 head_out_gate_vec_kernel(const float* __restrict__ o, int ldo, const float* __restrict__ g, long long ldg, const float* __restrict__ weight,
