@@ -6,7 +6,7 @@ achieved GB/s or TFLOP/s.  The same command under `ncu -k regex:<kernel>` gives 
 counters for that kernel.  (The reference has per-kernel event timing of the same kind behind
 HK_CUDA_EVENTS: src/cuda.zig:1212-1263.)
 
-Cases: gemm_tc (tcgen05 product, --swiglu / --add), gemm_smallm and gemm_stream (decode products), attn_decode
+Cases: gemm_tc and gemm_pair (tcgen05 products, one SM a tile and on pairs of SMs, --swiglu / --add), gemm_smallm and gemm_stream (decode products), attn_decode
 (paged decode attention), attn_prefill (paged causal attention of one prompt), decode (whole decode steps
 of a shallow random model with the 8B layer sizes, launched one kernel after the other without a graph: the
 launch list of a profiler then shows every kernel of a step with its time).
@@ -77,7 +77,7 @@ def _decode_steps(a, dev) -> int:
 
 def main(argv=None) -> int:
     ap = argparse.ArgumentParser(prog="hk_b200.profiling")
-    ap.add_argument("case", choices=["gemm_tc", "gemm_smallm", "gemm_stream", "attn_decode", "attn_prefill", "decode"])
+    ap.add_argument("case", choices=["gemm_tc", "gemm_pair", "gemm_smallm", "gemm_stream", "attn_decode", "attn_prefill", "decode"])
     ap.add_argument("--m", type=int, default=2048)
     ap.add_argument("--n", type=int, default=24576)
     ap.add_argument("--k", type=int, default=4096)
@@ -116,7 +116,7 @@ def main(argv=None) -> int:
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     if a.case == "decode":
         return _decode_steps(a, dev)
-    if a.case in ("gemm_tc", "gemm_smallm", "gemm_stream"):
+    if a.case in ("gemm_tc", "gemm_pair", "gemm_smallm", "gemm_stream"):
         x = (torch.randn(a.m, a.k, device=dev) / 8).to(torch.bfloat16)
         w = (torch.randn(a.n, a.k, device=dev) / 8).to(torch.bfloat16)
         if a.swiglu:
@@ -125,7 +125,7 @@ def main(argv=None) -> int:
         else:
             out = torch.zeros(a.m, a.n, dtype=torch.float32, device=dev)
             fn = lambda: ops.gemm(x, w, out, accumulate=a.add)
-        with ops.force(gemm={"gemm_tc": "tc", "gemm_smallm": "smallm", "gemm_stream": "stream"}[a.case]):
+        with ops.force(gemm={"gemm_tc": "tc", "gemm_pair": "pair", "gemm_smallm": "smallm", "gemm_stream": "stream"}[a.case]):
             us = _time(fn, a.reps, flush)
         flops = 2.0 * a.m * a.n * a.k
         nbytes = 2.0 * (a.n * a.k + a.m * a.k) + out.numel() * out.element_size()
