@@ -1,6 +1,7 @@
 // What the tcgen05 products share: the epilogues' arithmetic, barriers, TMA and tensor-memory instructions, tensor maps.
 #pragma once
 #include <cuda.h>
+#include <math_constants.h>
 
 #include <mutex>
 #include <unordered_map>
@@ -28,11 +29,16 @@ __device__ __forceinline__ bf16 squared_relu(float z, GluParams gp) {
   const float r = fmaxf(z, 0.f);
   return __float2bfloat16_rn(gp.slope * (r * r));
 }
-// x / d, d at least 1, rounded as the plain division rounds.  A zero, which every row that fills a tile up has for a gate, would take
-// the division's branch for unusual operands: 100 rows by 12,288 x 2,048 took 20 us, 128 rows 15.
+// x / d for d of 1 and more, without a branch for unusual operands, which a row that fills a tile up (all zeros) takes, and which keeps
+// one division from running beside the next: a quotient from the quick reciprocal and one step of iterative refinement, whose residual a
+// fused multiply-add gives exactly (P. Markstein, IBM Journal of Research and Development 34, 1990), so within 0.500001 units in the
+// last place of normal results (8 of 40 million differ from the plain division's).  The quick reciprocal is 0 above 2^126, so a large d
+// is divided down first; infinities stay what the first quotient makes of them.  Whole products, us, plain division / this: 64 rows by
+// 24,576 x 4,096 40.9 / 37.0, 100 by 12,288 x 2,048 14.6 / 13.6, 200 18.8 / 15.6.
 __device__ __forceinline__ float over(float x, float d) {
-  const float y = (x == 0.f ? 1.f : x) / d;
-  return x == 0.f ? x * y : y;
+  const float s = d > 0x1p64f ? 0x1p-64f : 1.0f, b = d * s, c = __fdividef(1.0f, b), q = x * c;
+  const float y = fmaf(fmaf(-q, b, x), c, q);
+  return (fabsf(q) < CUDART_INF_F && b < CUDART_INF_F ? y : q) * s;
 }
 template <int EPI>
 __device__ __forceinline__ float glu_pair(float g, float u, GluParams gp) {

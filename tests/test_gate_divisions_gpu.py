@@ -28,6 +28,44 @@ def test_gated_products(rows, K, act, gate):
     assert not bool(out[:, -1].any())
 
 
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "swish_clamped"])
+@pytest.mark.parametrize("kernel", ["tc", "pair"])
+def test_gated_epilogues_divide_like_the_streaming_product(kernel, act):
+    """Products of one exact term: the same gates and ups, so the same bits as from the kernel that divides plainly, but for the few that
+    lie on the edge between two bfloat16 numbers."""
+    from hk_b200.csrc import ops
+    rows, K, F, apart = 20, 64, 16384, 0
+    g = torch.Generator(DEV).manual_seed(11)
+    for low, high in ((-1.0, 1.0), (-20.0, 20.0), (-89.0, 89.0)):
+        a, w = torch.zeros(rows, K, dtype=torch.bfloat16, device=DEV), torch.zeros(2 * F, K, dtype=torch.bfloat16, device=DEV)
+        a[:, 0] = torch.rand(rows, generator=g, device=DEV) + 0.5
+        w[:F, 0] = torch.rand(F, generator=g, device=DEV) * (high - low) + low
+        w[F:, 0] = torch.randn(F, generator=g, device=DEV)
+        outs = []
+        for name in (kernel, "stream"):
+            outs.append(torch.empty(rows, F, dtype=torch.bfloat16, device=DEV))
+            with ops.force(gemm=name):
+                ops.gemm_swiglu(a, w, outs[-1], act=act, limit=60.0, slope=1.702)
+        assert bool(torch.isfinite(outs[1].float()).all())
+        apart += int((outs[0] != outs[1]).sum())
+        # normal results: one rounding to bfloat16 apart at most
+        assert bool(((outs[0].double() - outs[1].double()).abs() <= 2.0 ** -7 * outs[1].double().abs() + 2.0 ** -126).all())
+    assert apart <= 3 * rows * F * 1e-5
+
+
+@pytest.mark.parametrize("kernel", ["tc", "pair"])
+def test_gates_that_are_not_finite(kernel):
+    from hk_b200.csrc import ops
+    a, w, inf = torch.zeros(20, 64, dtype=torch.bfloat16, device=DEV), torch.zeros(64, 64, dtype=torch.bfloat16, device=DEV), float("inf")
+    a[:, 0] = 1.0
+    w[:32, 0], w[32:, 0] = torch.tensor([inf, -inf, float("nan"), 0.0, -200.0, 200.0, 3e38, -3e38] * 4), 1.0
+    out = torch.empty(20, 32, dtype=torch.bfloat16, device=DEV)
+    with ops.force(gemm=kernel):
+        ops.gemm_swiglu(a, w, out)
+    want = torch.tensor([inf, float("nan"), float("nan"), 0.0, 0.0, 200.0, 3e38, 0.0] * 4, device=DEV).bfloat16()
+    assert torch.equal(out.nan_to_num(nan=7.0), want.nan_to_num(nan=7.0).expand(20, 32))
+
+
 def test_short_convolution_and_norms():
     from hk_b200.csrc import ops
     n, C = 64, 4096
