@@ -1220,7 +1220,8 @@ HK_API int hk_attention_decode_tma(const void* q, const void* k_pages, const voi
 }
 
 // The same, for items that are `splits` (2 to 8) key ranges of every request side by side, merged by the kernel itself: no scratch, no
-// hk_attention_combine.  Refuses (HK_ERR_UNSUPPORTED) besides what does not fit on the GPU at once.
+// hk_attention_combine.  Refuses (HK_ERR_UNSUPPORTED) besides what does not fit on the GPU at once, and the few steps that launch_decode_merged
+// leaves to the separate merge.
 HK_API int hk_attention_decode_merged(const void* q, const void* k_pages, const void* v_pages, long long num_pages,
                                       const int* block_table, int table_stride, const void* items, int n_items, int splits, void* out,
                                       int H, int G, int hd, int page_tokens, int window, float scale_log2, int sink, int pages_cap,
